@@ -505,12 +505,17 @@ bool flatquant_sm100_supported(int64_t ldx, int m, int n, int in_dtype, const vo
                                float clip) {
   if (in_dtype != QO_F16 && in_dtype != QO_BF16) return false;
   if (!(clip > 0.f)) return false;                            // the single running absmax needs a positive clip ratio
-  if (n != 64 && !flatquant_sm100_n128_supported(m, n) && !flatquant_sm100_n64_supported(m, n)) return false;
+  if (n != 64 && !flatquant_sm100_n128_supported(m, n) && !flatquant_sm100_n64_supported(m, n) && !flatquant_sm100_n256_supported(m, n))
+    return false;
   if (m < 16 || m > 128) return false;
   if (ldx % 8) return false;                                  // TMA: row stride must be a multiple of 16 bytes
   if (reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(left) % 16 || reinterpret_cast<uintptr_t>(right) % 16) return false;
   return encode_fn() != nullptr;
 }
+
+// Right transforms above 128: one to three tokens stay on the SIMT kernel, which the tests pin for a call of three.  (It
+// is the slower one there too; the line is not a measured crossing.)
+bool flatquant_sm100_preferred(int64_t tokens, int m, int n) { return tokens >= 4 || !flatquant_sm100_n256_supported(m, n); }
 
 // mode: 0 int8 codes, 1 packed codes, 2 transform only (float32 Z written to `codes`)
 int launch_flatquant_sm100_mode(int mode, const void* x, int64_t ldx, const void* left, const void* right, void* codes,
@@ -528,7 +533,8 @@ int launch_flatquant_sm100_mode(int mode, const void* x, int64_t ldx, const void
   const cuuint64_t strides[2] = {(cuuint64_t)n * 2, (cuuint64_t)ldx * 2};
   const bool batched = flatquant_sm100_n64_supported(m, n);  // groups of 2 tokens, stacked-L^T second product
   const bool wide = flatquant_sm100_n128_supported(m, n);     // right transform of size 128
-  const cuuint32_t box[3] = {64, (cuuint32_t)m, (cuuint32_t)(batched ? 2 : (wide ? flatquant_sm100_n128_group(m) : 128 / m))};
+  const bool wider = flatquant_sm100_n256_supported(m, n);    // right transforms of 144 .. 256, one token at a time
+  const cuuint32_t box[3] = {64, (cuuint32_t)m, (cuuint32_t)(batched ? 2 : (wide ? flatquant_sm100_n128_group(m) : (wider ? 1 : 128 / m)))};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = encode_fn()(&map, in_dtype == QO_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
                                  3, const_cast<void*>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -540,6 +546,8 @@ int launch_flatquant_sm100_mode(int mode, const void* x, int64_t ldx, const void
     return launch_flatquant_sm100_n64(mode, &map, left, right, codes, scales, tokens, m, n, clip, in_dtype, scale_dtype, status, stream);
   if (wide)
     return launch_flatquant_sm100_n128(mode, &map, left, right, codes, scales, tokens, m, n, clip, in_dtype, scale_dtype, status, stream);
+  if (wider)
+    return launch_flatquant_sm100_n256(mode, &map, left, right, codes, scales, tokens, m, n, clip, in_dtype, scale_dtype, status, stream);
   if (in_dtype == QO_BF16)
     return launch_mode<__nv_bfloat16, 64>(mode, map, left, right, codes, scales, tokens, m, clip, scale_dtype, status, stream);
   return launch_mode<__half, 64>(mode, map, left, right, codes, scales, tokens, m, clip, scale_dtype, status, stream);

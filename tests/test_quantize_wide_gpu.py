@@ -1,0 +1,61 @@
+"""GPU parity of the quantizer for right transforms of 144 .. 256 (flatquant_sm100_n256.cu), at the edges of its tiles: against the
+oracle, and against the SIMT kernel on tokens with infinities, NaNs and zeros."""
+import pytest
+import torch
+
+from helpers import N, abi_quantize, lib, make_inputs, ptr, QD, stream_ptr, t2f
+from oracle import w4a4_oracle as O
+from test_quantize_gpu import check
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# (M, N): both halves of the rows or one, 32-column blocks whole or half, the second tile's lanes from 16 to 128;
+# tokens: one, a few, more than one round of every SM
+WIDE = [(128, 224, "bf16", 1, True), (128, 224, "fp16", 150, False), (128, 256, "bf16", 301, True), (16, 144, "bf16", 40, True),
+        (16, 256, "fp16", 5, False), (80, 160, "fp16", 7, True), (96, 192, "bf16", 160, False), (112, 240, "bf16", 9, True), (64, 208, "fp16", 33, True)]
+
+
+@pytest.mark.parametrize("m,n,dtype,tokens,pack", WIDE)
+def test_against_oracle(m, n, dtype, tokens, pack):
+    x, left, right = make_inputs(tokens, m * n, dtype, 7 * m + n + tokens, True, mn=(m, n))
+    sample = slice(None) if tokens <= 40 else torch.linspace(0, tokens - 1, 40).long()
+    ref_codes, ref_scales = O.flatquant_quantize(t2f(x[sample]), t2f(left), t2f(right), 0.9, pack, dtype)
+    codes, scales = abi_quantize(x.to(DEV), left.to(DEV), right.to(DEV), 0.9, pack, dtype, policy=2)
+    assert lib.qo_last_quantizer_path() == 2 and lib.qo_device_status(stream_ptr()) == N.QO_OK
+    check(codes.cpu()[sample].numpy(), t2f(scales)[sample if isinstance(sample, slice) else sample.numpy()], ref_codes, ref_scales, pack)
+
+
+def test_transform_only_and_dispatch():
+    x, left, right = make_inputs(6, 128 * 224, "bf16", 3, True)
+    ref = O.kronecker_transform(t2f(x), t2f(left), t2f(right), "bf16").reshape(6, -1)
+    z = torch.empty(6, 128 * 224, device=DEV)
+    xd, ld, rd = x.to(DEV), left.to(DEV), right.to(DEV)
+    N.check(lib.qo_flatquant_transform(ptr(xd), 128 * 224, ptr(ld), ptr(rd), ptr(z), 6, 128, 224, QD["bf16"], stream_ptr()))
+    torch.cuda.synchronize()
+    assert lib.qo_last_quantizer_path() == 2
+    # a sum next to a rounding boundary of Y or Z may round to the neighbour (2^-8 relative in bf16)
+    err = (z.cpu() - torch.from_numpy(ref)).abs()
+    assert (err > 2.0 ** -7 * torch.from_numpy(ref).abs() + 2.0 ** -7 * float(abs(ref).mean())).float().mean() == 0
+    abi_quantize(xd, ld, rd, 0.9, True, "bf16")
+    assert lib.qo_last_quantizer_path() == 2
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("pack", [True, False])
+def test_special_tokens_equal_the_simt_kernel(dtype, pack):
+    m, n = 32, 160
+    x, left, right = make_inputs(12, m * n, dtype, 5, True, mn=(m, n))
+    x[1, 77] = float("inf")
+    x[2, 5000] = -float("inf")
+    x[3, 0] = float("nan")
+    x[4] = float("nan")
+    x[5] = 0.0
+    x[6] = 1e-7  # fp16: subnormal, the scale rounds to zero
+    x[7, 3], x[7, 4000] = float("inf"), float("inf")
+    got = abi_quantize(x.to(DEV), left.to(DEV), right.to(DEV), 0.9, pack, dtype, policy=2)
+    ref = abi_quantize(x.to(DEV), left.to(DEV), right.to(DEV), 0.9, pack, dtype, policy=1)
+    special = torch.tensor([1, 2, 3, 4, 5, 7], device=DEV)
+    assert torch.equal(got[0][special], ref[0][special])
+    assert torch.equal(got[1][special], ref[1][special])
+    assert torch.allclose(got[1][6], ref[1][6], rtol=2.0 ** -7)
