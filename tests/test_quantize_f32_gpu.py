@@ -1,0 +1,46 @@
+"""The register-tiled float32 quantizer (flatquant_f32.cu) gives the bits of the shape-generic kernel: every sum is the same chain
+of fused multiply-adds."""
+import pytest
+import torch
+
+from helpers import N, QD, abi_quantize, lib, make_inputs, ptr, stream_ptr
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# M not a multiple of 8 or 16, N from one block to more than 256 threads' worth; one token, partial groups, many rounds
+SHAPES = [(3, 8, 5), (10, 24, 700), (32, 32, 1), (32, 32, 4801), (48, 64, 333), (64, 64, 1), (64, 64, 1300), (64, 80, 77), (86, 128, 301),
+          (112, 128, 299), (128, 192, 150), (24, 8, 40)]
+
+
+@pytest.mark.parametrize("m,n,tokens", SHAPES)
+@pytest.mark.parametrize("pack", [True, False])
+def test_same_bits_as_the_generic_kernel(m, n, tokens, pack):
+    x, left, right = make_inputs(tokens, m * n, "fp32", 3 * m + n + tokens, True, mn=(m, n))
+    if tokens >= 5:
+        x[0], x[1, 1], x[2, 2] = 0.0, float("inf"), float("nan")
+        x[3] *= 1e37
+        x[4] *= 1e-40
+    xd = torch.zeros(tokens, m * n + 4, device=DEV)
+    xd[:, : m * n] = x.to(DEV)
+    xd = xd[:, : m * n]
+    ld, rd = left.to(DEV), right.to(DEV)
+    ref = abi_quantize(xd, ld, rd, 0.9, pack, "fp32", policy=1)
+    got = abi_quantize(xd, ld, rd, 0.9, pack, "fp32", policy=0)
+    assert torch.equal(got[0], ref[0])
+    assert torch.equal(got[1].view(torch.int32), ref[1].view(torch.int32))
+
+
+@pytest.mark.parametrize("m,n,tokens", [(64, 64, 9), (86, 128, 3)])
+def test_transform_only_has_the_same_bits(m, n, tokens):
+    x, left, right = make_inputs(tokens, m * n, "fp32", m + n, True, mn=(m, n))
+    xd, ld, rd = x.to(DEV), left.to(DEV), right.to(DEV)
+    out = []
+    for policy in (1, 0):
+        z = torch.empty(tokens, m * n, device=DEV)
+        N.check(lib.qo_set_kernel_policy(policy))
+        N.check(lib.qo_flatquant_transform(ptr(xd), m * n, ptr(ld), ptr(rd), ptr(z), tokens, m, n, QD["fp32"], stream_ptr()))
+        lib.qo_set_kernel_policy(0)
+        torch.cuda.synchronize()
+        out.append(z)
+    assert torch.equal(out[0], out[1])
