@@ -261,7 +261,7 @@ static int int4_matmul_impl(const int32_t* a, int64_t lda, const int32_t* b, int
     if (workspace_bytes < need) return fail(QO_ERR_WORKSPACE, "int4_matmul: workspace of %zu bytes, need %zu", workspace_bytes, need);
     t_gemm_path = 2;
     return launch_gemm_sm100(a, lda, b, bsk, bsn, sa, sb, out, out_dtype, t, k, n, acc_out, bias, workspace,
-                             workspace_bytes, st);
+                             workspace_bytes, st, b_is_layer_weight);
   }
   t_gemm_path = 1;
   return launch_gemm_generic(a, lda, b, bsk, bsn, sa, sb, out, out_dtype, t, k, n, acc_out, bias, st);
@@ -356,7 +356,7 @@ int qo_w4a4_linear_gather(const void* x, int64_t ldx, const void* left, const vo
     workspace_bytes = need;
   }
   if (workspace_bytes < need) return fail(QO_ERR_WORKSPACE, "w4a4_linear_gather: workspace of %zu bytes, need %zu", workspace_bytes, need);
-  if (t_policy == 1 || !gemm_unpack_preferred(tokens, k, n_out) ||
+  if (t_policy == 1 || !gemm_unpack_prefill(tokens, n_out) ||
       !gemm_unpack_supported(tokens, k, n_out, workspace, k / 8, w_packed, 1, k / 8) || n_out % 16)
     return fail(QO_ERR_UNSUPPORTED, "w4a4_linear_gather: only prefill-sized products gather in the kernel (tokens=%lld k=%lld n_out=%lld)",
                 (long long)tokens, (long long)k, (long long)n_out);
@@ -373,8 +373,8 @@ int qo_w4a4_linear_gather(const void* x, int64_t ldx, const void* left, const vo
   uint32_t* status = device_status_word(dev);
   if (!status) return fail(QO_ERR_CUDA, "w4a4_linear_gather: could not allocate the device status word");
   t_gemm_path = 2;
-  rc = launch_gemm_unpack(a_packed, k / 8, w_packed, k / 8, a_scale, w_scale, nullptr, out_dtype, tokens, k, n_out, nullptr, bias,
-                          status, reinterpret_cast<cudaStream_t>(stream), &g);
+  rc = launch_gemm_unpack(a_packed, k / 8, w_packed, 1, k / 8, a_scale, w_scale, nullptr, out_dtype, tokens, k, n_out, nullptr, bias,
+                          status, reinterpret_cast<cudaStream_t>(stream), false, &g);
   if (rc == QO_ERR_UNSUPPORTED && qo_last_error()[0] == 0)
     return fail(QO_ERR_UNSUPPORTED, "w4a4_linear_gather: this device cannot co-schedule the CTA pairs of the kernel");
   return rc;
@@ -487,7 +487,9 @@ int qo_w4a4_linear_prepared(const void* x, int64_t ldx, const void* left, const 
   if (workspace_bytes < need) return fail(QO_ERR_WORKSPACE, "w4a4_linear: workspace of %zu bytes, need %zu", workspace_bytes, need);
   // few tokens (weight-streaming kernel), prefill sizes (the GEMM that unpacks in the kernel is the faster one there and
   // needs no int8 copy), or a shape / policy the int8 tensor-core kernel does not take: packed route
-  const bool unpack_route = t_policy != 1 && gemm_unpack_preferred(tokens, k, n_out) &&
+  // (above 128 rows the int8 kernels start a second row block: 256 x 4096 x 11008 29.1 us with the copy, 21.2 packed, 600 x
+  // 14336 x 4096 82 against 49; up to 128 rows the copy is the faster one, 22.6 against 26.9 us at 128 x 14336 x 4096)
+  const bool unpack_route = t_policy != 1 && (tokens > 128 ? gemm_unpack_preferred(tokens, k, n_out) : gemm_unpack_prefill(tokens, n_out)) &&
                             gemm_unpack_supported(tokens, k, n_out, workspace, k / 8, w_packed, 1, k / 8);
   const bool direct = !unpack_route && t_policy != 1 && tokens > 32 && gemm_sm100_supported(tokens, k, n_out, k / 8, 1, k / 8) &&
                       reinterpret_cast<uintptr_t>(prepared) % 256 == 0;

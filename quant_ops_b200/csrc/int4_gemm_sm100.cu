@@ -842,18 +842,17 @@ int launch_widen_rows(const int32_t* in, int64_t ld_words, int8_t* out, int64_t 
 
 int launch_gemm_sm100(const int32_t* a, int64_t lda, const int32_t* b, int64_t bsk, int64_t bsn, const float* sa,
                       const float* sb, void* out, int out_dtype, int64_t t, int64_t k, int64_t n, int32_t* acc_out,
-                      const void* bias, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+                      const void* bias, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool b_early) {
   if (workspace_bytes < gemm_sm100_workspace_bytes(t, k, n) || reinterpret_cast<uintptr_t>(workspace) % 256)
     return fail(QO_ERR_WORKSPACE, "int4_matmul: workspace missing, too small or not 256-byte aligned");
   int rc;
-  // prefill-sized products with K-contiguous operands: the kernel that unpacks the nibbles itself (no widening pass,
-  // the workspace stays untouched)
+  // the kernel that unpacks the nibbles itself, where it can (no widening pass, the workspace stays untouched)
   if (gemm_unpack_supported(t, k, n, a, lda, b, bsk, bsn) && gemm_unpack_preferred(t, k, n)) {
     int dev = 0;
     QO_CUDA_TRY(cudaGetDevice(&dev));
     uint32_t* status = device_status_word(dev);
     if (!status) return fail(QO_ERR_CUDA, "int4_matmul: could not allocate the device status word");
-    rc = launch_gemm_unpack(a, lda, b, bsn, sa, sb, out, out_dtype, t, k, n, acc_out, bias, status, stream);
+    rc = launch_gemm_unpack(a, lda, b, bsk, bsn, sa, sb, out, out_dtype, t, k, n, acc_out, bias, status, stream, b_early);
     if (rc != QO_ERR_UNSUPPORTED) return rc;
   }
   int8_t* a8 = reinterpret_cast<int8_t*>(workspace);

@@ -60,6 +60,7 @@ constexpr int kBM = 128;        // rows per CTA
 constexpr int kBN = 256;        // columns of the pair's tile
 constexpr int kBNh = kBN / 2;   // B rows staged per CTA
 constexpr int kKStage = 256;    // int4 values per stage = 128 packed bytes = 256 int8 bytes per row
+constexpr int kKWords = kKStage / 8;
 constexpr int kSets = 3;        // converter sets in rotation = ring depth: set g always works on slot g of both rings
 constexpr int kThreads = 28 * 32;
 constexpr int kPStages = kSets;     // packed ring
@@ -69,9 +70,17 @@ constexpr int kOAtomBytes = kBNh * 128;                 // one 128-byte K atom o
 constexpr int kOBBytes = 2 * kOAtomBytes;               // 32 KB per operand stage
 constexpr int kOffP = 0;
 constexpr int kOffO = kOffP + kPStages * kPStageBytes;  // 96 KB
-constexpr int kOffSb = kOffO + kOStages * kOBBytes;     // +96 KB; 8 epilogue warps x 128 floats
-constexpr int kOffBar = kOffSb + 8 * 128 * 4;
-constexpr int kSmemBytes = kOffBar + 512 + 1024;
+constexpr int kRingBytes = kOffO + kOStages * kOBBytes;  // +96 KB
+// Behind the rings: SPLIT = 1: column scales, 8 epilogue warps x 128 floats.  SPLIT > 1: the exchange of partial sums takes
+// 224 KB (the rings and 32 KB more), behind it 256 column and 128 row scales.
+template <int SPLIT>
+struct Smem {
+  static constexpr int kOffSb = SPLIT == 1 ? kRingBytes : 224 * 1024;
+  static constexpr int kOffSa = kOffSb + 256 * 4;  // SPLIT > 1 only
+  static constexpr int kOffBar = kOffSb + (SPLIT == 1 ? 8 * 128 * 4 : 384 * 4);
+  static constexpr int kBytes = kOffBar + 512 + 1024;
+  static_assert(kBytes <= 227 * 1024, "shared memory of one CTA");
+};
 constexpr int kColA = kBN;      // first tensor-memory column of the A operand stages (64 columns each)
 constexpr int kEpiWarp0 = 2, kAWarp0 = 10, kBWarp0 = 22;
 
@@ -79,6 +88,7 @@ struct Bars {
   uint64_t p_full[kPStages], p_empty[kPStages];
   uint64_t op_ready[kOStages], op_empty[kOStages];
   uint64_t acc_full, acc_empty;
+  uint64_t exchange;  // bytes of the other pairs' partial sums (SPLIT > 1)
   uint32_t tmem_base;
 };
 
@@ -159,21 +169,42 @@ __device__ __forceinline__ bool issue_stage(uint32_t d_tmem, uint32_t a_tmem, ui
 // GATHER: the outputs are not stored to `out` but, at row `row_offset + row`, into every buffer of `dsts` -- this GPU's
 // own copy of the gathered output and the peers' copies, mapped into this process (plain stores over NVLink; the
 // all-gather of a row-sharded layer's outputs costs no kernel of its own and no SMs).
-template <typename OutT, bool GATHER>
+//
+// SPLIT > 1 (few output tiles: a short activation matrix or a narrow layer): K is split over SPLIT CTA pairs which form
+// one cluster and work on one tile, one work item per pair.  Measured (graph replay, before: widening pass + int8 kernels):
+// 256 x 14336 x 4096 35.6 -> 21.7 us, 64 x 4096 x 4096 15.6 -> 11.2, 512 x 4096 x 4096 22.3 -> 13.9.  What is left behind the
+// last MMA is the exchange, about 5 us of which 2.5 are the copies (18 bytes per cycle and SM), and the first fill, 2 us.
+// At the end the pairs share out the tile's columns and send
+// each other their int32 partial sums through distributed shared memory (into the rings, which are idle by then).
+// Whole-number sums: exact in any order.
+// b_early: B was not written by the kernel ahead in the stream, so the first stages' B halves are requested before the
+// dependency wait.
+//
+// BCOLS: B is the reference layout [K/8, N] of packed words with N contiguous.  Its box is 32 words of K by 128
+// channels (333 x 4096 x 14336 50.0 -> 27.7 us), a channel's words lie 512 bytes apart in the stage, and a converter thread, which owns a channel, reads
+// them one by one without bank conflicts: no transposing pass over the weights.
+template <typename OutT, bool GATHER, int SPLIT, bool BCOLS>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap b_map,
                       const float* __restrict__ sa, const float* __restrict__ sb, OutT* __restrict__ out,
                       int32_t* __restrict__ acc_out, const OutT* __restrict__ bias, int t, int n, int k, int items, int cut_from,
-                      uint32_t* __restrict__ status, const __grid_constant__ GatherDsts dsts) {
+                      int b_early, uint32_t* __restrict__ status, const __grid_constant__ GatherDsts dsts) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  Bars* bars = reinterpret_cast<Bars*>(smem + kOffBar);
+  using S = Smem<SPLIT>;
+  Bars* bars = reinterpret_cast<Bars*>(smem + S::kOffBar);
   const uint32_t smem_base = smem_u32(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t rank = cluster_cta_rank();  // 0 = leader
-  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  const uint32_t crank = cluster_cta_rank();
+  const uint32_t rank = SPLIT == 1 ? crank : (crank & 1);             // in the pair: 0 = leader
+  const uint32_t leader = SPLIT == 1 ? 0u : (crank & ~1u), other = leader + 1;  // cluster ranks of the pair's CTAs
+  // (SPLIT > 1: `pair` counts clusters, each with one tile; kz is the pair's slice of K)
+  const int pair = SPLIT == 1 ? blockIdx.x >> 1 : blockIdx.x / (2 * SPLIT), npairs = SPLIT == 1 ? gridDim.x >> 1 : items;
   const int tiles_n = (n + kBN - 1) / kBN;
-  const int ksteps = k / kKStage;  // k is a multiple of 256 (checked by the host)
+  const int kstages = k / kKStage;  // k is a multiple of 256 (checked by the host)
+  const int kz = SPLIT == 1 ? 0 : (int)(crank >> 1);
+  const int ks_first = SPLIT == 1 ? 0 : kz * kstages / SPLIT;
+  const int ksteps = SPLIT == 1 ? kstages : (kz + 1) * kstages / SPLIT - ks_first;  // stages of this pair per item
   // Work items: whole tiles, except that the tiles of a last wave which would occupy at most half of the pairs are cut
   // into two halves of 128 columns (MMAs with N = 128), so that twice as many pairs share that wave: 256 tiles on 74
   // pairs take the time of 3.7 tiles instead of 4.
@@ -192,6 +223,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
     for (int i = 0; i < kOStages; ++i) { mbar_init(smem_u32(&bars->op_ready[i]), 12); mbar_init(smem_u32(&bars->op_empty[i]), 1); }
     mbar_init(smem_u32(&bars->acc_full), 1);
     mbar_init(smem_u32(&bars->acc_empty), 16);
+    mbar_init(smem_u32(&bars->exchange), 1);
     fence_barrier_init();
     prefetch_tensormap(&a_map);
     prefetch_tensormap(&b_map);
@@ -205,6 +237,18 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
   cluster_sync_all();  // both CTAs' barriers and tensor memory exist before either touches the other
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  int early = 0;  // stages whose B half is already on its way
+  if (SPLIT > 1 && b_early && tid == 0) {
+    early = min(kPStages, ksteps);
+    const int row_b = (pair % tiles_n) * kBN + (int)rank * kBNh;
+    for (int s = 0; s < early; ++s) {
+      const uint32_t bar = smem_u32(&bars->p_full[s]);
+      mbar_arrive_expect_tx(bar, kPStageBytes);
+      const uint32_t dst = smem_base + kOffP + s * kPStageBytes + kPABytes;
+      if (BCOLS) tma_load_2d(dst, &b_map, bar, row_b, (ks_first + s) * kKWords);
+      else tma_load_2d(dst, &b_map, bar, (ks_first + s) * 128, row_b);
+    }
+  }
   // Launched with programmatic stream serialization: everything above may overlap the tail of the preceding kernel.
   grid_dependency_wait();
 
@@ -221,12 +265,17 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
         const int row_a = mb * 2 * kBM + (int)rank * kBM, row_b = nb * kBN + col_in_tile + (int)rank * (width >> 1);
         for (int ks = 0; ks < ksteps; ++ks, ++step) {
           const int ps = step % kPStages, pph = (step / kPStages) & 1;
-          if (!mbar_wait(smem_u32(&bars->p_empty[ps]), pph ^ 1)) { atomicCAS(status, 0u, 0xA00u + ps); ok = false; break; }
           const uint32_t bar = smem_u32(&bars->p_full[ps]);
-          mbar_arrive_expect_tx(bar, kPStageBytes);
           const uint32_t dst = smem_base + kOffP + ps * kPStageBytes;
-          tma_load_2d(dst, &a_map, bar, ks * 128, row_a);
-          tma_load_2d(dst + kPABytes, &b_map, bar, ks * 128, row_b);
+          if (SPLIT > 1 && step < early) {  // first use of the stage: its barrier already expects the bytes
+            tma_load_2d(dst, &a_map, bar, (ks_first + ks) * 128, row_a);
+            continue;
+          }
+          if (!mbar_wait(smem_u32(&bars->p_empty[ps]), pph ^ 1)) { atomicCAS(status, 0u, 0xA00u + ps); ok = false; break; }
+          mbar_arrive_expect_tx(bar, kPStageBytes);
+          tma_load_2d(dst, &a_map, bar, (ks_first + ks) * 128, row_a);
+          if (BCOLS) tma_load_2d(dst + kPABytes, &b_map, bar, row_b, (ks_first + ks) * kKWords);
+          else tma_load_2d(dst + kPABytes, &b_map, bar, (ks_first + ks) * 128, row_b);
         }
       }
     }
@@ -238,8 +287,9 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       // one thread feeds the tensor cores of both SMs, so its instruction count per MMA matters: the B descriptor is
       // built once and advanced by adding to its address field (units of 16 bytes)
       const uint64_t b_desc0 = umma_smem_desc_sw128(smem_base + kOffO, 16, 1024);
-      const uint32_t op_empty0 = smem_u32(&bars->op_empty[0]), op_empty0_peer = cluster_map_shared(op_empty0, 1);
-      const uint32_t acc_full = smem_u32(&bars->acc_full), acc_full_peer = cluster_map_shared(acc_full, 1);
+      // (a shared::cta address is the same location's shared::cluster address)
+      const uint32_t op_empty0 = smem_u32(&bars->op_empty[0]), op_empty0_peer = cluster_map_shared(op_empty0, other);
+      const uint32_t acc_full = smem_u32(&bars->acc_full), acc_full_peer = cluster_map_shared(acc_full, other);
       int step = 0;
       bool ok = true, ready = false;  // ready: the operands of `step` were already seen complete by an early probe
       for (int lt = 0; ok && lt < mine; ++lt) {
@@ -266,7 +316,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
     // ---- epilogue: the CTA's own 128 rows of the tile; warp (q, half) takes columns 128 half .. of lanes 32 q .. ------
     const int q = warp & 3, half = (warp - kEpiWarp0) >> 2;
     const bool wide_stores = (n % 16) == 0 && (reinterpret_cast<uintptr_t>(out) % 32) == 0;  // rows start on 32-byte boundaries
-    float* sb_s = reinterpret_cast<float*>(smem + kOffSb) + (warp - kEpiWarp0) * 128;
+    float* sb_s = reinterpret_cast<float*>(smem + S::kOffSb) + (SPLIT == 1 ? warp - kEpiWarp0 : half) * 128;
     for (int lt = 0; lt < mine; ++lt) {
       int tile, col_in_tile, width;
       item_of(pair + lt * npairs, tile, col_in_tile, width);
@@ -279,9 +329,12 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       const float s_row = row_ok ? sa[row] * 0.00390625f : 0.f;
       const int colw = nb * kBN + col_in_tile + half * wcols;  // first column of this warp
       __syncwarp();
-      for (int i = lane; i < wcols; i += 32) sb_s[i] = (colw + i < n) ? sb[colw + i] : 0.f;
+      if (SPLIT == 1 || q == 0)
+        for (int i = lane; i < wcols; i += 32) sb_s[i] = (colw + i < n) ? sb[colw + i] : 0.f;
+      if (SPLIT > 1 && half == 0) reinterpret_cast<float*>(smem + S::kOffSa)[q * 32 + lane] = s_row;
       __syncwarp();
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_full), lt & 1))) { atomicCAS(status, 0u, 0xA30u); break; }
+      if (SPLIT > 1) break;  // every MMA of this pair is done; the partial sums are exchanged below
       tc_fence_after();
 #pragma unroll 1
       for (int cc = 0; cc < wcols; cc += 32) {
@@ -294,7 +347,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
           __syncwarp();
           if (lane == 0) {
             const uint32_t e = smem_u32(&bars->acc_empty);
-            if (rank == 0) mbar_arrive(e); else mbar_arrive_cluster(cluster_map_shared(e, 0));
+            if (rank == 0) mbar_arrive(e); else mbar_arrive_cluster(cluster_map_shared(e, leader));
           }
         }
         const int col0 = colw + cc;
@@ -386,7 +439,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       __syncwarp();
       if (lane == 0) {
         const uint32_t ready = smem_u32(&bars->op_ready[s]);
-        if (rank == 0) mbar_arrive(ready); else mbar_arrive_cluster(cluster_map_shared(ready, 0));
+        if (rank == 0) mbar_arrive(ready); else mbar_arrive_cluster(cluster_map_shared(ready, leader));
       }
     }
   } else {
@@ -412,7 +465,12 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
           const int task = (g * 4 + i) * 64 + bt;  // 0 .. 1023
           cc[i] = task >> 7;                        // packed piece 0 .. 7 (32 values each)
           rr[i] = task & 127;
-          p[i] = ld_shared_v4(src + (uint32_t)(rr[i] * 128) + (((uint32_t)cc[i] ^ (uint32_t)(rr[i] & 7)) << 4));
+          if (BCOLS) {
+            const uint32_t col = src + (uint32_t)(cc[i] * 4 * kBNh * 4 + rr[i] * 4);  // word 4c of this channel
+            p[i] = make_uint4(ld_shared_u32(col), ld_shared_u32(col + kBNh * 4), ld_shared_u32(col + 2 * kBNh * 4), ld_shared_u32(col + 3 * kBNh * 4));
+          } else {
+            p[i] = ld_shared_v4(src + (uint32_t)(rr[i] * 128) + (((uint32_t)cc[i] ^ (uint32_t)(rr[i] & 7)) << 4));
+          }
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -433,11 +491,101 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       __syncwarp();
       if (lane == 0) {
         const uint32_t ready = smem_u32(&bars->op_ready[s]);
-        if (rank == 0) mbar_arrive(ready); else mbar_arrive_cluster(cluster_map_shared(ready, 0));
+        if (rank == 0) mbar_arrive(ready); else mbar_arrive_cluster(cluster_map_shared(ready, leader));
       }
     }
   }
 
+  if (SPLIT > 1) {
+    // Exchange of the partial sums.  The tile's eight blocks of 32 columns belong to the pairs in turn (block c to pair
+    // c % SPLIT); the owner adds the pairs' sums of its blocks and writes the outputs.  A warp takes one block of 32
+    // rows x 32 columns out of tensor memory, lays it down as 4 KB (rows of 128 bytes, 16-byte pieces XOR-swizzled by the
+    // row) and sends it as ONE bulk copy into the owner's shared memory, which counts the bytes on a barrier: stores of
+    // single lines took 2.5 us for what the copies do in less than one.  Blocks without a real row are left out.
+    const int mb = pair / tiles_n, nb = pair - mb * tiles_n;
+    const int row0 = mb * 2 * kBM + (int)rank * kBM;
+    const int quads = max(0, min(4, (t - row0 + 31) >> 5));  // lane quadrants with real rows
+    auto owned = [](int z) { return (8 - z + SPLIT - 1) / SPLIT; };
+    const int own = owned(kz);
+    const uint32_t staging = smem_base + (uint32_t)(SPLIT * 4 * own) * 4096u;  // behind the slots the other pairs fill
+    static_assert((SPLIT * 4 * ((8 + SPLIT - 1) / SPLIT) + 4 * (8 - (8 + SPLIT - 1) / SPLIT)) * 4096 <= S::kOffSb, "slots and staging");
+    static_assert((SPLIT * 4 * (8 / SPLIT) + 4 * (8 - 8 / SPLIT)) * 4096 <= S::kOffSb, "slots and staging");
+    if (tid == 0) mbar_arrive_expect_tx(smem_u32(&bars->exchange), (uint32_t)((SPLIT - 1) * own * quads) * 4096u);
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncwarp();
+    // The epilogue warps come here after their accumulator barrier, so past this barrier no CTA of the cluster has an
+    // MMA in flight and the rings are free.  Every thread passes it, and the one at the end, on every path.
+    cluster_sync_all();
+    if (warp >= 2 && warp < 18 && (warp & 3) < quads) {
+      const int q = warp & 3;
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = (warp - 2) >> 2; c < 8; c += 4) {
+        uint32_t v[32];
+        tmem_ld_32x32b_x32(tmem + ((uint32_t)(q * 32) << 16) + c * 32, v);
+        tmem_ld_wait();
+        const int owner = c % SPLIT, j = c / SPLIT;
+        const int before = j + (c % SPLIT > kz ? 1 : 0);  // this pair's own blocks among the first c
+        const uint32_t slot = (uint32_t)((kz * 4 + q) * owned(owner) + j) * 4096u;  // in the owner's shared memory
+        const uint32_t dst = owner == kz ? smem_base + slot : staging + (uint32_t)(q * (8 - own) + c - before) * 4096u;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)(lane * 128 + ((i ^ (lane & 7)) << 4))), "r"(v[4 * i]),
+                       "r"(v[4 * i + 1]), "r"(v[4 * i + 2]), "r"(v[4 * i + 3]) : "memory");
+        if (owner != kz) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            const uint32_t peer = (uint32_t)owner * 2u + rank;
+            bulk_copy_s2cluster(cluster_map_shared(smem_base + slot, peer), dst, 4096u, cluster_map_shared(smem_u32(&bars->exchange), peer));
+          }
+        }
+      }
+      tc_fence_before();
+    }
+    __syncthreads();  // this CTA's own blocks are in place
+    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->exchange), 0))) atomicCAS(status, 0u, 0xA70u);
+    {
+      // eight rows of one block per warp and step: four lanes per row, eight columns per lane
+      const float* sbs = reinterpret_cast<const float*>(smem + S::kOffSb);
+      const float* sas = reinterpret_cast<const float*>(smem + S::kOffSa);
+      const int p0 = 2 * (lane & 3);
+      for (int unit = warp; unit < own * quads * 4; unit += kThreads / 32) {
+        const int j = unit / (quads * 4), rest = unit - j * quads * 4, q = rest >> 2, r = (rest & 3) * 8 + (lane >> 2);
+        const int row = row0 + q * 32 + r, cb = (j * SPLIT + kz) * 32 + 4 * p0, col = nb * kBN + cb;
+        if (row >= t || col >= n) continue;
+        int v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int z = 0; z < SPLIT; ++z) {
+          const uint32_t base = smem_base + (uint32_t)((z * 4 + q) * own + j) * 4096u + (uint32_t)(r * 128);
+          const uint4 a0 = ld_shared_v4(base + (uint32_t)((p0 ^ (r & 7)) << 4)), a1 = ld_shared_v4(base + (uint32_t)(((p0 + 1) ^ (r & 7)) << 4));
+          v[0] += (int)a0.x; v[1] += (int)a0.y; v[2] += (int)a0.z; v[3] += (int)a0.w;
+          v[4] += (int)a1.x; v[5] += (int)a1.y; v[6] += (int)a1.z; v[7] += (int)a1.w;
+        }
+        const float s_row = sas[q * 32 + r];  // (already without the factor 256)
+        const float4 c0 = *reinterpret_cast<const float4*>(sbs + cb), c1 = *reinterpret_cast<const float4*>(sbs + cb + 4);
+        uint32_t w[4] = {pack_out2<OutT>(((float)v[0] * s_row) * c0.x, ((float)v[1] * s_row) * c0.y),
+                         pack_out2<OutT>(((float)v[2] * s_row) * c0.z, ((float)v[3] * s_row) * c0.w),
+                         pack_out2<OutT>(((float)v[4] * s_row) * c1.x, ((float)v[5] * s_row) * c1.y),
+                         pack_out2<OutT>(((float)v[6] * s_row) * c1.z, ((float)v[7] * s_row) * c1.w)};
+        if (bias != nullptr) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 o = unpack_out2(w[i], OutT());
+            const float2 bb = unpack_out2(*reinterpret_cast<const uint32_t*>(bias + col + 2 * i), OutT());
+            w[i] = pack_out2<OutT>(o.x + bb.x, o.y + bb.y);
+          }
+        }
+        *reinterpret_cast<uint4*>(out + (int64_t)row * n + col) = make_uint4(w[0], w[1], w[2], w[3]);
+        if (acc_out != nullptr) {
+          uint4* arow = reinterpret_cast<uint4*>(acc_out + (int64_t)row * n + col);
+          arow[0] = make_uint4((uint32_t)(v[0] >> 8), (uint32_t)(v[1] >> 8), (uint32_t)(v[2] >> 8), (uint32_t)(v[3] >> 8));
+          arow[1] = make_uint4((uint32_t)(v[4] >> 8), (uint32_t)(v[5] >> 8), (uint32_t)(v[6] >> 8), (uint32_t)(v[7] >> 8));
+        }
+      }
+    }
+  }
   // Nobody leaves while the other CTA may still signal it: the leader's commits to the peer's barriers complete with
   // the MMAs, which both CTAs' epilogues have waited for (accumulator barrier); the peer's arrivals on the leader's
   // barriers were made before this barrier.  The last "operand stage free" commits are awaited by one thread below.
@@ -449,7 +597,11 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
   }
   tc_fence_before();
   __syncwarp();
-  cluster_sync_all();
+  // SPLIT = 1: the peer's last arrivals on the leader's barriers must have landed before the leader leaves, hence the
+  // releasing form.  SPLIT > 1: every remote arrival and copy has been waited for by its receiver, so no CTA's memory is
+  // written or read from outside any more, and the arrival need not wait for the output stores.
+  if (SPLIT == 1) cluster_sync_all();
+  else cluster_sync_relaxed();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem, 512);
@@ -475,6 +627,21 @@ EncodeTiledFn unpack_encode_fn() {
   return fn;
 }
 
+struct UnpackArgs {
+  const int32_t* a;
+  int64_t lda;
+  const int32_t* b;
+  int64_t ldb;  // words between the rows of B: [n, k/8], or [k/8, n] (BCOLS)
+  const float *sa, *sb;
+  void* out;
+  int32_t* acc_out;
+  const void* bias;
+  int64_t t, k, n;
+  bool b_early;
+};
+
+int64_t unpack_tiles(int64_t t, int64_t n) { return ((t + 2 * kBM - 1) / (2 * kBM)) * ((n + kBN - 1) / kBN); }
+
 // packed operand [rows, k / 2 bytes] with a row stride of ld_words 32-bit words; boxes of 128 bytes x box_rows rows
 int make_map_packed(CUtensorMap* map, const void* base, int64_t rows, int64_t k, int64_t ld_words, int box_rows) {
   const cuuint64_t dims[2] = {(cuuint64_t)(k / 2), (cuuint64_t)rows};
@@ -488,21 +655,34 @@ int make_map_packed(CUtensorMap* map, const void* base, int64_t rows, int64_t k,
   return QO_OK;
 }
 
-// CTA pairs of this kernel the device runs at once (0 if the query fails); cached per device
-template <typename OutT, bool GATHER>
-int max_pairs(int dev) {
+// packed operand [k / 8 words, n] with n contiguous and a row stride of ld_words words; boxes of 32 words of K x 128 channels
+int make_map_packed_cols(CUtensorMap* map, const void* base, int64_t n, int64_t k, int64_t ld_words) {
+  const cuuint64_t dims[2] = {(cuuint64_t)n, (cuuint64_t)(k / 8)};
+  const cuuint64_t strides[1] = {(cuuint64_t)(ld_words * 4)};
+  const cuuint32_t box[2] = {(cuuint32_t)kBNh, (cuuint32_t)kKWords};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = unpack_encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void*>(base), dims, strides, box, estr,
+                                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(QO_ERR_CUDA, "int4_matmul: cuTensorMapEncodeTiled failed with code %d", (int)r);
+  return QO_OK;
+}
+
+// clusters of 2 * SPLIT CTAs of this kernel the device runs at once (0 if the query fails); cached per device
+template <typename OutT, bool GATHER, int SPLIT, bool BCOLS>
+int max_clusters(int dev) {
   static int cached[64] = {};
   int& c = cached[dev & 63];
   if (c == 0) {
-    auto kern = gemm_s4_unpack_kernel<OutT, GATHER>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess) { (void)cudaGetLastError(); c = -1; return 0; }
+    auto kern = gemm_s4_unpack_kernel<OutT, GATHER, SPLIT, BCOLS>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<SPLIT>::kBytes) != cudaSuccess) { (void)cudaGetLastError(); c = -1; return 0; }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * 74);
+    cfg.gridDim = dim3(2 * SPLIT * 74);
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.dynamicSmemBytes = Smem<SPLIT>::kBytes;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.x = 2 * SPLIT;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
@@ -514,85 +694,110 @@ int max_pairs(int dev) {
   return c > 0 ? c : 0;
 }
 
-template <typename OutT, bool GATHER>
-int launch_typed(const int32_t* a, int64_t lda, const int32_t* b, int64_t ldb, const float* sa, const float* sb, void* out,
-                 int32_t* acc_out, const void* bias, int64_t t, int64_t k, int64_t n, uint32_t* status, const GatherDsts& dsts,
-                 cudaStream_t stream) {
+template <typename OutT, bool GATHER, int SPLIT, bool BCOLS>
+int launch_typed(const UnpackArgs& p, uint32_t* status, const GatherDsts& dsts, cudaStream_t stream) {
   int dev = 0;
   QO_CUDA_TRY(cudaGetDevice(&dev));
-  const int pairs_max = max_pairs<OutT, GATHER>(dev);
-  if (pairs_max <= 0) return QO_ERR_UNSUPPORTED;
+  const int clusters = max_clusters<OutT, GATHER, SPLIT, BCOLS>(dev);
+  if (clusters <= 0) return QO_ERR_UNSUPPORTED;
+  const int64_t ntiles = unpack_tiles(p.t, p.n);
+  if (SPLIT > 1 && ntiles > clusters) return QO_ERR_UNSUPPORTED;  // a second wave would cost more than the split saves
   CUtensorMap a_map, b_map;
-  int rc = make_map_packed(&a_map, a, t, k, lda, kBM);
+  int rc = make_map_packed(&a_map, p.a, p.t, p.k, p.lda, kBM);
   if (rc) return rc;
-  if ((rc = make_map_packed(&b_map, b, n, k, ldb, kBNh))) return rc;
-  const int64_t ntiles = ((t + 2 * kBM - 1) / (2 * kBM)) * ((n + kBN - 1) / kBN);
-  const int pairs = (int)(ntiles < pairs_max ? ntiles : pairs_max);
+  if ((rc = BCOLS ? make_map_packed_cols(&b_map, p.b, p.n, p.k, p.ldb) : make_map_packed(&b_map, p.b, p.n, p.k, p.ldb, kBNh))) return rc;
+  const int pairs = (int)(ntiles < clusters ? ntiles : clusters);
   // tiles of a last wave that would occupy at most half of the pairs are cut into halves of 128 columns
   const int64_t whole = (ntiles / pairs) * pairs, rest = ntiles - whole;
-  const bool cut = rest > 0 && 2 * rest <= pairs;
+  const bool cut = SPLIT == 1 && rest > 0 && 2 * rest <= pairs;
   const int items = (int)(cut ? whole + 2 * rest : ntiles), cut_from = cut ? (int)whole : 0x7fffffff;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(2 * pairs));
+  cfg.gridDim = dim3((unsigned)(2 * SPLIT * pairs));
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.dynamicSmemBytes = Smem<SPLIT>::kBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = 2;
+  attr[1].val.clusterDim.x = 2 * SPLIT;
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  QO_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_s4_unpack_kernel<OutT, GATHER>, a_map, b_map, sa, sb, reinterpret_cast<OutT*>(out), acc_out,
-                                 reinterpret_cast<const OutT*>(bias), (int)t, (int)n, (int)k, items, cut_from, status, dsts));
+  QO_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_s4_unpack_kernel<OutT, GATHER, SPLIT, BCOLS>, a_map, b_map, p.sa, p.sb, reinterpret_cast<OutT*>(p.out),
+                                 p.acc_out, reinterpret_cast<const OutT*>(p.bias), (int)p.t, (int)p.n, (int)p.k, items, cut_from,
+                                 p.b_early ? 1 : 0, status, dsts));
   return check_launch("gemm_s4_unpack_kernel");
+}
+
+// K slices per tile: as many as there are pairs for, while every pair keeps at least two stages of K and all clusters run at
+// once.  256 x 14336 x 4096 (16 tiles): 21.7 us with three slices, the most that run at once;
+// clusters of four pairs do not fit sixteen times on the device.
+template <typename OutT, bool BCOLS>
+int launch_split(const UnpackArgs& p, uint32_t* status, cudaStream_t stream) {
+  const GatherDsts none = {};
+  const int64_t tiles = unpack_tiles(p.t, p.n), kstages = p.k / kKStage;
+  int rc = QO_ERR_UNSUPPORTED;
+  if (4 * tiles <= 74 && kstages >= 8) rc = launch_typed<OutT, false, 4, BCOLS>(p, status, none, stream);
+  if (rc == QO_ERR_UNSUPPORTED && 3 * tiles <= 74 && kstages >= 6) rc = launch_typed<OutT, false, 3, BCOLS>(p, status, none, stream);
+  if (rc == QO_ERR_UNSUPPORTED && 2 * tiles <= 74 && kstages >= 4) rc = launch_typed<OutT, false, 2, BCOLS>(p, status, none, stream);
+  if (rc == QO_ERR_UNSUPPORTED) rc = launch_typed<OutT, false, 1, BCOLS>(p, status, none, stream);
+  return rc;
 }
 
 }  // namespace
 
-// shapes the in-kernel-unpack GEMM takes: both operands with K contiguous and 16-byte aligned rows, K a multiple of
-// 256 (a ragged stage would be filled with zero BYTES by TMA, which are not zero CODES in offset binary)
+// shapes the in-kernel-unpack GEMM takes: A with K contiguous, B with K or N contiguous, 16-byte aligned rows, K a multiple
+// of 256 (a ragged stage would be filled with zero BYTES by TMA, which are not zero CODES in offset binary)
 bool gemm_unpack_supported(int64_t t, int64_t k, int64_t n, const void* a, int64_t lda, const void* b, int64_t bsk, int64_t bsn) {
   if (k < kKStage || (k % kKStage) != 0 || k > 131072) return false;
   if (n % 8) return false;  // 16-byte output stores
-  if (bsk != 1 || (bsn % 4) != 0 || (lda % 4) != 0) return false;
+  const int64_t ldb = bsk == 1 ? bsn : bsk;
+  if ((bsk != 1 && bsn != 1) || ldb <= 0 || (ldb % 4) != 0 || (lda % 4) != 0) return false;
+  if (bsk != 1 && ldb < n) return false;  // overlapping rows
   if (reinterpret_cast<uintptr_t>(a) % 16 || reinterpret_cast<uintptr_t>(b) % 16) return false;
   if (t > 0x7fffff00LL || n > 0x7fffff00LL) return false;
   return unpack_encode_fn() != nullptr;
 }
 
-// Shapes for which the kernel is the better choice: enough 256 x 256 tiles to keep the CTA pairs busy, and a row count
-// that 256-row tiles do not pad by much.  Fewer rows run on the single-CTA kernels (which split K over clusters).
-bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n) {
-  (void)k;
+// Prefill sizes: enough 256 x 256 tiles to keep the CTA pairs busy without splitting K, and a row count that 256-row
+// tiles do not pad by much.
+bool gemm_unpack_prefill(int64_t t, int64_t n) {
   if (current_kernel_policy() == 3) return false;
-  const int64_t tiles = ((t + 2 * kBM - 1) / (2 * kBM)) * ((n + kBN - 1) / kBN);
   const int64_t rows256 = ((t + 255) / 256) * 256, rows128 = ((t + 127) / 128) * 128;
-  return n >= kBN && tiles >= 48 && rows256 * 8 <= rows128 * 9;
+  return n >= kBN && unpack_tiles(t, n) >= 48 && rows256 * 8 <= rows128 * 9;
+}
+
+// Shapes for which the kernel is the better choice: prefill sizes, and everything else with K of 2048 or more.  Measured against
+// widening both operands and multiplying int8 (graph replay): 256 x 14336 x 4096 21.7 against 35.6 us, 600 x 2048 x 1024 11.1
+// against 16.0, 100 x 2048 x 256 10.0 against 11.7, but 100 x 1024 x 1024 9.4 against 7.2 and 300 x 1024 x 2048 9.6 against 7.7:
+// with four stages of K the fill and the exchange outweigh a widening pass that is as short as the product.
+bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n) {
+  return gemm_unpack_prefill(t, n) || (current_kernel_policy() != 3 && n >= kBN && k >= 2048);
 }
 
 // returns QO_ERR_UNSUPPORTED without a message when the device cannot co-schedule CTA pairs of this kernel
-int launch_gemm_unpack(const int32_t* a, int64_t lda, const int32_t* b, int64_t ldb, const float* sa, const float* sb, void* out,
+int launch_gemm_unpack(const int32_t* a, int64_t lda, const int32_t* b, int64_t bsk, int64_t bsn, const float* sa, const float* sb, void* out,
                        int out_dtype, int64_t t, int64_t k, int64_t n, int32_t* acc_out, const void* bias, uint32_t* status,
-                       cudaStream_t stream, const GatherDsts* gather) {
+                       cudaStream_t stream, bool b_early, const GatherDsts* gather) {
   if (out_dtype != QO_F16 && out_dtype != QO_BF16) return fail(QO_ERR_INVALID_ARGUMENT, "int4_matmul: out_dtype must be QO_F16 or QO_BF16");
   if (bias && reinterpret_cast<uintptr_t>(bias) % 4) return fail(QO_ERR_INVALID_ARGUMENT, "int4_matmul: bias must be 4-byte aligned");
+  const bool cols = bsk != 1;
+  const UnpackArgs p = {a, lda, b, cols ? bsk : bsn, sa, sb, out, acc_out, bias, t, k, n, b_early};
   if (gather != nullptr) {
-    if (n % 16) return fail(QO_ERR_UNSUPPORTED, "w4a4_linear_gather: n_out must be a multiple of 16");
+    if (n % 16 || cols) return fail(QO_ERR_UNSUPPORTED, "w4a4_linear_gather: n_out must be a multiple of 16");
     for (int d = 0; d < gather->n_dst; ++d)
       if (!gather->ptr[d] || reinterpret_cast<uintptr_t>(gather->ptr[d]) % 32)
         return fail(QO_ERR_INVALID_ARGUMENT, "w4a4_linear_gather: destination %d is null or not 32-byte aligned", d);
-    if (out_dtype == QO_F16) return launch_typed<__half, true>(a, lda, b, ldb, sa, sb, nullptr, nullptr, bias, t, k, n, status, *gather, stream);
-    return launch_typed<__nv_bfloat16, true>(a, lda, b, ldb, sa, sb, nullptr, nullptr, bias, t, k, n, status, *gather, stream);
+    if (out_dtype == QO_F16) return launch_typed<__half, true, 1, false>(p, status, *gather, stream);
+    return launch_typed<__nv_bfloat16, true, 1, false>(p, status, *gather, stream);
   }
   if (reinterpret_cast<uintptr_t>(out) % 16 || (acc_out && reinterpret_cast<uintptr_t>(acc_out) % 16))
     return fail(QO_ERR_INVALID_ARGUMENT, "int4_matmul: outputs of the tcgen05 kernel must be 16-byte aligned");
-  const GatherDsts none = {};
-  if (out_dtype == QO_F16) return launch_typed<__half, false>(a, lda, b, ldb, sa, sb, out, acc_out, bias, t, k, n, status, none, stream);
-  return launch_typed<__nv_bfloat16, false>(a, lda, b, ldb, sa, sb, out, acc_out, bias, t, k, n, status, none, stream);
+  if (out_dtype == QO_F16)
+    return cols ? launch_split<__half, true>(p, status, stream) : launch_split<__half, false>(p, status, stream);
+  return cols ? launch_split<__nv_bfloat16, true>(p, status, stream) : launch_split<__nv_bfloat16, false>(p, status, stream);
 }
 
 }  // namespace qo

@@ -179,7 +179,7 @@ bool gemm_sm100_supported(int64_t t, int64_t k, int64_t n, int64_t lda, int64_t 
 int launch_gemm_sm100(const int32_t* a, int64_t lda, const int32_t* b, int64_t bsk, int64_t bsn,
                       const float* sa, const float* sb, void* out, int out_dtype, int64_t t, int64_t k,
                       int64_t n, int32_t* acc_out, const void* bias, void* workspace, size_t workspace_bytes,
-                      cudaStream_t stream);
+                      cudaStream_t stream, bool b_early = false);
 
 // kernel selection of the calling thread (qo_set_kernel_policy): 0 automatic, 1 generic SIMT only, 2 tcgen05 only,
 // 3 tcgen05 only and without the CTA-pair kernel
@@ -189,8 +189,9 @@ int launch_gemm_sm100_pair(const int8_t* a8, const int8_t* b8, const float* sa, 
                            int64_t t, int64_t k, int64_t n, int32_t* acc_out, const void* bias, uint32_t* status,
                            cudaStream_t stream);
 
-// packed-int4 GEMM that unpacks inside the kernel (int4_gemm_sm100_unpack.cu): b is [n, k/8] with row stride ldb words
+// packed-int4 GEMM that unpacks inside the kernel (int4_gemm_sm100_unpack.cu): b is [n, k/8] (bsk == 1) or [k/8, n] (bsn == 1)
 bool gemm_unpack_supported(int64_t t, int64_t k, int64_t n, const void* a, int64_t lda, const void* b, int64_t bsk, int64_t bsn);
+bool gemm_unpack_prefill(int64_t t, int64_t n);  // sizes that keep the CTA pairs busy without splitting K (the fused gather takes only these)
 bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n);
 // destinations of the fused all-gather (see gemm_s4_unpack_kernel): the buffers [total_rows, n] of this GPU and its
 // peers; this rank's rows start at row_offset
@@ -199,9 +200,10 @@ struct GatherDsts {
   int n_dst;
   long long row_offset;
 };
-int launch_gemm_unpack(const int32_t* a, int64_t lda, const int32_t* b, int64_t ldb, const float* sa, const float* sb, void* out,
+// b_early: B was not written by the kernel that precedes the GEMM in the stream
+int launch_gemm_unpack(const int32_t* a, int64_t lda, const int32_t* b, int64_t bsk, int64_t bsn, const float* sa, const float* sb, void* out,
                        int out_dtype, int64_t t, int64_t k, int64_t n, int32_t* acc_out, const void* bias, uint32_t* status,
-                       cudaStream_t stream, const GatherDsts* gather = nullptr);
+                       cudaStream_t stream, bool b_early = false, const GatherDsts* gather = nullptr);
 
 // pieces of the tcgen05 GEMM, used separately by the fused layer
 int launch_widen_rows(const int32_t* in, int64_t ld_words, int8_t* out, int64_t rows, int64_t k, cudaStream_t stream, bool blocked,

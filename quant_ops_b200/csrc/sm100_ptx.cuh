@@ -122,6 +122,15 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// the same without ordering memory: nobody reads anything because of this barrier
+__device__ __forceinline__ void cluster_sync_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// bulk copy from this CTA's shared memory into a peer's (shared::cluster addresses of the peer), bytes counted on a barrier there
+__device__ __forceinline__ void bulk_copy_s2cluster(uint32_t dst_cluster, uint32_t src_cta, uint32_t bytes, uint32_t bar_cluster) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst_cluster), "r"(src_cta), "r"(bytes), "r"(bar_cluster) : "memory");
+}
 // address of the same shared-memory location in the CTA with the given rank of this cluster
 __device__ __forceinline__ uint32_t cluster_map_shared(uint32_t cta_addr, uint32_t rank) {
   uint32_t r;
@@ -134,6 +143,12 @@ __device__ __forceinline__ void st_cluster_shared_v4(uint32_t cluster_addr, uint
 __device__ __forceinline__ uint4 ld_shared_v4(uint32_t cta_addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(cta_addr) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ uint32_t ld_shared_u32(uint32_t cta_addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(cta_addr) : "memory");
   return v;
 }
 

@@ -1,0 +1,61 @@
+"""The GEMM that unpacks inside the kernel, with K split over clusters of CTA pairs and with the weights in the [K/8, N] layout:
+accumulators and outputs are the bits of the kernels that multiply widened operands (policy 3) at the edges of its tiles."""
+import pytest
+import torch
+
+import quant_ops_b200 as q
+from helpers import N, abi_int4_matmul, lib, make_inputs, stream_ptr
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# rows: one, around a CTA's and a pair's rows; columns: one tile, ragged tiles, as many as leave two, one or no split;
+# K: a single stage, the shortest that are split in two and in four, odd numbers of stages
+SHAPES = [(1, 4096, 4096), (33, 256, 256), (100, 1024, 264), (128, 2048, 1024), (129, 2304, 1000), (256, 14336, 4096), (257, 4096, 4096),
+          (300, 2816, 520), (512, 1280, 4096), (200, 4096, 14336), (333, 4096, 14328), (700, 11008, 4088), (1030, 4096, 1024)]
+
+
+def problem(t, k, n, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    words = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, dtype=torch.int64, device=DEV, generator=g).to(torch.int32)
+    return words(t, k // 8), words(n, k // 8), torch.rand(t, device=DEV, generator=g) + 0.01, torch.rand(n, device=DEV, generator=g) * 1e-4
+
+
+@pytest.mark.parametrize("t,k,n", SHAPES)
+@pytest.mark.parametrize("layout", ["weights_t_view", "reference_contiguous"])
+def test_same_bits_as_the_widening_path(t, k, n, layout):
+    a, w, sa, sb = problem(t, k, n, t + k + n)
+    b = w.t() if layout == "weights_t_view" else w.t().contiguous()
+    for out_dtype in ("fp16", "bf16"):
+        ref, ref_acc = abi_int4_matmul(a, b, sa, sb, out_dtype, True, policy=3)
+        got, acc = abi_int4_matmul(a, b, sa, sb, out_dtype, True, policy=2)
+        assert lib.qo_device_status(stream_ptr()) == N.QO_OK
+        assert torch.equal(acc, ref_acc)
+        assert torch.equal(got.view(torch.int16), ref.view(torch.int16))
+
+
+def test_row_strides_and_repeated_calls():
+    a, w, sa, sb = problem(150, 4096, 2048, 9)
+    wide = torch.zeros(150, 516, dtype=torch.int32, device=DEV)
+    wide[:, :512] = a
+    cols = torch.zeros(512, 2056, dtype=torch.int32, device=DEV)
+    cols[:, :2048] = w.t()
+    ref = abi_int4_matmul(a, w.t(), sa, sb, "bf16", policy=3)
+    for _ in range(30):  # the rings are reused as exchange buffers: a leftover of one call must not reach the next
+        assert torch.equal(abi_int4_matmul(wide[:, :512], cols[:, :2048], sa, sb, "bf16"), ref)
+        assert torch.equal(abi_int4_matmul(a, w.t(), sa, sb, "bf16"), ref)
+
+
+@pytest.mark.parametrize("tokens,k,n_out", [(33, 4096, 4096), (64, 14336, 4096), (256, 14336, 4096), (130, 4096, 11008)])
+def test_layer_with_early_weight_loads(tokens, k, n_out):
+    """Inside the layer the first weight stages are requested before the quantizer ahead has finished: the same bits as the
+    two calls by hand, with bias, call after call."""
+    x, left, right = make_inputs(tokens, k, "bf16", tokens + n_out, True)
+    xd, ld, rd = x.to(DEV), left.to(DEV), right.to(DEV)
+    _, w, _, sb = problem(1, k, n_out, 4)
+    bias = torch.randn(n_out, device=DEV).bfloat16()
+    codes, scales = q.flatquant_dynamic_quantize(xd, ld, rd, 0.9, True)
+    want = (q.int4_matmul_ex(codes, w.t(), scales, sb, torch.bfloat16).float() + bias.float()).bfloat16()
+    for _ in range(10):
+        assert torch.equal(q.w4a4_linear(xd, ld, rd, w, sb, bias, 0.9), want)
+    q.device_status()
