@@ -15,6 +15,9 @@ import torch
 from . import ops
 from .decompose import get_decompose_dim
 
+_w4a4_linear = torch.ops.quant_ops.w4a4_linear.default
+_w4a4_linear_prepared = torch.ops.quant_ops.w4a4_linear_prepared.default
+
 
 class W4A4Linear(torch.nn.Module):
     def __init__(self, in_features: int, out_features: int, bias: bool = False, clip_ratio: float = 1.0,
@@ -68,15 +71,20 @@ class W4A4Linear(torch.nn.Module):
         return self.prepare()
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features)
-        if x2.dtype != self.left_trans.dtype:
-            raise RuntimeError(f"input dtype {x2.dtype} does not match the transforms' dtype {self.left_trans.dtype}")
-        out_dtype = x2.dtype if x2.dtype in (torch.float16, torch.bfloat16) else torch.float16
+        # The buffers by dictionary instead of module attribute lookups, and no reshape of an input that has two dimensions:
+        # in a decode step this method's own time is as long as the kernels'.
+        try:
+            b = self._buffers
+            left, right, w, ws, bias = b["left_trans"], b["right_trans"], b["weight_packed"], b["weight_scale"], b["bias"]
+        except KeyError:  # one of them was replaced by a parameter
+            left, right, w, ws, bias = self.left_trans, self.right_trans, self.weight_packed, self.weight_scale, self.bias
+        x2 = x if x.dim() == 2 and x.shape[1] == self.in_features else x.reshape(-1, self.in_features)
+        dtype = x2.dtype
+        if dtype != left.dtype:
+            raise RuntimeError(f"input dtype {dtype} does not match the transforms' dtype {left.dtype}")
+        out_dtype = dtype if dtype == torch.bfloat16 else torch.float16
         if self.weight_int8 is not None:
-            y = ops.w4a4_linear_prepared(x2, self.left_trans, self.right_trans, self.weight_packed, self.weight_int8,
-                                         self.weight_scale, self.bias, self.clip_ratio, out_dtype)
+            y = _w4a4_linear_prepared(x2, left, right, w, self.weight_int8, ws, bias, self.clip_ratio, out_dtype)
         else:
-            y = ops.w4a4_linear(x2, self.left_trans, self.right_trans, self.weight_packed, self.weight_scale, self.bias,
-                                self.clip_ratio, out_dtype)
-        return y.reshape(*lead, self.out_features)
+            y = _w4a4_linear(x2, left, right, w, ws, bias, self.clip_ratio, out_dtype)
+        return y if x2 is x else y.reshape(*x.shape[:-1], self.out_features)
