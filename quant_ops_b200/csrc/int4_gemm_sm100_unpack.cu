@@ -777,6 +777,9 @@ bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n) {
   return gemm_unpack_prefill(t, n) || (current_kernel_policy() != 3 && n >= kBN && k >= 2048);
 }
 
+// preferred, and all tiles on the 74 CTA pairs at once
+bool gemm_unpack_one_round(int64_t t, int64_t k, int64_t n) { return gemm_unpack_preferred(t, k, n) && unpack_tiles(t, n) <= 74; }
+
 // returns QO_ERR_UNSUPPORTED without a message when the device cannot co-schedule CTA pairs of this kernel
 int launch_gemm_unpack(const int32_t* a, int64_t lda, const int32_t* b, int64_t bsk, int64_t bsn, const float* sa, const float* sb, void* out,
                        int out_dtype, int64_t t, int64_t k, int64_t n, int32_t* acc_out, const void* bias, uint32_t* status,

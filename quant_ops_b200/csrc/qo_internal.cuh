@@ -193,6 +193,7 @@ int launch_gemm_sm100_pair(const int8_t* a8, const int8_t* b8, const float* sa, 
 bool gemm_unpack_supported(int64_t t, int64_t k, int64_t n, const void* a, int64_t lda, const void* b, int64_t bsk, int64_t bsn);
 bool gemm_unpack_prefill(int64_t t, int64_t n);  // sizes that keep the CTA pairs busy without splitting K (the fused gather takes only these)
 bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n);
+bool gemm_unpack_one_round(int64_t t, int64_t k, int64_t n);
 // destinations of the fused all-gather (see gemm_s4_unpack_kernel): the buffers [total_rows, n] of this GPU and its
 // peers; this rank's rows start at row_offset
 struct GatherDsts {
