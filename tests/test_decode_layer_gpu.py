@@ -1,0 +1,41 @@
+"""Decode-sized layers over the row lengths at which the resident-weights GEMM groups its warps differently (one, two, four or all
+sixteen to a barrier): the bits of quantize -> GEMM by hand, and the module's forward over input shapes and replaced buffers."""
+import pytest
+import torch
+
+import quant_ops_b200 as q
+from helpers import N, lib, make_inputs, stream_ptr
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def layer_inputs(tokens, k, n_out):
+    x, left, right = make_inputs(tokens, k, "bf16", tokens + k + n_out, True)
+    g = torch.Generator(device=DEV).manual_seed(k)
+    w = torch.randint(-2 ** 31, 2 ** 31, (n_out, k // 8), dtype=torch.int64, device=DEV, generator=g).to(torch.int32)
+    return x.to(DEV), left.to(DEV), right.to(DEV), w, torch.rand(n_out, device=DEV, generator=g) * 1e-3
+
+
+@pytest.mark.parametrize("k", [1024, 2560, 3072, 4096, 6144, 11008, 14336])
+@pytest.mark.parametrize("tokens,n_out", [(1, 4096), (9, 1032), (32, 520)])
+def test_same_bits_as_two_calls(tokens, k, n_out):
+    x, left, right, w, sw = layer_inputs(tokens, k, n_out)
+    codes, scales = q.flatquant_dynamic_quantize(x, left, right, 0.9, True)
+    want = q.int4_matmul_ex(codes, w.t(), scales, sw, torch.bfloat16)
+    for _ in range(5):
+        assert torch.equal(q.w4a4_linear(x, left, right, w, sw, None, 0.9), want)
+    assert lib.qo_device_status(stream_ptr()) == N.QO_OK
+
+
+def test_forward_over_input_shapes():
+    x, left, right, w, sw = layer_inputs(6, 4096, 256)
+    layer = q.W4A4Linear(4096, 256, clip_ratio=0.9, device=DEV)
+    layer.weight_packed.copy_(w), layer.weight_scale.copy_(sw), layer.left_trans.copy_(left), layer.right_trans.copy_(right)
+    want = q.w4a4_linear(x, left, right, w, sw, None, 0.9)
+    assert torch.equal(layer(x), want)
+    assert torch.equal(layer(x.reshape(2, 3, 4096)), want.reshape(2, 3, 256))
+    assert torch.equal(layer(x[0]), layer(x[:1])[0])
+    assert layer(x[:0]).shape == (0, 256)
+    layer.left_trans = torch.nn.Parameter(left.clone(), requires_grad=False)  # leaves the buffers
+    assert torch.equal(layer(x), want)
