@@ -11,16 +11,20 @@
 //
 //   warp 0        TMA: 3-D tensor map (n, m, token), boxes of 64 x M, 128-byte swizzle; ONE X stage: it is free again
 //                 as soon as the first product is done, so the next token's load runs under the rest of this token
-//   warp 1        issues both products, tile by tile, so that the Y pass of tile 0 runs under the first product of
-//                 tile 1 and the second product of tile 0 under the Y pass of tile 1
-//   warps 2-9     Y pass: warp (tile, q) rounds lanes 32q .. 32q+31 of its tile, in place
-//   warps 10-25   quantize pass: warp (tile, h, q) takes columns (rows of the token's matrix) 64h .. 64h+63 of lanes
+//   warps 1, 2    issue the two products, tile by tile, so that the Y pass of tile 0 runs under the first product of
+//                 tile 1 and the second product of tile 0 under the Y pass of tile 1; two issuers keep each other's
+//                 barrier latencies off the tensor core
+//   warps 4-11    Y pass: warp (tile, q) rounds lanes 32q .. 32q+31 of its tile, in place
+//   warps 12-27   quantize pass: warp (tile, h, q) takes columns (rows of the token's matrix) 64h .. 64h+63 of lanes
 //                 32q .. 32q+31; absmax through shared memory, scale, codes.  A lane holds one column of the token's
 //                 matrix, so the eight codes of a packed word lie in eight lanes: an 8 x 8 transposition of nibbles
 //                 (three shuffles) turns them round.
 //
-// Bound: HBM (57,344 bytes in and 14,340 out per token of 28672; 11 us for 1001 tokens).  Measured: 39.6 us for 1001 bf16
-// tokens to packed codes, 1.8 TB/s, where the SIMT kernel, until now the only one for such widths, takes 3608 us.
+// Bound: HBM (57,344 bytes in and 14,340 out per token of 28672; 11 us for 1001 tokens).  Measured in graph replay: 29.7 us
+// for 1001 bf16 tokens to packed codes, 2.4 TB/s, 112.7 us for 4000 (35.1 and 124.7 with one issuing warp and without the
+// register shares); the SIMT kernel, before the only one for such widths, takes 3600 us for the former.  A token is a
+// chain of load, first product, Y pass and second product; its X boxes given back one by one were measured slower (38 to
+// 41 us: more barrier polls and commits in the issuing thread).
 //
 // Numerics are those of flatquant_sm100_n128.cu (same packed arithmetic, same rounding points; reference:
 // src/quant_ops/ops/quantization/flatquant/ops.py:99-117).  Tokens with an infinity or a NaN among their transformed
@@ -34,8 +38,12 @@ namespace {
 using namespace ptx;
 using namespace fq;
 
-constexpr int kThreads = 832;  // 26 warps: TMA, MMA issuer, 8 (Y pass) + 16 (quantize pass)
-constexpr int kYWarp0 = 2, kQWarp0 = 10;
+constexpr int kThreads = 896;  // 28 warps: TMA, two MMA issuers, one idle, 8 (Y pass) + 16 (quantize pass)
+constexpr int kYWarp0 = 4, kQWarp0 = 12;
+// Registers per thread (by warpgroup, hence the idle warp): the block is launched with 896 x 72.  With 224 KB of shared
+// memory in use hardly any L1 is left, so a register spilled in the quantize pass is read back from L2.
+constexpr int kRegsQuant = 88, kRegsRest = 48;
+static_assert(512 * kRegsQuant + 384 * kRegsRest <= kThreads * 72, "the shares must fit the launch's registers");
 constexpr int kMaxM = 128, kMaxN = 256;
 constexpr int kOffX = 0;                              // four 64-column atoms of M rows
 constexpr int kOffL = kOffX + 4 * kAtomBytes;         // two 64-column blocks of M rows
@@ -183,80 +191,8 @@ flatquant_n256_kernel(const __grid_constant__ CUtensorMap x_map, const T* __rest
     asm volatile("bar.sync 1, %0;" ::"n"(kStagers) : "memory");
   }
 
-  if (warp == 0) {
-    if (lane == 0) {
-      const int boxes = (n + 63) >> 6;
-      long long tok = blockIdx.x;
-      for (int it = 0; it < mine; ++it, tok += gridDim.x) {
-        if (!mbar_wait(smem_u32(&misc->empty_x), (it & 1) ^ 1)) { atomicCAS(status, 0u, 0xC00u); break; }
-        const uint32_t bar = smem_u32(&misc->full_x);
-        mbar_arrive_expect_tx(bar, (uint32_t)(boxes * m * 128));
-        for (int b = 0; b < boxes; ++b) tma_load_3d(smem_base + kOffX + b * kAtomBytes, &x_map, bar, b * 64, 0, (int)tok);
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc1 = umma_idesc(1, Fmt<T>::id, Fmt<T>::id, 1, 0, 128, m);  // A = R^T: M-major, B = X rows: K-major
-      const uint32_t idesc2 = umma_idesc(1, Fmt<T>::id, Fmt<T>::id, 0, 1, 128, m);  // A = Y^T in tensor memory, B = L: N-major
-      const uint64_t desc_x = umma_smem_desc_sw128(smem_base + kOffX, 16, 1024);
-      const uint64_t desc_l = umma_smem_desc_sw128(smem_base + kOffL, kAtomBytes, 1024);
-      const int ks1 = n >> 4, ks2 = m >> 4;
-      bool ok = true;
-      for (int it = 0; ok && it < mine; ++it) {
-        const int ph = it & 1;
-        if (!mbar_wait(smem_u32(&misc->full_x), ph)) { atomicCAS(status, 0u, 0xC10u); break; }
-        for (int tl = 0; tl < 2; ++tl) {
-          if (!mbar_wait(smem_u32(&misc->y_free[tl]), ph ^ 1)) { atomicCAS(status, 0u, 0xC20u + tl); ok = false; break; }
-          tc_fence_after();
-          const uint64_t desc_r = umma_smem_desc_sw128(smem_base + kOffR + tl * 2 * (n * 128), (uint32_t)(n * 128), 1024);
-#pragma unroll 1
-          for (int ks = 0; ks < ks1; ++ks)  // 16 rows of R = 2048 bytes per step; X: 32 bytes inside a 64-column atom
-            mma_f16_ss(tmem + tl * 128, desc_r + (uint64_t)(ks * 128), desc_x + (uint64_t)((ks >> 2) * (kAtomBytes >> 4) + (ks & 3) * 2), idesc1, ks);
-          mma_commit(smem_u32(&misc->d1_full[tl]));
-        }
-        if (!ok) break;
-        mma_commit(smem_u32(&misc->empty_x));
-        for (int tl = 0; tl < 2; ++tl) {
-          if (const int w = mbar_wait2(smem_u32(&misc->y_ready[tl]), ph, smem_u32(&misc->d2_empty[tl]), ph ^ 1)) {
-            atomicCAS(status, 0u, 0xC20u + 0x10u * w + tl);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-#pragma unroll 1
-          for (int ks = 0; ks < ks2; ++ks)  // 16 values of Y^T = 8 tensor-memory columns per step
-            mma_f16_ts(tmem + kColZ + tl * 128, tmem + tl * 128 + ks * 8, desc_l + (uint64_t)(ks * 128), idesc2, ks);
-          mma_commit(smem_u32(&misc->y_free[tl]));
-          mma_commit(smem_u32(&misc->d2_full[tl]));
-        }
-      }
-    }
-  } else if (warp < kQWarp0) {
-    // ---- Y pass: 32 lanes of one tile; every 32 float32 columns become 16 packed ones, written below what is still to read
-    const int q = warp & 3, tl = (warp - kYWarp0) >> 2;
-    const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + tl * 128;
-    const bool works = tl * 128 + q * 32 < n;
-    for (int it = 0; it < (works ? mine : 0); ++it) {
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc->d1_full[tl]), it & 1))) { atomicCAS(status, 0u, 0xC50u + tl); break; }
-      tc_fence_after();
-#pragma unroll 1
-      for (int c = 0; c < m; c += 32) {
-        uint32_t v[32], a[8], b[8];
-        tmem_ld_32x32b_x32(base + c, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          a[i] = pack2<T>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-          b[i] = pack2<T>(__uint_as_float(v[16 + 2 * i]), __uint_as_float(v[16 + 2 * i + 1]));
-        }
-        tmem_st_32x32b_x8(base + (c >> 1), a);
-        if (c + 16 < m) tmem_st_32x32b_x8(base + (c >> 1) + 8, b);
-      }
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive_warp(smem_u32(&misc->y_ready[tl]));
-    }
-  } else {
+  if (warp >= kQWarp0) {
+    regs_inc<kRegsQuant>();
     // ---- quantize pass -----------------------------------------------------------------------------------------------
     const int q = warp & 3, idx = (warp - kQWarp0) >> 2, tl = idx >> 1, h = idx & 1;
     const int n0 = tl * 128 + q * 32, r0 = h * 64;   // first column / first row of the token's matrix in this warp
@@ -273,20 +209,16 @@ flatquant_n256_kernel(const __grid_constant__ CUtensorMap x_map, const T* __rest
       tc_fence_after();
       uint32_t zz[32];  // 64 rounded values as packed pairs; rows past the last one are zero
 #pragma unroll
-      for (int ch = 0; ch < 2; ++ch) {
-        if (ch * 32 < rows) {
-          uint32_t v[32];
-          tmem_ld_32x32b_x32(taddr + ch * 32, v);
+      for (int ch = 0; ch < 4; ++ch) {
+        if (ch * 16 < rows) {
+          uint32_t v[16];
+          tmem_ld_32x32b_x16(taddr + ch * 16, v);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) zz[16 * ch + i] = P2<T>::cvt(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-          if (rows < ch * 32 + 32) {
-#pragma unroll
-            for (int i = 8; i < 16; ++i) zz[16 * ch + i] = 0u;
-          }
+          for (int i = 0; i < 8; ++i) zz[8 * ch + i] = P2<T>::cvt(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
         } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) zz[16 * ch + i] = 0u;
+          for (int i = 0; i < 8; ++i) zz[8 * ch + i] = 0u;
         }
       }
       tc_fence_before();
@@ -393,6 +325,93 @@ flatquant_n256_kernel(const __grid_constant__ CUtensorMap x_map, const T* __rest
         }
       }
     }
+  } else {
+  regs_dec<kRegsRest>();
+  if (warp == 0) {
+    if (lane == 0) {
+      const int boxes = (n + 63) >> 6;
+      long long tok = blockIdx.x;
+      for (int it = 0; it < mine; ++it, tok += gridDim.x) {
+        if (!mbar_wait(smem_u32(&misc->empty_x), (it & 1) ^ 1)) { atomicCAS(status, 0u, 0xC00u); break; }
+        const uint32_t bar = smem_u32(&misc->full_x);
+        mbar_arrive_expect_tx(bar, (uint32_t)(boxes * m * 128));
+        for (int b = 0; b < boxes; ++b) tma_load_3d(smem_base + kOffX + b * kAtomBytes, &x_map, bar, b * 64, 0, (int)tok);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc1 = umma_idesc(1, Fmt<T>::id, Fmt<T>::id, 1, 0, 128, m);  // A = R^T: M-major, B = X rows: K-major
+      const uint64_t desc_x = umma_smem_desc_sw128(smem_base + kOffX, 16, 1024);
+      const int ks1 = n >> 4;
+      bool ok = true;
+      for (int it = 0; ok && it < mine; ++it) {
+        const int ph = it & 1;
+        for (int tl = 0; tl < 2; ++tl) {
+          if (const int w = tl == 0 ? mbar_wait2(smem_u32(&misc->full_x), ph, smem_u32(&misc->y_free[0]), ph ^ 1)
+                                    : (mbar_wait(smem_u32(&misc->y_free[1]), ph ^ 1) ? 0 : 3)) {
+            atomicCAS(status, 0u, 0xC10u + w);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint64_t desc_r = umma_smem_desc_sw128(smem_base + kOffR + tl * 2 * (n * 128), (uint32_t)(n * 128), 1024);
+#pragma unroll 2
+          for (int ks = 0; ks < ks1; ++ks)  // 16 rows of R = 2048 bytes per step; X: 32 bytes inside a 64-column atom
+            mma_f16_ss(tmem + tl * 128, desc_r + (uint64_t)(ks * 128), desc_x + (uint64_t)((ks >> 2) * (kAtomBytes >> 4) + (ks & 3) * 2), idesc1, ks);
+          mma_commit(smem_u32(&misc->d1_full[tl]));
+        }
+        if (ok) mma_commit(smem_u32(&misc->empty_x));
+      }
+    }
+  } else if (warp == 2) {
+    if (lane == 0) {
+      const uint32_t idesc2 = umma_idesc(1, Fmt<T>::id, Fmt<T>::id, 0, 1, 128, m);  // A = Y^T in tensor memory, B = L: N-major
+      const uint64_t desc_l = umma_smem_desc_sw128(smem_base + kOffL, kAtomBytes, 1024);
+      const int ks2 = m >> 4;
+      bool ok = true;
+      for (int it = 0; ok && it < mine; ++it) {
+        const int ph = it & 1;
+        for (int tl = 0; tl < 2; ++tl) {
+          if (const int w = mbar_wait2(smem_u32(&misc->y_ready[tl]), ph, smem_u32(&misc->d2_empty[tl]), ph ^ 1)) {
+            atomicCAS(status, 0u, 0xC20u + 0x10u * w + tl);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+#pragma unroll 2
+          for (int ks = 0; ks < ks2; ++ks)  // 16 values of Y^T = 8 tensor-memory columns per step
+            mma_f16_ts(tmem + kColZ + tl * 128, tmem + tl * 128 + ks * 8, desc_l + (uint64_t)(ks * 128), idesc2, ks);
+          mma_commit(smem_u32(&misc->y_free[tl]));
+          mma_commit(smem_u32(&misc->d2_full[tl]));
+        }
+      }
+    }
+  } else if (warp >= kYWarp0) {
+    // ---- Y pass: 32 lanes of one tile; every 32 float32 columns become 16 packed ones, written below what is still to read
+    const int q = warp & 3, tl = (warp - kYWarp0) >> 2;
+    const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + tl * 128;
+    const bool works = tl * 128 + q * 32 < n;
+    for (int it = 0; it < (works ? mine : 0); ++it) {
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc->d1_full[tl]), it & 1))) { atomicCAS(status, 0u, 0xC50u + tl); break; }
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; c < m; c += 32) {
+        uint32_t v[32], a[8], b[8];
+        tmem_ld_32x32b_x32(base + c, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          a[i] = pack2<T>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+          b[i] = pack2<T>(__uint_as_float(v[16 + 2 * i]), __uint_as_float(v[16 + 2 * i + 1]));
+        }
+        tmem_st_32x32b_x8(base + (c >> 1), a);
+        if (c + 16 < m) tmem_st_32x32b_x8(base + (c >> 1) + 8, b);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive_warp(smem_u32(&misc->y_ready[tl]));
+    }
+  }
   }
 
   tc_fence_before();
