@@ -17,7 +17,7 @@
 //     two's-complement nibbles, and a nibble placed in the HIGH half of a byte is the int8 value 16 * n.  The even
 //     and the odd elements of a word make one operand register each; activations are treated identically, so both
 //     sides agree on the (permuted) order of K, and every product carries the factor 256, removed exactly by an
-//     arithmetic shift at the end (|256 * acc| < 2^31 for K <= 131072);
+//     arithmetic shift at the end (|256 * acc| < 2^31 for K < 131072; at 131072 codes of -8 on both sides give 2^31);
 //   * the products run on mma.sync m16n8k32 (int8): channels are the 16 rows, 8 tokens the columns.
 //
 // Arithmetic as in the reference kernel (src/quant_ops/ops/quantization/int4_matmul/kernels/
@@ -449,7 +449,7 @@ int launch_t(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t ldb, con
 
 // few rows, weights contiguous along K, K a multiple of 128, rows of both operands 16-byte aligned
 bool gemm_skinny_supported(int64_t t, int64_t k, int64_t n, const void* a, int64_t lda, const void* b, int64_t bsk, int64_t bsn) {
-  return t >= 1 && t <= 32 && n >= 1 && k >= 128 && k <= 131072 && (k % 128) == 0 && bsk == 1 && (bsn % 4) == 0 && (lda % 4) == 0 &&
+  return t >= 1 && t <= 32 && n >= 1 && k >= 128 && k < 131072 && (k % 128) == 0 && bsk == 1 && (bsn % 4) == 0 && (lda % 4) == 0 &&
          (reinterpret_cast<uintptr_t>(a) % 16) == 0 && (reinterpret_cast<uintptr_t>(b) % 16) == 0 && n <= (int64_t)16 * 0x7fffffff;
 }
 

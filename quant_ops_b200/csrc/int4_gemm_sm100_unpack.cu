@@ -26,7 +26,8 @@
 // nibble in the HIGH half of a byte is the int8 value 16 * n.  Each packed word yields one word of its even elements
 // ((t << 4) & 0xF0F0F0F0) and one of its odd elements (t & 0xF0F0F0F0); both operands use the same (permuted) order
 // of K, a dot product does not care, and every product carries the factor 256, which an arithmetic shift removes
-// exactly in the epilogue (|256 * acc| < 2^31 for K <= 131072).  Four integer instructions per eight values.
+// exactly in the epilogue (codes of -8 on both sides give 256 * 64 * K, which is 2^31 at K = 131072: only shorter
+// products, |256 * acc| < 2^31, come here).  Four integer instructions per eight values.
 //
 // Roles (28 warps per CTA; both CTAs of a pair run the same code, only the leader issues MMAs):
 //   warp 0       TMA producer: packed A block + packed B half into a ring of 3 stages (local barriers)
@@ -751,7 +752,7 @@ int launch_split(const UnpackArgs& p, uint32_t* status, cudaStream_t stream) {
 // shapes the in-kernel-unpack GEMM takes: A with K contiguous, B with K or N contiguous, 16-byte aligned rows, K a multiple
 // of 256 (a ragged stage would be filled with zero BYTES by TMA, which are not zero CODES in offset binary)
 bool gemm_unpack_supported(int64_t t, int64_t k, int64_t n, const void* a, int64_t lda, const void* b, int64_t bsk, int64_t bsn) {
-  if (k < kKStage || (k % kKStage) != 0 || k > 131072) return false;
+  if (k < kKStage || (k % kKStage) != 0 || k >= 131072) return false;  // 256 * acc must fit an int32
   if (n % 8) return false;  // 16-byte output stores
   const int64_t ldb = bsk == 1 ? bsn : bsk;
   if ((bsk != 1 && bsn != 1) || ldb <= 0 || (ldb % 4) != 0 || (lda % 4) != 0) return false;

@@ -34,6 +34,22 @@ def test_same_bits_as_the_widening_path(t, k, n, layout):
         assert torch.equal(got.view(torch.int16), ref.view(torch.int16))
 
 
+@pytest.mark.parametrize("t,n", [(4, 256), (40, 256), (40, 264), (300, 1024), (1024, 3072)])
+@pytest.mark.parametrize("k", [131072 - 256, 131072])
+def test_extreme_codes_of_the_longest_reductions(t, n, k):
+    """Zeroed operands are codes of -8 on both sides.  With the factor 256 of the kernels that keep the nibbles in the high
+    half of a byte the sum is 2^31 at K = 131072, one more than an int32 holds: those kernels take the shorter products only
+    (few rows, split K, prefill), and longer ones run on widened operands."""
+    a, w = torch.zeros(t, k // 8, dtype=torch.int32, device=DEV), torch.zeros(n, k // 8, dtype=torch.int32, device=DEV)
+    sa, sb = torch.full((t,), 2.0 ** -10, device=DEV), torch.ones(n, device=DEV)
+    for b in (w.t(), w.t().contiguous()):
+        before = lib.qo_kernel_launch_count()
+        out, acc = abi_int4_matmul(a, b, sa, sb, "fp16", True)
+        assert (lib.qo_kernel_launch_count() - before == 1) == (k < 131072)  # one launch: no widening pass
+        assert int(acc.min()) == int(acc.max()) == 64 * k
+        assert float(out.min()) == float(out.max()) == 64 * k / 1024
+
+
 def test_row_strides_and_repeated_calls():
     a, w, sa, sb = problem(150, 4096, 2048, 9)
     wide = torch.zeros(150, 516, dtype=torch.int32, device=DEV)
