@@ -28,7 +28,8 @@
 //
 // Numerics are those of flatquant_sm100_n128.cu (same packed arithmetic, same rounding points; reference:
 // src/quant_ops/ops/quantization/flatquant/ops.py:99-117).  Tokens with an infinity or a NaN among their transformed
-// values, and fp16 tokens whose scale rounds to zero, take the scalar route of the SIMT kernel, code by code.
+// values, and tokens whose scale is zero (fp16), infinite (fp16 with a clip ratio above 1) or 2^100 and more (bf16: the
+// second term of 1/s would be subnormal), take the scalar route of the SIMT kernel, code by code.
 // Every mbarrier wait is bounded.
 #include "flatquant_sm100_common.cuh"
 
@@ -282,7 +283,7 @@ flatquant_n256_kernel(const __grid_constant__ CUtensorMap x_map, const T* __rest
       uint32_t rhi2, rlo2;
       P2<T>::recip2(inv_s, rhi2, rlo2);
       if (first && lane == 0) store_scale(scales, tok, s, scale_dtype);
-      const bool careful = special || s == 0.f;
+      const bool careful = special || s == 0.f || !(s < 0x1p100f);
       // a quotient can only leave [-8, 7] after rounding if some |z| / s reaches 7.5
       const bool clamp_needed = !(__uint_as_float(warp_bits) * inv_s < 7.4f);
 

@@ -3,7 +3,7 @@ oracle, and against the SIMT kernel on tokens with infinities, NaNs and zeros.""
 import pytest
 import torch
 
-from helpers import N, abi_quantize, lib, make_inputs, ptr, QD, stream_ptr, t2f
+from helpers import N, abi_quantize, lib, make_inputs, ptr, QD, stream_ptr, t2f, TD
 from oracle import w4a4_oracle as O
 from test_quantize_gpu import check
 
@@ -59,3 +59,21 @@ def test_special_tokens_equal_the_simt_kernel(dtype, pack):
     assert torch.equal(got[0][special], ref[0][special])
     assert torch.equal(got[1][special], ref[1][special])
     assert torch.allclose(got[1][6], ref[1][6], rtol=2.0 ** -7)
+
+
+@pytest.mark.parametrize("dtype,clip", [("bf16", 0.9), ("bf16", 1e6), ("fp16", 1.0), ("fp16", 1.3), ("fp16", 1e6)])
+@pytest.mark.parametrize("pack", [True, False])
+def test_scales_over_the_whole_range_of_the_type(dtype, clip, pack):
+    """Identity transforms, so that every kernel quantizes the same values: from the smallest to the largest scales, and
+    infinite ones (the row's largest value times the clip ratio leaves the type), the codes are those of the SIMT kernel."""
+    m, n = 32, 160
+    g = torch.Generator().manual_seed(11)
+    z = torch.randn(64, m * n, dtype=torch.float64, generator=g).clamp_(-1.99, 1.99)
+    low, high = (-130, 126) if dtype == "bf16" else (-23, 15)
+    x = (z * torch.exp2(torch.linspace(low, high, 64).round().double())[:, None]).to(TD[dtype]).to(DEV)
+    assert bool(x.isfinite().all())
+    left, right = torch.eye(m, dtype=x.dtype, device=DEV), torch.eye(n, dtype=x.dtype, device=DEV)
+    got = abi_quantize(x, left, right, clip, pack, dtype, policy=2)
+    ref = abi_quantize(x, left, right, clip, pack, dtype, policy=1)
+    assert bool(ref[1].isinf().any()) == (clip > 1)
+    assert torch.equal(got[1], ref[1]) and torch.equal(got[0], ref[0])
