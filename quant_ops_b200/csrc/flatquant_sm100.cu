@@ -514,8 +514,11 @@ bool flatquant_sm100_supported(int64_t ldx, int m, int n, int in_dtype, const vo
 }
 
 // Right transforms above 128: one to three tokens stay on the SIMT kernel, which the tests pin for a call of three.  (It
-// is the slower one there too; the line is not a measured crossing.)
-bool flatquant_sm100_preferred(int64_t tokens, int m, int n) { return tokens >= 4 || !flatquant_sm100_n256_supported(m, n); }
+// is the slower one there too; the line is not a measured crossing.)  So do outputs that are not 16-byte aligned, which that
+// kernel takes and this one refuses (narrower widths always refused them).
+bool flatquant_sm100_preferred(int64_t tokens, int m, int n, const void* codes) {
+  return (tokens >= 4 && reinterpret_cast<uintptr_t>(codes) % 16 == 0) || !flatquant_sm100_n256_supported(m, n);
+}
 
 // mode: 0 int8 codes, 1 packed codes, 2 transform only (float32 Z written to `codes`)
 int launch_flatquant_sm100_mode(int mode, const void* x, int64_t ldx, const void* left, const void* right, void* codes,

@@ -1,5 +1,7 @@
 """GPU parity of the quantizer for right transforms of 144 .. 256 (flatquant_sm100_n256.cu), at the edges of its tiles: against the
 oracle, and against the SIMT kernel on tokens with infinities, NaNs and zeros."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -77,3 +79,30 @@ def test_scales_over_the_whole_range_of_the_type(dtype, clip, pack):
     ref = abi_quantize(x, left, right, clip, pack, dtype, policy=1)
     assert bool(ref[1].isinf().any()) == (clip > 1)
     assert torch.equal(got[1], ref[1]) and torch.equal(got[0], ref[0])
+
+
+@pytest.mark.parametrize("mode,shift", [("packed", 4), ("int8", 1), ("transform", 4)])
+def test_outputs_off_a_16_byte_boundary(mode, shift):
+    """The C entry points take outputs of these widths at any boundary of their element type, on the SIMT kernel."""
+    m, n, tokens = 16, 160, 9
+    x, left, right = (t.to(DEV) for t in make_inputs(tokens, m * n, "bf16", 8, True, mn=(m, n)))
+    size = tokens * m * n * {"packed": 1, "int8": 2, "transform": 8}[mode] // 2
+    results = []
+    for policy, at in ((1, 0), (0, shift)):
+        raw = torch.full((size + 32,), 77, dtype=torch.uint8, device=DEV)
+        scales = torch.zeros(tokens, device=DEV)
+        out = C.c_void_p(raw.data_ptr() + at)
+        N.check(lib.qo_set_kernel_policy(policy))
+        try:
+            if mode == "transform":
+                N.check(lib.qo_flatquant_transform(ptr(x), m * n, ptr(left), ptr(right), out, tokens, m, n, QD["bf16"], stream_ptr()))
+            else:
+                N.check(lib.qo_flatquant_quantize(ptr(x), m * n, ptr(left), ptr(right), out, ptr(scales), tokens, m, n, 0.9, QD["bf16"],
+                                                  int(mode == "packed"), QD["fp32"], stream_ptr()))
+        finally:
+            lib.qo_set_kernel_policy(0)
+        torch.cuda.synchronize()
+        assert lib.qo_last_quantizer_path() == 1
+        assert bool((raw[:at] == 77).all()) and bool((raw[at + size:] == 77).all())
+        results.append((raw[at:at + size].clone(), scales))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
