@@ -163,7 +163,7 @@ int qo_flatquant_quantize(const void* x, int64_t ldx, const void* left, const vo
   const bool fast_ok = flatquant_sm100_supported(ldx, m, n, in_dtype, x, left, right, clip_ratio);
   if (t_policy >= 2 && !fast_ok)
     return fail(QO_ERR_UNSUPPORTED, "flatquant: no tcgen05 kernel for m=%d n=%d dtype=%d ldx=%lld", m, n, in_dtype, (long long)ldx);
-  if (fast_ok && t_policy != 1 && (t_policy >= 2 || flatquant_sm100_preferred(tokens, m, n, codes))) {
+  if (fast_ok && t_policy != 1 && (t_policy >= 2 || flatquant_sm100_preferred(m, n, codes))) {
     t_quant_path = 2;
     return launch_flatquant_sm100(x, ldx, left, right, codes, scales, tokens, m, n, clip_ratio, in_dtype, pack_int32,
                                   scale_dtype, st);
@@ -184,7 +184,7 @@ int qo_flatquant_transform(const void* x, int64_t ldx, const void* left, const v
   const bool fast_ok = flatquant_sm100_supported(ldx, m, n, in_dtype, x, left, right, 1.0f);
   if (t_policy >= 2 && !fast_ok)
     return fail(QO_ERR_UNSUPPORTED, "flatquant_transform: no tcgen05 kernel for m=%d n=%d dtype=%d", m, n, in_dtype);
-  if (fast_ok && t_policy != 1 && (t_policy >= 2 || flatquant_sm100_preferred(tokens, m, n, z))) {
+  if (fast_ok && t_policy != 1 && (t_policy >= 2 || flatquant_sm100_preferred(m, n, z))) {
     t_quant_path = 2;
     return launch_flatquant_sm100_mode(2, x, ldx, left, right, z, nullptr, tokens, m, n, 1.0f, in_dtype, QO_F32, st);
   }

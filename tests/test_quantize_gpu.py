@@ -136,14 +136,14 @@ def test_right_transform_of_size_64_small_left(m, dtype, tokens, pack):
         check(codes, scales, ref_codes, ref_scales, pack)
 
 
-@pytest.mark.parametrize("feat,dtype", [(28672, "bf16"), (32768, "fp16"), (24576, "fp32")])
-def test_very_wide_rows_take_the_generic_kernel(feat, dtype):
-    """28672 = 128 x 224 (the down-projection input of the 70B-class models) and 32768 = 128 x 256 have no tensor-core
-    kernel (right transform above 128); the SIMT kernel must take them."""
+@pytest.mark.parametrize("feat,dtype,path", [(28672, "bf16", 2), (32768, "fp16", 2), (24576, "fp32", 1)])
+def test_very_wide_rows(feat, dtype, path):
+    """28672 = 128 x 224 (the down-projection input of the 70B-class models) and 32768 = 128 x 256 run on the tensor cores at
+    any token count; float32 rows on a SIMT kernel."""
     x, left, right = make_inputs(3, feat, dtype, feat + 3, True)
     ref_codes, ref_scales = O.flatquant_quantize(t2f(x), t2f(left), t2f(right), 0.9, True, dtype)
     codes, scales = abi_quantize(x.to(DEV), left.to(DEV), right.to(DEV), 0.9, True, dtype, policy=0)
-    assert lib.qo_last_quantizer_path() == 1
+    assert lib.qo_last_quantizer_path() == path
     check(codes.cpu().numpy(), t2f(scales), ref_codes, ref_scales, True)
 
 

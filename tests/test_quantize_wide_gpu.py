@@ -106,3 +106,13 @@ def test_outputs_off_a_16_byte_boundary(mode, shift):
         assert bool((raw[:at] == 77).all()) and bool((raw[at + size:] == 77).all())
         results.append((raw[at:at + size].clone(), scales))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+def test_a_token_has_the_same_codes_alone_and_in_a_batch():
+    """Rows are independent: one token, three and all of them give the same bits."""
+    x, left, right = (t.to(DEV) for t in make_inputs(64, 128 * 224, "bf16", 17, True, mn=(128, 224)))
+    codes, scales = abi_quantize(x, left, right, 0.9, True, "bf16")
+    for size in (1, 3):
+        for i in range(0, 64 - size + 1, size):
+            c, s = abi_quantize(x[i:i + size], left, right, 0.9, True, "bf16")
+            assert torch.equal(c, codes[i:i + size]) and torch.equal(s, scales[i:i + size])
