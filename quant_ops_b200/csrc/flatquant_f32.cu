@@ -313,6 +313,26 @@ bool flatquant_f32_supported(int64_t ldx, int m, int n, const void* x, const voi
          reinterpret_cast<uintptr_t>(codes) % 16 == 0;
 }
 
+// Small matrices of few tokens are left to the generic kernel (the same bits).  Its threads compute 8 values at a time, those
+// of this kernel 64: as long as a token has no more than 256 such groups of 8 and the SM's threads are not used up, the
+// shorter chains are done first.  The lines follow measurements of both kernels over the tokens an SM has at once and the
+// threads they occupy (graph replay, generic / this kernel, us): 32 x 32 packed 8.7 / 12.0 for 148 tokens and 12.3 / 12.4
+// for 592; 32 x 64 packed 11.6 / 14.7 for 148, 15.0 / 15.0 for 296; 64 x 32 packed 14.2 / 14.5 for 148, 17.1 / 14.4 for
+// 149; 148 tokens to int8: 24 x 24 10.2 / 10.9, 32 x 32 12.2 / 11.9.  The generic kernel stores int8 codes byte by byte, and a
+// tall matrix costs it more (L is read from memory, eight values a step): hence the limits by mode and M.
+bool flatquant_f32_preferred(int mode, int64_t tokens, int m, int n) {
+  const int groups = ((m + 7) / 8) * n;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return true; }
+  const int64_t per_sm = (tokens + sm_count(dev) - 1) / sm_count(dev);
+  if (groups > 256 || per_sm > 4) return true;  // more than a group per thread; more tokens than the generic kernel takes at once
+  int most = 0;  // threads of an SM with work up to which the generic kernel is the faster one
+  if (mode == 1) most = m <= 24 ? 768 : (m <= 32 ? 512 : (m <= 48 ? 360 : (m <= 64 ? 256 : 0)));
+  else if (mode == 0) most = m <= 16 ? 768 : (m <= 24 ? 576 : 0);
+  else most = m <= 8 ? 384 : 0;
+  return per_sm * groups > most;
+}
+
 int launch_flatquant_f32(int mode, const void* x, int64_t ldx, const void* left, const void* right, void* codes, void* scales,
                          int64_t tokens, int m, int n, float clip, int scale_dtype, cudaStream_t stream) {
   const float* xf = reinterpret_cast<const float*>(x);

@@ -156,7 +156,7 @@ int launch_flatquant_generic(const void* x, int64_t ldx, const void* left, const
   switch (in_dtype) {
     case QO_F32:
       // the register-tiled kernel gives the same bits; policy 1 keeps this one, so that the tests compare the two
-      if (current_kernel_policy() != 1 && flatquant_f32_supported(ldx, m, n, x, right, codes))
+      if (current_kernel_policy() != 1 && flatquant_f32_supported(ldx, m, n, x, right, codes) && flatquant_f32_preferred(pack, tokens, m, n))
         return launch_flatquant_f32(pack, x, ldx, left, right, codes, scales, tokens, m, n, clip, scale_dtype, stream);
       return launch_typed<float>(x, ldx, left, right, codes, scales, tokens, m, n, clip, pack, scale_dtype, stream);
     case QO_F16:

@@ -136,6 +136,7 @@ int launch_flatquant_generic(const void* x, int64_t ldx, const void* left, const
                              int scale_dtype, cudaStream_t stream);
 // float32 activations, register-tiled (flatquant_f32.cu); mode: 0 int8 codes, 1 packed codes, 2 transform only
 bool flatquant_f32_supported(int64_t ldx, int m, int n, const void* x, const void* right, const void* codes);
+bool flatquant_f32_preferred(int mode, int64_t tokens, int m, int n);
 int launch_flatquant_f32(int mode, const void* x, int64_t ldx, const void* left, const void* right, void* codes, void* scales,
                          int64_t tokens, int m, int n, float clip, int scale_dtype, cudaStream_t stream);
 // returns QO_ERR_UNSUPPORTED (without setting an error) when the shape has no tcgen05 kernel

@@ -3,7 +3,8 @@ of fused multiply-adds."""
 import pytest
 import torch
 
-from helpers import N, QD, abi_quantize, lib, make_inputs, ptr, stream_ptr
+import quant_ops_b200 as q
+from helpers import N, QD, abi_quantize, launched_kernels, lib, make_inputs, ptr, stream_ptr
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -44,3 +45,21 @@ def test_transform_only_has_the_same_bits(m, n, tokens):
         torch.cuda.synchronize()
         out.append(z)
     assert torch.equal(out[0], out[1])
+
+
+# small matrices of few tokens keep the generic kernel, which is the faster one there: either side of each line
+ROUTES = [(32, 32, 1, True, False), (32, 32, 148 * 4, True, False), (32, 32, 148 * 4 + 1, True, True), (32, 32, 1, False, True),
+          (32, 64, 148 * 2, True, False), (32, 64, 148 * 2 + 1, True, True), (24, 24, 148 * 4, False, False), (28, 24, 1, False, True),
+          (16, 128, 148 * 3, False, False), (16, 128, 148 * 3 + 1, False, True), (64, 32, 148, True, False), (64, 32, 149, True, True),
+          (72, 24, 1, True, True), (48, 48, 1, True, True), (64, 64, 1, True, True), (3, 8, 148 * 4, True, False), (3, 8, 148 * 4 + 1, True, True)]
+
+
+@pytest.mark.parametrize("m,n,tokens,pack,tiled", ROUTES)
+def test_route_and_bits_at_the_lines(m, n, tokens, pack, tiled):
+    assert torch.cuda.get_device_properties(0).multi_processor_count == 148
+    x, left, right = (t.to(DEV) for t in make_inputs(tokens, m * n, "fp32", m + n + tokens, True, mn=(m, n)))
+    ref = abi_quantize(x, left, right, 0.9, pack, "fp32", policy=1)
+    got = abi_quantize(x, left, right, 0.9, pack, "fp32")
+    assert torch.equal(got[0], ref[0]) and torch.equal(got[1].view(torch.int32), ref[1].view(torch.int32))
+    names = launched_kernels(lambda: q.flatquant_dynamic_quantize(x, left, right, 0.9, pack))
+    assert len(names) == 1 and ("flatquant_f32_kernel" if tiled else "flatquant_generic_kernel") in names[0]
