@@ -304,7 +304,7 @@ int qo_w4a4_linear(const void* x, int64_t ldx, const void* left, const void* rig
   char* ws = reinterpret_cast<char*>(workspace);
   // prefill sizes: the quantizer packs, and the GEMM that unpacks in the kernel takes the packed codes and the packed
   // weights as they are (the packed route below); otherwise ...
-  const bool unpack_route = t_policy != 1 && gemm_unpack_preferred(tokens, k, n_out) &&
+  const bool unpack_route = t_policy != 1 && gemm_unpack_preferred(tokens, k, n_out, Widening::kWeightsBeside) &&
                             gemm_unpack_supported(tokens, k, n_out, workspace, k / 8, w_packed, 1, k / 8);
   if (!unpack_route && t_policy != 1 && tokens > 32 && gemm_sm100_supported(tokens, k, n_out, k / 8, 1, k / 8)) {
     // ... tensor-core route with int8 operands: the quantizer writes int8 codes, which is that GEMM's A operand as it

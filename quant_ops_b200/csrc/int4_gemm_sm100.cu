@@ -847,7 +847,7 @@ int launch_gemm_sm100(const int32_t* a, int64_t lda, const int32_t* b, int64_t b
     return fail(QO_ERR_WORKSPACE, "int4_matmul: workspace missing, too small or not 256-byte aligned");
   int rc;
   // the kernel that unpacks the nibbles itself, where it can (no widening pass, the workspace stays untouched)
-  if (gemm_unpack_supported(t, k, n, a, lda, b, bsk, bsn) && gemm_unpack_preferred(t, k, n)) {
+  if (gemm_unpack_supported(t, k, n, a, lda, b, bsk, bsn) && gemm_unpack_preferred(t, k, n, bsk == 1 ? Widening::kRows : Widening::kColumns)) {
     int dev = 0;
     QO_CUDA_TRY(cudaGetDevice(&dev));
     uint32_t* status = device_status_word(dev);

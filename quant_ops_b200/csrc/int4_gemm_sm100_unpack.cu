@@ -774,12 +774,28 @@ bool gemm_unpack_prefill(int64_t t, int64_t n) {
 // widening both operands and multiplying int8 (graph replay): 256 x 14336 x 4096 21.7 against 35.6 us, 600 x 2048 x 1024 11.1
 // against 16.0, 100 x 2048 x 256 10.0 against 11.7, but 100 x 1024 x 1024 9.4 against 7.2 and 300 x 1024 x 2048 9.6 against 7.7:
 // with four stages of K the fill and the exchange outweigh a widening pass that is as short as the product.
-bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n) {
-  return gemm_unpack_prefill(t, n) || (current_kernel_policy() != 3 && n >= kBN && k >= 2048);
+//
+// Few column tiles and a long K are the exception.  K is split four ways at most here, so 1 to 4 tiles occupy 8 to 32 of the
+// 148 SMs; the int8 kernels split it up to eight ways, half as wide tiles for one block of 128 rows, and there is little to
+// widen.  How little depends on what runs beside it (`instead`).  Measured, unpacking / int8: layer 128 x 4096 -> 256 15.0 /
+// 13.8 us, 128 x 4096 -> 1024 15.2 / 14.3, 128 x 8192 -> 256 1.21 apart, 96 x 8192 -> 512 1.11, 256 x 14336 -> 256 1.02; rows 128 x
+// 14336 x 512 17.4 / 14.6 us, 128 x 11008 x 1024 16.1 / 15.1, 33 x 14336 x 512 15.4 / 14.6; columns 128 x 14336 x 512 17.4 /
+// 16.5.  On the other side of the lines: layer 96 x 4096 -> 1024 and 128 x 6144 -> 1024 alike, 96 x 8192 -> 1024 0.98, 129 x
+// 8192 -> 1024 0.91; rows 128 x 5120 x 512 1.01, 96 x 11008 x 1024 0.99; columns 96 x 8192 x 512 0.99.
+bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n, Widening instead) {
+  if (gemm_unpack_prefill(t, n)) return true;
+  if (current_kernel_policy() == 3 || n < kBN || k < 2048) return false;
+  const int64_t tiles = unpack_tiles(t, n);
+  const bool upper_half = t > 96 && t <= 128;
+  if (instead == Widening::kColumns) return !(k >= 8192 && tiles <= 2 && upper_half) && !(k >= 14336 && tiles == 1);
+  if (k >= 8192 && (tiles == 1 || (t <= 128 && tiles <= (t > 96 ? 4 : 2)))) return false;
+  return !(instead == Widening::kWeightsBeside && upper_half && k >= 4096 && (tiles <= 3 || (tiles == 4 && k < 6144)));
 }
 
 // preferred, and all tiles on the 74 CTA pairs at once
-bool gemm_unpack_one_round(int64_t t, int64_t k, int64_t n) { return gemm_unpack_preferred(t, k, n) && unpack_tiles(t, n) <= 74; }
+bool gemm_unpack_one_round(int64_t t, int64_t k, int64_t n) {
+  return gemm_unpack_preferred(t, k, n, Widening::kWeightsBeside) && unpack_tiles(t, n) <= 74;
+}
 
 // returns QO_ERR_UNSUPPORTED without a message when the device cannot co-schedule CTA pairs of this kernel
 int launch_gemm_unpack(const int32_t* a, int64_t lda, const int32_t* b, int64_t bsk, int64_t bsn, const float* sa, const float* sb, void* out,

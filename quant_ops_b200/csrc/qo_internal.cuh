@@ -193,7 +193,10 @@ int launch_gemm_sm100_pair(const int8_t* a8, const int8_t* b8, const float* sa, 
 // packed-int4 GEMM that unpacks inside the kernel (int4_gemm_sm100_unpack.cu): b is [n, k/8] (bsk == 1) or [k/8, n] (bsn == 1)
 bool gemm_unpack_supported(int64_t t, int64_t k, int64_t n, const void* a, int64_t lda, const void* b, int64_t bsk, int64_t bsn);
 bool gemm_unpack_prefill(int64_t t, int64_t n);  // sizes that keep the CTA pairs busy without splitting K (the fused gather takes only these)
-bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n);
+// what the int8 kernels would need first: the weights widened beside the quantizer (the layer), both operands in one pass, or
+// the weights transposed as well ([K/8, N])
+enum class Widening { kWeightsBeside, kRows, kColumns };
+bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n, Widening instead);
 bool gemm_unpack_one_round(int64_t t, int64_t k, int64_t n);
 // destinations of the fused all-gather (see gemm_s4_unpack_kernel): the buffers [total_rows, n] of this GPU and its
 // peers; this rank's rows start at row_offset

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import quant_ops_b200 as q
-from helpers import N, abi_int4_matmul, lib, make_inputs, stream_ptr
+from helpers import N, abi_int4_matmul, launched_kernels, lib, make_inputs, stream_ptr
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -34,7 +34,7 @@ def test_same_bits_as_the_widening_path(t, k, n, layout):
         assert torch.equal(got.view(torch.int16), ref.view(torch.int16))
 
 
-@pytest.mark.parametrize("t,n", [(4, 256), (40, 256), (40, 264), (300, 1024), (1024, 3072)])
+@pytest.mark.parametrize("t,n", [(4, 1288), (40, 1280), (40, 1288), (300, 1024), (1024, 3072)])
 @pytest.mark.parametrize("k", [131072 - 256, 131072])
 def test_extreme_codes_of_the_longest_reductions(t, n, k):
     """Zeroed operands are codes of -8 on both sides.  With the factor 256 of the kernels that keep the nibbles in the high
@@ -75,3 +75,29 @@ def test_layer_with_early_weight_loads(tokens, k, n_out):
     for _ in range(10):
         assert torch.equal(q.w4a4_linear(xd, ld, rd, w, sb, bias, 0.9), want)
     q.device_status()
+
+
+# few column tiles and a long K run on widened operands; either side of each line
+FEW_TILES = [("layer", 96, 4096, 256, True), ("layer", 97, 4096, 256, False), ("layer", 128, 4096, 1024, False), ("layer", 128, 4096, 1032, True),
+             ("layer", 128, 3072, 256, True), ("layer", 129, 4096, 1024, True), ("layer", 128, 6144, 1024, True), ("layer", 64, 8192, 512, False),
+             ("layer", 64, 8192, 520, True), ("layer", 256, 8192, 256, False), ("layer", 257, 8192, 256, True), ("rows", 128, 8192, 1024, False),
+             ("rows", 128, 7168, 1024, True), ("rows", 96, 8192, 768, True), ("rows", 40, 14336, 512, False), ("columns", 128, 8192, 512, False),
+             ("columns", 96, 8192, 512, True), ("columns", 20, 14336, 256, False), ("columns", 20, 14336, 264, True)]
+
+
+@pytest.mark.parametrize("form,t,k,n,unpacks", FEW_TILES)
+def test_route_and_bits_at_the_lines(form, t, k, n, unpacks):
+    a, w, sa, sb = problem(t, k, n, t + k + n)
+    if form == "layer":
+        x, left, right = (v.to(DEV) for v in make_inputs(t, k, "bf16", t + n, True))
+        codes, scales = q.flatquant_dynamic_quantize(x, left, right, 0.9, True)
+        want = q.int4_matmul_ex(codes, w.t(), scales, sb, torch.bfloat16)
+        call = lambda: q.w4a4_linear(x, left, right, w, sb, None, 0.9)
+    else:
+        b = w.t() if form == "rows" else w.t().contiguous()
+        want = abi_int4_matmul(a, b, sa, sb, "fp16", policy=3)
+        call = lambda: q.int4_matmul(a, b, sa, sb)
+    assert torch.equal(call(), want)
+    names = launched_kernels(call)
+    assert any("gemm_s4_unpack_kernel" in name for name in names) == unpacks
+    assert any("widen" in name for name in names) != unpacks
