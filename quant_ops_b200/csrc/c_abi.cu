@@ -485,12 +485,10 @@ int qo_w4a4_linear_prepared(const void* x, int64_t ldx, const void* left, const 
     workspace_bytes = need;
   }
   if (workspace_bytes < need) return fail(QO_ERR_WORKSPACE, "w4a4_linear: workspace of %zu bytes, need %zu", workspace_bytes, need);
-  // few tokens (weight-streaming kernel), prefill sizes (the GEMM that unpacks in the kernel is the faster one there and
-  // needs no int8 copy), or a shape / policy the int8 tensor-core kernel does not take: packed route
-  // ... and, above 160 rows, products whose tiles the packed kernel runs at once (300 x 14336 x 4096 39.8 us with the copy,
-  // 32.0 packed; 200 x 4096 x 11008 28.2 against 21.0).  With fewer rows (130 x 14336 x 4096 25.9 against 27.0) or a second
-  // round of tiles (300 x 4096 x 11008 22.5 against 30.2) the copy is the faster one.
-  const bool unpack_route = t_policy != 1 && (gemm_unpack_prefill(tokens, n_out) || (tokens > 160 && gemm_unpack_one_round(tokens, k, n_out))) &&
+  // few tokens (weight-streaming kernel), sizes at which the GEMM that unpacks in the kernel is the faster one (prefill, and
+  // most sizes above 128 rows, see gemm_unpack_beats_copy), or a shape / policy the int8 tensor-core kernel does not take:
+  // packed route
+  const bool unpack_route = t_policy != 1 && gemm_unpack_beats_copy(tokens, k, n_out) &&
                             gemm_unpack_supported(tokens, k, n_out, workspace, k / 8, w_packed, 1, k / 8);
   const bool direct = !unpack_route && t_policy != 1 && tokens > 32 && gemm_sm100_supported(tokens, k, n_out, k / 8, 1, k / 8) &&
                       reinterpret_cast<uintptr_t>(prepared) % 256 == 0;

@@ -792,9 +792,23 @@ bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n, Widening instead) {
   return !(instead == Widening::kWeightsBeside && upper_half && k >= 4096 && (tiles <= 3 || (tiles == 4 && k < 6144)));
 }
 
-// preferred, and all tiles on the 74 CTA pairs at once
-bool gemm_unpack_one_round(int64_t t, int64_t k, int64_t n) {
-  return gemm_unpack_preferred(t, k, n, Widening::kWeightsBeside) && unpack_tiles(t, n) <= 74;
+// Layers whose weights are kept as an int8 copy as well (no widening pass on the other side): above 128 rows, where the int8
+// kernels start a second row block, if all tiles run on the 74 CTA pairs at once.  Measured over 129 to 2048 rows, 512 to 14336
+// outputs and K of 2048 to 14336, packed / copy (graph replay): mostly 0.62 to 0.95 (160 x 4096 -> 11008 20.8 / 26.6 us, 300 x 14336
+// -> 4096 32.0 / 39.8, 600 x 11008 -> 4096 0.65), alike for 4096 x 4096 up to 256 rows.  The copy stays
+//   * for K of 8192 and more with few tiles, which the int8 kernels spread over more SMs: up to 14 tiles of 128 x 256
+//     1.02 to 1.15 (256 x 14336 -> 1024 24.6 / 22.2 us); at 16 such tiles 0.88 to 0.93;
+//   * for the same K between 34 tiles of 256 x 256, from which on K is not split here any more (33 clusters of four CTAs fit), and
+//     74 of 128 x 256, up to which it is there: 300 x 8192 -> 4352 1.08, 600 x 14336 -> 3072 1.16; on either side 600 x 14336 -> 2816
+//     0.84, 450 x 14336 -> 5120 0.63;
+//   * for K of 4096 with 16 tiles and up to 32 of 128 x 256, 1.02 to 1.05 (1024 x 4096 -> 1024 20.2 / 19.3 us).
+// A second round of tiles: 300 x 4096 -> 11008 30.2 / 22.5.  Up to 128 rows the sides change from shape to shape, 0.80 to 1.31.
+bool gemm_unpack_beats_copy(int64_t t, int64_t k, int64_t n) {
+  if (gemm_unpack_prefill(t, n)) return true;
+  const int64_t tiles = unpack_tiles(t, n), tiles8 = ((t + 127) / 128) * ((n + 255) / 256);
+  if (t <= 128 || tiles > 74 || !gemm_unpack_preferred(t, k, n, Widening::kWeightsBeside)) return false;
+  if (k >= 8192) return tiles8 > 14 && (tiles < 34 || tiles8 > 74);
+  return !(k >= 4096 && k < 5120 && tiles >= 16 && tiles8 <= 32);
 }
 
 // returns QO_ERR_UNSUPPORTED without a message when the device cannot co-schedule CTA pairs of this kernel

@@ -197,7 +197,7 @@ bool gemm_unpack_prefill(int64_t t, int64_t n);  // sizes that keep the CTA pair
 // the weights transposed as well ([K/8, N])
 enum class Widening { kWeightsBeside, kRows, kColumns };
 bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n, Widening instead);
-bool gemm_unpack_one_round(int64_t t, int64_t k, int64_t n);
+bool gemm_unpack_beats_copy(int64_t t, int64_t k, int64_t n);  // against weights that are kept widened
 // destinations of the fused all-gather (see gemm_s4_unpack_kernel): the buffers [total_rows, n] of this GPU and its
 // peers; this rank's rows start at row_offset
 struct GatherDsts {

@@ -101,3 +101,21 @@ def test_route_and_bits_at_the_lines(form, t, k, n, unpacks):
     names = launched_kernels(call)
     assert any("gemm_s4_unpack_kernel" in name for name in names) == unpacks
     assert any("widen" in name for name in names) != unpacks
+
+
+# layers that keep an int8 copy of their weights: packed weights where the unpacking kernel is the faster one, else the copy
+KEPT = [(128, 4096, 2048, False), (129, 4096, 2048, True), (160, 4096, 11008, True), (257, 4096, 11008, False), (1024, 4096, 1024, False),
+        (1040, 4096, 1024, True), (384, 8192, 1024, False), (400, 8192, 1024, True), (256, 8192, 1792, False), (300, 8192, 4352, False), (600, 8192, 3072, False), (520, 8192, 2816, True),
+        (900, 8192, 3072, True), (600, 2048, 1024, True), (256, 1024, 1024, False)]
+
+
+@pytest.mark.parametrize("t,k,n,packed", KEPT)
+def test_route_and_bits_with_kept_weights(t, k, n, packed):
+    _, w, _, sb = problem(1, k, n, t + n)
+    x, left, right = (v.to(DEV) for v in make_inputs(t, k, "bf16", t + n, True))
+    kept = q.prepare_weights(w)
+    codes, scales = q.flatquant_dynamic_quantize(x, left, right, 0.9, True)
+    call = lambda: q.w4a4_linear_prepared(x, left, right, w, kept, sb, None, 0.9)
+    assert torch.equal(call(), abi_int4_matmul(codes, w.t(), scales, sb, "bf16", policy=3))
+    names = launched_kernels(call)
+    assert len(names) == 2 and any("gemm_s4_unpack_kernel" in name for name in names) == packed
