@@ -84,7 +84,7 @@ class W4A4Linear(torch.nn.Module):
             raise RuntimeError(f"input dtype {dtype} does not match the transforms' dtype {left.dtype}")
         out_dtype = dtype if dtype == torch.bfloat16 else torch.float16
         if self.weight_int8 is not None:
-            y = _w4a4_linear_prepared(x2, left, right, w, self.weight_int8, ws, bias, self.clip_ratio, out_dtype)
+            y = _w4a4_linear_prepared(x2, left, right, w, self.weight_int8, ws, bias, float(self.clip_ratio), out_dtype)
         else:
-            y = _w4a4_linear(x2, left, right, w, ws, bias, self.clip_ratio, out_dtype)
+            y = _w4a4_linear(x2, left, right, w, ws, bias, float(self.clip_ratio), out_dtype)
         return y if x2 is x else y.reshape(*x.shape[:-1], self.out_features)

@@ -1,4 +1,5 @@
 """Host-side behaviour of the Python operator layer (no GPU needed): names, fake kernels, no CPU fallback."""
+import numpy as np
 import pytest
 import torch
 
@@ -41,3 +42,12 @@ def test_fake_kernels_give_the_reference_shapes_and_dtypes():
         wp = torch.empty(96, 512, device="cuda", dtype=torch.int32)
         y = q.w4a4_linear(x, lr, lr, wp, torch.empty(96, device="cuda"), None, 0.9)
         assert y.shape == (8, 96) and y.dtype == torch.bfloat16
+
+
+def test_layer_takes_any_clip_ratio_that_float_takes():
+    """The attribute can be set after construction, from a configuration for instance; shapes only (meta device)."""
+    for keep in (False, True):
+        layer = q.W4A4Linear(256, 32, device="meta", keep_int8_weights=keep).prepare()
+        for clip in (0.9, 1, np.float32(0.9), torch.tensor(0.9), "0.9"):
+            layer.clip_ratio = clip
+            assert layer(torch.empty(3, 256, dtype=torch.bfloat16, device="meta")).shape == (3, 32)
