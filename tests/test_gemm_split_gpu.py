@@ -9,10 +9,12 @@ from helpers import N, abi_int4_matmul, launched_kernels, lib, make_inputs, stre
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
-# rows: one, around a CTA's and a pair's rows; columns: one tile, ragged tiles, as many as leave two, one or no split;
-# K: a single stage, the shortest that are split in two and in four, odd numbers of stages
+# rows: one, around a CTA's and a pair's rows; columns: one tile, ragged tiles, as many as leave four to one slices of K;
+# K: the shortest that are split, odd numbers of stages, a single stage and three of them unsplit at prefill sizes, and three shapes
+# whose K of less than 2048 keeps them on widened operands
 SHAPES = [(1, 4096, 4096), (33, 256, 256), (100, 1024, 264), (128, 2048, 1024), (129, 2304, 1000), (256, 14336, 4096), (257, 4096, 4096),
-          (300, 2816, 520), (512, 1280, 4096), (200, 4096, 14336), (333, 4096, 14328), (700, 11008, 4088), (1030, 4096, 1024)]
+          (300, 2816, 520), (512, 1280, 4096), (200, 4096, 14336), (333, 4096, 14328), (700, 11008, 4088), (1030, 4096, 1024),
+          (33, 2048, 256), (100, 2304, 264), (1536, 256, 2048), (1500, 768, 2056)]
 
 
 def problem(t, k, n, seed):
@@ -28,7 +30,9 @@ def test_same_bits_as_the_widening_path(t, k, n, layout):
     b = w.t() if layout == "weights_t_view" else w.t().contiguous()
     for out_dtype in ("fp16", "bf16"):
         ref, ref_acc = abi_int4_matmul(a, b, sa, sb, out_dtype, True, policy=3)
+        before = lib.qo_kernel_launch_count()
         got, acc = abi_int4_matmul(a, b, sa, sb, out_dtype, True, policy=2)
+        assert (lib.qo_kernel_launch_count() - before == 1) == (k >= 2048 or t >= 1500)  # one launch: no widening pass
         assert lib.qo_device_status(stream_ptr()) == N.QO_OK
         assert torch.equal(acc, ref_acc)
         assert torch.equal(got.view(torch.int16), ref.view(torch.int16))

@@ -11,7 +11,7 @@ DEV = "cuda:0"
 
 # M not a multiple of 8 or 16, N from one block to more than 256 threads' worth; one token, partial groups, many rounds
 SHAPES = [(3, 8, 5), (10, 24, 700), (32, 32, 1), (32, 32, 4801), (48, 64, 333), (64, 64, 1), (64, 64, 1300), (64, 80, 77), (86, 128, 301),
-          (112, 128, 299), (128, 192, 150), (24, 8, 40)]
+          (112, 128, 299), (128, 192, 150), (24, 8, 40), (3, 8, 601), (24, 8, 700)]
 
 
 @pytest.mark.parametrize("m,n,tokens", SHAPES)
@@ -30,6 +30,8 @@ def test_same_bits_as_the_generic_kernel(m, n, tokens, pack):
     got = abi_quantize(xd, ld, rd, 0.9, pack, "fp32", policy=0)
     assert torch.equal(got[0], ref[0])
     assert torch.equal(got[1].view(torch.int32), ref[1].view(torch.int32))
+    if tokens > 592 or m * n >= 3072:  # (smaller ones may keep the generic kernel, see below)
+        assert "flatquant_f32_kernel" in launched_kernels(lambda: q.flatquant_dynamic_quantize(xd, ld, rd, 0.9, pack))[0]
 
 
 @pytest.mark.parametrize("m,n,tokens", [(64, 64, 9), (86, 128, 3)])
@@ -45,6 +47,39 @@ def test_transform_only_has_the_same_bits(m, n, tokens):
         torch.cuda.synchronize()
         out.append(z)
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("which,tiled", [("none", True), ("left", True), ("x", False), ("stride", False), ("right", False), ("codes", False)])
+def test_operands_off_a_16_byte_boundary(which, tiled):
+    """Rows, right transforms and outputs that are not 16-byte aligned fall back to the generic kernel; left transforms need not be."""
+    m, n, tokens = 64, 64, 5
+    x, left, right = (t.to(DEV) for t in make_inputs(tokens, m * n, "fp32", 21, True, mn=(m, n)))
+    ref = abi_quantize(x, left, right, 0.9, True, "fp32", policy=1)
+
+    def shifted(t, words):
+        raw = torch.zeros(t.numel() + 8, device=DEV, dtype=t.dtype)
+        view = raw[words:words + t.numel()].view(t.shape)
+        view.copy_(t)
+        return view
+
+    ldx = m * n
+    if which == "x":
+        x = shifted(x, 1)
+    if which == "stride":
+        wide = torch.zeros(tokens, m * n + 2, device=DEV)
+        wide[:, : m * n] = x
+        x, ldx = wide, m * n + 2
+    left, right = shifted(left, which == "left"), shifted(right, which == "right")
+    codes, scales = shifted(torch.zeros_like(ref[0]), which == "codes"), torch.zeros(tokens, device=DEV)
+
+    def call():
+        N.check(lib.qo_flatquant_quantize(ptr(x), ldx, ptr(left), ptr(right), ptr(codes), ptr(scales), tokens, m, n, 0.9, QD["fp32"], 1,
+                                          QD["fp32"], stream_ptr()))
+
+    call()
+    torch.cuda.synchronize()
+    assert torch.equal(codes, ref[0]) and torch.equal(scales, ref[1])
+    assert ("flatquant_f32_kernel" if tiled else "flatquant_generic_kernel") in launched_kernels(call)[0]
 
 
 # small matrices of few tokens keep the generic kernel, which is the faster one there: either side of each line

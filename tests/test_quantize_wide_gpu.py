@@ -53,7 +53,7 @@ def test_special_tokens_equal_the_simt_kernel(dtype, pack):
     x[3, 0] = float("nan")
     x[4] = float("nan")
     x[5] = 0.0
-    x[6] = 1e-7  # fp16: subnormal, the scale rounds to zero
+    x[6] = 1e-7  # fp16: subnormal values and scale (the codes depend on the order of the sums, hence the scale only)
     x[7, 3], x[7, 4000] = float("inf"), float("inf")
     got = abi_quantize(x.to(DEV), left.to(DEV), right.to(DEV), 0.9, pack, dtype, policy=2)
     ref = abi_quantize(x.to(DEV), left.to(DEV), right.to(DEV), 0.9, pack, dtype, policy=1)
@@ -106,6 +106,21 @@ def test_outputs_off_a_16_byte_boundary(mode, shift):
         assert bool((raw[:at] == 77).all()) and bool((raw[at + size:] == 77).all())
         results.append((raw[at:at + size].clone(), scales))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("pack", [True, False])
+def test_a_scale_that_rounds_to_zero(pack):
+    """fp16 tokens of up to three subnormal steps: three steps over 7 round to a scale of 0, and the quotients' limits are the
+    codes: 7, -8, and 0 for 0.  Identity transforms keep the values."""
+    m, n = 32, 160
+    g = torch.Generator().manual_seed(3)
+    x = (torch.randint(-3, 4, (6, m * n), generator=g) * 2.0 ** -24).half().to(DEV)
+    left, right = torch.eye(m, dtype=x.dtype, device=DEV), torch.eye(n, dtype=x.dtype, device=DEV)
+    codes, scales = abi_quantize(x, left, right, 1.0, pack, "fp16", policy=2)
+    assert bool((scales == 0).all())
+    if pack:
+        codes = ((codes[:, :, None] >> (4 * torch.arange(8, dtype=torch.int32, device=DEV))) & 15).reshape(6, m * n) - 8
+    assert torch.equal(codes.int(), torch.where(x > 0, 7, torch.where(x < 0, -8, 0)).int())
 
 
 def test_a_token_has_the_same_codes_alone_and_in_a_batch():
