@@ -269,7 +269,8 @@ QO_API int qo_flatquant_quantize_host(const void* x_host, const void* left_host,
 
 /* Number of kernels this library has launched in this process (all threads); used by the benchmark. */
 QO_API uint64_t qo_kernel_launch_count(void);
-/* Which quantizer kernel the last qo_flatquant_quantize on this thread used: 0 none, 1 generic SIMT, 2 tcgen05. */
+/* Which quantizer kernel the last qo_flatquant_quantize on this thread used: 0 none, 1 SIMT (the
+ * shape-generic kernel or the register-tiled one for float32), 2 tcgen05. */
 QO_API int qo_last_quantizer_path(void);
 /* Which GEMM kernel the last qo_int4_matmul on this thread used: 0 none, 1 generic SIMT, 2 tcgen05,
  * 3 weight-streaming kernel for 1 .. 32 rows (automatic policy only). */

@@ -14,8 +14,9 @@
 //   * small matrices are batched, as many tokens per CTA as fill its threads (64 x 64: four) unless there are too few
 //     tokens to give every SM two CTAs.
 //
-// Measured: 77.7 us for 2048 x 4096 to int8 codes in graph replay (37 % of the FMA pipe), 158 us for 700 x 14336; the
-// shape-generic kernel takes 257 us for the former.
+// Measured: 77.7 us for 2048 x 4096 to int8 codes in graph replay (the 29 us of multiply-adds are 37 % of that), 158 us for
+// 700 x 14336; the shape-generic kernel takes 257 us for the former.  Bound by the issue slots: 71 % used while an SM is active,
+// for 52 % of the FMA pipe (8192 x 4096; shared-memory reads 32 %).
 //
 // Every sum is one chain of fused multiply-adds in ascending k, as in flatquant_generic.cu: the results are the same
 // bits (reference: src/quant_ops/ops/quantization/flatquant/ops.py:99-117).

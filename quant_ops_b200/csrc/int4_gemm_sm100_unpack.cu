@@ -37,6 +37,9 @@
 //   warps 10-21  A converters: three sets of four warps, set g takes the stages g, g + 3, ...; thread = row, lane
 //                quadrant = warp % 4
 //   warps 22-27  B converters: three sets of two warps, same rotation
+//   With K split over the pairs of a cluster (SPLIT > 1, see the kernel) each pair has its own leader and rings, the epilogue
+//   warps stop at the accumulator barrier, and then every warp takes part in the exchange: warps 2-17 lay the blocks down and
+//   send them, all 28 add and store.
 //   Converters of both CTAs report to the leader's "operands ready" barrier (remote arrivals from the peer).
 //   A converter's work per stage is a chain of fixed latencies (barrier poll, shared-memory loads, the tensor-memory
 //   or shared-memory stores, a proxy fence, the arrival); sets in rotation keep one chain per set off the critical
