@@ -782,9 +782,10 @@ bool gemm_unpack_prefill(int64_t t, int64_t n) {
 // 148 SMs; the int8 kernels split it up to eight ways, half as wide tiles for one block of 128 rows, and there is little to
 // widen.  How little depends on what runs beside it (`instead`).  Measured, unpacking / int8: layer 128 x 4096 -> 256 15.0 /
 // 13.8 us, 128 x 4096 -> 1024 15.2 / 14.3, 128 x 8192 -> 256 1.21 apart, 96 x 8192 -> 512 1.11, 256 x 14336 -> 256 1.02; rows 128 x
-// 14336 x 512 17.4 / 14.6 us, 128 x 11008 x 1024 16.1 / 15.1, 33 x 14336 x 512 15.4 / 14.6; columns 128 x 14336 x 512 17.4 /
-// 16.5.  On the other side of the lines: layer 96 x 4096 -> 1024 and 128 x 6144 -> 1024 alike, 96 x 8192 -> 1024 0.98, 129 x
-// 8192 -> 1024 0.91; rows 128 x 5120 x 512 1.01, 96 x 11008 x 1024 0.99; columns 96 x 8192 x 512 0.99.
+// 4096 x 256 11.8 / 11.3 us, 128 x 14336 x 512 17.4 / 14.6, 128 x 11008 x 1024 16.1 / 15.1, 33 x 14336 x 512 15.4 / 14.6;
+// columns 128 x 14336 x 512 17.4 / 16.5.  On the other side of the lines: layer 96 x 4096 -> 1024 and 128 x 6144 -> 1024
+// alike, 96 x 8192 -> 1024 0.98, 129 x 8192 -> 1024 0.91; rows 128 x 5120 x 512 1.01, 96 x 11008 x 1024 0.99; columns 96 x
+// 8192 x 512 0.99.
 bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n, Widening instead) {
   if (gemm_unpack_prefill(t, n)) return true;
   if (current_kernel_policy() == 3 || n < kBN || k < 2048) return false;
@@ -792,7 +793,8 @@ bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n, Widening instead) {
   const bool upper_half = t > 96 && t <= 128;
   if (instead == Widening::kColumns) return !(k >= 8192 && tiles <= 2 && upper_half) && !(k >= 14336 && tiles == 1);
   if (k >= 8192 && (tiles == 1 || (t <= 128 && tiles <= (t > 96 ? 4 : 2)))) return false;
-  return !(instead == Widening::kWeightsBeside && upper_half && k >= 4096 && (tiles <= 3 || (tiles == 4 && k < 6144)));
+  const int64_t most = instead == Widening::kRows ? 1 : (k < 6144 ? 4 : 3);
+  return !(upper_half && k >= 4096 && tiles <= most);
 }
 
 // Layers whose weights are kept as an int8 copy as well (no widening pass on the other side): above 128 rows, where the int8

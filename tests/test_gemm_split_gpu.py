@@ -84,7 +84,7 @@ def test_layer_with_early_weight_loads(tokens, k, n_out):
 # few column tiles and a long K run on widened operands; either side of each line
 FEW_TILES = [("layer", 96, 4096, 256, True), ("layer", 97, 4096, 256, False), ("layer", 128, 4096, 1024, False), ("layer", 128, 4096, 1032, True),
              ("layer", 128, 3072, 256, True), ("layer", 129, 4096, 1024, True), ("layer", 128, 6144, 1024, True), ("layer", 64, 8192, 512, False),
-             ("layer", 64, 8192, 520, True), ("layer", 256, 8192, 256, False), ("layer", 257, 8192, 256, True), ("rows", 128, 8192, 1024, False),
+             ("layer", 64, 8192, 520, True), ("layer", 256, 8192, 256, False), ("layer", 257, 8192, 256, True), ("rows", 128, 4096, 256, False), ("rows", 128, 4096, 264, True), ("rows", 128, 8192, 1024, False),
              ("rows", 128, 7168, 1024, True), ("rows", 96, 8192, 768, True), ("rows", 40, 14336, 512, False), ("columns", 128, 8192, 512, False),
              ("columns", 96, 8192, 512, True), ("columns", 20, 14336, 256, False), ("columns", 20, 14336, 264, True)]
 
