@@ -537,8 +537,8 @@ int launch_flatquant_sm100_mode(int mode, const void* x, int64_t ldx, const void
   const cuuint64_t strides[2] = {(cuuint64_t)n * 2, (cuuint64_t)ldx * 2};
   const bool batched = flatquant_sm100_n64_supported(m, n);  // groups of 2 tokens, stacked-L^T second product
   const bool wide = flatquant_sm100_n128_supported(m, n);     // right transform of size 128
-  const bool wider = flatquant_sm100_n256_supported(m, n);    // right transforms of 144 .. 256, one token at a time
-  const cuuint32_t box[3] = {64, (cuuint32_t)m, (cuuint32_t)(batched ? 2 : (wide ? flatquant_sm100_n128_group(m) : (wider ? 1 : 128 / m)))};
+  const bool wider = flatquant_sm100_n256_supported(m, n);    // right transforms of 144 .. 256, a CTA pair per token
+  const cuuint32_t box[3] = {64, (cuuint32_t)(wider ? flatquant_sm100_n256_box_rows(m) : m), (cuuint32_t)(batched ? 2 : (wide ? flatquant_sm100_n128_group(m) : (wider ? 1 : 128 / m)))};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = encode_fn()(&map, in_dtype == QO_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
                                  3, const_cast<void*>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -231,7 +231,9 @@ int launch_flatquant_sm100_n128(int mode, const void* x_map, const void* left, c
                                 int64_t tokens, int m, int n, float clip, int in_dtype, int scale_dtype, uint32_t* status,
                                 cudaStream_t stream);
 
-// one launch of the kernel for right transforms of 144 .. 256 (flatquant_sm100_n256.cu)
+// one launch of the kernel for right transforms of 144 .. 256 (flatquant_sm100_n256.cu); the tensor map's boxes have
+// flatquant_sm100_n256_box_rows(m) rows
+int flatquant_sm100_n256_box_rows(int m);
 bool flatquant_sm100_n256_supported(int m, int n);
 int launch_flatquant_sm100_n256(int mode, const void* x_map, const void* left, const void* right, void* out, void* scales,
                                 int64_t tokens, int m, int n, float clip, int in_dtype, int scale_dtype, uint32_t* status,

@@ -1,30 +1,33 @@
 // FlatQuant quantizer for sm_100a, right transform of size 144 .. 256 (features = M x N, M and N multiples of 16,
 // 16 <= M <= 128): 28672 = 128 x 224, 32768 = 128 x 256, 24576 = 128 x 192, 20480 = 128 x 160, 18432 = 128 x 144.
 //
-// One persistent CTA per SM, one token at a time.  Both products are computed TRANSPOSED, because neither the rounded
-// Y nor a second copy of X would fit in shared memory beside a 256 x 256 R (128 KB) and X (64 KB):
+// A CTA PAIR (cta_group::2) per token, 74 persistent pairs.  Both products are computed TRANSPOSED and each CTA owns up to 128
+// of the token's N columns, as the rows of its tensor memory:
 //
-//   Y^T = R^T . X^T   A = R as it lies in memory (M-major), two tiles of 128 rows (the N dimension of the token),
-//                     B = X rows as the TMA brings them (K-major), N = M columns, K = N
+//   Y^T = R^T . X^T   A = R as it lies in memory (M-major): each CTA keeps its 128 columns of R; B = X rows as the TMA
+//                     brings them (K-major): each CTA loads half of the token's rows
 //   Z^T = Y^T . L     A = Y^T, rounded to the activation dtype, from TENSOR MEMORY: it overwrites the first half of its
-//                     own float32 accumulators; B = L as it lies in memory (N-major); K = M
+//                     own float32 accumulators; B = L as it lies in memory (N-major), half of its columns per CTA
 //
-//   warp 0        TMA: 3-D tensor map (n, m, token), boxes of 64 x M, 128-byte swizzle; ONE X stage: it is free again
-//                 as soon as the first product is done, so the next token's load runs under the rest of this token
-//   warps 1, 2    issue the two products, tile by tile, so that the Y pass of tile 0 runs under the first product of
-//                 tile 1 and the second product of tile 0 under the Y pass of tile 1; two issuers keep each other's
-//                 barrier latencies off the tensor core
-//   warps 4-11    Y pass: warp (tile, q) rounds lanes 32q .. 32q+31 of its tile, in place
-//   warps 12-27   quantize pass: warp (tile, h, q) takes columns (rows of the token's matrix) 64h .. 64h+63 of lanes
-//                 32q .. 32q+31; absmax through shared memory, scale, codes.  A lane holds one column of the token's
-//                 matrix, so the eight codes of a packed word lie in eight lanes: an 8 x 8 transposition of nibbles
-//                 (three shuffles) turns them round.
+// A pair holds one R (128 KB) in two shared memories, so four tokens' X fit beside it, and the accumulators of two tokens
+// fit tensor memory: loads, products, Y pass and quantize pass of different tokens overlap.
 //
-// Bound: HBM (57,344 bytes in and 14,340 out per token of 28672; 11 us for 1001 tokens).  Measured in graph replay: 29.7 us
-// for 1001 bf16 tokens to packed codes, 2.4 TB/s, 112.7 us for 4000 (35.1 and 124.7 with one issuing warp and without the
-// register shares); the SIMT kernel, before the only one for such widths, takes 3600 us for the former.  A token is a
-// chain of load, first product, Y pass and second product; its X boxes given back one by one were measured slower (38 to
-// 41 us: more barrier polls and commits in the issuing thread).
+//   warp 0        TMA: 3-D tensor map (n, m, token), boxes of 64 columns x half of the rows, 128-byte swizzle, 4 stages
+//   warps 3, 2    (leader) issue the two products; two issuers keep each other's barrier latencies off the tensor core
+//   warps 4-11    Y pass: warp (h, q) rounds columns 64h .. 64h+63 of lanes 32q .. 32q+31, in place
+//   warps 12-27   quantize pass, two sets of eight that alternate between tokens: warp (h, q) takes columns (rows of the
+//                 token's matrix) 64h .. 64h+63 of lanes 32q .. 32q+31; absmax through both CTAs' shared memory, scale,
+//                 codes.  A lane holds one column of the token's matrix, so the eight codes of a packed word lie in
+//                 eight lanes: an 8 x 8 transposition of nibbles (three shuffles a word) turns them round.
+//
+// Bound: HBM (57,344 bytes in and 14,340 out per token of 28672; 11 us for 1001 tokens).  Measured in graph replay, bf16 to
+// packed codes, one CTA per token with one X stage (all that fits beside a whole R) / this: 1001 x 28672 29.6 / 26.9 us,
+// 4000 112 / 92, 64 10.3 / 7.8, one token 9.9 / 6.3; 301 x 32768 17.0 / 13.2, 1001 x 18432 24.7 / 21.5; 500 x 2304 (16 x
+// 144) alike.  Without any product or code the loads alone take 13 us at 1001 tokens, without the codes 23, without the products 24:
+// the issuing thread (14 + 8 MMAs a token, 85 to 140 cycles each where the tensor core needs 64) and the chain of the
+// quantize pass (about 4400 cycles a visit, 2 sets) are equally long, both stretched by the instruction fetches of
+// seven roles on an SM (1.7 warps wait for instructions per instruction issued).  Measured and slower: three quantize sets of 72 registers
+// (28.6), four sets of four warps (spills, 44), Y pass in two sets of four warps (27.5).
 //
 // Numerics are those of flatquant_sm100_n128.cu (same packed arithmetic, same rounding points; reference:
 // src/quant_ops/ops/quantization/flatquant/ops.py:99-117).  Tokens with an infinity or a NaN among their transformed
@@ -39,30 +42,35 @@ namespace {
 using namespace ptx;
 using namespace fq;
 
-constexpr int kThreads = 896;  // 28 warps: TMA, two MMA issuers, one idle, 8 (Y pass) + 16 (quantize pass)
+constexpr int kThreads = 896;  // 28 warps: TMA, two MMA issuers, one idle, 2 x 4 (Y pass) + 2 x 8 (quantize pass)
 constexpr int kYWarp0 = 4, kQWarp0 = 12;
-// Registers per thread (by warpgroup, hence the idle warp): the block is launched with 896 x 72.  With 224 KB of shared
-// memory in use hardly any L1 is left, so a register spilled in the quantize pass is read back from L2.
+// Registers per thread (by warpgroup, hence the idle warp): the block is launched with 896 x 72.
 constexpr int kRegsQuant = 88, kRegsRest = 48;
 static_assert(512 * kRegsQuant + 384 * kRegsRest <= kThreads * 72, "the shares must fit the launch's registers");
 constexpr int kMaxM = 128, kMaxN = 256;
-constexpr int kOffX = 0;                              // four 64-column atoms of M rows
-constexpr int kOffL = kOffX + 4 * kAtomBytes;         // two 64-column blocks of M rows
-constexpr int kOffR = kOffL + 2 * kAtomBytes;         // four 64-column blocks of N rows
-constexpr int kOffMisc = kOffR + 4 * kMaxN * 128;
-constexpr int kSmemBytes = kOffMisc + 256 + 1024;
+constexpr int kXStages = 4;
+constexpr int kBoxBytes = 64 * 128;                   // up to 64 rows of 64 columns
+constexpr int kXBytes = 4 * kBoxBytes;                // a CTA's rows of one token
+constexpr int kOffX = 0;
+constexpr int kOffL = kOffX + kXStages * kXBytes;     // M rows of up to 64 columns
+constexpr int kOffR = kOffL + kMaxM * 128;            // two 64-column blocks of N rows
+constexpr int kOffMisc = kOffR + 2 * kMaxN * 128;
+constexpr int kSmemBytes = kOffMisc + 512 + 1024;
 static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
-constexpr int kTmemCols = 512;                        // first product: 2 tiles x 128 columns; second product: the same
+constexpr int kTmemCols = 512;                        // first product (then Y): 2 tokens x 128 columns; second product: the same
 constexpr int kColZ = 256;
 
 struct Misc {
-  uint64_t full_x, empty_x;
-  uint64_t d1_full[2], y_ready[2], y_free[2], d2_full[2], d2_empty[2], set_sync;
+  uint64_t full_x[kXStages];                          // leader's: both CTAs' boxes
+  uint64_t empty_x[kXStages];
+  uint64_t d1_full[2], d2_full[2];
+  uint64_t y_ready[2], y_free[2], d2_empty[2];        // leader's
+  uint64_t staged;                                    // leader's: both CTAs' transforms are in place
+  uint64_t meet[2][2];                                // [set][use % 2], see the quantize pass
   uint32_t tmem_base;
-  uint32_t absmax_bits[3];  // bits of the token's largest |z|; a NaN among them is larger than any number
-  uint32_t finite_bits[3];  // the same without the NaNs, plus one (0: every value is a NaN)
+  alignas(16) uint32_t part[2][2][2][8];              // [set][use % 2][CTA][warp]: what the warps of a token tell each other
 };
-static_assert(sizeof(Misc) <= 256, "misc area");
+static_assert(sizeof(Misc) <= 512, "misc area");
 
 // NaN-propagating |max| of packed pairs (the sign is ignored by the caller)
 template <typename T> __device__ __forceinline__ uint32_t absmax_nan(uint32_t a, uint32_t b);
@@ -77,35 +85,43 @@ template <> __device__ __forceinline__ uint32_t absmax_nan<__half>(uint32_t a, u
   return d;
 }
 
-// Transposition inside groups of 8 lanes: lane i's nibble j becomes lane j's nibble i.
-struct NibbleTurn {
-  uint32_t sel4, sel2, mask1, shr1, shl1;
-  __device__ __forceinline__ explicit NibbleTurn(int lane) {
-    sel4 = (lane & 4) ? 0x3276u : 0x5410u;  // halves
-    sel2 = (lane & 2) ? 0x3715u : 0x6240u;  // bytes
-    mask1 = (lane & 1) ? 0xF0F0F0F0u : 0x0F0F0F0Fu;
-    shr1 = (lane & 1) ? 4u : 0u;
-    shl1 = (lane & 1) ? 0u : 4u;
-  }
-  __device__ __forceinline__ uint32_t operator()(uint32_t x) const {
-    x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 4), sel4);
-    x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 2), sel2);
-    const uint32_t r = __shfl_xor_sync(0xffffffffu, x, 1);
-    return (x & mask1) | (((r >> shr1) << shl1) & ~mask1);
-  }
-};
+// Transposition inside groups of 8 lanes: lane i's nibble j becomes lane j's nibble i.  COUNT words at a time, exchange by
+// exchange: a shuffle's latency is hidden by the other words' shuffles, and there are few warps to hide it.
+template <int COUNT>
+__device__ __forceinline__ void turn_nibbles(uint32_t* x, int stride, int lane) {
+  const uint32_t sel4 = (lane & 4) ? 0x3276u : 0x5410u;  // halves
+  const uint32_t sel2 = (lane & 2) ? 0x3715u : 0x6240u;  // bytes
+  const uint32_t mask1 = (lane & 1) ? 0xF0F0F0F0u : 0x0F0F0F0Fu;
+  const uint32_t shr1 = (lane & 1) ? 4u : 0u, shl1 = (lane & 1) ? 0u : 4u;
+  uint32_t r[COUNT];
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) r[i] = __shfl_xor_sync(0xffffffffu, x[i * stride], 4);
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) x[i * stride] = __byte_perm(x[i * stride], r[i], sel4);
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) r[i] = __shfl_xor_sync(0xffffffffu, x[i * stride], 2);
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) x[i * stride] = __byte_perm(x[i * stride], r[i], sel2);
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) r[i] = __shfl_xor_sync(0xffffffffu, x[i * stride], 1);
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) x[i * stride] = (x[i * stride] & mask1) | (((r[i] >> shr1) << shl1) & ~mask1);
+}
 // The same for the four bytes of groups of 4 lanes.
-struct ByteTurn {
-  uint32_t sel2, sel1;
-  __device__ __forceinline__ explicit ByteTurn(int lane) {
-    sel2 = (lane & 2) ? 0x3276u : 0x5410u;
-    sel1 = (lane & 1) ? 0x3715u : 0x6240u;
-  }
-  __device__ __forceinline__ uint32_t operator()(uint32_t x) const {
-    x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 2), sel2);
-    return __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 1), sel1);
-  }
-};
+template <int COUNT>
+__device__ __forceinline__ void turn_bytes(uint32_t* x, int stride, int lane) {
+  const uint32_t sel2 = (lane & 2) ? 0x3276u : 0x5410u;
+  const uint32_t sel1 = (lane & 1) ? 0x3715u : 0x6240u;
+  uint32_t r[COUNT];
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) r[i] = __shfl_xor_sync(0xffffffffu, x[i * stride], 2);
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) x[i * stride] = __byte_perm(x[i * stride], r[i], sel2);
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) r[i] = __shfl_xor_sync(0xffffffffu, x[i * stride], 1);
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) x[i * stride] = __byte_perm(x[i * stride], r[i], sel1);
+}
 
 // eight codes (offset binary, a nibble each) one by one: any z and s
 template <typename T>
@@ -121,7 +137,7 @@ __device__ __noinline__ uint32_t careful_word(uint32_t z0, uint32_t z1, uint32_t
 }
 
 template <typename T, int MODE>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
 flatquant_n256_kernel(const __grid_constant__ CUtensorMap x_map, const T* __restrict__ left, const T* __restrict__ right,
                       void* __restrict__ out, void* __restrict__ scales, long long tokens, int m, int n, float clip,
                       int scale_dtype, uint32_t* __restrict__ status) {
@@ -130,100 +146,147 @@ flatquant_n256_kernel(const __grid_constant__ CUtensorMap x_map, const T* __rest
   Misc* misc = reinterpret_cast<Misc*>(smem + kOffMisc);
   const uint32_t smem_base = smem_u32(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = (int)cluster_cta_rank();
+  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const int feat = m * n;
-  const int quads1 = (n - 128 + 31) >> 5;  // lane quadrants of tile 1 with real rows (tile 0 has four)
+  // The leader owns the columns from 128 on, the other CTA 0 .. 127: lane quadrants without columns (N = 224: one) leave the
+  // leader's issuing warps a scheduler of their own.
+  const int col0 = rank == 0 ? 128 : 0;
+  const int quads_leader = (n - 128 + 31) >> 5;       // lane quadrants of the leader with real columns (the other CTA has four)
+  const int quads = rank == 0 ? quads_leader : 4;
   const int halves = m > 64 ? 2 : 1;
-  int mine = 0;  // tokens of this CTA
-  if ((long long)blockIdx.x < tokens) mine = (int)((tokens - blockIdx.x + gridDim.x - 1) / gridDim.x);
+  const int np = (m + 31) & ~31, rows_cta = np >> 1;  // the pair's MMAs take N in steps of 32; each CTA brings half of it
+  int mine = 0;                                       // tokens of this pair
+  if ((long long)pair < tokens) mine = (int)((tokens - pair + npairs - 1) / npairs);
 
   if (tid == 0) {
-    mbar_init(smem_u32(&misc->full_x), 1);
-    mbar_init(smem_u32(&misc->empty_x), 1);
+    for (int i = 0; i < kXStages; ++i) {
+      mbar_init(smem_u32(&misc->full_x[i]), 1);
+      mbar_init(smem_u32(&misc->empty_x[i]), 1);
+    }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&misc->d1_full[i]), 1);
-      mbar_init(smem_u32(&misc->y_ready[i]), i == 0 ? 4 : quads1);  // one arrival per working warp
-      mbar_init(smem_u32(&misc->y_free[i]), 1);
       mbar_init(smem_u32(&misc->d2_full[i]), 1);
-      mbar_init(smem_u32(&misc->d2_empty[i]), halves * (i == 0 ? 4 : quads1));
+      mbar_init(smem_u32(&misc->y_ready[i]), halves * (4 + quads_leader));  // one arrival per working warp of both CTAs
+      mbar_init(smem_u32(&misc->y_free[i]), 1);
+      mbar_init(smem_u32(&misc->d2_empty[i]), halves * (4 + quads_leader));
+      for (int j = 0; j < 2; ++j) mbar_init(smem_u32(&misc->meet[i][j]), halves * quads);
     }
-    mbar_init(smem_u32(&misc->set_sync), halves * (4 + quads1));
-    for (int i = 0; i < 3; ++i) misc->absmax_bits[i] = misc->finite_bits[i] = 0u;
+    mbar_init(smem_u32(&misc->staged), 2);
+    for (int i = 0; i < 2 * 2 * 2 * 8; ++i) (&misc->part[0][0][0][0])[i] = 0u;  // the slots of warps without work stay 0
     fence_barrier_init();
     prefetch_tensormap(&x_map);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&misc->tmem_base), kTmemCols);
-    tmem_relinquish();
+    tmem_alloc_pair(smem_u32(&misc->tmem_base), kTmemCols);
+    tmem_relinquish_pair();
   }
   tc_fence_before();
-  __syncthreads();
+  __syncwarp();
+  cluster_sync_all();  // both CTAs' barriers and tensor memory exist before either touches the other
   tc_fence_after();
   const uint32_t tmem = misc->tmem_base;
   grid_dependency_wait();    // nothing below touches global memory before the kernel ahead in the stream has completed
   grid_launch_dependents();  // (after the wait: see flatquant_sm100_n128.cu)
 
   if (warp != 0) {
-    // Both transforms as they lie in memory, 16 bytes at a time with the 128-byte XOR swizzle.  R: rows k < n in four
-    // 64-column blocks, columns past n zero; L: rows k < m in two blocks, columns past m zero (never read: N = m).
+    // This CTA's part of both transforms as it lies in memory, 16 bytes at a time with the 128-byte XOR swizzle.  R: rows
+    // k < n of columns col0 .. col0 + 127 in two 64-column blocks; L: rows k < m of columns rows_cta rank .. + rows_cta - 1.
+    // Columns past the last one are zero.
     constexpr int kStagers = kThreads - 32;
     const int t1 = tid - 32;
-    constexpr int kPer = 6;  // pieces requested by a thread before it stores them: the loads' latencies overlap
-    for (int base = t1; base < n * 32; base += kStagers * kPer) {
-      uint4 w[kPer];
+    constexpr int kPer = 5;  // pieces requested by a thread before it stores them: the loads' latencies overlap
+    static_assert(kStagers * kPer >= kMaxN * 16, "one round");
+    uint4 w[kPer], wl[2];
 #pragma unroll
-      for (int j = 0; j < kPer; ++j) {
-        const int idx = base + j * kStagers, k = idx >> 5, c = idx & 31;
-        w[j] = make_uint4(0, 0, 0, 0);
-        if (idx < n * 32 && 8 * c < n) w[j] = *reinterpret_cast<const uint4*>(right + k * n + 8 * c);
-      }
-#pragma unroll
-      for (int j = 0; j < kPer; ++j) {
-        const int idx = base + j * kStagers, k = idx >> 5, c = idx & 31;
-        if (idx < n * 32) *reinterpret_cast<uint4*>(smem + kOffR + (c >> 3) * (n * 128) + k * 128 + (((c & 7) ^ (k & 7)) << 4)) = w[j];
-      }
+    for (int j = 0; j < kPer; ++j) {
+      const int idx = t1 + j * kStagers, k = idx >> 4, c = col0 + 8 * (idx & 15);
+      w[j] = make_uint4(0, 0, 0, 0);
+      if (idx < n * 16 && c < n) w[j] = *reinterpret_cast<const uint4*>(right + k * n + c);
     }
-    for (int idx = t1; idx < m * 16; idx += kStagers) {
-      const int k = idx >> 4, c = idx & 15;
-      uint4 w = make_uint4(0, 0, 0, 0);
-      if (8 * c < m) w = *reinterpret_cast<const uint4*>(left + k * m + 8 * c);
-      *reinterpret_cast<uint4*>(smem + kOffL + (c >> 3) * kAtomBytes + k * 128 + (((c & 7) ^ (k & 7)) << 4)) = w;
+    static_assert(kStagers * 2 >= kMaxM * 8, "one round");
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int idx = t1 + j * kStagers, k = idx >> 3, c = 8 * (idx & 7);
+      wl[j] = make_uint4(0, 0, 0, 0);
+      if (idx < m * 8 && c < rows_cta && rank * rows_cta + c < m) wl[j] = *reinterpret_cast<const uint4*>(left + k * m + rank * rows_cta + c);
+    }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int idx = t1 + j * kStagers, k = idx >> 4, c = idx & 15;
+      if (idx < n * 16) *reinterpret_cast<uint4*>(smem + kOffR + (c >> 3) * (n * 128) + k * 128 + (((c & 7) ^ (k & 7)) << 4)) = w[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int idx = t1 + j * kStagers, k = idx >> 3, c = idx & 7;
+      if (idx < m * 8) *reinterpret_cast<uint4*>(smem + kOffL + k * 128 + ((c ^ (k & 7)) << 4)) = wl[j];
     }
     fence_proxy_async_smem();
     asm volatile("bar.sync 1, %0;" ::"n"(kStagers) : "memory");
+    if (tid == 32) mbar_arrive_cluster(cluster_map_shared(smem_u32(&misc->staged), 0));
   }
 
   if (warp >= kQWarp0) {
     regs_inc<kRegsQuant>();
-    // ---- quantize pass -----------------------------------------------------------------------------------------------
-    const int q = warp & 3, idx = (warp - kQWarp0) >> 2, tl = idx >> 1, h = idx & 1;
-    const int n0 = tl * 128 + q * 32, r0 = h * 64;   // first column / first row of the token's matrix in this warp
-    const int rows = min(64, m - r0);                // rows of this warp (a multiple of 16)
+    // ---- quantize pass: set e takes the tokens e, e + 2, ... of this pair ---------------------------------------------
+    const int q = warp & 3, idx = (warp - kQWarp0) >> 2, e = idx >> 1, h = idx & 1;
+    const int n0 = col0 + q * 32, r0 = h * 64;  // first column / first row of the token's matrix in this warp
+    const int rows = min(64, m - r0);                 // rows of this warp (a multiple of 16)
     const bool valid = n0 + lane < n;
-    const bool first = tl == 0 && h == 0 && q == 0;
-    const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + kColZ + tl * 128 + r0;
-    const uint32_t gs = smem_u32(&misc->set_sync);
+    const bool first = h == 0 && q == 0;              // of this CTA
+    const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + kColZ + e * 128 + r0;
+    const uint32_t d2_empty = cluster_map_shared(smem_u32(&misc->d2_empty[e]), 0);
+    const uint32_t peer_bytes = 4u * (uint32_t)(halves * (rank == 0 ? 4 : quads_leader));
     int meets = 0;
-    long long tok = blockIdx.x;
-    for (int it = 0; it < (n0 < n && rows > 0 ? mine : 0); ++it, tok += gridDim.x) {
-      const int buf = it % 3;
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc->d2_full[tl]), it & 1))) { atomicCAS(status, 0u, 0xC60u + tl); break; }
+    // Every warp of the token gives a value, and gets the largest of all of them.  A value goes into the warp's slot in both
+    // CTAs, into the other one together with the bytes that its barrier counts.  Barriers and slots alternate: a warp
+    // that is already at the next meeting must not be counted for this one, and it can be at the one after next only
+    // when every warp has left this one.
+    auto meet_max = [&](uint32_t value, uint32_t& largest) -> bool {
+      const int b = meets & 1;
+      const uint32_t bar = smem_u32(&misc->meet[e][b]);
+      if (lane == 0) {
+        const uint32_t slot = smem_u32(&misc->part[e][b][rank][h * 4 + q]);
+        st_async_cluster(cluster_map_shared(slot, rank ^ 1), value, cluster_map_shared(bar, rank ^ 1));
+        misc->part[e][b][rank][h * 4 + q] = value;
+        if (first) mbar_arrive_expect_tx(bar, peer_bytes);
+        else mbar_arrive(bar);
+      }
+      __syncwarp();
+      if (!__all_sync(0xffffffffu, mbar_wait_cluster(bar, (meets >> 1) & 1))) return false;
+      ++meets;
+      largest = __reduce_max_sync(0xffffffffu, *(volatile uint32_t*)&misc->part[e][b][(lane >> 3) & 1][lane & 7]);
+      return true;
+    };
+    for (int it = e; it < (n0 < n && rows > 0 ? mine : 0); it += 2) {
+      const long long tok = pair + (long long)it * npairs;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc->d2_full[e]), (it >> 1) & 1))) { atomicCAS(status, 0u, 0xC60u + e); break; }
       tc_fence_after();
       uint32_t zz[32];  // 64 rounded values as packed pairs; rows past the last one are zero
+      // (rows is a multiple of 16: the second half of a last block of 16 is zero, as R's missing columns are)
+      if (rows > 32) {
+        uint32_t va[32], vb[32];
+        tmem_ld_32x32b_x32(taddr, va);
+        tmem_ld_32x32b_x32(taddr + 32, vb);
+        tmem_ld_wait();
 #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        if (ch * 16 < rows) {
-          uint32_t v[16];
-          tmem_ld_32x32b_x16(taddr + ch * 16, v);
-          tmem_ld_wait();
+        for (int i = 0; i < 16; ++i) {
+          zz[i] = P2<T>::cvt(__uint_as_float(va[2 * i]), __uint_as_float(va[2 * i + 1]));
+          zz[16 + i] = P2<T>::cvt(__uint_as_float(vb[2 * i]), __uint_as_float(vb[2 * i + 1]));
+        }
+      } else {
+        uint32_t va[32];
+        tmem_ld_32x32b_x32(taddr, va);
+        tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 8; ++i) zz[8 * ch + i] = P2<T>::cvt(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) zz[8 * ch + i] = 0u;
+        for (int i = 0; i < 16; ++i) {
+          zz[i] = P2<T>::cvt(__uint_as_float(va[2 * i]), __uint_as_float(va[2 * i + 1]));
+          zz[16 + i] = 0u;
         }
       }
       tc_fence_before();
-      mbar_arrive_warp(smem_u32(&misc->d2_empty[tl]));  // the accumulators are free again
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(d2_empty);  // the accumulators are free again
 
       if (MODE == kTransform) {
         float* dst = reinterpret_cast<float*>(out) + tok * feat + (int64_t)r0 * n + n0 + lane;
@@ -249,14 +312,10 @@ flatquant_n256_kernel(const __grid_constant__ CUtensorMap x_map, const T* __rest
       // bits of non-negative floats order as integers, and those of a NaN are above those of an infinity
       const uint32_t row_bits = valid ? max(__float_as_uint(fabsf(P2<T>::lo(m0))), __float_as_uint(fabsf(P2<T>::hi(m0)))) : 0u;
       const uint32_t warp_bits = __reduce_max_sync(0xffffffffu, row_bits);
-      if (lane == 0) atomicMax(&misc->absmax_bits[buf], warp_bits);
-      mbar_arrive_warp(gs);
-      if (!__all_sync(0xffffffffu, mbar_wait(gs, meets & 1))) { atomicCAS(status, 0u, 0xC70u); break; }
-      ++meets;
-      const uint32_t token_bits = misc->absmax_bits[buf];
-      if (first && lane == 0) misc->absmax_bits[(it + 2) % 3] = misc->finite_bits[(it + 2) % 3] = 0u;
+      uint32_t token_bits;
+      if (!meet_max(warp_bits, token_bits)) { atomicCAS(status, 0u, 0xC70u); break; }
       float amax = __uint_as_float(token_bits);
-      const bool special = token_bits >= 0x7F800000u;  // the same for every warp of the token
+      const bool special = token_bits >= 0x7F800000u;  // the same for every warp of the token, in both CTAs
       if (special) {
         // an infinity or a NaN in this token: the SIMT kernel's extremes skip NaNs (and start from +-3.4e38)
         float a = -1.f;
@@ -270,11 +329,8 @@ flatquant_n256_kernel(const __grid_constant__ CUtensorMap x_map, const T* __rest
             if (2 * i < rows) a = fmaxf(a, fmaxf(fabsf(P2<T>::lo(zz[i])), fabsf(P2<T>::hi(zz[i]))));
         }
         const uint32_t fb = __reduce_max_sync(0xffffffffu, valid && a >= 0.f ? __float_as_uint(a) + 1u : 0u);
-        if (lane == 0) atomicMax(&misc->finite_bits[buf], fb);
-        mbar_arrive_warp(gs);
-        if (!__all_sync(0xffffffffu, mbar_wait(gs, meets & 1))) { atomicCAS(status, 0u, 0xC71u); break; }
-        ++meets;
-        const uint32_t tb = misc->finite_bits[buf];
+        uint32_t tb;
+        if (!meet_max(fb, tb)) { atomicCAS(status, 0u, 0xC71u); break; }
         amax = tb == 0u ? 3.4e38f : __uint_as_float(tb - 1u);
       }
       const float top = rnd1<T>(amax * clip);
@@ -282,144 +338,177 @@ flatquant_n256_kernel(const __grid_constant__ CUtensorMap x_map, const T* __rest
       const float inv_s = __frcp_rn(s);
       uint32_t rhi2, rlo2;
       P2<T>::recip2(inv_s, rhi2, rlo2);
-      if (first && lane == 0) store_scale(scales, tok, s, scale_dtype);
+      if (first && rank == 0 && lane == 0) store_scale(scales, tok, s, scale_dtype);
       const bool careful = special || s == 0.f || !(s < 0x1p100f);
       // a quotient can only leave [-8, 7] after rounding if some |z| / s reaches 7.5
       const bool clamp_needed = !(__uint_as_float(warp_bits) * inv_s < 7.4f);
 
       if (MODE == kPacked) {
-        const NibbleTurn turn(lane);
         uint32_t* dst = reinterpret_cast<uint32_t*>(out) + tok * (feat / 8) + (int64_t)(r0 + (lane & 7)) * (n / 8) + n0 / 8 + (lane >> 3);
-        const bool store = n0 + 8 * (lane >> 3) < n;
+        // (one choice for all words: the branches and the code of the other cases stay out of the usual one)
+        if (careful) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (8 * j >= rows) break;
-          uint32_t w;
-          if (careful) w = careful_word<T>(zz[4 * j], zz[4 * j + 1], zz[4 * j + 2], zz[4 * j + 3], s);
-          else if (clamp_needed) w = quantize8<T, true>(&zz[4 * j], s, inv_s, rhi2, rlo2);
-          else w = quantize8<T, false>(&zz[4 * j], s, inv_s, rhi2, rlo2);
-          w = turn(w);
-          if (store) dst[(8 * j) * (n / 8)] = w;
+          for (int j = 0; j < 8; ++j) zz[4 * j] = careful_word<T>(zz[4 * j], zz[4 * j + 1], zz[4 * j + 2], zz[4 * j + 3], s);
+        } else if (clamp_needed) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) zz[4 * j] = quantize8<T, true>(&zz[4 * j], s, inv_s, rhi2, rlo2);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) zz[4 * j] = quantize8<T, false>(&zz[4 * j], s, inv_s, rhi2, rlo2);
+        }
+        turn_nibbles<8>(zz, 4, lane);
+        if (n0 + 8 * (lane >> 3) < n) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (8 * j < rows) dst[(8 * j) * (n / 8)] = zz[4 * j];
         }
       } else {
-        const ByteTurn turn(lane);
         uint8_t* dst = reinterpret_cast<uint8_t*>(out) + tok * feat + (int64_t)(r0 + (lane & 3)) * n + n0 + 4 * (lane >> 2);
-        const bool store = n0 + 4 * (lane >> 2) < n;
+        if (careful) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (8 * j >= rows) break;
-          uint32_t pb, qb;
-          if (careful) {
+          for (int j = 0; j < 8; ++j) {
             const uint32_t w = careful_word<T>(zz[4 * j], zz[4 * j + 1], zz[4 * j + 2], zz[4 * j + 3], s);
             const uint32_t even = w & 0x0F0F0F0Fu, odd = (w >> 4) & 0x0F0F0F0Fu;
-            pb = __byte_perm(even, odd, 0x5140);
-            qb = __byte_perm(even, odd, 0x7362);
-          } else {
+            zz[4 * j] = bytes4(__byte_perm(even, odd, 0x5140));
+            zz[4 * j + 2] = bytes4(__byte_perm(even, odd, 0x7362));
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            uint32_t pb, qb;
             nibble_bytes_packed<T>(&zz[4 * j], s, inv_s, rhi2, rlo2, pb, qb);
+            zz[4 * j] = bytes4(pb);
+            zz[4 * j + 2] = bytes4(qb);
           }
-          pb = turn(bytes4(pb));
-          qb = turn(bytes4(qb));
-          if (store) {
-            *reinterpret_cast<uint32_t*>(dst + (8 * j) * n) = pb;
-            *reinterpret_cast<uint32_t*>(dst + (8 * j + 4) * n) = qb;
-          }
+        }
+        turn_bytes<8>(zz, 2, lane);
+        turn_bytes<8>(zz + 16, 2, lane);
+        if (n0 + 4 * (lane >> 2) < n) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (4 * j < rows) *reinterpret_cast<uint32_t*>(dst + (4 * j) * n) = zz[2 * j];
         }
       }
     }
   } else {
   regs_dec<kRegsRest>();
   if (warp == 0) {
+    // ---- TMA: each CTA brings its half of the token's rows; the leader's barrier counts both ----------------------------
     if (lane == 0) {
       const int boxes = (n + 63) >> 6;
-      long long tok = blockIdx.x;
-      for (int it = 0; it < mine; ++it, tok += gridDim.x) {
-        if (!mbar_wait(smem_u32(&misc->empty_x), (it & 1) ^ 1)) { atomicCAS(status, 0u, 0xC00u); break; }
-        const uint32_t bar = smem_u32(&misc->full_x);
-        mbar_arrive_expect_tx(bar, (uint32_t)(boxes * m * 128));
-        for (int b = 0; b < boxes; ++b) tma_load_3d(smem_base + kOffX + b * kAtomBytes, &x_map, bar, b * 64, 0, (int)tok);
+      const uint32_t bytes = (uint32_t)(2 * boxes * rows_cta * 128);
+      int it = 0;
+      bool ok = true;
+      for (; it < mine; ++it) {
+        const int s = it % kXStages, ph = (it / kXStages) & 1;
+        if (!mbar_wait(smem_u32(&misc->empty_x[s]), ph ^ 1)) { atomicCAS(status, 0u, 0xC00u + s); ok = false; break; }
+        const uint32_t bar = cluster_map_shared(smem_u32(&misc->full_x[s]), 0);
+        if (rank == 0) mbar_arrive_expect_tx(smem_u32(&misc->full_x[s]), bytes);
+        const int tok = (int)(pair + (long long)it * npairs);
+        for (int b = 0; b < boxes; ++b) tma_load_3d_pair(smem_base + kOffX + s * kXBytes + b * kBoxBytes, &x_map, bar, b * 64, rank * rows_cta, tok);
+      }
+      // The last commits to this CTA's barriers have landed before it can leave; after a wait that gave up, the loads still in
+      // flight have (their bytes are counted in the leader, out of this CTA's sight).
+      if (!ok)
+        for (int i = 0; i < 100; ++i) __nanosleep(1000);
+      for (int back = 1; ok && back <= kXStages && back <= mine; ++back) {
+        const int u = mine - back;
+        if (!mbar_wait(smem_u32(&misc->empty_x[u % kXStages]), (u / kXStages) & 1)) { atomicCAS(status, 0u, 0xC08u); break; }
       }
     }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc1 = umma_idesc(1, Fmt<T>::id, Fmt<T>::id, 1, 0, 128, m);  // A = R^T: M-major, B = X rows: K-major
-      const uint64_t desc_x = umma_smem_desc_sw128(smem_base + kOffX, 16, 1024);
+  } else if (warp == 3) {
+    if (lane == 0 && rank == 0) {
+      const uint32_t idesc1 = umma_idesc(1, Fmt<T>::id, Fmt<T>::id, 1, 0, 256, np);  // A = R^T: M-major, B = X rows: K-major
+      const uint64_t desc_r = umma_smem_desc_sw128(smem_base + kOffR, (uint32_t)(n * 128), 1024);
+      const uint64_t desc_x0 = umma_smem_desc_sw128(smem_base + kOffX, 16, 1024);
       const int ks1 = n >> 4;
-      bool ok = true;
-      for (int it = 0; ok && it < mine; ++it) {
-        const int ph = it & 1;
-        for (int tl = 0; tl < 2; ++tl) {
-          if (const int w = tl == 0 ? mbar_wait2(smem_u32(&misc->full_x), ph, smem_u32(&misc->y_free[0]), ph ^ 1)
-                                    : (mbar_wait(smem_u32(&misc->y_free[1]), ph ^ 1) ? 0 : 3)) {
-            atomicCAS(status, 0u, 0xC10u + w);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t desc_r = umma_smem_desc_sw128(smem_base + kOffR + tl * 2 * (n * 128), (uint32_t)(n * 128), 1024);
-#pragma unroll 2
-          for (int ks = 0; ks < ks1; ++ks)  // 16 rows of R = 2048 bytes per step; X: 32 bytes inside a 64-column atom
-            mma_f16_ss(tmem + tl * 128, desc_r + (uint64_t)(ks * 128), desc_x + (uint64_t)((ks >> 2) * (kAtomBytes >> 4) + (ks & 3) * 2), idesc1, ks);
-          mma_commit(smem_u32(&misc->d1_full[tl]));
+      const uint32_t d1_full = smem_u32(&misc->d1_full[0]), d1_full_peer = cluster_map_shared(d1_full, 1);
+      const uint32_t empty_x = smem_u32(&misc->empty_x[0]), empty_x_peer = cluster_map_shared(empty_x, 1);
+      int left_to_do = mine;
+      if (!mbar_wait(smem_u32(&misc->staged), 0)) { atomicCAS(status, 0u, 0xC18u); left_to_do = 0; }
+      for (int it = 0; it < left_to_do; ++it) {
+        const int s = it % kXStages, e = it & 1;
+        if (const int w = mbar_wait2(smem_u32(&misc->full_x[s]), (it / kXStages) & 1, smem_u32(&misc->y_free[e]), ((it >> 1) & 1) ^ 1)) {
+          atomicCAS(status, 0u, 0xC10u + w);
+          break;
         }
-        if (ok) mma_commit(smem_u32(&misc->empty_x));
+        tc_fence_after();
+        const uint64_t dx = desc_x0 + (uint64_t)(s * (kXBytes >> 4));
+        // 16 rows of R = 2048 bytes per step; X: 32 bytes inside a 64-column box
+        int ks = 0;
+        for (; ks + 4 <= ks1; ks += 4)
+          mma_f16_ss_pair_x4<128, 2>(tmem + e * 128, desc_r + (uint64_t)(ks * 128), dx + (uint64_t)(ks * (kBoxBytes >> 6)), idesc1, ks);
+        for (; ks < ks1; ++ks)
+          mma_f16_ss_pair(tmem + e * 128, desc_r + (uint64_t)(ks * 128), dx + (uint64_t)((ks >> 2) * (kBoxBytes >> 4) + (ks & 3) * 2), idesc1, ks);
+        mma_commit_pair(d1_full + 8 * e);
+        mma_commit_pair(d1_full_peer + 8 * e);
+        mma_commit_pair(empty_x + 8 * s);
+        mma_commit_pair(empty_x_peer + 8 * s);
       }
     }
   } else if (warp == 2) {
-    if (lane == 0) {
-      const uint32_t idesc2 = umma_idesc(1, Fmt<T>::id, Fmt<T>::id, 0, 1, 128, m);  // A = Y^T in tensor memory, B = L: N-major
-      const uint64_t desc_l = umma_smem_desc_sw128(smem_base + kOffL, kAtomBytes, 1024);
+    if (lane == 0 && rank == 0) {
+      const uint32_t idesc2 = umma_idesc(1, Fmt<T>::id, Fmt<T>::id, 0, 1, 256, np);  // A = Y^T in tensor memory, B = L: N-major
+      const uint64_t desc_l = umma_smem_desc_sw128(smem_base + kOffL, 16, 1024);
       const int ks2 = m >> 4;
-      bool ok = true;
-      for (int it = 0; ok && it < mine; ++it) {
-        const int ph = it & 1;
-        for (int tl = 0; tl < 2; ++tl) {
-          if (const int w = mbar_wait2(smem_u32(&misc->y_ready[tl]), ph, smem_u32(&misc->d2_empty[tl]), ph ^ 1)) {
-            atomicCAS(status, 0u, 0xC20u + 0x10u * w + tl);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-#pragma unroll 2
-          for (int ks = 0; ks < ks2; ++ks)  // 16 values of Y^T = 8 tensor-memory columns per step
-            mma_f16_ts(tmem + kColZ + tl * 128, tmem + tl * 128 + ks * 8, desc_l + (uint64_t)(ks * 128), idesc2, ks);
-          mma_commit(smem_u32(&misc->y_free[tl]));
-          mma_commit(smem_u32(&misc->d2_full[tl]));
+      const uint32_t d2_full = smem_u32(&misc->d2_full[0]), d2_full_peer = cluster_map_shared(d2_full, 1);
+      for (int it = 0; it < mine; ++it) {
+        const int e = it & 1, ph = (it >> 1) & 1;
+        if (const int w = mbar_wait2(smem_u32(&misc->y_ready[e]), ph, smem_u32(&misc->d2_empty[e]), ph ^ 1)) {
+          atomicCAS(status, 0u, 0xC20u + 0x10u * w + e);
+          break;
         }
+        tc_fence_after();
+        // 16 values of Y^T = 8 tensor-memory columns per step, four steps at the start of every 64 columns
+        int ks = 0;
+        for (; ks + 4 <= ks2; ks += 4)
+          mma_f16_ts_pair_x4<8, 128>(tmem + kColZ + e * 128, tmem + e * 128 + ks * 16, desc_l + (uint64_t)(ks * 128), idesc2, ks);
+        for (; ks < ks2; ++ks)
+          mma_f16_ts_pair(tmem + kColZ + e * 128, tmem + e * 128 + (ks & 4) * 16 + (ks & 3) * 8, desc_l + (uint64_t)(ks * 128), idesc2, ks);
+        mma_commit_pair(smem_u32(&misc->y_free[e]));
+        mma_commit_pair(d2_full + 8 * e);
+        mma_commit_pair(d2_full_peer + 8 * e);
       }
     }
   } else if (warp >= kYWarp0) {
-    // ---- Y pass: 32 lanes of one tile; every 32 float32 columns become 16 packed ones, written below what is still to read
-    const int q = warp & 3, tl = (warp - kYWarp0) >> 2;
-    const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + tl * 128;
-    const bool works = tl * 128 + q * 32 < n;
-    for (int it = 0; it < (works ? mine : 0); ++it) {
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc->d1_full[tl]), it & 1))) { atomicCAS(status, 0u, 0xC50u + tl); break; }
+    // ---- Y pass: warp (h, q) rounds columns 64h .. 64h+63 of lanes 32q .. 32q+31; every 32 float32 columns become 16 packed
+    // ones at the start of the warp's own 64, below what it has still to read
+    const int q = warp & 3, h = (warp - kYWarp0) >> 2;
+    const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + h * 64;
+    const uint32_t y_ready = cluster_map_shared(smem_u32(&misc->y_ready[0]), 0);
+    const int cols = min(64, m - 64 * h);  // (a multiple of 16)
+    for (int it = 0; it < (q < quads && cols > 0 ? mine : 0); ++it) {
+      const int e = it & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc->d1_full[e]), (it >> 1) & 1))) { atomicCAS(status, 0u, 0xC50u + e); break; }
       tc_fence_after();
-#pragma unroll 1
-      for (int c = 0; c < m; c += 32) {
+#pragma unroll
+      for (int c = 0; c < 64; c += 32) {
+        if (c >= cols) break;
         uint32_t v[32], a[8], b[8];
-        tmem_ld_32x32b_x32(base + c, v);
+        tmem_ld_32x32b_x32(base + e * 128 + c, v);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           a[i] = pack2<T>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
           b[i] = pack2<T>(__uint_as_float(v[16 + 2 * i]), __uint_as_float(v[16 + 2 * i + 1]));
         }
-        tmem_st_32x32b_x8(base + (c >> 1), a);
-        if (c + 16 < m) tmem_st_32x32b_x8(base + (c >> 1) + 8, b);
+        tmem_st_32x32b_x8(base + e * 128 + (c >> 1), a);
+        if (c + 16 < cols) tmem_st_32x32b_x8(base + e * 128 + (c >> 1) + 8, b);
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive_warp(smem_u32(&misc->y_ready[tl]));
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(y_ready + 8 * e);
     }
   }
   }
 
   tc_fence_before();
-  __syncthreads();
+  __syncwarp();
+  cluster_sync_all();  // the other CTA's last arrivals and words have landed before this one leaves
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, kTmemCols);
+    tmem_dealloc_pair(tmem, kTmemCols);
   }
 }
 
@@ -436,7 +525,7 @@ int launch_one(const CUtensorMap& map, const void* left, const void* right, void
   }
   const int sms = sm_count(dev);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tokens < sms ? tokens : sms));
+  cfg.gridDim = dim3(2u * (unsigned)(tokens < sms / 2 ? tokens : sms / 2));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = stream;
@@ -463,6 +552,9 @@ int launch_mode(int mode, const CUtensorMap& map, const void* left, const void* 
 }  // namespace
 
 bool flatquant_sm100_n256_supported(int m, int n) { return n > 128 && n <= kMaxN && (n % 16) == 0 && m >= 16 && m <= kMaxM && (m % 16) == 0; }
+
+// the rows of a token are shared out between the two CTAs of a pair, whose MMAs take them in steps of 32
+int flatquant_sm100_n256_box_rows(int m) { return ((m + 31) & ~31) / 2; }
 
 int launch_flatquant_sm100_n256(int mode, const void* x_map, const void* left, const void* right, void* out, void* scales,
                                 int64_t tokens, int m, int n, float clip, int in_dtype, int scale_dtype, uint32_t* status,

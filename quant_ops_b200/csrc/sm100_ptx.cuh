@@ -297,6 +297,63 @@ __device__ __forceinline__ void mma_i8_ts_pair(uint32_t d_tmem, uint32_t a_tmem,
       "tcgen05.mma.cta_group::2.kind::i8 [%0], [%1], %2, %3, p;\n\t}\n"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// the same for 16-bit operands, A from shared memory and from tensor memory
+__device__ __forceinline__ void mma_f16_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void mma_f16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Four steps of K in one instruction sequence: one thread issues for the tensor cores of two SMs and shares its scheduler with busy
+// warps, so every instruction between the MMAs counts.  A advances by A_STEP per step (descriptor units of 16 bytes, or
+// tensor-memory columns), B by B_STEP.
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void mma_f16_ss_pair_x4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      ".reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "add.u64 a1, %1, %5;\n\t"
+      "add.u64 a2, %1, %6;\n\t"
+      "add.u64 a3, %1, %7;\n\t"
+      "add.u64 b1, %2, %8;\n\t"
+      "add.u64 b2, %2, %9;\n\t"
+      "add.u64 b3, %2, %10;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %3, 1;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a2, b2, %3, 1;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, 1;\n\t}\n"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(2 * A_STEP), "n"(3 * A_STEP),
+        "n"(B_STEP), "n"(2 * B_STEP), "n"(3 * B_STEP) : "memory");
+}
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void mma_f16_ts_pair_x4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      ".reg .b32 a1, a2, a3;\n\t"
+      ".reg .b64 b1, b2, b3;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "add.u32 a1, %1, %5;\n\t"
+      "add.u32 a2, %1, %6;\n\t"
+      "add.u32 a3, %1, %7;\n\t"
+      "add.u64 b1, %2, %8;\n\t"
+      "add.u64 b2, %2, %9;\n\t"
+      "add.u64 b3, %2, %10;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], b1, %3, 1;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a2], b2, %3, 1;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a3], b3, %3, 1;\n\t}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(2 * A_STEP), "n"(3 * A_STEP),
+        "n"(B_STEP), "n"(2 * B_STEP), "n"(3 * B_STEP) : "memory");
+}
 // the barrier (a shared::cluster address: this CTA's or, through cluster_map_shared, the peer's) gets one arrival
 // once every MMA issued so far by this thread has finished in both CTAs
 __device__ __forceinline__ void mma_commit_pair(uint32_t bar_cluster_addr) {
@@ -308,6 +365,35 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+// one word into a CTA of the cluster, its four bytes counted on a barrier of that CTA (shared::cluster addresses)
+__device__ __forceinline__ void st_async_cluster(uint32_t dst_cluster, uint32_t value, uint32_t bar_cluster) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];" ::"r"(dst_cluster), "r"(value), "r"(bar_cluster) : "memory");
+}
+// mbar_wait for a barrier behind which data written by other CTAs of the cluster is read
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t limit_polls = 1u << 26) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .u32 n;\n\t"
+      "mov.u32 n, %3;\n"
+      "QO_WAITC_AGAIN:\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra.uni QO_WAITC_DONE;\n\t"
+      "sub.u32 n, n, 1;\n\t"
+      "setp.gt.s32 p, n, 0;\n\t"
+      "@p bra.uni QO_WAITC_AGAIN;\n"
+      "QO_WAITC_DONE:\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit_polls) : "memory");
+  return ok != 0;
 }
 // one arrival on a barrier of any CTA of the cluster (shared::cluster address)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {

@@ -28,6 +28,16 @@ def test_against_oracle(m, n, dtype, tokens, pack):
     check(codes.cpu()[sample].numpy(), t2f(scales)[sample if isinstance(sample, slice) else sample.numpy()], ref_codes, ref_scales, pack)
 
 
+# row counts that a pair's MMAs (32 rows a step, half from each CTA) pad, and columns of the second CTA from one quadrant to four;
+# a pair with one token, two pairs, one pair more than the device has, and pairs with uneven shares
+PAIR = [(48, 176, "bf16", 2, True), (80, 144, "fp16", 75, True), (112, 256, "bf16", 149, False), (16, 192, "bf16", 74, True), (96, 224, "fp16", 3, True)]
+
+
+@pytest.mark.parametrize("m,n,dtype,tokens,pack", PAIR)
+def test_cta_pairs_against_oracle(m, n, dtype, tokens, pack):
+    test_against_oracle(m, n, dtype, tokens, pack)
+
+
 def test_transform_only_and_dispatch():
     x, left, right = make_inputs(6, 128 * 224, "bf16", 3, True)
     ref = O.kronecker_transform(t2f(x), t2f(left), t2f(right), "bf16").reshape(6, -1)
