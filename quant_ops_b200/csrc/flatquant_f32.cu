@@ -5,18 +5,21 @@
 // tokens, HBM 6 us, so the kernel is built to keep the FMA pipe fed:
 //
 //   * a thread owns an 8 x 8 block of a token's M x N matrix through both products; per step of k it reads 8 + 8 values
-//     from shared memory for 64 FMAs, all as 16-byte loads without bank conflicts (X and Y rows are padded by 16
-//     bytes; a warp's threads are neighbours along N first);
+//     from shared memory for 64 FMAs, all as 16-byte or 8-byte loads without bank conflicts (X and Y rows are padded by 16
+//     bytes; a warp's threads are neighbours along N first), and two neighbouring columns go through one instruction;
 //   * Y overwrites X in shared memory (every Y value is in registers when the last X value has been read), and Z never
 //     leaves the registers: extremes, scale and codes come straight from the accumulators;
-//   * R and L pass through shared memory in chunks of 16 rows, two buffers, cp.async: a CTA needs room for its
-//     tokens' X only, so two CTAs of 256 threads share an SM and one computes while the other loads or quantizes;
-//   * small matrices are batched, as many tokens per CTA as fill its threads (64 x 64: four) unless there are too few
-//     tokens to give every SM two CTAs.
+//   * where R and L fit shared memory beside as many tokens as the SM has registers for (512 threads), they stay there: one CTA
+//     per SM, whose teams of a few warps, with a named barrier each, work on tokens of their own, so that one team computes
+//     while another loads or quantizes;
+//   * otherwise (112 x 128) R and L pass through shared memory in chunks, two buffers, cp.async, with two CTAs per SM.
 //
-// Measured: 77.7 us for 2048 x 4096 to int8 codes in graph replay (the 29 us of multiply-adds are 37 % of that), 158 us for
-// 700 x 14336; the shape-generic kernel takes 257 us for the former.  Bound by the issue slots: 71 % used while an SM is active,
-// for 52 % of the FMA pipe (8192 x 4096; shared-memory reads 32 %).
+// Measured in graph replay, one kernel of the second kind for all shapes with scalar FMAs, groups of four tokens / this: 2048 x
+// 4096 to int8 codes 77.3 / 50.5 us, 8192 x 4096 267 / 190, 8192 x 1024 49.3 / 32, 2000 x 5120 107 / 79, 700 x 11008 148 / 90,
+// 700 x 14336 158 / 129, one token of 4096 17.1 / 11.4.  The multiply-adds alone need 29 us at 2048 x 4096 at 1965 MHz, but
+// FMAs at the full rate draw the clock down (a loop of nothing but outer products fed from shared memory: 1.46 GHz at
+// 128 a cycle and SM, 720 us for what takes 798 us at 98 a cycle and 1.71 GHz with scalar FMAs), to 39 us.  The rest is a
+// token's loads and its codes.  Loading the next token's X under the codes of this one was measured slower (53.0 us).
 //
 // Every sum is one chain of fused multiply-adds in ascending k, as in flatquant_generic.cu: the results are the same
 // bits (reference: src/quant_ops/ops/quantization/flatquant/ops.py:99-117).
@@ -25,8 +28,10 @@
 namespace qo {
 namespace {
 
-constexpr int kChunk = 16;    // rows of R or L per stage
-constexpr int kMaxGroup = 32; // tokens per CTA
+constexpr int kMinChunk = 16; // rows of R or L per stage: this, or twice as many where they fit
+constexpr int kMaxGroup = 32; // tokens per team
+constexpr int kMaxTeams = 15; // named barriers 1 .. 15
+constexpr int kMaxSmem = 220 * 1024;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -44,263 +49,369 @@ __device__ __forceinline__ uint32_t ordered(float f) {
 }
 __device__ __forceinline__ float unordered(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k); }
 
-// quantize_one<float> without a division for values that are not next to a rounding boundary: z * (1/s) is within
-// 2^-21 of round(z / s) relative, which cannot move rint() unless the quotient is within 1e-5 of a half
-// (values that large are clamped anyway).  NaNs and infinities fail the comparison and take the division.
-__device__ __forceinline__ int quantize_f32(float z, float s, float inv_s, bool exact_all) {
-  const float q = z * inv_s, r = rintf(q);
-  if (exact_all || !(fabsf(fabsf(q - r) - 0.5f) > 1e-5f)) return quantize_one<float>(z, s);
-  return (int)fminf(fmaxf(r, -8.f), 7.f);
+// Eight codes, offset binary, a nibble each.  t = z * (1/s) + 1.5 * 2^23 holds rint(z/s) in its low bits and t - 1.5 * 2^23 is it
+// as a float; clamped, four such words add up with weights 1, 16, 256, 4096 to their four nibbles and a constant.  z * (1/s)
+// is within 2^-21 of round(z / s) relative, which cannot move rint() unless the quotient is within 1e-5 of a half (values
+// that large are clamped anyway): such groups of eight, and those with a NaN or an infinity, take the division.
+__device__ __forceinline__ uint32_t quantize8_f32(const float (&z)[8], float s, float inv_s, bool exact_all) {
+  constexpr float kMagic = 12582912.f;                        // 0x4B400000
+  float t[8];
+  bool unsure = exact_all;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    t[j] = fmaf(z[j], inv_s, kMagic);
+    const float d = fmaf(z[j], inv_s, kMagic - t[j]);
+    unsure = unsure || !(fabsf(d) < 0.49999f);
+    t[j] = fminf(fmaxf(t[j], kMagic - 8.f), kMagic + 7.f);
+  }
+  if (unsure) {
+    uint32_t w = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w |= (uint32_t)(quantize_one<float>(z[j], s) + 8) << (4 * j);
+    return w;
+  }
+  constexpr uint32_t kBase = (0x4B400000u - 8u) * 0x1111u;
+  uint32_t w[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float* q = t + 4 * h;
+    w[h] = ((__float_as_uint(q[3]) * 16u + __float_as_uint(q[2])) * 16u + __float_as_uint(q[1])) * 16u + __float_as_uint(q[0]) - kBase;
+  }
+  return w[0] | (w[1] << 16);
 }
 
-// MODE 0: int8 codes, 1: packed codes, 2: transform only (float32 Z written to `codes`)
-template <int MODE, int THREADS>
+// An 8 x 8 block of accumulators, two neighbouring columns to a pair: one instruction multiplies and adds both (each as fmaf
+// does).  The FMA pipe takes as many multiply-adds a cycle either way, but half the issue slots (outer products fed from shared memory,
+// nothing else running: 105 against 96 a cycle and SM).
+typedef unsigned long long Pair;
+struct Block {
+  Pair v[8][4];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[i][j] = 0ull;
+  }
+  // row i += a * (b0, b1)
+  __device__ __forceinline__ void add_row(int i, float a, const ulonglong2& b0, const ulonglong2& b1) {
+    Pair aa;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v[i][0]) : "l"(aa), "l"(b0.x));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v[i][1]) : "l"(aa), "l"(b0.y));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v[i][2]) : "l"(aa), "l"(b1.x));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v[i][3]) : "l"(aa), "l"(b1.y));
+  }
+  __device__ __forceinline__ void row(int i, float (&z)[8]) const {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=f"(z[2 * j]), "=f"(z[2 * j + 1]) : "l"(v[i][j]));
+  }
+  __device__ __forceinline__ void store_row(int i, float* lo, float* hi) const {
+    *reinterpret_cast<ulonglong2*>(lo) = make_ulonglong2(v[i][0], v[i][1]);
+    *reinterpret_cast<ulonglong2*>(hi) = make_ulonglong2(v[i][2], v[i][3]);
+  }
+};
+
+// Y += X . R over kc rows of R (a multiple of 4): rows xa + i * xstep, columns of R at r and r + half
+__device__ __forceinline__ void product_right(Block& acc, const float* xa, int xstep, const float* r, int n, int half, int kc) {
+#pragma unroll 2
+  for (int k = 0; k < kc; k += 2, xa += 2) {
+    float2 a[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float2*>(xa + i * xstep);
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk, r += n) {
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(r), b1 = *reinterpret_cast<const ulonglong2*>(r + half);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc.add_row(i, kk == 0 ? a[i].x : a[i].y, b0, b1);
+    }
+  }
+}
+// Z += L^T . Y over kc rows of both: columns l .. l + 7 of L's rows, columns of Y at y and y + half
+__device__ __forceinline__ void product_left(Block& acc, const float* l, int m8, const float* y, int ldy, int half, int kc) {
+#pragma unroll 4
+  for (int k = 0; k < kc; ++k, l += m8, y += ldy) {
+    const float4 a0 = *reinterpret_cast<const float4*>(l), a1 = *reinterpret_cast<const float4*>(l + 4);
+    const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(y), b1 = *reinterpret_cast<const ulonglong2*>(y + half);
+    const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc.add_row(i, av[i], b0, b1);
+  }
+}
+
+// MODE 0: int8 codes, 1: packed codes, 2: transform only (float32 Z written to `codes`).  RESIDENT: R and L stay in shared memory and
+// the CTA's teams of `team` threads work on their own groups of tokens; otherwise the CTA is one team.
+template <int MODE, int THREADS, bool RESIDENT>
 __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
 flatquant_f32_kernel(const float* __restrict__ x, int64_t ldx, const float* __restrict__ left, const float* __restrict__ right,
-                     void* __restrict__ codes, void* __restrict__ scales, int64_t tokens, int m, int n, int group, float clip,
-                     int scale_dtype) {
+                     void* __restrict__ codes, void* __restrict__ scales, int64_t tokens, int m, int n, int group, int team, int chunk_rows,
+                     float clip, int scale_dtype) {
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
-  __shared__ uint32_t ext[2][kMaxGroup];  // extremes of the CTA's tokens, as ordered integers
-  const int tid = threadIdx.x;
+  __shared__ uint32_t ext_all[kMaxTeams][2][kMaxGroup];  // extremes of the teams' tokens
+  const int which = RESIDENT ? threadIdx.x / team : 0;   // team of this thread (the launch has whole teams only)
+  const int tid = RESIDENT ? threadIdx.x - which * team : threadIdx.x, threads = RESIDENT ? team : blockDim.x;
+  auto sync = [&]() {
+    if (RESIDENT) asm volatile("bar.sync %0, %1;" ::"r"(which + 1), "r"(team) : "memory");
+    else __syncthreads();
+  };
+  uint32_t (&ext)[2][kMaxGroup] = ext_all[which];
   const int nb = n >> 3, mb = (m + 7) >> 3, m8 = mb * 8, ldy = n + 4;
   const int bpt = nb * mb;                // 8 x 8 blocks of a token = threads of a token
   const int cw = n > m8 ? n : m8;
-  float* xs = smem;                       // [group][m][ldy]: X, then Y
-  float* chunk = smem + (size_t)group * m * ldy;  // two buffers of kChunk rows
+  // Shared memory: [team][group][m][ldy] X, then Y; behind it R [n][n] and L [m][m8], or two buffers of chunk_rows rows.  The rows that pad
+  // a token's M to a multiple of 8 are read from what follows it and come to nothing.
+  const int per_team = group * m * ldy;
+  float* xs = smem + (size_t)which * per_team;
+  float* chunk = smem + (size_t)(RESIDENT ? blockDim.x / team : 1) * per_team;
   const int g = tid / bpt, b = tid - g * bpt, ty = b / nb, tx = b - ty * nb;
   const bool worker = g < group;
   float* mine = xs + (size_t)(worker ? g : 0) * m * ldy;
-  const int ca = 4 * tx, cb = (n >> 1) + 4 * tx;  // this thread's columns: ca .. ca + 3 and cb .. cb + 3
+  const int half = n >> 1, ca = 4 * tx, r0 = 8 * ty;  // this thread's columns: ca .. ca + 3 and half + the same; its rows of Z
   const bool l_vec = (m & 7) == 0 && (reinterpret_cast<uintptr_t>(left) & 15) == 0;
   const int64_t feat = (int64_t)m * n;
+  // one running maximum of |z| is enough for a positive clip ratio: max(|min * clip|, max * clip) = max |z| * clip
+  const bool one_sided = clip > 0.f;
 
-  auto load_r = [&](int buf, int k0) {
-    const int rows = min(kChunk, n - k0), pieces = rows * (n >> 2);
+  // rows k0 .. k0 + rows - 1 of R and of L (there m8 wide, zero past m) into dst, by the threads t0, t0 + step, ...
+  auto load_r = [&](float* dst, int k0, int rows, int t0, int step) {
+    const int pieces = rows * (n >> 2);
     const float* src = right + (int64_t)k0 * n;
-    float* dst = chunk + buf * (kChunk * cw);
-    for (int i = tid; i < pieces; i += THREADS) cp_async16(dst + 4 * i, src + 4 * i);
+    for (int i = t0; i < pieces; i += step) cp_async16(dst + 4 * i, src + 4 * i);
   };
-  auto load_l = [&](int buf, int k0) {
-    const int rows = min(kChunk, m - k0);
+  auto load_l = [&](float* dst, int k0, int rows, int t0, int step) {
     const float* src = left + (int64_t)k0 * m;
-    float* dst = chunk + buf * (kChunk * cw);
     if (l_vec) {
       const int pieces = rows * (m >> 2);
-      for (int i = tid; i < pieces; i += THREADS) cp_async16(dst + 4 * i, src + 4 * i);
+      for (int i = t0; i < pieces; i += step) cp_async16(dst + 4 * i, src + 4 * i);
     } else {
-      for (int i = tid; i < rows * m8; i += THREADS) {
+      for (int i = t0; i < rows * m8; i += step) {
         const int k = i / m8, r = i - k * m8;
         cp_async4_zfill(dst + i, src + (r < m ? k * m + r : 0), r < m);
       }
     }
   };
+  float* const r_all = chunk;
+  float* const l_all = chunk + n * n;
+  if (RESIDENT) {
+    load_r(r_all, 0, n, threadIdx.x, blockDim.x);
+    load_l(l_all, 0, m, threadIdx.x, blockDim.x);
+    cp_async_commit();
+    cp_async_wait_all();
+    __syncthreads();
+  }
 
   const int64_t groups = (tokens + group - 1) / group;
-  for (int64_t grp = blockIdx.x; grp < groups; grp += gridDim.x) {
+  const int64_t teams = (int64_t)gridDim.x * (RESIDENT ? blockDim.x / team : 1);
+  for (int64_t grp = blockIdx.x + (int64_t)which * gridDim.x; grp < groups; grp += teams) {
     const int64_t t0 = grp * group;
     const int here = (int)min((int64_t)group, tokens - t0);
-    // X: rows of n floats into rows of ldy
+    // X: rows of n floats into rows of ldy; a thread keeps its column and steps through the rows
     {
-      const int q = n >> 2, per = m * q;
-      for (int i = tid; i < here * per; i += THREADS) {
-        const int tk = i / per, e = i - tk * per, r = e / q, c = e - r * q;
-        cp_async16(xs + ((size_t)tk * m + r) * ldy + 4 * c, x + (t0 + tk) * ldx + (int64_t)r * n + 4 * c);
+      const int q = n >> 2, step = q < threads ? threads / q : 1, row0 = q < threads ? tid / q : 0;
+      for (int tk = 0; tk < here; ++tk) {
+        const float* src = x + (t0 + tk) * ldx;
+        float* dst = xs + (size_t)tk * m * ldy;
+        if (row0 < step)
+          for (int c = tid - row0 * q; c < q; c += threads)
+            for (int r = row0; r < m; r += step) cp_async16(dst + r * ldy + 4 * c, src + r * n + 4 * c);
       }
     }
-    load_r(0, 0);
+    if (!RESIDENT) load_r(chunk, 0, min(chunk_rows, n), tid, threads);
     cp_async_commit();
     if (tid < kMaxGroup) {
-      ext[0][tid] = 0xFFFFFFFFu;
+      ext[0][tid] = one_sided ? 0u : 0xFFFFFFFFu;
       ext[1][tid] = 0u;
     }
     const bool active = worker && g < here;
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    Block acc;
+    acc.clear();
 
     // Y = X . R: rows ty + mb i
     int buf = 0;
-    for (int k0 = 0; k0 < n; k0 += kChunk, buf ^= 1) {
+    if (RESIDENT) {
       cp_async_wait_all();
-      __syncthreads();
-      if (k0 + kChunk < n) load_r(buf ^ 1, k0 + kChunk);
-      else load_l(buf ^ 1, 0);
-      cp_async_commit();
-      if (active) {
-        const float* rc = chunk + buf * (kChunk * cw);
-        const int kc = min(kChunk, n - k0);
-#pragma unroll 1
-        for (int k = 0; k < kc; k += 4) {
-          float4 a[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(mine + min(ty + mb * i, m - 1) * ldy + k0 + k);
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            const float4 b0 = *reinterpret_cast<const float4*>(rc + (k + kk) * n + ca);
-            const float4 b1 = *reinterpret_cast<const float4*>(rc + (k + kk) * n + cb);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const float av = kk == 0 ? a[i].x : (kk == 1 ? a[i].y : (kk == 2 ? a[i].z : a[i].w));
-              acc[i][0] = fmaf(av, b0.x, acc[i][0]);
-              acc[i][1] = fmaf(av, b0.y, acc[i][1]);
-              acc[i][2] = fmaf(av, b0.z, acc[i][2]);
-              acc[i][3] = fmaf(av, b0.w, acc[i][3]);
-              acc[i][4] = fmaf(av, b1.x, acc[i][4]);
-              acc[i][5] = fmaf(av, b1.y, acc[i][5]);
-              acc[i][6] = fmaf(av, b1.z, acc[i][6]);
-              acc[i][7] = fmaf(av, b1.w, acc[i][7]);
-            }
-          }
-        }
+      sync();
+      if (active) product_right(acc, mine + ty * ldy, mb * ldy, r_all + ca, n, half, n);
+    } else {
+      for (int k0 = 0; k0 < n; k0 += chunk_rows, buf ^= 1) {
+        cp_async_wait_all();
+        sync();
+        float* other = chunk + (buf ^ 1) * (chunk_rows * cw);
+        if (k0 + chunk_rows < n) load_r(other, k0 + chunk_rows, min(chunk_rows, n - k0 - chunk_rows), tid, threads);
+        else load_l(other, 0, min(chunk_rows, m), tid, threads);
+        cp_async_commit();
+        if (active) product_right(acc, mine + ty * ldy + k0, mb * ldy, chunk + buf * (chunk_rows * cw) + ca, n, half, min(chunk_rows, n - k0));
       }
     }
-    __syncthreads();  // every X value has been read
+    sync();  // every X value has been read
     if (active) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int r = ty + mb * i;
-        if (r < m) {
-          *reinterpret_cast<float4*>(mine + r * ldy + ca) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-          *reinterpret_cast<float4*>(mine + r * ldy + cb) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
-        }
+        if (r < m) acc.store_row(i, mine + r * ldy + ca, mine + r * ldy + half + ca);
       }
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    acc.clear();
 
-    // Z = L^T . Y: rows 4 ty .. 4 ty + 3 and m8 / 2 + the same
-    const int ra = 4 * ty, rb = (m8 >> 1) + 4 * ty;
-    for (int k0 = 0; k0 < m; k0 += kChunk, buf ^= 1) {
-      cp_async_wait_all();
-      __syncthreads();
-      if (k0 + kChunk < m) {
-        load_l(buf ^ 1, k0 + kChunk);
-        cp_async_commit();
-      }
-      if (active) {
-        const float* lc = chunk + buf * (kChunk * cw);
-        const int kc = min(kChunk, m - k0);
-#pragma unroll 2
-        for (int k = 0; k < kc; ++k) {
-          const float4 a0 = *reinterpret_cast<const float4*>(lc + k * m8 + ra), a1 = *reinterpret_cast<const float4*>(lc + k * m8 + rb);
-          const float4 b0 = *reinterpret_cast<const float4*>(mine + (k0 + k) * ldy + ca), b1 = *reinterpret_cast<const float4*>(mine + (k0 + k) * ldy + cb);
-          const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            acc[i][0] = fmaf(av[i], b0.x, acc[i][0]);
-            acc[i][1] = fmaf(av[i], b0.y, acc[i][1]);
-            acc[i][2] = fmaf(av[i], b0.z, acc[i][2]);
-            acc[i][3] = fmaf(av[i], b0.w, acc[i][3]);
-            acc[i][4] = fmaf(av[i], b1.x, acc[i][4]);
-            acc[i][5] = fmaf(av[i], b1.y, acc[i][5]);
-            acc[i][6] = fmaf(av[i], b1.z, acc[i][6]);
-            acc[i][7] = fmaf(av[i], b1.w, acc[i][7]);
-          }
+    // Z = L^T . Y: rows r0 .. r0 + 7
+    if (RESIDENT) {
+      sync();
+      if (active) product_left(acc, l_all + r0, m8, mine + ca, ldy, half, m);
+    } else {
+      for (int k0 = 0; k0 < m; k0 += chunk_rows, buf ^= 1) {
+        cp_async_wait_all();
+        sync();
+        if (k0 + chunk_rows < m) {
+          load_l(chunk + (buf ^ 1) * (chunk_rows * cw), k0 + chunk_rows, min(chunk_rows, m - k0 - chunk_rows), tid, threads);
+          cp_async_commit();
         }
+        if (active) product_left(acc, chunk + buf * (chunk_rows * cw) + r0, m8, mine + k0 * ldy + ca, ldy, half, min(chunk_rows, m - k0));
       }
     }
 
     const int64_t tok = t0 + g;
+    const int rows = active ? min(8, m - r0) : 0;  // real rows of this thread
     if (MODE == 2) {
-      if (active) {
-        float* z = reinterpret_cast<float*>(codes) + tok * feat;
+      float* z = reinterpret_cast<float*>(codes) + tok * feat + (int64_t)r0 * n + ca;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int r = (i < 4 ? ra : rb) + (i & 3);
-          if (r < m) {
-            *reinterpret_cast<float4*>(z + (int64_t)r * n + ca) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-            *reinterpret_cast<float4*>(z + (int64_t)r * n + cb) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
-          }
-        }
-      }
-      __syncthreads();  // the next group overwrites Y
+      for (int i = 0; i < 8; ++i)
+        if (i < rows) acc.store_row(i, z + i * n, z + i * n + half);
+      sync();  // the next group overwrites Y
       continue;
     }
-    if (active) {
+    if (one_sided) {
+      float top = -1.f;  // (fmaxf skips NaNs; below zero: no value that is a number)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (i < rows) {
+          float z[8];
+          acc.row(i, z);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) top = fmaxf(top, fabsf(z[j]));
+        }
+      }
+      // the lanes of one token first, then one atomic operation for them
+      const unsigned same = __match_any_sync(0xffffffffu, active ? g : kMaxGroup);
+      const uint32_t key = __reduce_max_sync(same, top < 0.f ? 0u : __float_as_uint(top) + 1u);
+      if (active && (tid & 31) == __ffs(same) - 1) atomicMax(&ext[0][g], key);
+    } else if (active) {
       float lmin = 3.4e38f, lmax = -3.4e38f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        if ((i < 4 ? ra : rb) + (i & 3) < m) {
+        if (i < rows) {
+          float z[8];
+          acc.row(i, z);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            lmin = fminf(lmin, acc[i][j]);
-            lmax = fmaxf(lmax, acc[i][j]);
+            lmin = fminf(lmin, z[j]);
+            lmax = fmaxf(lmax, z[j]);
           }
         }
       }
       atomicMin(&ext[0][g], ordered(lmin));
       atomicMax(&ext[1][g], ordered(lmax));
     }
-    __syncthreads();  // also: every Y value has been read, the next group may overwrite it
+    sync();  // also: every Y value has been read, the next group may overwrite it
     if (active) {
-      const float s = token_scale<float>(unordered(ext[0][g]), unordered(ext[1][g]), clip);
+      float zmin, zmax;
+      if (one_sided) {
+        zmax = ext[0][g] == 0u ? 3.4e38f : __uint_as_float(ext[0][g] - 1u);
+        zmin = -zmax;
+      } else {
+        zmin = unordered(ext[0][g]);
+        zmax = unordered(ext[1][g]);
+      }
+      const float s = token_scale<float>(zmin, zmax, clip);
       const float inv_s = __frcp_rn(s);
       const bool exact_all = !(s < 1e37f);  // 1/s would be subnormal
       if (b == 0) store_scale(scales, tok, s, scale_dtype);
+      const int64_t at = tok * feat + (int64_t)r0 * n + ca;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const int r = (i < 4 ? ra : rb) + (i & 3);
-        if (r >= m) continue;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int64_t at = tok * feat + (int64_t)r * n + (h ? cb : ca);
-          int q[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) q[j] = quantize_f32(acc[i][4 * h + j], s, inv_s, exact_all);
+        if (i < rows) {
+          float z[8];
+          acc.row(i, z);
+          const uint32_t w = quantize8_f32(z, s, inv_s, exact_all);  // (the low half: columns ca .. ca + 3)
           if (MODE == 1) {
-            reinterpret_cast<uint16_t*>(codes)[at >> 2] =
-                (uint16_t)((q[0] + 8) | ((q[1] + 8) << 4) | ((q[2] + 8) << 8) | ((q[3] + 8) << 12));
+            uint16_t* dst = reinterpret_cast<uint16_t*>(codes) + ((at + i * n) >> 2);
+            dst[0] = (uint16_t)w;
+            dst[n >> 3] = (uint16_t)(w >> 16);
           } else {
-            reinterpret_cast<char4*>(codes)[at >> 2] = make_char4((char)q[0], (char)q[1], (char)q[2], (char)q[3]);
+            // nibbles to bytes: (even, odd) interleaved, then less 8 per byte without a borrow
+            const uint32_t even = w & 0x0F0F0F0Fu, odd = (w >> 4) & 0x0F0F0F0Fu;
+            const uint32_t lo = __byte_perm(even, odd, 0x5140), hi = __byte_perm(even, odd, 0x7362);
+            uint32_t* dst = reinterpret_cast<uint32_t*>(codes) + ((at + i * n) >> 2);
+            dst[0] = ((lo | 0x80808080u) - 0x08080808u) ^ 0x80808080u;
+            dst[n >> 3] = ((hi | 0x80808080u) - 0x08080808u) ^ 0x80808080u;
           }
         }
       }
     }
-    __syncthreads();  // the extremes are reset by the next group
+    sync();  // the extremes are reset by the next group
   }
 }
 
-template <int MODE, int THREADS>
-int launch_sized(const float* x, int64_t ldx, const float* left, const float* right, void* codes, void* scales, int64_t tokens,
-                 int m, int n, float clip, int scale_dtype, cudaStream_t stream) {
-  auto kern = flatquant_f32_kernel<MODE, THREADS>;
-  constexpr int kSmem = THREADS == 256 ? 112 * 1024 : 200 * 1024;
-  int dev = 0;
-  QO_CUDA_TRY(cudaGetDevice(&dev));
+// The shape of a launch: tokens per team, threads per team, teams per CTA, CTAs per SM, threads with work per SM.
+struct Shape {
+  int group, team, teams, per_sm, busy, chunk_rows;
+  size_t smem;
+};
+
+// A team has whole warps for its tokens' 8 x 8 blocks and an SM the registers of 512 threads: the group that leaves the fewest of those
+// idle, and of several such the smallest, whose last round of groups is shared out best (64 x 64, 2048 tokens: 13.8 per SM;
+// groups of four, two CTAs of 256 threads, take 16).
+Shape shape_of(bool resident, int m, int n, int64_t tokens, int sms, int most_threads, int chunk_rows = 0) {
+  const int mb = (m + 7) / 8, m8 = mb * 8, bpt = mb * (n / 8), cw = n > m8 ? n : m8;
+  const size_t token_bytes = (size_t)m * (n + 4) * 4;
+  const size_t transforms = resident ? ((size_t)n * n + (size_t)m * m8 + 8 * (n + 4)) * 4 : (size_t)2 * chunk_rows * cw * 4;
+  const int64_t share = (tokens + sms - 1) / sms;  // of one SM
+  Shape best = {};
+  for (int g = 1; g <= kMaxGroup && (g == 1 || g <= share); ++g) {
+    const int team = (g * bpt + 31) / 32 * 32;
+    if (team > most_threads || transforms + g * token_bytes > (size_t)kMaxSmem) break;
+    int count = 512 / team;  // teams of an SM
+    const size_t fit = resident ? (kMaxSmem - transforms) / (g * token_bytes) : (size_t)(228 * 1024) / (transforms + g * token_bytes + sizeof(uint32_t) * kMaxTeams * 2 * kMaxGroup + 1024);
+    if ((size_t)count > fit) count = (int)fit;
+    if (resident && count > kMaxTeams) count = kMaxTeams;
+    const int busy = count * g * bpt;
+    if (busy > best.busy)
+      best = {g, team, resident ? count : 1, resident ? 1 : count, busy, chunk_rows, transforms + (resident ? count : 1) * g * token_bytes};
+  }
+  return best;
+}
+
+template <int MODE, int THREADS, bool RESIDENT>
+int launch_sized(const Shape& c, const float* x, int64_t ldx, const float* left, const float* right, void* codes, void* scales, int64_t tokens,
+                 int m, int n, float clip, int scale_dtype, int dev, cudaStream_t stream) {
+  auto kern = flatquant_f32_kernel<MODE, THREADS, RESIDENT>;
   static bool configured[64] = {};
   if (!configured[dev & 63]) {
-    QO_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    QO_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
     configured[dev & 63] = true;
   }
-  const int sms = sm_count(dev), per_sm = THREADS == 256 ? 2 : 1;
-  const int mb = (m + 7) / 8, bpt = mb * (n / 8), cw = n > mb * 8 ? n : mb * 8;
-  const size_t token_bytes = (size_t)m * (n + 4) * 4, chunk_bytes = (size_t)2 * kChunk * cw * 4;
-  // tokens per CTA: as many as fill its threads and fit, but no more than it takes to give every SM its CTAs
-  int group = THREADS / bpt;
-  if (group > kMaxGroup) group = kMaxGroup;
-  while (group > 1 && group * token_bytes + chunk_bytes > (size_t)kSmem) --group;
-  const int64_t spread = (tokens + (int64_t)sms * per_sm - 1) / ((int64_t)sms * per_sm);
-  if (spread < group) group = (int)spread;
-  const size_t smem = group * token_bytes + chunk_bytes;
-  const int64_t groups = (tokens + group - 1) / group;
-  const int grid = (int)(groups < (int64_t)sms * per_sm ? groups : (int64_t)sms * per_sm);
-  kern<<<grid, THREADS, smem, stream>>>(x, ldx, left, right, codes, scales, tokens, m, n, group, clip, scale_dtype);
+  // (resident: a CTA for every group as long as there are SMs, its other teams idle, then a second group for every CTA, ...)
+  const int64_t groups = (tokens + c.group - 1) / c.group, room = (int64_t)sm_count(dev) * c.per_sm;
+  kern<<<(unsigned)(groups < room ? groups : room), c.team * c.teams, c.smem, stream>>>(x, ldx, left, right, codes, scales, tokens, m, n, c.group, c.team,
+                                                                                       c.chunk_rows, clip, scale_dtype);
   return check_launch("flatquant_f32_kernel");
 }
 
-template <int THREADS>
-int launch_mode(int mode, const float* x, int64_t ldx, const float* left, const float* right, void* codes, void* scales,
-                int64_t tokens, int m, int n, float clip, int scale_dtype, cudaStream_t stream) {
-  switch (mode) {
-    case 0: return launch_sized<0, THREADS>(x, ldx, left, right, codes, scales, tokens, m, n, clip, scale_dtype, stream);
-    case 1: return launch_sized<1, THREADS>(x, ldx, left, right, codes, scales, tokens, m, n, clip, scale_dtype, stream);
-    default: return launch_sized<2, THREADS>(x, ldx, left, right, codes, scales, tokens, m, n, clip, scale_dtype, stream);
-  }
+template <int MODE>
+int launch_mode(const float* x, int64_t ldx, const float* left, const float* right, void* codes, void* scales, int64_t tokens, int m, int n,
+                float clip, int scale_dtype, cudaStream_t stream) {
+  int dev = 0;
+  QO_CUDA_TRY(cudaGetDevice(&dev));
+  const int bpt = ((m + 7) / 8) * (n / 8), sms = sm_count(dev);
+  const int most = bpt <= 256 ? 256 : 512;
+  // (longer chunks mean fewer barriers: 700 x 14336 133 / 128 us; on kMinChunk alone what this kernel takes depends)
+  Shape stream_shape = shape_of(false, m, n, tokens, sms, most, 2 * kMinChunk);
+  const Shape shorter = shape_of(false, m, n, tokens, sms, most, kMinChunk), resident = shape_of(true, m, n, tokens, sms, 512);
+  if (shorter.busy > stream_shape.busy) stream_shape = shorter;
+  if (resident.busy >= stream_shape.busy)
+    return launch_sized<MODE, 512, true>(resident, x, ldx, left, right, codes, scales, tokens, m, n, clip, scale_dtype, dev, stream);
+  if (bpt <= 256)
+    return launch_sized<MODE, 256, false>(stream_shape, x, ldx, left, right, codes, scales, tokens, m, n, clip, scale_dtype, dev, stream);
+  return launch_sized<MODE, 512, false>(stream_shape, x, ldx, left, right, codes, scales, tokens, m, n, clip, scale_dtype, dev, stream);
 }
 
 }  // namespace
@@ -309,7 +420,7 @@ int launch_mode(int mode, const float* x, int64_t ldx, const float* left, const 
 // buffers of M N floats in 200 KB), so that what that kernel refuses stays refused
 bool flatquant_f32_supported(int64_t ldx, int m, int n, const void* x, const void* right, const void* codes) {
   return (n % 8) == 0 && (int64_t)m * n * 8 <= 200 * 1024 && ((m + 7) / 8) * (n / 8) <= 512 &&
-         (size_t)m * (n + 4) * 4 + (size_t)2 * kChunk * (n > m + 7 ? n : m + 7) * 4 <= 200 * 1024 && (ldx % 4) == 0 &&
+         (size_t)m * (n + 4) * 4 + (size_t)2 * kMinChunk * (n > m + 7 ? n : m + 7) * 4 <= 200 * 1024 && (ldx % 4) == 0 &&
          reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(right) % 16 == 0 &&
          reinterpret_cast<uintptr_t>(codes) % 16 == 0;
 }
@@ -339,10 +450,11 @@ int launch_flatquant_f32(int mode, const void* x, int64_t ldx, const void* left,
   const float* xf = reinterpret_cast<const float*>(x);
   const float* lf = reinterpret_cast<const float*>(left);
   const float* rf = reinterpret_cast<const float*>(right);
-  const int bpt = ((m + 7) / 8) * (n / 8);
-  const size_t one = (size_t)m * (n + 4) * 4 + (size_t)2 * kChunk * (n > m + 7 ? n : m + 7) * 4;
-  if (bpt <= 256 && one <= 112 * 1024) return launch_mode<256>(mode, xf, ldx, lf, rf, codes, scales, tokens, m, n, clip, scale_dtype, stream);
-  return launch_mode<512>(mode, xf, ldx, lf, rf, codes, scales, tokens, m, n, clip, scale_dtype, stream);
+  switch (mode) {
+    case 0: return launch_mode<0>(xf, ldx, lf, rf, codes, scales, tokens, m, n, clip, scale_dtype, stream);
+    case 1: return launch_mode<1>(xf, ldx, lf, rf, codes, scales, tokens, m, n, clip, scale_dtype, stream);
+    default: return launch_mode<2>(xf, ldx, lf, rf, codes, scales, tokens, m, n, clip, scale_dtype, stream);
+  }
 }
 
 }  // namespace qo

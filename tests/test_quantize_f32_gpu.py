@@ -98,3 +98,20 @@ def test_route_and_bits_at_the_lines(m, n, tokens, pack, tiled):
     assert torch.equal(got[0], ref[0]) and torch.equal(got[1].view(torch.int32), ref[1].view(torch.int32))
     names = launched_kernels(lambda: q.flatquant_dynamic_quantize(x, left, right, 0.9, pack))
     assert len(names) == 1 and ("flatquant_f32_kernel" if tiled else "flatquant_generic_kernel") in names[0]
+
+
+# transforms kept in shared memory (teams of one or more tokens, some without any) and streamed, in long chunks and in short ones;
+# a clip ratio that is not positive needs both extremes, and signs and ties at the limits of the codes
+@pytest.mark.parametrize("m,n,tokens,clip", [(64, 64, 3, -0.7), (32, 32, 700, 0.0), (48, 64, 1483, 1.7), (61, 72, 299, 0.9), (64, 128, 149, -1.0),
+                                             (112, 128, 5, -0.7), (9, 1000, 150, 0.9), (128, 192, 3, 1.0)])
+@pytest.mark.parametrize("pack", [True, False])
+def test_teams_chunks_and_clip_ratios(m, n, tokens, clip, pack):
+    x, left, right = (t.to(DEV) for t in make_inputs(tokens, m * n, "fp32", 5 * m + n + tokens, True, mn=(m, n)))
+    x[0] = 3e38
+    x[1, ::2] = -float("inf")
+    x[2] = float("nan")
+    ref = abi_quantize(x, left, right, clip, pack, "fp32", policy=1)
+    names = launched_kernels(lambda: q.flatquant_dynamic_quantize(x, left, right, clip, pack))
+    got = abi_quantize(x, left, right, clip, pack, "fp32", policy=0)
+    assert torch.equal(got[0], ref[0]) and torch.equal(got[1].view(torch.int32), ref[1].view(torch.int32))
+    assert m * n < 3072 or "flatquant_f32_kernel" in names[0]
