@@ -87,7 +87,7 @@ def build_torch_binding(verbose: bool = False) -> str:
            "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            *[f"-isystem{i}" for i in incs], src, "-o", out,
            f"-L{PKG}", "-l:libquant_ops_b200.so", "-Wl,-rpath,$ORIGIN",
-           f"-L{torch_lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", f"-Wl,-rpath,{torch_lib}"]
+           f"-L{torch_lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-ltorch", f"-Wl,-rpath,{torch_lib}"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode:
         raise RuntimeError("g++ failed for torch_binding.cpp:\n" + res.stdout + res.stderr)

@@ -6,8 +6,15 @@
 //   quant_ops::int4_matmul                 src/quant_ops/ops/quantization/int4_matmul/kernels/cuda_int4_matmul_kernel.cu:207-214
 // Only the CUDA dispatch key gets an implementation: CPU tensors raise, there is no fallback.
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/core/dispatch/Dispatcher.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
 #include <tuple>
@@ -37,6 +44,13 @@ at::Tensor row_major(const at::Tensor& t) {
   return t.contiguous();
 }
 
+// an output or a workspace on the device of `like` (the guard is set, so the allocator is asked without another dispatch)
+at::Tensor empty_like_device(at::IntArrayRef sizes, at::ScalarType dtype, const at::Tensor& like) {
+  return at::Tensor(at::detail::empty_cuda(sizes, dtype, like.device(), c10::nullopt));
+}
+// one value per row or channel, as a contiguous vector; a contiguous vector is taken as it is
+at::Tensor as_vector(const at::Tensor& t) { return t.dim() == 1 && t.is_contiguous() ? t : t.reshape({-1}).contiguous(); }
+
 // scale_dtype: dtype of the returned per-token scales; float32 (what the reference's CUDA op returns) when absent
 std::tuple<at::Tensor, at::Tensor> flatquant_dynamic_quantize_ex(const at::Tensor& input, const at::Tensor& left_trans,
                                                                  const at::Tensor& right_trans, double clip_ratio,
@@ -62,9 +76,8 @@ std::tuple<at::Tensor, at::Tensor> flatquant_dynamic_quantize_ex(const at::Tenso
   x2 = row_major(x2);
   at::Tensor left = left_trans.contiguous(), right = right_trans.contiguous();
   const int64_t tokens = x2.size(0);
-  at::Tensor codes = pack_int32 ? at::empty({tokens, features / 8}, input.options().dtype(at::kInt))
-                                : at::empty({tokens, features}, input.options().dtype(at::kChar));
-  at::Tensor scales = at::empty({tokens}, input.options().dtype(scale_dtype));
+  at::Tensor codes = pack_int32 ? empty_like_device({tokens, features / 8}, at::kInt, input) : empty_like_device({tokens, features}, at::kChar, input);
+  at::Tensor scales = empty_like_device({tokens}, scale_dtype, input);
   check_status(qo_flatquant_quantize(x2.data_ptr(), tokens > 1 ? x2.stride(0) : features, left.data_ptr(),
                                      right.data_ptr(), codes.data_ptr(), scales.data_ptr(), tokens, (int)m, (int)n,
                                      (float)clip_ratio, dt, pack_int32 ? 1 : 0, sdt, current_stream()),
@@ -78,9 +91,8 @@ std::tuple<at::Tensor, at::Tensor> flatquant_dynamic_quantize(const at::Tensor& 
   return flatquant_dynamic_quantize_ex(input, left_trans, right_trans, clip_ratio, pack_int32, c10::nullopt);
 }
 
-std::tuple<at::Tensor, at::Tensor> int4_matmul_ex(const at::Tensor& a, const at::Tensor& b, const at::Tensor& scale_a,
-                                                  const at::Tensor& scale_b, at::ScalarType out_dtype,
-                                                  bool return_acc) {
+std::tuple<at::Tensor, at::Tensor> matmul(const at::Tensor& a, const at::Tensor& b, const at::Tensor& scale_a, const at::Tensor& scale_b,
+                                          at::ScalarType out_dtype, bool return_acc) {
   TORCH_CHECK(a.is_cuda(), "a_packed must be on CUDA");
   TORCH_CHECK(b.is_cuda(), "b_packed must be on CUDA");
   TORCH_CHECK(scale_a.is_cuda(), "scale_a must be on CUDA");
@@ -99,23 +111,30 @@ std::tuple<at::Tensor, at::Tensor> int4_matmul_ex(const at::Tensor& a, const at:
   at::Tensor a2 = row_major(a);
   // b may be the canonical [K/8, N] layout or the transposed view of a [N, K/8] weight; both go through as strides
   at::Tensor b2 = (b.stride(0) == 1 || b.stride(1) == 1 || b.numel() == 0) ? b : b.contiguous();
-  at::Tensor sa = scale_a.reshape({-1}).contiguous(), sb = scale_b.reshape({-1}).contiguous();
-  at::Tensor out = at::empty({t, n}, a.options().dtype(out_dtype));
-  at::Tensor acc = return_acc ? at::empty({t, n}, a.options().dtype(at::kInt)) : at::Tensor();
+  at::Tensor sa = as_vector(scale_a), sb = as_vector(scale_b);
+  at::Tensor out = empty_like_device({t, n}, out_dtype, a);
+  at::Tensor acc = return_acc ? empty_like_device({t, n}, at::kInt, a) : at::Tensor();
   const size_t ws_bytes = qo_int4_matmul_workspace_bytes(t, kp * 8, n);
-  at::Tensor ws = at::empty({(int64_t)ws_bytes}, a.options().dtype(at::kByte));
+  at::Tensor ws = ws_bytes ? empty_like_device({(int64_t)ws_bytes}, at::kByte, a) : at::Tensor();
   check_status(qo_int4_matmul(a2.data_ptr<int32_t>(), t > 1 ? a2.stride(0) : kp, b2.data_ptr<int32_t>(), b2.stride(0),
                               b2.stride(1), sa.data_ptr<float>(), sb.data_ptr<float>(), out.data_ptr(),
                               out_dtype == at::kHalf ? QO_F16 : QO_BF16, t, kp * 8, n,
                               return_acc ? acc.data_ptr<int32_t>() : nullptr, ws_bytes ? ws.data_ptr() : nullptr, ws_bytes,
                               current_stream()),
                "int4_matmul");
-  if (!return_acc) acc = at::empty({0}, a.options().dtype(at::kInt));
   return {out, acc};
 }
 
+std::tuple<at::Tensor, at::Tensor> int4_matmul_ex(const at::Tensor& a, const at::Tensor& b, const at::Tensor& scale_a,
+                                                  const at::Tensor& scale_b, at::ScalarType out_dtype,
+                                                  bool return_acc) {
+  std::tuple<at::Tensor, at::Tensor> r = matmul(a, b, scale_a, scale_b, out_dtype, return_acc);
+  if (!return_acc) std::get<1>(r) = at::empty({0}, a.options().dtype(at::kInt));
+  return r;
+}
+
 at::Tensor int4_matmul(const at::Tensor& a, const at::Tensor& b, const at::Tensor& scale_a, const at::Tensor& scale_b) {
-  return std::get<0>(int4_matmul_ex(a, b, scale_a, scale_b, at::kHalf, false));
+  return std::get<0>(matmul(a, b, scale_a, scale_b, at::kHalf, false));
 }
 
 at::Tensor dequantize_int4(const at::Tensor& quantized, const at::Tensor& scales, bool packed_int32) {
@@ -127,8 +146,8 @@ at::Tensor dequantize_int4(const at::Tensor& quantized, const at::Tensor& scales
   TORCH_CHECK(scales.numel() == tokens, "dequantize_int4: one scale per token expected");
   const int sdt = to_qo_dtype(scales.scalar_type(), "scales");
   c10::cuda::CUDAGuard guard(quantized.device());
-  at::Tensor q = quantized.contiguous(), s = scales.reshape({-1}).contiguous();
-  at::Tensor out = at::empty({tokens, features}, quantized.options().dtype(at::kFloat));
+  at::Tensor q = quantized.contiguous(), s = as_vector(scales);
+  at::Tensor out = empty_like_device({tokens, features}, at::kFloat, quantized);
   check_status(qo_dequantize_int4(q.data_ptr(), s.data_ptr(), out.data_ptr<float>(), tokens, features,
                                   packed_int32 ? 1 : 0, sdt, current_stream()),
                "dequantize_int4");
@@ -154,16 +173,16 @@ at::Tensor w4a4_linear(const at::Tensor& x, const at::Tensor& left_trans, const 
   const int dt = to_qo_dtype(x.scalar_type(), "x");
   c10::cuda::CUDAGuard guard(x.device());
   at::Tensor x2 = row_major(x), left = left_trans.contiguous(), right = right_trans.contiguous();
-  at::Tensor w = w_packed.contiguous(), ws_ = w_scale.reshape({-1}).contiguous();
+  at::Tensor w = w_packed.contiguous(), ws_ = as_vector(w_scale);
   at::Tensor b;
   if (bias.has_value() && bias->defined()) {
     TORCH_CHECK(bias->numel() == w.size(0), "w4a4_linear: bias must have n_out elements");
-    b = bias->to(out_dtype).contiguous();
+    b = bias->scalar_type() == out_dtype ? bias->contiguous() : bias->to(out_dtype).contiguous();
   }
   const int64_t tokens = x2.size(0), n_out = w.size(0);
-  at::Tensor out = at::empty({tokens, n_out}, x.options().dtype(out_dtype));
+  at::Tensor out = empty_like_device({tokens, n_out}, out_dtype, x);
   const size_t ws_bytes = qo_w4a4_linear_workspace_bytes(tokens, k, n_out);
-  at::Tensor ws = at::empty({(int64_t)ws_bytes}, x.options().dtype(at::kByte));
+  at::Tensor ws = ws_bytes ? empty_like_device({(int64_t)ws_bytes}, at::kByte, x) : at::Tensor();
   check_status(qo_w4a4_linear(x2.data_ptr(), tokens > 1 ? x2.stride(0) : k, left.data_ptr(), right.data_ptr(),
                               w.data_ptr<int32_t>(), ws_.data_ptr<float>(), b.defined() ? b.data_ptr() : nullptr,
                               out.data_ptr(), tokens, (int)m, (int)n, n_out, (float)clip_ratio, dt,
@@ -207,16 +226,16 @@ at::Tensor w4a4_linear_prepared(const at::Tensor& x, const at::Tensor& left_tran
   const int dt = to_qo_dtype(x.scalar_type(), "x");
   c10::cuda::CUDAGuard guard(x.device());
   at::Tensor x2 = row_major(x), left = left_trans.contiguous(), right = right_trans.contiguous();
-  at::Tensor w = w_packed.contiguous(), ws_ = w_scale.reshape({-1}).contiguous();
+  at::Tensor w = w_packed.contiguous(), ws_ = as_vector(w_scale);
   at::Tensor b;
   if (bias.has_value() && bias->defined()) {
     TORCH_CHECK(bias->numel() == w.size(0), "w4a4_linear_prepared: bias must have n_out elements");
-    b = bias->to(out_dtype).contiguous();
+    b = bias->scalar_type() == out_dtype ? bias->contiguous() : bias->to(out_dtype).contiguous();
   }
   const int64_t tokens = x2.size(0), n_out = w.size(0);
-  at::Tensor out = at::empty({tokens, n_out}, x.options().dtype(out_dtype));
+  at::Tensor out = empty_like_device({tokens, n_out}, out_dtype, x);
   const size_t ws_bytes = qo_w4a4_linear_prepared_workspace_bytes(tokens, k, n_out);
-  at::Tensor ws = at::empty({(int64_t)ws_bytes}, x.options().dtype(at::kByte));
+  at::Tensor ws = ws_bytes ? empty_like_device({(int64_t)ws_bytes}, at::kByte, x) : at::Tensor();
   check_status(qo_w4a4_linear_prepared(x2.data_ptr(), tokens > 1 ? x2.stride(0) : k, left.data_ptr(), right.data_ptr(),
                                        w.data_ptr<int32_t>(), w_prepared.data_ptr(), ws_.data_ptr<float>(),
                                        b.defined() ? b.data_ptr() : nullptr, out.data_ptr(), tokens, (int)m, (int)n, n_out,
@@ -258,6 +277,153 @@ std::tuple<at::Tensor, at::Tensor> quantize_weights_int4(const at::Tensor& w) {
   return {packed, scale};
 }
 
+// ---- direct calls ------------------------------------------------------------------------------------------------------
+// torch.ops parses its arguments against the schema, boxes them and, without an autograd kernel, passes them boxed through the
+// autograd fallback: about 5 us of a decode-sized layer's 13.4, whose two launches take 4.9.  These functions unpack the arguments
+// of the Python layer and call the same operators through the dispatcher, unboxed, so that modes, transforms, tracing, the
+// profiler and other registrations see them as before.  They return NotImplemented where Python has a say that the
+// dispatcher does not know of (tensor subclasses, __torch_function__ modes) and for anything that is not a tensor where one is expected;
+// the caller then goes through torch.ops.
+using TensorRef = const at::Tensor&;
+using OptTensor = const c10::optional<at::Tensor>&;
+using OptType = c10::optional<at::ScalarType>;
+
+template <typename Sig>
+c10::TypedOperatorHandle<Sig> find_op(const char* name) {
+  return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<Sig>();
+}
+
+struct Args {
+  PyObject* const* v;
+  bool wants_grad = false;  // some input asks for a gradient: the autograd fallback has to see the call
+  bool tensor(int i) {
+    if (!THPVariable_CheckExact(v[i])) return false;
+    wants_grad = wants_grad || THPVariable_Unpack(v[i]).requires_grad();
+    return true;
+  }
+  bool tensor_or_none(int i) { return v[i] == Py_None || tensor(i); }
+  bool type(int i) const { return THPDtype_Check(v[i]); }
+  bool type_or_none(int i) const { return v[i] == Py_None || THPDtype_Check(v[i]); }
+  TensorRef get(int i) const { return THPVariable_Unpack(v[i]); }
+  c10::optional<at::Tensor> get_optional(int i) const { return v[i] == Py_None ? c10::optional<at::Tensor>() : THPVariable_Unpack(v[i]); }
+  at::ScalarType get_type(int i) const { return reinterpret_cast<THPDtype*>(v[i])->scalar_type; }
+  OptType get_optional_type(int i) const { return v[i] == Py_None ? OptType() : OptType(get_type(i)); }
+};
+
+// calls with the GIL released, below autograd where no gradient is asked for
+template <typename F>
+auto call_op(const Args& a, F f) {
+  pybind11::gil_scoped_release no_gil;
+  if (a.wants_grad && at::GradMode::is_enabled()) return f();
+  at::AutoDispatchBelowADInplaceOrView below;
+  return f();
+}
+
+bool direct_ok(Py_ssize_t given, Py_ssize_t wanted) { return given == wanted && !at::impl::torch_function_mode_enabled(); }
+
+PyObject* not_implemented() { Py_RETURN_NOTIMPLEMENTED; }
+
+PyObject* wrap_pair(std::tuple<at::Tensor, at::Tensor>&& r) {
+  PyObject* first = THPVariable_Wrap(std::get<0>(std::move(r)));
+  PyObject* second = first ? THPVariable_Wrap(std::get<1>(std::move(r))) : nullptr;
+  PyObject* pair = second ? PyTuple_New(2) : nullptr;
+  if (!pair) {
+    Py_XDECREF(first);
+    Py_XDECREF(second);
+    return nullptr;
+  }
+  PyTuple_SET_ITEM(pair, 0, first);
+  PyTuple_SET_ITEM(pair, 1, second);
+  return pair;
+}
+
+// (input, left_trans, right_trans, clip_ratio: float, pack_int32: bool)
+PyObject* py_quantize(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{v};
+  if (!direct_ok(n, 5) || !a.tensor(0) || !a.tensor(1) || !a.tensor(2) || !PyFloat_CheckExact(v[3]) || !PyBool_Check(v[4])) return not_implemented();
+  static const auto op = find_op<std::tuple<at::Tensor, at::Tensor>(TensorRef, TensorRef, TensorRef, double, bool)>("quant_ops::flatquant_dynamic_quantize");
+  const double clip = PyFloat_AS_DOUBLE(v[3]);
+  const bool pack = v[4] == Py_True;
+  return wrap_pair(call_op(a, [&] { return op.call(a.get(0), a.get(1), a.get(2), clip, pack); }));
+  END_HANDLE_TH_ERRORS
+}
+
+// (a_packed, b_packed, scale_a, scale_b)
+PyObject* py_matmul(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{v};
+  if (!direct_ok(n, 4) || !a.tensor(0) || !a.tensor(1) || !a.tensor(2) || !a.tensor(3)) return not_implemented();
+  static const auto op = find_op<at::Tensor(TensorRef, TensorRef, TensorRef, TensorRef)>("quant_ops::int4_matmul");
+  return THPVariable_Wrap(call_op(a, [&] { return op.call(a.get(0), a.get(1), a.get(2), a.get(3)); }));
+  END_HANDLE_TH_ERRORS
+}
+
+// (a_packed, b_packed, scale_a, scale_b, out_dtype): the output only
+PyObject* py_matmul_typed(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{v};
+  if (!direct_ok(n, 5) || !a.tensor(0) || !a.tensor(1) || !a.tensor(2) || !a.tensor(3) || !a.type(4)) return not_implemented();
+  static const auto op =
+      find_op<std::tuple<at::Tensor, at::Tensor>(TensorRef, TensorRef, TensorRef, TensorRef, at::ScalarType, bool)>("quant_ops::int4_matmul_ex");
+  return THPVariable_Wrap(std::get<0>(call_op(a, [&] { return op.call(a.get(0), a.get(1), a.get(2), a.get(3), a.get_type(4), false); })));
+  END_HANDLE_TH_ERRORS
+}
+
+// (quantized, scales, packed_int32: bool)
+PyObject* py_dequantize(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{v};
+  if (!direct_ok(n, 3) || !a.tensor(0) || !a.tensor(1) || !PyBool_Check(v[2])) return not_implemented();
+  static const auto op = find_op<at::Tensor(TensorRef, TensorRef, bool)>("quant_ops::dequantize_int4");
+  const bool packed = v[2] == Py_True;
+  return THPVariable_Wrap(call_op(a, [&] { return op.call(a.get(0), a.get(1), packed); }));
+  END_HANDLE_TH_ERRORS
+}
+
+// (x, left_trans, right_trans, w_packed, w_scale, bias, clip_ratio: float, out_dtype)
+PyObject* py_linear(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{v};
+  if (!direct_ok(n, 8) || !a.tensor(0) || !a.tensor(1) || !a.tensor(2) || !a.tensor(3) || !a.tensor(4) || !a.tensor_or_none(5) ||
+      !PyFloat_CheckExact(v[6]) || !a.type_or_none(7))
+    return not_implemented();
+  static const auto op =
+      find_op<at::Tensor(TensorRef, TensorRef, TensorRef, TensorRef, TensorRef, OptTensor, double, OptType)>("quant_ops::w4a4_linear");
+  const double clip = PyFloat_AS_DOUBLE(v[6]);
+  const c10::optional<at::Tensor> bias = a.get_optional(5);
+  const OptType type = a.get_optional_type(7);
+  return THPVariable_Wrap(call_op(a, [&] { return op.call(a.get(0), a.get(1), a.get(2), a.get(3), a.get(4), bias, clip, type); }));
+  END_HANDLE_TH_ERRORS
+}
+
+// (x, left_trans, right_trans, w_packed, w_prepared, w_scale, bias, clip_ratio: float, out_dtype)
+PyObject* py_linear_prepared(PyObject*, PyObject* const* v, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{v};
+  if (!direct_ok(n, 9) || !a.tensor(0) || !a.tensor(1) || !a.tensor(2) || !a.tensor(3) || !a.tensor(4) || !a.tensor(5) || !a.tensor_or_none(6) ||
+      !PyFloat_CheckExact(v[7]) || !a.type_or_none(8))
+    return not_implemented();
+  static const auto op =
+      find_op<at::Tensor(TensorRef, TensorRef, TensorRef, TensorRef, TensorRef, TensorRef, OptTensor, double, OptType)>("quant_ops::w4a4_linear_prepared");
+  const double clip = PyFloat_AS_DOUBLE(v[7]);
+  const c10::optional<at::Tensor> bias = a.get_optional(6);
+  const OptType type = a.get_optional_type(8);
+  return THPVariable_Wrap(call_op(a, [&] { return op.call(a.get(0), a.get(1), a.get(2), a.get(3), a.get(4), a.get(5), bias, clip, type); }));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef kMethods[] = {
+    {"flatquant_dynamic_quantize", (PyCFunction)(void (*)(void))&py_quantize, METH_FASTCALL, nullptr},
+    {"int4_matmul", (PyCFunction)(void (*)(void))&py_matmul, METH_FASTCALL, nullptr},
+    {"int4_matmul_typed", (PyCFunction)(void (*)(void))&py_matmul_typed, METH_FASTCALL, nullptr},
+    {"dequantize_int4", (PyCFunction)(void (*)(void))&py_dequantize, METH_FASTCALL, nullptr},
+    {"w4a4_linear", (PyCFunction)(void (*)(void))&py_linear, METH_FASTCALL, nullptr},
+    {"w4a4_linear_prepared", (PyCFunction)(void (*)(void))&py_linear_prepared, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_torch_binding", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
 }  // namespace
 
 TORCH_LIBRARY(quant_ops, m) {
@@ -287,3 +453,6 @@ TORCH_LIBRARY_IMPL(quant_ops, CUDA, m) {
   m.impl("unpack_int4", &unpack_int4);
   m.impl("quantize_weights_int4", &quantize_weights_int4);
 }
+
+// the same file is loaded as the library of the operators above and imported as quant_ops_b200._torch_binding
+PyMODINIT_FUNC PyInit__torch_binding(void) { return PyModule_Create(&kModule); }

@@ -15,6 +15,8 @@ import torch
 from . import ops
 from .decompose import get_decompose_dim
 
+_direct = ops._direct
+_is_dynamo_compiling = torch.compiler.is_dynamo_compiling
 _w4a4_linear = torch.ops.quant_ops.w4a4_linear.default
 _w4a4_linear_prepared = torch.ops.quant_ops.w4a4_linear_prepared.default
 
@@ -83,8 +85,11 @@ class W4A4Linear(torch.nn.Module):
         if dtype != left.dtype:
             raise RuntimeError(f"input dtype {dtype} does not match the transforms' dtype {left.dtype}")
         out_dtype = dtype if dtype == torch.bfloat16 else torch.float16
-        if self.weight_int8 is not None:
-            y = _w4a4_linear_prepared(x2, left, right, w, self.weight_int8, ws, bias, float(self.clip_ratio), out_dtype)
-        else:
-            y = _w4a4_linear(x2, left, right, w, ws, bias, float(self.clip_ratio), out_dtype)
+        clip, copy, y = float(self.clip_ratio), self.weight_int8, NotImplemented
+        if not _is_dynamo_compiling():  # (see ops.py: the same operators, called without boxing)
+            y = (_direct.w4a4_linear(x2, left, right, w, ws, bias, clip, out_dtype) if copy is None else
+                 _direct.w4a4_linear_prepared(x2, left, right, w, copy, ws, bias, clip, out_dtype))
+        if y is NotImplemented:
+            y = (_w4a4_linear(x2, left, right, w, ws, bias, clip, out_dtype) if copy is None else
+                 _w4a4_linear_prepared(x2, left, right, w, copy, ws, bias, clip, out_dtype))
         return y if x2 is x else y.reshape(*x.shape[:-1], self.out_features)

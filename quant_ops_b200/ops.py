@@ -15,7 +15,12 @@ import torch
 from . import _native
 
 _native.load_torch_binding()
+from . import _torch_binding as _direct  # noqa: E402  (the library just loaded, as a module)
+
 _ops = torch.ops.quant_ops
+_is_dynamo_compiling = torch.compiler.is_dynamo_compiling
+# Functions of _direct call the operators of _ops without boxing their arguments, and return NotImplemented for arguments that
+# need torch.ops (tensor subclasses, __torch_function__ modes, wrong types).  torch.compile and torch.jit.script see torch.ops only.
 
 
 def flatquant_dynamic_quantize(input_tensor: torch.Tensor, left_trans: torch.Tensor, right_trans: torch.Tensor,
@@ -28,6 +33,10 @@ def flatquant_dynamic_quantize(input_tensor: torch.Tensor, left_trans: torch.Ten
     the input dtype already (float16 scales of bfloat16 inputs are rounded once more).
     """
     if scale_dtype is None:
+        if not _is_dynamo_compiling():
+            out = _direct.flatquant_dynamic_quantize(input_tensor, left_trans, right_trans, float(clip_ratio), bool(pack_int32))
+            if out is not NotImplemented:
+                return out
         return _ops.flatquant_dynamic_quantize(input_tensor, left_trans, right_trans, float(clip_ratio), bool(pack_int32))
     return _ops.flatquant_dynamic_quantize_ex(input_tensor, left_trans, right_trans, float(clip_ratio), bool(pack_int32), scale_dtype)
 
@@ -53,12 +62,26 @@ def flatquant_cuda(input_tensor, left_trans, right_trans, clip_ratio: float = 1.
 
 def dequantize_int4(quantized: torch.Tensor, scales: torch.Tensor, packed_int32: bool = False) -> torch.Tensor:
     """codes * per-token scale as float32 [tokens, features]."""
-    return _ops.dequantize_int4(quantized, scales, bool(packed_int32))
+    if torch.jit.is_scripting():
+        return _ops.dequantize_int4(quantized, scales, bool(packed_int32))
+    else:
+        if not _is_dynamo_compiling():
+            out = _direct.dequantize_int4(quantized, scales, bool(packed_int32))
+            if out is not NotImplemented:
+                return out
+        return _ops.dequantize_int4(quantized, scales, bool(packed_int32))
 
 
 def int4_matmul(a_packed: torch.Tensor, b_packed: torch.Tensor, scale_a: torch.Tensor, scale_b: torch.Tensor) -> torch.Tensor:
     """[T, K/8] x [K/8, N] packed int4 -> float16 [T, N] = (int32 acc * scale_a[row]) * scale_b[col]."""
-    return _ops.int4_matmul(a_packed, b_packed, scale_a, scale_b)
+    if torch.jit.is_scripting():
+        return _ops.int4_matmul(a_packed, b_packed, scale_a, scale_b)
+    else:
+        if not _is_dynamo_compiling():
+            out = _direct.int4_matmul(a_packed, b_packed, scale_a, scale_b)
+            if out is not NotImplemented:
+                return out
+        return _ops.int4_matmul(a_packed, b_packed, scale_a, scale_b)
 
 
 def int4_matmul_cuda(a_packed, b_packed, scale_a, scale_b):
@@ -69,6 +92,10 @@ def int4_matmul_cuda(a_packed, b_packed, scale_a, scale_b):
 def int4_matmul_ex(a_packed, b_packed, scale_a, scale_b, out_dtype: torch.dtype = torch.float16,
                    return_accumulators: bool = False):
     """int4_matmul with a choice of output dtype (float16 / bfloat16) and optional raw int32 accumulators."""
+    if not return_accumulators and not _is_dynamo_compiling():
+        out = _direct.int4_matmul_typed(a_packed, b_packed, scale_a, scale_b, out_dtype)
+        if out is not NotImplemented:
+            return out
     out, acc = _ops.int4_matmul_ex(a_packed, b_packed, scale_a, scale_b, out_dtype, bool(return_accumulators))
     return (out, acc) if return_accumulators else out
 
@@ -77,7 +104,14 @@ def w4a4_linear(x: torch.Tensor, left_trans: torch.Tensor, right_trans: torch.Te
                 w_scale: torch.Tensor, bias: Optional[torch.Tensor] = None, clip_ratio: float = 1.0,
                 out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """Fused quantize -> int4 GEMM.  w_packed is [n_out, K/8] (K contiguous), w_scale float32 [n_out]."""
-    return _ops.w4a4_linear(x, left_trans, right_trans, w_packed, w_scale, bias, float(clip_ratio), out_dtype)
+    if torch.jit.is_scripting():
+        return _ops.w4a4_linear(x, left_trans, right_trans, w_packed, w_scale, bias, float(clip_ratio), out_dtype)
+    else:
+        if not _is_dynamo_compiling():
+            out = _direct.w4a4_linear(x, left_trans, right_trans, w_packed, w_scale, bias, float(clip_ratio), out_dtype)
+            if out is not NotImplemented:
+                return out
+        return _ops.w4a4_linear(x, left_trans, right_trans, w_packed, w_scale, bias, float(clip_ratio), out_dtype)
 
 
 def prepare_weights(w_packed: torch.Tensor) -> torch.Tensor:
@@ -91,7 +125,14 @@ def w4a4_linear_prepared(x: torch.Tensor, left_trans: torch.Tensor, right_trans:
                          clip_ratio: float = 1.0, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """w4a4_linear with the weights also given as the int8 copy made by prepare_weights: same results, no per-call
     rewriting of either operand (the activations are quantized straight to int8 codes)."""
-    return _ops.w4a4_linear_prepared(x, left_trans, right_trans, w_packed, w_prepared, w_scale, bias, float(clip_ratio), out_dtype)
+    if torch.jit.is_scripting():
+        return _ops.w4a4_linear_prepared(x, left_trans, right_trans, w_packed, w_prepared, w_scale, bias, float(clip_ratio), out_dtype)
+    else:
+        if not _is_dynamo_compiling():
+            out = _direct.w4a4_linear_prepared(x, left_trans, right_trans, w_packed, w_prepared, w_scale, bias, float(clip_ratio), out_dtype)
+            if out is not NotImplemented:
+                return out
+        return _ops.w4a4_linear_prepared(x, left_trans, right_trans, w_packed, w_prepared, w_scale, bias, float(clip_ratio), out_dtype)
 
 
 def pack_int4_to_int32(tensor: torch.Tensor) -> torch.Tensor:

@@ -197,3 +197,63 @@ def test_scale_dtype_keyword_and_device_status():
     assert sh.dtype == torch.float16 and torch.equal(ch, c32) and torch.equal(sh, s32.half())
     assert torch.equal(q.dequantize_int4(cb, sb, True), q.dequantize_int4(c32, s32, True))
     q.device_status()
+
+
+def test_direct_calls_behave_as_the_operators_do():
+    """The Python layer calls the operators without boxing: modes, the profiler, autograd, tensor subclasses and vmap still
+    find them, and results and errors are those of torch.ops."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    x = torch.randn(3, 4096, device=DEV, dtype=torch.bfloat16)
+    layer = q.W4A4Linear(4096, 256, device=DEV, bias=True).load_float(torch.randn(256, 4096) * 0.02, torch.eye(64), torch.eye(64), torch.randn(256))
+    b = layer._buffers
+    args = (b["left_trans"], b["right_trans"], b["weight_packed"], b["weight_scale"], b["bias"], 1.0, torch.bfloat16)
+    want = torch.ops.quant_ops.w4a4_linear(x, *args)
+    assert torch.equal(layer(x), want) and torch.equal(q.w4a4_linear(x, *args), want)
+    codes, scales = torch.ops.quant_ops.flatquant_dynamic_quantize(x, *args[:2], 1.0, True)
+    calls = {
+        "quant_ops::flatquant_dynamic_quantize": lambda v: q.flatquant_dynamic_quantize(v, *args[:2], 1.0, True),
+        "quant_ops::w4a4_linear": lambda v: layer(v),
+        "quant_ops::int4_matmul": lambda v: q.int4_matmul(codes, args[2].t(), scales, args[3]),
+        "quant_ops::int4_matmul_ex": lambda v: q.int4_matmul_ex(codes, args[2].t(), scales, args[3], torch.bfloat16),
+        "quant_ops::dequantize_int4": lambda v: q.dequantize_int4(codes, scales, True),
+    }
+    seen = []
+
+    class Log(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func.name())
+            return func(*args, **(kwargs or {}))
+
+    class Sub(torch.Tensor):
+        @classmethod
+        def __torch_function__(cls, func, types, args=(), kwargs=None):
+            seen.append("sub")
+            return super().__torch_function__(func, types, args, kwargs or {})
+
+    for name, call in calls.items():
+        with Log():
+            call(x)
+        assert name in seen
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+            call(x)
+        assert name in [e.name for e in prof.events()]
+    seen.clear()
+    calls["quant_ops::flatquant_dynamic_quantize"](x.as_subclass(Sub))
+    assert "sub" in seen
+    with torch.inference_mode():
+        y = layer(x)
+    assert y.is_inference() and torch.equal(y, want)
+    xg = x.clone().requires_grad_()
+    direct, boxed = layer(xg), torch.ops.quant_ops.w4a4_linear(xg, *args)
+    assert direct.requires_grad == boxed.requires_grad and type(direct.grad_fn) is type(boxed.grad_fn)
+    with torch.no_grad():
+        assert not layer(xg).requires_grad
+    errors = []
+    for call in (lambda v: layer(v), lambda v: torch.ops.quant_ops.w4a4_linear(v, *args)):
+        try:
+            torch.vmap(call)(x[None])
+            errors.append(None)
+        except RuntimeError as e:
+            errors.append(type(e))
+    assert errors[0] == errors[1]
