@@ -4,7 +4,7 @@
 // 128-row tcgen05 tile would spend at least three quarters of its rows on padding and would need the weights widened
 // to int8 in memory first, which doubles the bytes.  Here the weights stay packed all the way into registers:
 //
-//   * one CTA owns 16 or 32 output channels (rows of the [Nout, K/8] weight matrix); per 16 channels, 8 warps split
+//   * one CTA owns 16 or 32 output channels (many channels: an even share of them, int4_gemm_even_kernel) (rows of the [Nout, K/8] weight matrix); per 16 channels, 8 warps split
 //     K into 8 contiguous slices and add their partial sums through shared memory at the end;
 //   * a lane loads 16 bytes of a weight row at a time (four lanes cover 64 contiguous bytes of one row, a warp 16
 //     rows, consecutive loads of a warp walk along the rows), four chunks of 128 values per batch, and the next
@@ -395,6 +395,211 @@ int launch_resident(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t l
 #undef QO_RES
 }
 
+// ---- many channels ------------------------------------------------------------------------------------------------------
+// One CTA per SM, and the output channels shared out evenly: 97 for 14336 channels, where blocks of 16, two CTAs an SM, come to
+// 3.03 rounds.  The 16 warps split the CTA's channels into up to four groups, so that a warp's accumulators stay in
+// registers, and K into 16 / groups slices.  The codes come through the read-only path: a copy into shared memory comes
+// before the first product, and with more tokens it costs an SM its second CTA.
+constexpr int kEvenWarps = 16;
+constexpr int kMaxTileProducts = 8;  // 16-channel tiles x 8-token tiles of a warp: 32 accumulators a lane
+constexpr int kMaxTiles = 4;         // of them 16-channel tiles, whose weights are held in registers
+constexpr int kMaxChannels = 4 * kMaxTiles * 16;  // of a CTA at a time
+
+// NT = 8-token column tiles, TILES = 16-channel row tiles of a warp, DEPTH / XDEPTH = chunks of weights / codes in flight per warp.
+// cpc = channels of a CTA at a time, cpg = those of one of its `groups` groups of warps.
+template <int NT, int TILES, int DEPTH, int XDEPTH, typename OutT>
+__global__ void __launch_bounds__(kEvenWarps * 32, 1)
+int4_gemm_even_kernel(const uint32_t* __restrict__ a, int64_t lda, const uint32_t* __restrict__ b, int64_t ldb,
+                      const float* __restrict__ sa, const float* __restrict__ sb, OutT* __restrict__ out,
+                      int32_t* __restrict__ acc_out, const OutT* __restrict__ bias, int tokens, int nchunks, int64_t n, int cpc,
+                      int cpg, int groups, int weights_first) {
+  static_assert(DEPTH % XDEPTH == 0, "buffers are indexed at compile time");
+  extern __shared__ int red[];  // partial sums [warp][tile][nt][16][9]
+  __shared__ float sb_s[kMaxChannels], sa_s[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int slices = kEvenWarps / groups, grp = warp / slices, slice = warp - grp * slices;
+  const int per = (nchunks + slices - 1) / slices;
+  const int cb = slice * per, ce = min(nchunks, cb + per);
+  const uint4 zero4 = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);  // eight zeros per word
+  // weights_first: see int4_gemm_skinny_kernel; the first weights and the channels' scales are requested before the wait
+  bool waited = false;
+  if (!weights_first) {
+    ptx::grid_dependency_wait();
+    waited = true;
+  }
+  for (int64_t c0 = (int64_t)blockIdx.x * cpc; c0 < n; c0 += (int64_t)gridDim.x * cpc) {
+    const int nch = (int)min((int64_t)cpc, n - c0);
+    const int first = grp * cpg, mine = max(0, min(cpg, nch - first));  // this warp's channels of the CTA
+    for (int i = threadIdx.x; i < nch; i += kEvenWarps * 32) sb_s[i] = sb[c0 + i];
+    const uint32_t* wrow = b + (c0 + first + g) * ldb + 4 * t4;
+    uint4 w[DEPTH][TILES][2], x[XDEPTH][NT];
+    auto load_w = [&](int u, int c) {
+#pragma unroll
+      for (int tl = 0; tl < TILES; ++tl)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = tl * 16 + 8 * h;
+          w[u][tl][h] = (c < ce && r + g < mine) ? ld_stream(wrow + (int64_t)r * ldb + (int64_t)c * kChunkWords) : zero4;
+        }
+    };
+    auto load_x = [&](int u, int c) {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int tok = nt * 8 + g;
+        x[u][nt] = (c < ce && tok < tokens) ? __ldg(reinterpret_cast<const uint4*>(a + (int64_t)tok * lda + (int64_t)c * kChunkWords + 4 * t4)) : zero4;
+      }
+    };
+#pragma unroll
+    for (int u = 0; u < DEPTH; ++u) load_w(u, cb + u);
+    if (!waited) ptx::grid_dependency_wait();
+    waited = true;
+#pragma unroll
+    for (int u = 0; u < XDEPTH; ++u) load_x(u, cb + u);
+    if (threadIdx.x < tokens) sa_s[threadIdx.x] = sa[threadIdx.x];
+
+    int acc[TILES][NT][4];
+#pragma unroll
+    for (int tl = 0; tl < TILES; ++tl)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[tl][nt][i] = 0;
+    for (int c = cb; c < ce; c += DEPTH) {
+#pragma unroll
+      for (int u = 0; u < DEPTH; ++u) {
+        if (c + u < ce) {
+          uint32_t xe[NT][4], xo[NT][4];
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            const uint4 xx = x[u % XDEPTH][nt];
+            split16(xx.x, xe[nt][0], xo[nt][0]);
+            split16(xx.y, xe[nt][1], xo[nt][1]);
+            split16(xx.z, xe[nt][2], xo[nt][2]);
+            split16(xx.w, xe[nt][3], xo[nt][3]);
+          }
+#pragma unroll
+          for (int tl = 0; tl < TILES; ++tl) {
+            if (tl * 16 >= mine) break;  // uniform: this tile has no channel
+            const uint4 w0 = w[u][tl][0], w1 = w[u][tl][1];
+            const uint32_t w0w[4] = {w0.x, w0.y, w0.z, w0.w}, w1w[4] = {w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint32_t a0, a1, a2, a3;
+              split16(w0w[j], a0, a2);
+              split16(w1w[j], a1, a3);
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt) mma_s8(acc[tl][nt], a0, a1, a2, a3, xe[nt][j], xo[nt][j]);
+            }
+          }
+        }
+        load_w(u, c + u + DEPTH);
+        load_x(u % XDEPTH, c + u + XDEPTH);
+      }
+    }
+
+    // partial sums of the slices through shared memory (fragment layout: see int4_gemm_skinny_kernel)
+#pragma unroll
+    for (int tl = 0; tl < TILES; ++tl)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        int* p = red + (((warp * TILES + tl) * NT + nt) * 16) * 9;
+        p[g * 9 + 2 * t4] = acc[tl][nt][0];
+        p[g * 9 + 2 * t4 + 1] = acc[tl][nt][1];
+        p[(g + 8) * 9 + 2 * t4] = acc[tl][nt][2];
+        p[(g + 8) * 9 + 2 * t4 + 1] = acc[tl][nt][3];
+      }
+    __syncthreads();
+    for (int w0 = 0, f = 0; w0 < kEvenWarps; w0 += slices, f += cpg) {  // group by group
+      for (int idx = threadIdx.x; idx < TILES * NT * 128; idx += kEvenWarps * 32) {
+        const int r = idx & 15, col = (idx >> 4) & 7, nt = (idx >> 7) % NT, tl = idx / (NT * 128);
+        const int tok = nt * 8 + col, chl = f + tl * 16 + r;
+        if (tok >= tokens || tl * 16 + r >= cpg || chl >= nch) continue;
+        int sum = 0;
+#pragma unroll 4
+        for (int v = w0; v < w0 + slices; ++v) sum += red[(((v * TILES + tl) * NT + nt) * 16 + r) * 9 + col];
+        sum >>= 8;  // both operands carried the factor 16
+        const int64_t ch = c0 + chl;
+        OutT v = to_out<OutT>(((float)sum * sa_s[tok]) * sb_s[chl]);
+        if (bias != nullptr) v = to_out<OutT>(from_out(v) + from_out(bias[ch]));
+        out[(int64_t)tok * n + ch] = v;
+        if (acc_out != nullptr) acc_out[(int64_t)tok * n + ch] = sum;
+      }
+    }
+    __syncthreads();  // the next turn overwrites the scales and the partial sums
+  }
+}
+
+struct EvenArgs {
+  const uint32_t *a, *b;
+  int64_t lda, ldb;
+  const float *sa, *sb;
+  void* out;
+  int32_t* acc_out;
+  const void* bias;
+  int tokens, nchunks;
+  int64_t n;
+  int weights_first;
+  int cpc, cpg, groups, grid;
+};
+
+template <int NT, int TILES, typename OutT>
+int launch_even_cfg(const EvenArgs& p, int dev, cudaStream_t stream) {
+  // chunks in flight, as many as the registers allow: 8 to 16 weight loads of 16 bytes a lane
+  constexpr int kDepth = TILES == 4 ? (NT == 1 ? 2 : 1) : (TILES == 2 ? (NT == 4 ? 2 : 4) : 4);
+  constexpr int kXDepth = NT == 4 || kDepth == 1 ? 1 : 2;
+  constexpr int kRed = kEvenWarps * TILES * NT * 16 * 9 * (int)sizeof(int);
+  auto kern = int4_gemm_even_kernel<NT, TILES, kDepth, kXDepth, OutT>;
+  static bool configured[64] = {};
+  if (!configured[dev & 63]) {
+    QO_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRed));
+    configured[dev & 63] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)p.grid);
+  cfg.blockDim = dim3(kEvenWarps * 32);
+  cfg.dynamicSmemBytes = kRed;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  QO_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p.a, p.lda, p.b, p.ldb, p.sa, p.sb, reinterpret_cast<OutT*>(p.out), p.acc_out,
+                                 reinterpret_cast<const OutT*>(p.bias), p.tokens, p.nchunks, p.n, p.cpc, p.cpg, p.groups, p.weights_first));
+  return check_launch("int4_gemm_even_kernel");
+}
+
+template <typename OutT>
+int launch_even(EvenArgs p, int dev, cudaStream_t stream) {
+  const int sms = sm_count(dev), nt = p.tokens <= 8 ? 1 : (p.tokens <= 16 ? 2 : 4), most_tiles = min(kMaxTiles, kMaxTileProducts / nt);
+  // channels per CTA: the same share for every SM, in several turns if the warps could not hold the sums; groups of warps: as few
+  // as hold them
+  const int64_t most = 4 * 16 * most_tiles, turns = (p.n + sms * most - 1) / (sms * most);
+  p.cpc = (int)((p.n + sms * turns - 1) / (sms * turns));
+  const int64_t blocks = (p.n + p.cpc - 1) / p.cpc;
+  p.grid = (int)(blocks < sms ? blocks : sms);
+  int tiles = 0;
+  for (p.groups = 1;; p.groups *= 2) {
+    p.cpg = (p.cpc + p.groups - 1) / p.groups;
+    tiles = (p.cpg + 15) / 16;
+    if (tiles <= most_tiles || p.groups == 4) break;
+  }
+#define QO_EVEN(NTV, TLV) return launch_even_cfg<NTV, TLV, OutT>(p, dev, stream)
+  if (nt == 1) {
+    if (tiles <= 1) QO_EVEN(1, 1);
+    if (tiles <= 2) QO_EVEN(1, 2);
+    QO_EVEN(1, 4);
+  }
+  if (nt == 2) {
+    if (tiles <= 1) QO_EVEN(2, 1);
+    if (tiles <= 2) QO_EVEN(2, 2);
+    QO_EVEN(2, 4);
+  }
+  if (tiles <= 1) QO_EVEN(4, 1);
+  QO_EVEN(4, 2);
+#undef QO_EVEN
+}
+
 template <int NT, int RT, bool STAGED, typename OutT>
 int launch_cfg(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t ldb, const float* sa, const float* sb, void* out,
                int32_t* acc_out, const void* bias, int tokens, int nchunks, int64_t n, size_t smem, int weights_first,
@@ -440,6 +645,17 @@ int launch_nt(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t ldb, co
 template <typename OutT>
 int launch_t(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t ldb, const float* sa, const float* sb, void* out,
              int32_t* acc_out, const void* bias, int tokens, int nchunks, int64_t n, int weights_first, cudaStream_t stream) {
+  // Even shares where blocks of 16 channels would need more than one round of two CTAs per SM.  Measured, blocks / even shares (graph
+  // replay, weights from HBM): 4 x 4096 x 14336 11.8 / 10.1 us, 16 x 4096 x 14336 15.5 / 11.5, 16 x 4096 x 8192 9.6 / 8.7, 12 x 4096 x
+  // 5120 8.0 / 7.1, 16 x 14336 x 5120 24.3 / 14.5, 16 x 14336 x 28672 86.7 / 49.4, 3 x 8192 x 6144 10.6 / 9.5; at 4096 channels
+  // the blocks stay: 1 x 14336 x 4096 8.8 / 10.6, 16 x 4096 x 4096 5.9 / 7.3 (small CTAs of successive launches overlap).  Up to
+  // 8 tokens the line is a little higher (1 x 4096 x 5120 6.1 / 6.3); above 16, where a warp holds two blocks of weights only, it
+  // lies at three rounds, for K up to 8192: 32 x 4096 x 14336 23.3 / 19.1, but 20 x 4096 x 11008 16.0 / 17.6 and 32 x 14336 x 28672 99 / 102.
+  int dev = 0;
+  QO_CUDA_TRY(cudaGetDevice(&dev));
+  const int64_t per_sm = tokens <= 8 ? 36 : (tokens <= 16 ? 32 : 96);
+  if (n > per_sm * sm_count(dev) && (tokens <= 16 || nchunks <= 64))
+    return launch_even<OutT>({a, b, lda, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, 0, 0, 0, 0}, dev, stream);
   if (tokens <= 8) return launch_nt<1, OutT>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, stream);
   if (tokens <= 16) return launch_nt<2, OutT>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, stream);
   return launch_nt<4, OutT>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, stream);

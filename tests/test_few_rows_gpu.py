@@ -1,0 +1,48 @@
+"""The packed product of 1 to 32 rows with many channels, shared out evenly over the SMs: accumulators and outputs are the bits of
+the shape-generic kernel."""
+import pytest
+import torch
+
+import quant_ops_b200 as q
+from helpers import N, abi_int4_matmul, launched_kernels, lib, stream_ptr
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# tokens: either side of 8 and 16; channels: the first past each line, ragged last CTAs and tiles, every split into groups of warps, two
+# turns of all SMs; K: one chunk, fewer chunks than slices, ragged slices
+SHAPES = [(1, 128, 5329), (8, 2304, 14336), (5, 4096, 9473), (1, 256, 37893), (9, 128, 4737), (16, 1152, 18944), (13, 4096, 9500), (16, 256, 38001),
+          (17, 384, 14209), (32, 4096, 18944), (25, 512, 18945), (32, 1024, 40000)]
+
+
+def problem(t, k, n, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    words = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, dtype=torch.int64, device=DEV, generator=g).to(torch.int32)
+    return words(t, k // 8), words(n, k // 8), torch.rand(t, device=DEV, generator=g) + 0.01, torch.rand(n, device=DEV, generator=g) * 1e-3
+
+
+@pytest.mark.parametrize("t,k,n", SHAPES)
+def test_same_bits_as_the_generic_kernel(t, k, n):
+    a, w, sa, sb = problem(t, k, n, t + k + n)
+    for out_dtype in ("fp16", "bf16"):
+        ref, ref_acc = abi_int4_matmul(a, w.t(), sa, sb, out_dtype, True, policy=1)
+        got, acc = abi_int4_matmul(a, w.t(), sa, sb, out_dtype, True)
+        assert lib.qo_device_status(stream_ptr()) == N.QO_OK
+        assert torch.equal(acc, ref_acc) and torch.equal(got.view(torch.int16), ref.view(torch.int16))
+    assert "int4_gemm_even_kernel" in launched_kernels(lambda: q.int4_matmul(a, w.t(), sa, sb))[0]
+
+
+@pytest.mark.parametrize("tokens,n_out", [(16, 14336), (32, 14336), (12, 37893)])
+def test_inside_the_layer(tokens, n_out):
+    """More channels than the resident-weights kernel holds: the layer streams them, its first weights before the codes are there."""
+    g = torch.Generator().manual_seed(tokens + n_out)
+    x = torch.randn(tokens, 4096, generator=g).bfloat16().to(DEV)
+    l = torch.linalg.qr(torch.randn(64, 64, dtype=torch.float64, generator=g)).Q.bfloat16().contiguous().to(DEV)
+    _, w, _, sb = problem(1, 4096, n_out, 4)
+    bias = torch.randn(n_out, generator=g).bfloat16().to(DEV)
+    codes, scales = q.flatquant_dynamic_quantize(x, l, l, 0.9, True)
+    want = q.int4_matmul_ex(codes, w.t(), scales, sb, torch.bfloat16)
+    want = (want.float() + bias.float()).bfloat16()
+    for _ in range(10):
+        assert torch.equal(q.w4a4_linear(x, l, l, w, sb, bias, 0.9, torch.bfloat16), want)
+    assert "int4_gemm_even_kernel" in launched_kernels(lambda: q.w4a4_linear(x, l, l, w, sb, bias, 0.9, torch.bfloat16))[1]
