@@ -302,6 +302,13 @@ int qo_w4a4_linear(const void* x, int64_t ldx, const void* left, const void* rig
   }
   if (workspace_bytes < need) return fail(QO_ERR_WORKSPACE, "w4a4_linear: workspace of %zu bytes, need %zu", workspace_bytes, need);
   char* ws = reinterpret_cast<char*>(workspace);
+  // one to four tokens of 64-wide right transforms: every CTA quantizes them itself and multiplies its share of the channels
+  if (t_policy == 0 && decode_layer_supported(x, ldx, left, right, w_packed, tokens, m, n, n_out, clip_ratio, in_dtype)) {
+    t_quant_path = 2;
+    t_gemm_path = 3;
+    return launch_decode_layer(x, ldx, left, right, w_packed, w_scale, bias, out, tokens, m, n_out, clip_ratio, in_dtype, out_dtype,
+                               reinterpret_cast<cudaStream_t>(stream));
+  }
   // prefill sizes: the quantizer packs, and the GEMM that unpacks in the kernel takes the packed codes and the packed
   // weights as they are (the packed route below); otherwise ...
   const bool unpack_route = t_policy != 1 && gemm_unpack_preferred(tokens, k, n_out, Widening::kWeightsBeside) &&

@@ -1,0 +1,404 @@
+// The fused layer for one to four tokens in ONE kernel: right transform of 64, left transform of 16, 32, 48 or 64 (4096 = 64 x 64, 3072 =
+// 48 x 64).  Every CTA quantizes all tokens itself and multiplies the codes with its own share of the output channels.
+//
+// A decode step is latency from end to end: the launch of the quantizer, its chain of products and passes on one or two SMs, the
+// hand-over to the GEMM on all SMs, the codes through L2 and back.  The transform of four tokens is 4 x 1 MFLOP on the tensor
+// core; 148 repetitions of it cost nothing that another SM would have done meanwhile, and spare a launch, the hand-over and the
+// trip of the codes.  The weights of a CTA (28 rows of 2 KB for 4096 -> 4096) are fetched with bulk copies while it quantizes.
+//
+//   all warps     stage X (two tokens to a group, two groups side by side), R and L^T (twice, as flatquant_sm100_n64.cu)
+//   one thread    Y = X . R, then Z = LL . Y2 per group (tcgen05, the instruction shapes of flatquant_sm100_n64.cu, hence its bits)
+//   8 warps       per group: Y pass (Y overwrites X, which its product has read), quantize pass; the codes stay in shared memory
+//   16 warps      each a sixteenth of K of all channels of the CTA, mma.sync m16n8k32 as in int4_gemm_skinny.cu; the partial sums
+//                 are added through the memory that held the weights
+//
+// Measured in graph replay, weights from HBM, quantizer and GEMM / this: 1 x 4096 -> 4096 7.2 / 6.7 us, 4 tokens 7.8 / 7.4, 1 x
+// 4096 -> 1024 6.4 / 5.2, 4 tokens 6.5 / 5.9, 1 x 4096 -> 11008 10.8 / 11.0; a call's launches take the host 2.3 us less.  Bound by
+// latency: launch, staging, two products with a pass after each, the weights' arrival (8.4 MB in 1.3 us at the copy rate), the sums.
+// More tokens take the quantizer's pipeline, and a share of channels that does not fit beside the stages (14336: 97 rows) two kernels.
+//
+// Numerics: flatquant_sm100_n64.cu and int4_gemm_skinny.cu (reference: src/quant_ops/ops/quantization/flatquant/ops.py:99-117 and
+// src/quant_ops/ops/quantization/int4_matmul/kernels/cuda_int4_matmul_kernel.cu:49-118).  Every mbarrier wait is bounded.
+#include "flatquant_sm100_common.cuh"
+
+namespace qo {
+namespace {
+
+using namespace ptx;
+using namespace fq;
+
+constexpr int kThreads = 512, kWarps = 16;
+constexpr int kMaxTokens = 4;
+constexpr int kStageBytes = 128 * 128;                    // two tokens: 2 x 64 rows of 128 bytes
+constexpr int kOffR = 0;
+constexpr int kOffLL = kOffR + 64 * 128;
+constexpr int kOffX = kOffLL + kAtomBytes;                // one stage per group
+constexpr int kTmemCols = 512;                            // first product: 2 x 64 columns; second product: 2 x 128
+constexpr int kColZ = 256;
+constexpr size_t kSmemLimit = 227 * 1024 - 1024;          // beside the static part
+
+struct Misc {
+  uint64_t d1_full[2], d2_full[2], weights;
+  uint32_t tmem_base;
+  alignas(16) float absmax[2][2][4];                      // [group][token][warp of the token]; slots without a warp stay 0
+  float scale[kMaxTokens];
+};
+
+__device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+// packed word -> (even elements, odd elements) as int8 bytes holding 16 * value
+__device__ __forceinline__ void split16(uint32_t w, uint32_t& even, uint32_t& odd) {
+  const uint32_t t = w ^ 0x88888888u;
+  even = (t << 4) & 0xF0F0F0F0u;
+  odd = t & 0xF0F0F0F0u;
+}
+__device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+template <typename T> __device__ __forceinline__ T to_type(float v);
+template <> __device__ __forceinline__ __half to_type<__half>(float v) { return __float2half_rn(v); }
+template <> __device__ __forceinline__ __nv_bfloat16 to_type<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+__device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
+__device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+// TILES = 16-channel tiles of a CTA's share
+template <typename T, int TILES, typename OutT>
+__global__ void __launch_bounds__(kThreads, 1)
+decode_layer_n64_kernel(const T* __restrict__ x, int64_t ldx, const T* __restrict__ left, const T* __restrict__ right,
+                        const uint32_t* __restrict__ w, const float* __restrict__ sw, const OutT* __restrict__ bias,
+                        OutT* __restrict__ out, int tokens, int m, int64_t n, int cpc, float clip, uint32_t* __restrict__ status) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ Misc misc;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t smem_base = smem_u32(smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nchunks = m >> 1, stride4 = nchunks * 4 + 4;  // 128 values per chunk; row stride of codes and weights in 16-byte units
+  const int groups = (tokens + 1) >> 1;
+  uint4* codes = reinterpret_cast<uint4*>(smem + kOffX + groups * kStageBytes);
+  uint4* wsm = codes + 2 * groups * stride4;
+  const int64_t c0 = (int64_t)blockIdx.x * cpc;
+  const int nch = (int)min((int64_t)cpc, n - c0);         // the grid is sized so that every CTA has at least one channel
+  const uint4 zero4 = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);  // eight zeros per word
+
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&misc.d1_full[i]), 1);
+      mbar_init(smem_u32(&misc.d2_full[i]), 1);
+    }
+    mbar_init(smem_u32(&misc.weights), 1);
+    fence_barrier_init();
+  }
+  if (tid < 16) (&misc.absmax[0][0][0])[tid] = 0.f;
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&misc.tmem_base), kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = misc.tmem_base;
+  grid_dependency_wait();    // nothing above touches global memory; the weights, too, may come from the kernel ahead
+  grid_launch_dependents();
+
+  // ---- weights: rows of K / 2 bytes, padded by 64 so that the fragment reads are conflict-free -------------------------
+  if (warp == 0) {
+    const uint32_t bar = smem_u32(&misc.weights), row_bytes = (uint32_t)nchunks * 64u;
+    if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)nch * row_bytes);
+    __syncwarp();
+    for (int r = lane; r < nch; r += 32) bulk_copy_g2s(smem_u32(wsm + r * stride4), w + (c0 + r) * (int64_t)(nchunks * 16), row_bytes, bar);
+  }
+  // ---- X, R and LL in the 128-byte swizzle, every load of a thread requested before its first store ---------------------
+  {
+    uint4 wx[4], wl[2], wr;
+    const int rows_group = 2 * m, pieces_x = groups * rows_group * 8;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int idx = tid + j * kThreads, gr = idx >> 3, grp = gr / rows_group, r = gr - grp * rows_group;
+      const int tok = 2 * grp + (r >= m ? 1 : 0), row = r >= m ? r - m : r;
+      wx[j] = make_uint4(0, 0, 0, 0);
+      if (idx < pieces_x && tok < tokens) wx[j] = *reinterpret_cast<const uint4*>(x + tok * ldx + row * 64 + (idx & 7) * 8);
+    }
+    wr = *reinterpret_cast<const uint4*>(right + tid * 8);  // 64 rows of 8 pieces
+    const int mpad = (m + 31) & ~31;                        // each copy of L^T starts on a 32-row boundary
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int idx = tid + j * kThreads, k = idx >> 4, c = idx & 15, cpy = (8 * c) / mpad, i0 = 8 * c - cpy * mpad;
+      wl[j] = make_uint4(0, 0, 0, 0);
+      if (k < m && cpy < 2 && i0 < m) wl[j] = *reinterpret_cast<const uint4*>(left + k * m + i0);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int idx = tid + j * kThreads, gr = idx >> 3, c = idx & 7, grp = gr / rows_group, r = gr - grp * rows_group;
+      if (idx < pieces_x) *reinterpret_cast<uint4*>(smem + kOffX + grp * kStageBytes + r * 128 + ((c ^ (r & 7)) << 4)) = wx[j];
+    }
+    *reinterpret_cast<uint4*>(smem + kOffR + (tid >> 3) * 128 + (((tid & 7) ^ ((tid >> 3) & 7)) << 4)) = wr;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int idx = tid + j * kThreads, k = idx >> 4, c = idx & 15;
+      if (k < m) *reinterpret_cast<uint4*>(smem + kOffLL + (c >> 3) * (kAtomBytes / 2) + k * 128 + (((c & 7) ^ (k & 7)) << 4)) = wl[j];
+    }
+    fence_proxy_async_smem();
+  }
+  __syncthreads();
+
+  const int grp = warp >> 3, q = warp & 3, h = (warp >> 2) & 1;  // warp (q, h) of its group's eight
+  if (grp < groups) {
+    // ---- first product, by one thread of the group ---------------------------------------------------------------------
+    if ((warp & 7) == 0 && lane == 0) {
+      const uint32_t idesc1 = umma_idesc(1, Fmt<T>::id, Fmt<T>::id, 0, 1, 128, 64);  // A = X rows: K-major, B = R as it lies in memory: N-major
+      const uint64_t da = umma_smem_desc_sw128(smem_base + kOffX + grp * kStageBytes, 16, 1024), db = umma_smem_desc_sw128(smem_base + kOffR, 16, 1024);
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) mma_f16_ss(tmem + grp * 64, da + ks * 2, db + ks * 128, idesc1, ks);
+      mma_commit(smem_u32(&misc.d1_full[grp]));
+    }
+    __syncwarp();
+    // ---- Y pass: columns 32h .. of lanes 32q .., rounded, over the X rows ------------------------------------------------
+    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc.d1_full[grp]), 0))) atomicCAS(status, 0u, 0xD10u + grp);
+    tc_fence_after();
+    const int r = q * 32 + lane;
+    if (q * 32 < 2 * m) {
+      uint32_t v[32];
+      tmem_ld_32x32b_x32(tmem + ((uint32_t)(q * 32) << 16) + grp * 64 + h * 32, v);
+      tmem_ld_wait();
+      const uint32_t yrow = (smem_base + kOffX + grp * kStageBytes + r * 128) | (uint32_t)((r & 7) << 4);
+      if (r < 2 * m) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint4 y;
+          y.x = pack2<T>(__uint_as_float(v[8 * j + 0]), __uint_as_float(v[8 * j + 1]));
+          y.y = pack2<T>(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]));
+          y.z = pack2<T>(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]));
+          y.w = pack2<T>(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]));
+          asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(yrow ^ (uint32_t)((h * 4 + j) << 4)), "r"(y.x), "r"(y.y), "r"(y.z), "r"(y.w) : "memory");
+        }
+      }
+      fence_proxy_async_smem();
+    }
+    tc_fence_before();
+    asm volatile("bar.sync %0, 256;" ::"r"(1 + grp) : "memory");
+    // ---- second product --------------------------------------------------------------------------------------------------
+    if ((warp & 7) == 0 && lane == 0) {
+      tc_fence_after();
+      const uint32_t idesc2 = umma_idesc(1, Fmt<T>::id, Fmt<T>::id, 1, 1, 128, 128);  // A = LL: M-major, B = the two tokens' Y side by side: N-major
+      uint64_t da = umma_smem_desc_sw128(smem_base + kOffLL, kAtomBytes / 2, 1024);
+      uint64_t db = umma_smem_desc_sw128(smem_base + kOffX + grp * kStageBytes, (uint32_t)(m * 128), 1024);
+#pragma unroll 1
+      for (int ks = 0; ks < (m >> 4); ++ks, da += 128, db += 128) mma_f16_ss(tmem + kColZ + grp * 128, da, db, idesc2, ks);
+      mma_commit(smem_u32(&misc.d2_full[grp]));
+    }
+    __syncwarp();
+    // ---- quantize pass: lane block c holds the Z rows of token c, see flatquant_sm100_n64.cu ------------------------------
+    const int mpad = (m + 31) & ~31, c = r / mpad, mi = r - c * mpad, tok = 2 * grp + c;
+    const bool has_rows = c < 2 && q * 32 - c * mpad < m;   // of this warp
+    const bool valid = c < 2 && mi < m && tok < tokens;
+    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&misc.d2_full[grp]), 0))) atomicCAS(status, 0u, 0xD20u + grp);
+    tc_fence_after();
+    uint32_t zz[16];
+    float row_amax = 0.f;
+    if (has_rows) {
+      uint32_t v[32];
+      tmem_ld_32x32b_x32(tmem + ((uint32_t)(q * 32) << 16) + kColZ + grp * 128 + c * 64 + h * 32, v);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 16; ++i) zz[i] = P2<T>::cvt(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+      uint32_t m0 = zz[0], m1 = zz[1], m2 = zz[2], m3 = zz[3];
+#pragma unroll
+      for (int i = 4; i < 16; i += 4) {
+        m0 = P2<T>::absmax(m0, zz[i]);
+        m1 = P2<T>::absmax(m1, zz[i + 1]);
+        m2 = P2<T>::absmax(m2, zz[i + 2]);
+        m3 = P2<T>::absmax(m3, zz[i + 3]);
+      }
+      m0 = P2<T>::absmax(P2<T>::absmax(m0, m1), P2<T>::absmax(m2, m3));
+      row_amax = valid ? fmaxf(fabsf(P2<T>::lo(m0)), fabsf(P2<T>::hi(m0))) : 0.f;
+      const float warp_amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(row_amax)));
+      if (lane == 0) misc.absmax[grp][c][((q * 32 - c * mpad) >> 5) * 2 + h] = warp_amax;
+    }
+    tc_fence_before();
+    asm volatile("bar.sync %0, 256;" ::"r"(1 + grp) : "memory");
+    if (has_rows) {
+      const float4 p4 = *reinterpret_cast<const float4*>(&misc.absmax[grp][c][0]);
+      const float amax = fmaxf(fmaxf(p4.x, p4.y), fmaxf(p4.z, p4.w));
+      const float top = rnd1<T>(amax * clip);
+      const float s = fmaxf(rnd1<T>(top * 0.142857149f), DT<T>::floor_scale());
+      const float inv_s = __frcp_rn(s);
+      uint32_t rhi2, rlo2;
+      P2<T>::recip2(inv_s, rhi2, rlo2);
+      if (valid && mi == 0 && h == 0) misc.scale[tok] = s;
+      const bool clamp_needed = __any_sync(0xffffffffu, !(row_amax * inv_s < 7.4f));
+      uint32_t o[4];
+      if (s != 0.f) {
+        if (clamp_needed) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[j] = quantize8<T, true>(&zz[4 * j], s, inv_s, rhi2, rlo2);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[j] = quantize8<T, false>(&zz[4 * j], s, inv_s, rhi2, rlo2);
+        }
+      } else {
+        // the reference divides by zero here: +-inf clamps to 7 / -8, 0/0 counts as 0
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          o[j] = 0;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t pz = zz[4 * j + (i >> 1)];
+            const float z = (i & 1) ? P2<T>::hi(pz) : P2<T>::lo(pz);
+            o[j] |= (uint32_t)(z > 0.f ? 15 : (z < 0.f ? 0 : 8)) << (4 * i);
+          }
+        }
+      }
+      if (valid) codes[tok * stride4 + mi * 2 + h] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+  // ---- product ------------------------------------------------------------------------------------------------------------
+  const bool landed = mbar_wait(smem_u32(&misc.weights), 0);
+  tc_fence_before();
+  const bool all_landed = __syncthreads_and(landed);  // (also: codes and scales are complete, tensor memory has been read)
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, kTmemCols);
+  }
+  if (!all_landed) {  // one decision for the whole CTA
+    if (tid == 0) atomicCAS(status, 0u, 0xD30u);
+    return;  // the outputs stay unwritten; qo_device_status reports the timeout
+  }
+  const int g = lane >> 2, t4 = lane & 3;
+  const int per = (nchunks + kWarps - 1) / kWarps, cb = warp * per, ce = min(nchunks, cb + per);
+  int acc[TILES][4];
+#pragma unroll
+  for (int tl = 0; tl < TILES; ++tl)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[tl][i] = 0;
+  for (int c = cb; c < ce; ++c) {
+    const uint4 xx = g < tokens ? codes[g * stride4 + c * 4 + t4] : zero4;
+    const uint32_t xw[4] = {xx.x, xx.y, xx.z, xx.w};
+    uint32_t xe[4], xo[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) split16(xw[j], xe[j], xo[j]);
+#pragma unroll
+    for (int tl = 0; tl < TILES; ++tl) {
+      if (tl * 16 >= nch) break;  // uniform: this tile has no channel
+      const int r0 = tl * 16 + g, r1 = r0 + 8;
+      const uint4 w0 = r0 < nch ? wsm[r0 * stride4 + c * 4 + t4] : zero4;
+      const uint4 w1 = r1 < nch ? wsm[r1 * stride4 + c * 4 + t4] : zero4;
+      const uint32_t w0w[4] = {w0.x, w0.y, w0.z, w0.w}, w1w[4] = {w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t a0, a1, a2, a3;
+        split16(w0w[j], a0, a2);
+        split16(w1w[j], a1, a3);
+        mma_s8(acc[tl], a0, a1, a2, a3, xe[j], xo[j]);
+      }
+    }
+  }
+  __syncthreads();  // every weight has been read
+  int* red = reinterpret_cast<int*>(wsm);  // [warp][tile][16][5]: the columns of four tokens
+  if (t4 < 2) {
+#pragma unroll
+    for (int tl = 0; tl < TILES; ++tl) {
+      int* p = red + ((warp * TILES + tl) * 16) * 5;
+      p[g * 5 + 2 * t4] = acc[tl][0];
+      p[g * 5 + 2 * t4 + 1] = acc[tl][1];
+      p[(g + 8) * 5 + 2 * t4] = acc[tl][2];
+      p[(g + 8) * 5 + 2 * t4 + 1] = acc[tl][3];
+    }
+  }
+  __syncthreads();
+  for (int idx = tid; idx < TILES * 64; idx += kThreads) {
+    const int r = idx & 15, tok = (idx >> 4) & 3, tl = idx >> 6, chl = tl * 16 + r;
+    if (tok >= tokens || chl >= nch) continue;
+    const int64_t ch = c0 + chl;
+    const float scale = sw[ch];
+    int sum = 0;
+#pragma unroll
+    for (int v = 0; v < kWarps; ++v) sum += red[((v * TILES + tl) * 16 + r) * 5 + tok];
+    sum >>= 8;  // both operands carried the factor 16
+    OutT o = to_type<OutT>(((float)sum * misc.scale[tok]) * scale);
+    if (bias != nullptr) o = to_type<OutT>(to_float(o) + to_float(bias[ch]));
+    out[(int64_t)tok * n + ch] = o;
+  }
+}
+
+// shared memory of a CTA with cpc channels
+size_t smem_bytes(int64_t tokens, int m, int64_t cpc, int tiles) {
+  const size_t groups = (size_t)(tokens + 1) / 2, row = (size_t)(m / 2) * 64 + 64;
+  const size_t weights = cpc * row, red = (size_t)kWarps * tiles * 16 * 5 * sizeof(int);
+  return 1024 + kOffX + groups * kStageBytes + 2 * groups * row + (weights > red ? weights : red);
+}
+
+int tiles_of(int64_t cpc) { return cpc <= 16 ? 1 : (cpc <= 32 ? 2 : (cpc <= 64 ? 4 : 8)); }
+
+template <typename T, int TILES, typename OutT>
+int launch_cfg(const void* x, int64_t ldx, const void* left, const void* right, const int32_t* w, const float* sw, const void* bias, void* out,
+               int64_t tokens, int m, int64_t n, int cpc, size_t smem, float clip, uint32_t* status, int dev, cudaStream_t stream) {
+  auto kern = decode_layer_n64_kernel<T, TILES, OutT>;
+  static bool configured[64] = {};
+  if (!configured[dev & 63]) {
+    QO_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
+    configured[dev & 63] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((n + cpc - 1) / cpc));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  QO_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, reinterpret_cast<const T*>(x), ldx, reinterpret_cast<const T*>(left), reinterpret_cast<const T*>(right),
+                                 reinterpret_cast<const uint32_t*>(w), sw, reinterpret_cast<const OutT*>(bias), reinterpret_cast<OutT*>(out), (int)tokens,
+                                 m, n, cpc, clip, status));
+  return check_launch("decode_layer_n64_kernel");
+}
+
+template <typename T, typename OutT>
+int launch_typed(const void* x, int64_t ldx, const void* left, const void* right, const int32_t* w, const float* sw, const void* bias, void* out,
+                 int64_t tokens, int m, int64_t n, float clip, uint32_t* status, int dev, cudaStream_t stream) {
+  const int64_t cpc = (n + sm_count(dev) - 1) / sm_count(dev);
+  const int tiles = tiles_of(cpc);
+  const size_t smem = smem_bytes(tokens, m, cpc, tiles);
+#define QO_DEC(TL) return launch_cfg<T, TL, OutT>(x, ldx, left, right, w, sw, bias, out, tokens, m, n, (int)cpc, smem, clip, status, dev, stream)
+  if (tiles == 1) QO_DEC(1);
+  if (tiles == 2) QO_DEC(2);
+  if (tiles == 4) QO_DEC(4);
+  QO_DEC(8);
+#undef QO_DEC
+}
+
+}  // namespace
+
+// what the tcgen05 quantizer takes (flatquant_sm100_supported), with these transforms, and a share of the channels that fits
+bool decode_layer_supported(const void* x, int64_t ldx, const void* left, const void* right, const void* w, int64_t tokens, int m, int n,
+                            int64_t n_out, float clip, int in_dtype) {
+  if (tokens < 1 || tokens > kMaxTokens || n != 64 || m < 16 || m > 64 || m % 16 != 0) return false;
+  if (ldx < (int64_t)m * n || !flatquant_sm100_supported(ldx, m, n, in_dtype, x, left, right, clip) || reinterpret_cast<uintptr_t>(w) % 16) return false;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+  const int64_t cpc = (n_out + sm_count(dev) - 1) / sm_count(dev);
+  return cpc <= 128 && smem_bytes(tokens, m, cpc, tiles_of(cpc)) <= kSmemLimit;
+}
+
+int launch_decode_layer(const void* x, int64_t ldx, const void* left, const void* right, const int32_t* w, const float* sw, const void* bias, void* out,
+                        int64_t tokens, int m, int64_t n_out, float clip, int in_dtype, int out_dtype, cudaStream_t stream) {
+  int dev = 0;
+  QO_CUDA_TRY(cudaGetDevice(&dev));
+  uint32_t* status = device_status_word(dev);
+  if (!status) return fail(QO_ERR_CUDA, "w4a4_linear: could not allocate the device status word");
+  if (in_dtype == QO_BF16) {
+    if (out_dtype == QO_BF16)
+      return launch_typed<__nv_bfloat16, __nv_bfloat16>(x, ldx, left, right, w, sw, bias, out, tokens, m, n_out, clip, status, dev, stream);
+    return launch_typed<__nv_bfloat16, __half>(x, ldx, left, right, w, sw, bias, out, tokens, m, n_out, clip, status, dev, stream);
+  }
+  if (out_dtype == QO_BF16)
+    return launch_typed<__half, __nv_bfloat16>(x, ldx, left, right, w, sw, bias, out, tokens, m, n_out, clip, status, dev, stream);
+  return launch_typed<__half, __half>(x, ldx, left, right, w, sw, bias, out, tokens, m, n_out, clip, status, dev, stream);
+}
+
+}  // namespace qo

@@ -1,0 +1,67 @@
+"""The layer of one to four tokens in one kernel (decode_layer_sm100.cu): the bits of quantize -> GEMM by hand, at the edges of its
+shares of channels and of its groups of tokens."""
+import pytest
+import torch
+
+import quant_ops_b200 as q
+from helpers import N, launched_kernels, lib, make_inputs, stream_ptr, TD
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def problem(tokens, mn, n_out, dtype, seed=0):
+    m, n = mn
+    x, left, right = make_inputs(tokens, m * n, dtype, tokens + m + n_out + seed, True, mn=mn)
+    g = torch.Generator(device=DEV).manual_seed(n_out)
+    w = torch.randint(-2 ** 31, 2 ** 31, (n_out, m * n // 8), dtype=torch.int64, device=DEV, generator=g).to(torch.int32)
+    return x.to(DEV), left.to(DEV), right.to(DEV), w, torch.rand(n_out, device=DEV, generator=g) * 1e-3
+
+
+def by_hand(x, left, right, w, sw, clip, out_dtype, bias=None):
+    codes, scales = q.flatquant_dynamic_quantize(x, left, right, clip, True)
+    y = q.int4_matmul_ex(codes, w.t(), scales, sw, out_dtype)
+    return y if bias is None else (y.float() + bias.float()).to(out_dtype)
+
+
+@pytest.mark.parametrize("mn", [(64, 64), (48, 64), (32, 64), (16, 64)])
+@pytest.mark.parametrize("tokens,n_out,dtype,out", [(1, 1, "bf16", "bf16"), (2, 149, "fp16", "fp16"), (3, 1032, "bf16", "fp16"), (4, 4096, "fp16", "bf16"),
+                                                    (4, 4747, "bf16", "bf16"), (1, 9000, "bf16", "bf16"), (2, 11008, "fp16", "fp16")])
+def test_same_bits_as_two_calls(mn, tokens, n_out, dtype, out):
+    x, left, right, w, sw = problem(tokens, mn, n_out, dtype)
+    bias = torch.randn(n_out, device=DEV).to(TD[out])
+    want = by_hand(x, left, right, w, sw, 0.9, TD[out], bias)
+    call = lambda: q.w4a4_linear(x, left, right, w, sw, bias, 0.9, TD[out])
+    for _ in range(5):
+        assert torch.equal(call(), want)
+    assert lib.qo_device_status(stream_ptr()) == N.QO_OK
+    names = launched_kernels(call)
+    assert len(names) == 1 and "decode_layer_n64_kernel" in names[0]
+
+
+def test_special_tokens_and_strides():
+    """Zero tokens, subnormal ones whose float16 scale rounds to zero, clipped ones; rows with a stride; five tokens take two kernels."""
+    x, left, right, w, sw = problem(4, (64, 64), 520, "fp16")
+    wide = torch.zeros(4, 4104, device=DEV, dtype=torch.float16)
+    wide[:, :4096] = x
+    wide[1] = 0
+    wide[2, :4096] = (torch.randint(-3, 4, (4096,), device=DEV) * 2.0 ** -24).half()
+    wide[3, 5] = 3000.0
+    x = wide[:, :4096]
+    eye = torch.eye(64, device=DEV, dtype=torch.float16)
+    for l, r in ((left, right), (eye, eye)):
+        assert torch.equal(q.w4a4_linear(x, l, r, w, sw, None, 0.5), by_hand(x, l, r, w, sw, 0.5, torch.float16))
+    five = torch.cat([x, x[:1]])
+    assert torch.equal(q.w4a4_linear(five, left, right, w, sw, None, 0.5)[:4], q.w4a4_linear(x, left, right, w, sw, None, 0.5))
+    assert len(launched_kernels(lambda: q.w4a4_linear(five, left, right, w, sw, None, 0.5))) == 2
+
+
+def test_a_layer_behind_the_kernel_that_writes_its_weights():
+    """Inputs, weights and scales come from the kernels right ahead in the stream."""
+    x, left, right, w, sw = problem(2, (64, 64), 4096, "bf16")
+    want = by_hand(x, left, right, w, sw, 0.9, torch.bfloat16)
+    xs, ws, ss = torch.zeros_like(x), torch.zeros_like(w), torch.zeros_like(sw)
+    for _ in range(20):
+        xs.zero_(), ws.zero_(), ss.zero_()
+        xs.copy_(x), ss.copy_(sw), ws.copy_(w)
+        assert torch.equal(q.w4a4_linear(xs, left, right, ws, ss, None, 0.9), want)
