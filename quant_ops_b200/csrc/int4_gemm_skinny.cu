@@ -398,7 +398,7 @@ int launch_resident(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t l
 // ---- many channels ------------------------------------------------------------------------------------------------------
 // One CTA per SM, and the output channels shared out evenly: 97 for 14336 channels, where blocks of 16, two CTAs an SM, come to
 // 3.03 rounds.  The 16 warps split the CTA's channels into up to four groups, so that a warp's accumulators stay in
-// registers, and K into 16 / groups slices.  The codes come through the read-only path: a copy into shared memory comes
+// registers, and K into 16 / groups slices.  The codes come straight into registers: a copy into shared memory comes
 // before the first product, and with more tokens it costs an SM its second CTA.
 constexpr int kEvenWarps = 16;
 constexpr int kMaxTileProducts = 8;  // 16-channel tiles x 8-token tiles of a warp: 32 accumulators a lane
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(kEvenWarps * 32, 1)
 int4_gemm_even_kernel(const uint32_t* __restrict__ a, int64_t lda, const uint32_t* __restrict__ b, int64_t ldb,
                       const float* __restrict__ sa, const float* __restrict__ sb, OutT* __restrict__ out,
                       int32_t* __restrict__ acc_out, const OutT* __restrict__ bias, int tokens, int nchunks, int64_t n, int cpc,
-                      int cpg, int groups, int weights_first) {
+                      int cpg, int groups) {
   static_assert(DEPTH % XDEPTH == 0, "buffers are indexed at compile time");
   extern __shared__ int red[];  // partial sums [warp][tile][nt][16][9]
   __shared__ float sb_s[kMaxChannels], sa_s[32];
@@ -421,12 +421,7 @@ int4_gemm_even_kernel(const uint32_t* __restrict__ a, int64_t lda, const uint32_
   const int per = (nchunks + slices - 1) / slices;
   const int cb = slice * per, ce = min(nchunks, cb + per);
   const uint4 zero4 = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);  // eight zeros per word
-  // weights_first: see int4_gemm_skinny_kernel; the first weights and the channels' scales are requested before the wait
-  bool waited = false;
-  if (!weights_first) {
-    ptx::grid_dependency_wait();
-    waited = true;
-  }
+  ptx::grid_dependency_wait();
   for (int64_t c0 = (int64_t)blockIdx.x * cpc; c0 < n; c0 += (int64_t)gridDim.x * cpc) {
     const int nch = (int)min((int64_t)cpc, n - c0);
     const int first = grp * cpg, mine = max(0, min(cpg, nch - first));  // this warp's channels of the CTA
@@ -446,16 +441,14 @@ int4_gemm_even_kernel(const uint32_t* __restrict__ a, int64_t lda, const uint32_
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
         const int tok = nt * 8 + g;
-        x[u][nt] = (c < ce && tok < tokens) ? __ldg(reinterpret_cast<const uint4*>(a + (int64_t)tok * lda + (int64_t)c * kChunkWords + 4 * t4)) : zero4;
+        x[u][nt] = (c < ce && tok < tokens) ? ptx::ld_behind_wait(a + (int64_t)tok * lda + (int64_t)c * kChunkWords + 4 * t4) : zero4;
       }
     };
 #pragma unroll
     for (int u = 0; u < DEPTH; ++u) load_w(u, cb + u);
-    if (!waited) ptx::grid_dependency_wait();
-    waited = true;
 #pragma unroll
     for (int u = 0; u < XDEPTH; ++u) load_x(u, cb + u);
-    if (threadIdx.x < tokens) sa_s[threadIdx.x] = sa[threadIdx.x];
+    if (threadIdx.x < tokens) sa_s[threadIdx.x] = ptx::ld_behind_wait_f32(sa + threadIdx.x);
 
     int acc[TILES][NT][4];
 #pragma unroll
@@ -538,7 +531,6 @@ struct EvenArgs {
   const void* bias;
   int tokens, nchunks;
   int64_t n;
-  int weights_first;
   int cpc, cpg, groups, grid;
 };
 
@@ -565,7 +557,7 @@ int launch_even_cfg(const EvenArgs& p, int dev, cudaStream_t stream) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   QO_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p.a, p.lda, p.b, p.ldb, p.sa, p.sb, reinterpret_cast<OutT*>(p.out), p.acc_out,
-                                 reinterpret_cast<const OutT*>(p.bias), p.tokens, p.nchunks, p.n, p.cpc, p.cpg, p.groups, p.weights_first));
+                                 reinterpret_cast<const OutT*>(p.bias), p.tokens, p.nchunks, p.n, p.cpc, p.cpg, p.groups));
   return check_launch("int4_gemm_even_kernel");
 }
 
@@ -655,7 +647,7 @@ int launch_t(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t ldb, con
   QO_CUDA_TRY(cudaGetDevice(&dev));
   const int64_t per_sm = tokens <= 8 ? 36 : (tokens <= 16 ? 32 : 96);
   if (n > per_sm * sm_count(dev) && (tokens <= 16 || nchunks <= 64))
-    return launch_even<OutT>({a, b, lda, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, 0, 0, 0, 0}, dev, stream);
+    return launch_even<OutT>({a, b, lda, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, 0, 0, 0, 0}, dev, stream);
   if (tokens <= 8) return launch_nt<1, OutT>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, stream);
   if (tokens <= 16) return launch_nt<2, OutT>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, stream);
   return launch_nt<4, OutT>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, stream);

@@ -34,7 +34,7 @@ def test_same_bits_as_the_generic_kernel(t, k, n):
 
 @pytest.mark.parametrize("tokens,n_out", [(16, 14336), (32, 14336), (12, 37893)])
 def test_inside_the_layer(tokens, n_out):
-    """More channels than the resident-weights kernel holds: the layer streams them, its first weights before the codes are there."""
+    """More channels than the resident-weights kernel holds: the layer streams them behind the quantizer."""
     g = torch.Generator().manual_seed(tokens + n_out)
     x = torch.randn(tokens, 4096, generator=g).bfloat16().to(DEV)
     l = torch.linalg.qr(torch.randn(64, 64, dtype=torch.float64, generator=g)).Q.bfloat16().contiguous().to(DEV)
