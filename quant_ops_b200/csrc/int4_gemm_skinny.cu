@@ -646,7 +646,8 @@ int launch_t(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t ldb, con
   int dev = 0;
   QO_CUDA_TRY(cudaGetDevice(&dev));
   const int64_t per_sm = tokens <= 8 ? 36 : (tokens <= 16 ? 32 : 96);
-  if (n > per_sm * sm_count(dev) && (tokens <= 16 || nchunks <= 64))
+  // (not inside the layer, whose first weights come before the wait for the codes)
+  if (!weights_first && n > per_sm * sm_count(dev) && (tokens <= 16 || nchunks <= 64))
     return launch_even<OutT>({a, b, lda, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, 0, 0, 0, 0}, dev, stream);
   if (tokens <= 8) return launch_nt<1, OutT>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, stream);
   if (tokens <= 16) return launch_nt<2, OutT>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, stream);
