@@ -18,9 +18,11 @@
 //     the NEXT stage's barrier before it issues the MMAs of this one and looks at the answer afterwards.
 //   * A TMA load of a 32 KB stage takes about 1400 cycles from request to arrival (operands in L2), longer than a
 //     stage's MMAs (about 1100): the packed ring is three stages deep, as is the operand ring behind it.
-//   * Tensor memory (512 columns) holds ONE 256-column accumulator and three A stages of 64 columns; the epilogue (8
-//     warps) therefore does not overlap the next tile's main loop, but frees the accumulator as soon as its last
-//     values are in registers.
+//   * Tensor memory (512 columns) holds three A stages of 64 columns and ONE 256-column accumulator that starts at column 0
+//     and 64 in turn.  The next tile's main loop starts when the 192 columns that both use are in the registers of the
+//     epilogue (8 warps), and the conversion, the stores and the other 64 columns overlap it.
+//   * The converters run on 48 registers and the epilogue on 128 (setmaxnreg): a spill in a converter loop, or addresses of
+//     all slots kept in registers there, cost 5 to 12 % of every shape.
 //
 // Unpacking without sign extension: x ^ 0x88888888 turns the offset-binary nibbles into two's-complement nibbles, and a
 // nibble in the HIGH half of a byte is the int8 value 16 * n.  Each packed word yields one word of its even elements
@@ -33,10 +35,10 @@
 //   warp 0       TMA producer: packed A block + packed B half into a ring of 3 stages (local barriers)
 //   warp 1       leader: tcgen05.mma.cta_group::2, M = 256, N = 256, eight K = 32 slices per stage; commits release the
 //                operand stage in BOTH CTAs (one commit per CTA, the peer's barrier addressed through mapa)
-//   warps 2-9    epilogue of the CTA's own 128 accumulator rows (two warps per lane quadrant, 128 columns each)
-//   warps 10-21  A converters: three sets of four warps, set g takes the stages g, g + 3, ...; thread = row, lane
+//   warps 4-11   epilogue of the CTA's own 128 accumulator rows (two warps per lane quadrant, 128 columns each)
+//   warps 12-23  A converters: three sets of four warps, set g takes the stages g, g + 3, ...; thread = row, lane
 //                quadrant = warp % 4
-//   warps 22-27  B converters: three sets of two warps, same rotation
+//   warps 2-3 and 24-27  B converters: three sets of two warps, same rotation
 //   With K split over the pairs of a cluster (SPLIT > 1, see the kernel) each pair has its own leader and rings, the epilogue
 //   warps stop at the accumulator barrier, and then every warp takes part in the exchange: warps 2-17 lay the blocks down and
 //   send them, all 28 add and store.
@@ -51,6 +53,7 @@
 // Every mbarrier wait is bounded; a wait that runs out records a code in the device status word and its role leaves.
 // The cluster barriers at set-up and tear-down are hardware barriers that every thread of both CTAs reaches.
 #include <mutex>
+#include <type_traits>
 
 #include "qo_internal.cuh"
 #include "sm100_ptx.cuh"
@@ -75,18 +78,25 @@ constexpr int kOBBytes = 2 * kOAtomBytes;               // 32 KB per operand sta
 constexpr int kOffP = 0;
 constexpr int kOffO = kOffP + kPStages * kPStageBytes;  // 96 KB
 constexpr int kRingBytes = kOffO + kOStages * kOBBytes;  // +96 KB
-// Behind the rings: SPLIT = 1: column scales, 8 epilogue warps x 128 floats.  SPLIT > 1: the exchange of partial sums takes
-// 224 KB (the rings and 32 KB more), behind it 256 column and 128 row scales.
+constexpr int kStoreBytes = 4096;                        // an epilogue warp's outputs on their way: 32 rows x 64 columns
+// Behind the rings: SPLIT = 1: outputs and 64 column scales of each of the 8 epilogue warps.  SPLIT > 1: the exchange of partial
+// sums takes 224 KB (the rings and 32 KB more), behind it 256 column and 128 row scales.
 template <int SPLIT>
 struct Smem {
-  static constexpr int kOffSb = SPLIT == 1 ? kRingBytes : 224 * 1024;
+  static constexpr int kOffOut = kRingBytes;       // SPLIT = 1 only
+  static constexpr int kOffSb = SPLIT == 1 ? kOffOut + 8 * kStoreBytes : 224 * 1024;
   static constexpr int kOffSa = kOffSb + 256 * 4;  // SPLIT > 1 only
-  static constexpr int kOffBar = kOffSb + (SPLIT == 1 ? 8 * 128 * 4 : 384 * 4);
-  static constexpr int kBytes = kOffBar + 512 + 1024;
+  static constexpr int kOffBar = kOffSb + (SPLIT == 1 ? 8 * 64 * 4 : 384 * 4);
+  static constexpr int kBytes = kOffBar + 128 + 896;  // barriers; room to start on a 1024-byte boundary (the window itself starts on 128)
   static_assert(kBytes <= 227 * 1024, "shared memory of one CTA");
 };
-constexpr int kColA = kBN;      // first tensor-memory column of the A operand stages (64 columns each)
-constexpr int kEpiWarp0 = 2, kAWarp0 = 10, kBWarp0 = 22;
+constexpr int kAccShift = 64;   // the accumulators of successive items start at tensor-memory columns 0 and 64 in turn
+constexpr int kColA = kBN + kAccShift;  // first tensor-memory column of the A operand stages (64 columns each)
+constexpr int kShortSums = 65536;  // up to this K a sum fits 22 bits and a sign
+constexpr int kBPiecesA = 3;
+constexpr int kEpiWarp0 = 4, kAWarp0 = 12, kBWarp0 = 24;
+// registers per thread behind the role split (SPLIT = 1), by warpgroup: 2 x 128 + 5 x 48 = 496 of the 7 x 72 = 504 of the launch
+constexpr int kRegsEpilogue = 128, kRegsRest = 48;
 
 struct Bars {
   uint64_t p_full[kPStages], p_empty[kPStages];
@@ -95,6 +105,7 @@ struct Bars {
   uint64_t exchange;  // bytes of the other pairs' partial sums (SPLIT > 1)
   uint32_t tmem_base;
 };
+static_assert(sizeof(Bars) <= 128, "barriers");
 
 template <typename OutT>
 __device__ __forceinline__ uint32_t pack_out2(float a, float b);
@@ -111,6 +122,77 @@ __device__ __forceinline__ uint32_t pack_out2<__nv_bfloat16>(float a, float b) {
 __device__ __forceinline__ float2 unpack_out2(uint32_t w, __half) { return __half22float2(*reinterpret_cast<__half2*>(&w)); }
 __device__ __forceinline__ float2 unpack_out2(uint32_t w, __nv_bfloat16) { return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w)); }
 
+// Two sums (float bits, see below) -> ((sum + shift) * row) * column, packed; two operations to an instruction, each rounded by itself.
+template <typename OutT>
+__device__ __forceinline__ uint32_t scale_out2(uint32_t a, uint32_t b, float shift, float row, float ca, float cb) {
+  float x = __uint_as_float(a), y = __uint_as_float(b);
+  asm("{\n\t"
+      ".reg .b64 v, m, r, c;\n\t"
+      "mov.b64 v, {%0, %1};\n\t"
+      "mov.b64 m, {%5, %5};\n\t"
+      "mov.b64 r, {%2, %2};\n\t"
+      "mov.b64 c, {%3, %4};\n\t"
+      "add.rn.f32x2 v, v, m;\n\t"
+      "mul.rn.f32x2 v, v, r;\n\t"
+      "mul.rn.f32x2 v, v, c;\n\t"
+      "mov.b64 {%0, %1}, v;\n\t"
+      "}\n"
+      : "+f"(x), "+f"(y) : "f"(row), "f"(ca), "f"(cb), "f"(shift));
+  return pack_out2<OutT>(x, y);
+}
+__device__ __forceinline__ uint32_t add_out2(uint32_t a, uint32_t b, __half) {
+  const __half2 r = __hadd2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t add_out2(uint32_t a, uint32_t b, __nv_bfloat16) {
+  const __nv_bfloat162 r = __hadd2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// 16 accumulators of one row -> 16-bit outputs, laid down in shared memory as the 16-byte pieces `piece`, + 1 of the row's 64 bytes, XOR-
+// swizzled by bits 1 and 2 of the row (TMA's 64-byte swizzle).  The accumulators hold 256 times the sum (both operands carried the
+// factor 16).  Sums of at most 22 bits (K of 65536 and less) become floats by the shift and the addition of
+// 1.5 * 2^23's bit pattern, which are one integer instruction, and a subtraction; longer ones by a conversion.
+template <typename OutT>
+__device__ __forceinline__ void lay_down(const uint32_t* v, bool short_sums, float row, const float* columns, bool add_bias,
+                                         uint32_t bias_w, int bias_lane, uint32_t stage_row, int lane, int piece) {
+  constexpr int NV = 16;
+  uint32_t f[NV];
+  if (short_sums) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) f[i] = (uint32_t)(((int)v[i] >> 8) + 0x4B400000);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) f[i] = __float_as_uint((float)((int)v[i] >> 8));
+  }
+  const float shift = short_sums ? -12582912.f : -0.f;
+  uint32_t w[NV / 2];
+#pragma unroll
+  for (int j = 0; j < NV / 4; ++j) {
+    const float4 c = *reinterpret_cast<const float4*>(columns + 4 * j);
+    w[2 * j] = scale_out2<OutT>(f[4 * j], f[4 * j + 1], shift, row, c.x, c.y);
+    w[2 * j + 1] = scale_out2<OutT>(f[4 * j + 2], f[4 * j + 3], shift, row, c.z, c.w);
+  }
+  if (add_bias) {  // lane `bias_lane` + j holds the pair of columns of word j
+#pragma unroll
+    for (int j = 0; j < NV / 2; ++j) w[j] = add_out2(w[j], __shfl_sync(0xffffffffu, bias_w, bias_lane + j), OutT());
+  }
+#pragma unroll
+  for (int j = 0; j < NV / 8; ++j)
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(stage_row + (uint32_t)(((piece + j) ^ ((lane >> 1) & 3)) << 4)), "r"(w[4 * j]),
+                 "r"(w[4 * j + 1]), "r"(w[4 * j + 2]), "r"(w[4 * j + 3]) : "memory");
+}
+
+// the accumulators themselves as a second output
+template <int NV>
+__device__ __forceinline__ void store_sums(const uint32_t (&v)[NV], int32_t* row, int col, int n) {
+#pragma unroll
+  for (int j = 0; j < NV / 4; ++j)
+    if (col + 4 * j < n)
+      reinterpret_cast<uint4*>(row + col)[j] = make_uint4((uint32_t)((int)v[4 * j] >> 8), (uint32_t)((int)v[4 * j + 1] >> 8),
+                                                          (uint32_t)((int)v[4 * j + 2] >> 8), (uint32_t)((int)v[4 * j + 3] >> 8));
+}
+
 // packed word -> (even elements, odd elements) as int8 bytes holding 16 * value
 __device__ __forceinline__ void split16(uint32_t w, uint32_t& even, uint32_t& odd) {
   // the shift as an integer multiply-add (FMA pipe), the mask and the sign flip of each operand as one three-input
@@ -119,6 +201,28 @@ __device__ __forceinline__ void split16(uint32_t w, uint32_t& even, uint32_t& od
   asm("mad.lo.u32 %0, %1, 16, 0;" : "=r"(w16) : "r"(w));
   asm("lop3.b32 %0, %1, 0xF0F0F0F0, 0x80808080, 0x6A;" : "=r"(even) : "r"(w16));  // (a & b) ^ c
   asm("lop3.b32 %0, %1, 0xF0F0F0F0, 0x80808080, 0x6A;" : "=r"(odd) : "r"(w));
+}
+
+// Piece c (0 .. 7) of a packed B row: 16 bytes, 32 values.  `src` is the stage's B block: rows of 128 bytes, 128-byte swizzle, or
+// (BCOLS) 32 rows of words of K.  (smem offsets of a row: its start on 128 bytes | swizzle, so that a piece is one XOR away)
+template <bool BCOLS>
+__device__ __forceinline__ uint4 load_b_piece(uint32_t src, int row, int c) {
+  if (BCOLS) {
+    const uint32_t col = src + (uint32_t)(row * 4 + c * 4 * kBNh * 4);  // word 4c of this channel
+    return make_uint4(ld_shared_u32(col), ld_shared_u32(col + kBNh * 4), ld_shared_u32(col + 2 * kBNh * 4), ld_shared_u32(col + 3 * kBNh * 4));
+  }
+  return ld_shared_v4((src + (uint32_t)(row * 128) | (uint32_t)((row & 7) << 4)) ^ (uint32_t)(c << 4));
+}
+// the same piece as int8 into the operand stage: K values 32c .. 32c + 31 are K atom c >> 2, 16-byte pieces 2 (c & 3) and the next
+__device__ __forceinline__ void store_b_piece(uint32_t dst, int row, int c, uint4 p) {
+  uint32_t o[8];
+  split16(p.x, o[0], o[1]);
+  split16(p.y, o[2], o[3]);
+  split16(p.z, o[4], o[5]);
+  split16(p.w, o[6], o[7]);
+  const uint32_t at = ((dst + (uint32_t)((c >> 2) * kOAtomBytes + row * 128)) | (uint32_t)((row & 7) << 4)) ^ (uint32_t)((2 * (c & 3)) << 4);
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at ^ 16u), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
 }
 
 // One stage of the leader's issue loop as a single instruction sequence: probe the NEXT stage's "operands ready"
@@ -190,10 +294,11 @@ __device__ __forceinline__ bool issue_stage(uint32_t d_tmem, uint32_t a_tmem, ui
 template <typename OutT, bool GATHER, int SPLIT, bool BCOLS>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap b_map,
+                      const __grid_constant__ CUtensorMap out_map,
                       const float* sa, const float* sb, OutT* __restrict__ out,
                       int32_t* __restrict__ acc_out, const OutT* bias, int t, int n, int k, int items, int cut_from,
                       int b_early, uint32_t* __restrict__ status, const __grid_constant__ GatherDsts dsts) {
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(128) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   using S = Smem<SPLIT>;
   Bars* bars = reinterpret_cast<Bars*>(smem + S::kOffBar);
@@ -231,6 +336,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
     fence_barrier_init();
     prefetch_tensormap(&a_map);
     prefetch_tensormap(&b_map);
+    if (SPLIT == 1 && !GATHER) prefetch_tensormap(&out_map);
   }
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(&bars->tmem_base), 512);
@@ -253,20 +359,176 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       else tma_load_2d(dst, &b_map, bar, (ks_first + s) * 128, row_b);
     }
   }
-  // Launched with programmatic stream serialization: everything above may overlap the tail of the preceding kernel.
-  grid_dependency_wait();
+  // Launched with programmatic stream serialization: everything above may overlap the tail of the preceding kernel.  Each role that
+  // touches global memory waits for that kernel first (with K split, every warp does in the end).
 
+  if (SPLIT > 1) grid_dependency_wait();
+  // A block of 32 rows x 32 columns that the warp has laid down at `stage`, to the outputs.
+  auto send_block = [&](uint32_t stage, int row0, int col0) {
+    if (GATHER) {
+      // (plain stores, four lanes to the 64 bytes of a row; the host admits only buffers whose rows start on 32 bytes)
+      __syncwarp();
+      for (int r = lane >> 2; r < 32 && row0 + r < t; r += 8) {
+        const int p = lane & 3;
+        const uint4 o = ld_shared_v4(stage + (uint32_t)(r * 64 + ((p ^ ((r >> 1) & 3)) << 4)));
+        if (col0 + 8 * p < n)
+          for (int d = 0; d < dsts.n_dst; ++d)
+            *reinterpret_cast<uint4*>(reinterpret_cast<OutT*>(dsts.ptr[d]) + (int64_t)(row0 + r + dsts.row_offset) * n + col0 + 8 * p) = o;
+      }
+      __syncwarp();
+    } else {
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&out_map, stage, col0, row0);  // (rows and columns past the end are not written)
+        bulk_commit();
+      }
+    }
+  };
+  if (warp >= kEpiWarp0 && warp < kAWarp0) {
+    if constexpr (SPLIT == 1) regs_inc<kRegsEpilogue>();
+    // ---- epilogue: the CTA's own 128 rows of the tile; warp (q, half) takes four blocks of 32 columns of lanes 32 q .. ------
+    // The next item's MMAs cannot start before this item's accumulators have been read out of the columns that both use: all but
+    // 64.  A warp therefore takes its three blocks of the shared columns into registers at once, says that the accumulator is free,
+    // and converts and stores under the next item's main loop.  A block leaves through shared memory by TMA: stores by the
+    // lanes that own the rows touched 32 lines at a time, a line per cycle.
+    // Measured at 16 stages per item (about 17000 cycles of MMAs): from the last MMA's issue to the first of the next item 5500
+    // cycles with the blocks one after the other and stores by row, 1900 now; graph replay, before / now: 500 x 4096 x 9472 (one item per
+    // pair) 18.7 / 18.2 us, 2048 x 4096 x 9472 (four) 57.0 / 52.2, 4096 x 4096 x 4096 54.4 / 49.1, 777 x 4096 x 11008 41.2 / 38.2.
+    // What overlaps costs the main loop about 1000 cycles per item (shared memory is as busy as the tensor cores).
+    const int q = warp & 3, half = (warp - kEpiWarp0) >> 2;
+    float* sb_s = reinterpret_cast<float*>(smem + S::kOffSb) + (SPLIT == 1 ? (warp - kEpiWarp0) * 64 : half * 128);
+    const uint32_t staging = smem_base + S::kOffOut + (warp - kEpiWarp0) * kStoreBytes;
+    grid_dependency_wait();
+#pragma unroll 1
+    for (int lt = 0; lt < mine; ++lt) {
+      int tile, col_in_tile, width;
+      item_of(pair + lt * npairs, tile, col_in_tile, width);
+      const int mb = tile / tiles_n, nb = tile - mb * tiles_n;
+      const int row0 = mb * 2 * kBM + (int)rank * kBM + q * 32;  // first row of this warp
+      const int colt = nb * kBN + col_in_tile;                   // first column of the item
+      const float s_row = row0 + lane < t ? (SPLIT == 1 ? sa[row0 + lane] : sa[row0 + lane] * 0.00390625f) : 0.f;
+      // blocks of 32 columns in the order in which this warp takes them (a half item has two for each warp)
+      const bool last = lt == mine - 1;
+      const bool whole = width == kBN;
+      const int shared_from = (lt & 1) ? 0 : kAccShift / 32;  // first block of those that the next accumulator overlaps
+      auto block = [&](int i) {
+        if (!whole) return 2 * half + i;
+        return i < 2 ? shared_from + 4 * half + i : i == 2 ? shared_from + 2 + half : ((lt & 1) ? 6 : 0) + half;
+      };
+      // scales and biases of blocks i and i + 1: a lane has one column of each, and a pair of columns of one of them (lanes 0 .. 15 of
+      // block i)
+      float sb_r[2];
+      uint32_t bias_w = 0u;
+      auto load_columns = [&](int i) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int c = colt + 32 * block(i + h) + lane;
+          sb_r[h] = c < n ? sb[c] : 0.f;
+        }
+        const int cb = colt + 32 * block(i + (lane >> 4)) + 2 * (lane & 15);
+        return bias != nullptr && cb < n ? *reinterpret_cast<const uint32_t*>(bias + cb) : 0u;
+      };
+      auto share_columns = [&] {
+        __syncwarp();
+        sb_s[lane] = sb_r[0];
+        sb_s[32 + lane] = sb_r[1];
+        __syncwarp();
+      };
+      __syncwarp();
+      if (SPLIT == 1) {
+        bias_w = load_columns(0);
+        if (lane == 0) bulk_wait_read<0>();  // the item before has left
+        share_columns();
+      } else if (q == 0) {
+        for (int i = lane; i < 128; i += 32) sb_s[i] = colt + half * 128 + i < n ? sb[colt + half * 128 + i] : 0.f;
+      }
+      if (SPLIT > 1 && half == 0) reinterpret_cast<float*>(smem + S::kOffSa)[q * 32 + lane] = s_row;
+      __syncwarp();
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_full), lt & 1))) { atomicCAS(status, 0u, 0xA30u); break; }
+      if (SPLIT > 1) break;  // every MMA of this pair is done; the partial sums are exchanged below
+      tc_fence_after();
+      const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (lt & 1) * kAccShift;
+      auto release = [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          const uint32_t e = smem_u32(&bars->acc_empty);
+          if (rank == 0) mbar_arrive(e); else mbar_arrive_cluster(cluster_map_shared(e, leader));
+        }
+      };
+      // block i, whose accumulators are in v, to the outputs
+      auto emit = [&](int i, const uint32_t (&v)[32], bool short_sums) {
+        const int col0 = colt + 32 * block(i);
+        if (row0 >= t || col0 >= n) {
+          if (lane == 0) bulk_commit();  // an empty group: the waits count one per block
+          return;
+        }
+        const uint32_t stage = staging + (uint32_t)(i & 1) * (kStoreBytes / 2);
+        if (i >= 2) {
+          if (lane == 0) bulk_wait_read<1>();  // the block that was laid down here before has left
+          __syncwarp();
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          lay_down<OutT>(v + 16 * h, short_sums, s_row, sb_s + 32 * (i & 1) + 16 * h, bias != nullptr, bias_w, 16 * (i & 1) + 8 * h,
+                         stage + (uint32_t)(lane * 64), lane, 2 * h);
+        send_block(stage, row0, col0);
+      };
+      if (acc_out == nullptr && k <= kShortSums) {
+        uint32_t v[3][32];
+        tmem_ld_32x32b_x32(acc + 32 * block(0), v[0]);
+        tmem_ld_32x32b_x32(acc + 32 * block(1), v[1]);
+        if (whole) tmem_ld_32x32b_x32(acc + 32 * block(2), v[2]);
+        tmem_ld_wait_for(v[0]);
+        tmem_ld_wait_for(v[1]);
+        tmem_ld_wait_for(v[2]);
+        if (!last) release();
+        emit(0, v[0], true);
+        const uint32_t bias_late = whole ? load_columns(2) : 0u;
+        emit(1, v[1], true);
+        if (whole) {
+          tmem_ld_32x32b_x32(acc + 32 * block(3), v[0]);
+          share_columns();
+          bias_w = bias_late;
+          emit(2, v[2], true);
+          tmem_ld_wait_for(v[0]);
+          emit(3, v[0], true);
+        }
+      } else {
+        // with the accumulators themselves as a second output, or sums of more bits: block by block
+#pragma unroll 1
+        for (int i = 0; i < (whole ? 4 : 2); ++i) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(acc + 32 * block(i), v);
+          tmem_ld_wait_for(v);
+          if (!last && i == 3) release();  // (a half item is always a pair's last)
+          if (i == 2) {
+            bias_w = load_columns(2);
+            share_columns();
+          }
+          if (acc_out != nullptr && row0 + lane < t) store_sums(v, acc_out + (int64_t)(row0 + lane) * n, colt + 32 * block(i), n);
+          emit(i, v, k <= kShortSums);
+        }
+      }
+    }
+    if (SPLIT == 1 && lane == 0) bulk_wait_read<0>();  // the outputs have left before the block's shared memory goes
+  } else {
+  if constexpr (SPLIT == 1) regs_dec<kRegsRest>();
   if (warp == 0) {
     // ---- TMA producer -------------------------------------------------------------------------------------------
+    grid_dependency_wait();
     if (lane == 0) {
       int step = 0;
       bool ok = true;
+#pragma unroll 1
       for (int item = pair; ok && item < items; item += npairs) {
         int tile, col_in_tile, width;
         item_of(item, tile, col_in_tile, width);
         const int mb = tile / tiles_n, nb = tile - mb * tiles_n;
         // a CTA stages its half of the item's B rows; the box always has 128 rows, of which a half item uses the first 64
         const int row_a = mb * 2 * kBM + (int)rank * kBM, row_b = nb * kBN + col_in_tile + (int)rank * (width >> 1);
+#pragma unroll 1
         for (int ks = 0; ks < ksteps; ++ks, ++step) {
           const int ps = step % kPStages, pph = (step / kPStages) & 1;
           const uint32_t bar = smem_u32(&bars->p_full[ps]);
@@ -296,9 +558,15 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       const uint32_t acc_full = smem_u32(&bars->acc_full), acc_full_peer = cluster_map_shared(acc_full, other);
       int step = 0;
       bool ok = true, ready = false;  // ready: the operands of `step` were already seen complete by an early probe
+#pragma unroll 1
       for (int lt = 0; ok && lt < mine; ++lt) {
-        if (!mbar_wait(smem_u32(&bars->acc_empty), (lt & 1) ^ 1)) { atomicCAS(status, 0u, 0xA10u); break; }
+        // the item's first operands are looked for before the accumulator, so that the answer comes while that is being drained
+        if (!ready && !mbar_wait(smem_u32(&bars->op_ready[step % kOStages]), (step / kOStages) & 1)) { atomicCAS(status, 0u, 0xA20u); break; }
+        ready = true;
+        if (lt > 0 && !mbar_wait(smem_u32(&bars->acc_empty), (lt & 1) ^ 1)) { atomicCAS(status, 0u, 0xA10u); break; }
+        const uint32_t d_tmem = tmem + (lt & 1) * kAccShift;
         const uint32_t idesc = pair + lt * npairs >= cut_from ? idesc_half : idesc_whole;
+#pragma unroll 1
         for (int ks = 0; ks < ksteps; ++ks, ++step) {
           const int s = step % kOStages, ph = (step / kOStages) & 1;
           if (!ready && !mbar_wait(smem_u32(&bars->op_ready[s]), ph)) { atomicCAS(status, 0u, 0xA20u + s); ok = false; break; }
@@ -307,7 +575,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
           const bool last = step + 1 >= total_steps;
           const int sn = last ? s : (step + 1) % kOStages, phn = last ? ph : ((step + 1) / kOStages) & 1;
           tc_fence_after();
-          ready = issue_stage(tmem, tmem + kColA + s * 64, b_desc0 + (uint64_t)(s * (kOBBytes >> 4)), idesc, ks != 0,
+          ready = issue_stage(d_tmem, tmem + kColA + s * 64, b_desc0 + (uint64_t)(s * (kOBBytes >> 4)), idesc, ks != 0,
                               op_empty0 + s * 8, op_empty0_peer + s * 8, smem_u32(&bars->op_ready[sn]), phn) && !last;
         }
         if (ok) {
@@ -316,128 +584,49 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
         }
       }
     }
-  } else if (warp < kAWarp0) {
-    // ---- epilogue: the CTA's own 128 rows of the tile; warp (q, half) takes columns 128 half .. of lanes 32 q .. ------
-    const int q = warp & 3, half = (warp - kEpiWarp0) >> 2;
-    const bool wide_stores = (n % 16) == 0 && (reinterpret_cast<uintptr_t>(out) % 32) == 0;  // rows start on 32-byte boundaries
-    float* sb_s = reinterpret_cast<float*>(smem + S::kOffSb) + (SPLIT == 1 ? warp - kEpiWarp0 : half) * 128;
-    for (int lt = 0; lt < mine; ++lt) {
-      int tile, col_in_tile, width;
-      item_of(pair + lt * npairs, tile, col_in_tile, width);
-      const int mb = tile / tiles_n, nb = tile - mb * tiles_n;
-      const int wcols = width >> 1;  // columns of this warp: 128, or 64 of a half item
-      const int row = mb * 2 * kBM + (int)rank * kBM + q * 32 + lane;
-      const bool row_ok = row < t;
-      // Both operands carried the factor 16.  float(256 * acc) is exact (|acc| < 2^23) and scaling by a power of two
-      // commutes with rounding, so the factor is taken out of the row scale instead of out of every accumulator.
-      const float s_row = row_ok ? sa[row] * 0.00390625f : 0.f;
-      const int colw = nb * kBN + col_in_tile + half * wcols;  // first column of this warp
-      __syncwarp();
-      if (SPLIT == 1 || q == 0)
-        for (int i = lane; i < wcols; i += 32) sb_s[i] = (colw + i < n) ? sb[colw + i] : 0.f;
-      if (SPLIT > 1 && half == 0) reinterpret_cast<float*>(smem + S::kOffSa)[q * 32 + lane] = s_row;
-      __syncwarp();
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_full), lt & 1))) { atomicCAS(status, 0u, 0xA30u); break; }
-      if (SPLIT > 1) break;  // every MMA of this pair is done; the partial sums are exchanged below
-      tc_fence_after();
-#pragma unroll 1
-      for (int cc = 0; cc < wcols; cc += 32) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(tmem + ((uint32_t)(q * 32) << 16) + half * wcols + cc, v);
-        tmem_ld_wait();
-        if (cc + 32 == wcols) {
-          // the last accumulator values of this warp are in registers: the next tile's MMAs may overwrite them
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            const uint32_t e = smem_u32(&bars->acc_empty);
-            if (rank == 0) mbar_arrive(e); else mbar_arrive_cluster(cluster_map_shared(e, leader));
-          }
-        }
-        const int col0 = colw + cc;
-        if (row_ok && col0 < n) {
-          const int64_t off = (int64_t)(GATHER ? row + dsts.row_offset : row) * n + col0;
-          // 16 columns at a time: eight packed words live beside the 32 accumulators, not sixteen
-#pragma unroll
-          for (int jh = 0; jh < 2; ++jh) {
-            if (col0 + 16 * jh >= n) break;
-            uint32_t w[8];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float4 sc = *reinterpret_cast<const float4*>(sb_s + cc + 16 * jh + 4 * j);
-              const uint32_t* vv = v + 16 * jh + 4 * j;
-              w[2 * j] = pack_out2<OutT>(((float)(int)vv[0] * s_row) * sc.x, ((float)(int)vv[1] * s_row) * sc.y);
-              w[2 * j + 1] = pack_out2<OutT>(((float)(int)vv[2] * s_row) * sc.z, ((float)(int)vv[3] * s_row) * sc.w);
-            }
-            if (bias != nullptr) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                if (col0 + 16 * jh + 2 * j < n) {
-                  const float2 o = unpack_out2(w[j], OutT());
-                  const float2 bb = unpack_out2(*reinterpret_cast<const uint32_t*>(bias + col0 + 16 * jh + 2 * j), OutT());
-                  w[j] = pack_out2<OutT>(o.x + bb.x, o.y + bb.y);
-                }
-              }
-            }
-            // A lane owns a row, so a warp's store instruction touches 32 different lines; the exposed part of the
-            // epilogue is bound by those line accesses.  32-byte stores (whole sectors) halve their number.
-            if (GATHER) {
-              // (the host admits only row lengths and buffers that make every piece a whole 32-byte sector)
-              for (int d = 0; d < dsts.n_dst; ++d)
-                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(reinterpret_cast<OutT*>(dsts.ptr[d]) + off + 16 * jh),
-                             "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
-            } else if (wide_stores) {
-              asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + off + 16 * jh), "r"(w[0]), "r"(w[1]), "r"(w[2]),
-                           "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
-            } else {
-              reinterpret_cast<uint4*>(out + off + 16 * jh)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-              if (col0 + 16 * jh + 8 < n) reinterpret_cast<uint4*>(out + off + 16 * jh)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-            }
-          }
-          if (acc_out != nullptr) {
-            int32_t* arow = acc_out + (int64_t)row * n + col0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              if (col0 + 4 * j < n)
-                reinterpret_cast<uint4*>(arow)[j] = make_uint4((uint32_t)((int)v[4 * j] >> 8), (uint32_t)((int)v[4 * j + 1] >> 8),
-                                                               (uint32_t)((int)v[4 * j + 2] >> 8), (uint32_t)((int)v[4 * j + 3] >> 8));
-          }
-        }
-        __syncwarp();
-      }
-    }
-  } else if (warp < kBWarp0) {
-    // ---- A converters: set e takes the stages e, e + 3, ...; thread = one row of the CTA's A block ---------------------
+  } else if (warp >= kAWarp0 && warp < kBWarp0) {
+    // ---- A converters: set e takes the stages e, e + 3, ...; thread = one row of the CTA's A block, and the last pieces of
+    // the same row of B, so that a stage's converters take about the same time -----------------------------------------------
     const int e = (warp - kAWarp0) >> 2, q = warp & 3, r = q * 32 + lane;  // set 0 .. 2
-    const uint32_t row_off = (uint32_t)(r * 128), sw = (uint32_t)(r & 7);
-    for (int step = e; step < total_steps; step += kSets) {
-      const int ps = step % kPStages, pph = (step / kPStages) & 1;
-      const int s = step % kOStages, ph = (step / kOStages) & 1;
-      if (__any_sync(0xffffffffu, mbar_wait2(smem_u32(&bars->p_full[ps]), pph, smem_u32(&bars->op_empty[s]), ph ^ 1) != 0)) {
-        atomicCAS(status, 0u, 0xA40u + ps);
+    const uint32_t sw = (uint32_t)((r & 7) << 4);
+#pragma unroll 1
+    for (int step = e, ph = 0; step < total_steps; step += kSets, ph ^= 1) {
+      int s = e;  // the slot of both rings; not known to the compiler, which would keep all of the stage's addresses in registers
+      asm volatile("" : "+r"(s));
+      if (__any_sync(0xffffffffu, mbar_wait2(smem_u32(&bars->p_full[s]), ph, smem_u32(&bars->op_empty[s]), ph ^ 1) != 0)) {
+        atomicCAS(status, 0u, 0xA40u + s);
         break;
       }
       tc_fence_after();
-      const uint32_t src = smem_base + kOffP + ps * kPStageBytes + row_off;
+      const uint32_t stage = smem_base + kOffP + s * kPStageBytes;
+      const uint32_t src = (stage + (uint32_t)(r * 128)) | sw;  // (rows start on 128 bytes: piece c is at src ^ 16 c)
+      // four 16-byte pieces in flight, two of them (16 tensor-memory columns) converted at a time
+      uint4 p[4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint4 p[4];
+      for (int c = 0; c < 4; ++c) p[c] = ld_shared_v4(src ^ (uint32_t)(c << 4));
 #pragma unroll
-        for (int c = 0; c < 4; ++c) p[c] = ld_shared_v4(src + (((uint32_t)(4 * h + c) ^ sw) << 4));
-        uint32_t v[32];
+      for (int h = 0; h < 4; ++h) {
+        uint32_t v[16];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          split16(p[c].x, v[8 * c + 0], v[8 * c + 1]);
-          split16(p[c].y, v[8 * c + 2], v[8 * c + 3]);
-          split16(p[c].z, v[8 * c + 4], v[8 * c + 5]);
-          split16(p[c].w, v[8 * c + 6], v[8 * c + 7]);
+        for (int c = 0; c < 2; ++c) {
+          const int o = (2 * h + c) & 3;
+          split16(p[o].x, v[8 * c + 0], v[8 * c + 1]);
+          split16(p[o].y, v[8 * c + 2], v[8 * c + 3]);
+          split16(p[o].z, v[8 * c + 4], v[8 * c + 5]);
+          split16(p[o].w, v[8 * c + 6], v[8 * c + 7]);
+          if (h < 2) p[o] = ld_shared_v4(src ^ (uint32_t)((2 * h + c + 4) << 4));
+          else if (2 * h + c - 4 < kBPiecesA) p[o] = load_b_piece<BCOLS>(stage + kPABytes, r, 8 - kBPiecesA + 2 * h + c - 4);
         }
-        tmem_st_32x32b_x32(tmem + ((uint32_t)(q * 32) << 16) + kColA + s * 64 + h * 32, v);
+        tmem_st_32x32b_x16(tmem + ((uint32_t)(q * 32) << 16) + kColA + s * 64 + h * 16, v);
       }
+#pragma unroll
+      for (int i = 0; i < kBPiecesA; ++i) store_b_piece(smem_base + kOffO + s * kOBBytes, r, 8 - kBPiecesA + i, p[i]);
       // The packed stage is released only here, after instructions that consume every loaded value: an arrival placed
       // right behind the ld.shared instructions was measured to let the next TMA overwrite rows that some lanes had
       // not read yet (nothing orders another lane's outstanding loads before lane 0's arrival).
-      mbar_arrive_warp(smem_u32(&bars->p_empty[ps]));
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bars->p_empty[s]));
+      fence_proxy_async_smem();  // the tensor core reads the int8 stage through the async proxy
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -447,57 +636,39 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       }
     }
   } else {
-    // ---- B converters: 128 rows x 8 packed 16-byte pieces per stage, sixteen per thread of the set on duty; eight
-    // consecutive lanes take eight consecutive rows of one piece, which is conflict-free for the 128-byte-swizzled
-    // reads and writes ---------------------------------------------------------------------------------------------
-    const int f = (warp - kBWarp0) >> 1, bt = ((warp - kBWarp0) & 1) * 32 + lane;  // set 0 .. 2, thread within the set (0 .. 63)
-    for (int step = f; step < total_steps; step += kSets) {
-      const int ps = step % kPStages, pph = (step / kPStages) & 1;
-      const int s = step % kOStages, ph = (step / kOStages) & 1;
-      if (__any_sync(0xffffffffu, mbar_wait2(smem_u32(&bars->p_full[ps]), pph, smem_u32(&bars->op_empty[s]), ph ^ 1) != 0)) {
-        atomicCAS(status, 0u, 0xA50u + ps);
+    // ---- B converters: the first pieces of B's 128 rows, two rows per thread of the set on duty; eight consecutive lanes take
+    // eight consecutive rows of one piece, which is conflict-free for the 128-byte-swizzled reads and writes ---------------
+    const int f = warp < kBWarp0 ? 0 : 1 + ((warp - kBWarp0) >> 1), bt = (warp & 1) * 32 + lane;  // set 0 .. 2, thread within the set (0 .. 63)
+#pragma unroll 1
+    for (int step = f, ph = 0; step < total_steps; step += kSets, ph ^= 1) {
+      int s = f;  // (as above)
+      asm volatile("" : "+r"(s));
+      if (__any_sync(0xffffffffu, mbar_wait2(smem_u32(&bars->p_full[s]), ph, smem_u32(&bars->op_empty[s]), ph ^ 1) != 0)) {
+        atomicCAS(status, 0u, 0xA50u + s);
         break;
       }
-      const uint32_t src = smem_base + kOffP + ps * kPStageBytes + kPABytes;
+      const uint32_t src = smem_base + kOffP + s * kPStageBytes + kPABytes;
       const uint32_t dst = smem_base + kOffO + s * kOBBytes;
+      // piece c of rows bt and bt + 64; two pieces of a row ahead of the conversion
+      constexpr int kTasks = 2 * (8 - kBPiecesA);
+      uint4 p[4];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        uint4 p[4];
-        int rr[4], cc[4];
+      for (int i = 0; i < 4; ++i) p[i] = load_b_piece<BCOLS>(src, bt + 64 * (i & 1), i >> 1);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int task = (g * 4 + i) * 64 + bt;  // 0 .. 1023
-          cc[i] = task >> 7;                        // packed piece 0 .. 7 (32 values each)
-          rr[i] = task & 127;
-          if (BCOLS) {
-            const uint32_t col = src + (uint32_t)(cc[i] * 4 * kBNh * 4 + rr[i] * 4);  // word 4c of this channel
-            p[i] = make_uint4(ld_shared_u32(col), ld_shared_u32(col + kBNh * 4), ld_shared_u32(col + 2 * kBNh * 4), ld_shared_u32(col + 3 * kBNh * 4));
-          } else {
-            p[i] = ld_shared_v4(src + (uint32_t)(rr[i] * 128) + (((uint32_t)cc[i] ^ (uint32_t)(rr[i] & 7)) << 4));
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint32_t o[8];
-          split16(p[i].x, o[0], o[1]);
-          split16(p[i].y, o[2], o[3]);
-          split16(p[i].z, o[4], o[5]);
-          split16(p[i].w, o[6], o[7]);
-          // piece c holds K values 32c .. 32c+31 = int8 bytes 32c .. of the row: K atom c >> 2, 16-byte pieces 2(c & 3), +1
-          const uint32_t rowp = dst + (uint32_t)((cc[i] >> 2) * kOAtomBytes + rr[i] * 128), x = (uint32_t)(rr[i] & 7);
-          const uint32_t j0 = (uint32_t)(2 * (cc[i] & 3));
-          asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(rowp + ((j0 ^ x) << 4)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-          asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(rowp + (((j0 + 1) ^ x) << 4)), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
-        }
+      for (int i = 0; i < kTasks; ++i) {
+        store_b_piece(dst, bt + 64 * (i & 1), i >> 1, p[i & 3]);
+        if (i + 4 < kTasks) p[i & 3] = load_b_piece<BCOLS>(src, bt + 64 * (i & 1), (i + 4) >> 1);
       }
-      mbar_arrive_warp(smem_u32(&bars->p_empty[ps]));  // every loaded value has been consumed by the stores above
-      fence_proxy_async_smem();  // the tensor core reads the stage through the async proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bars->p_empty[s]));  // every loaded value has been consumed by the stores above
+      fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
         const uint32_t ready = smem_u32(&bars->op_ready[s]);
         if (rank == 0) mbar_arrive(ready); else mbar_arrive_cluster(cluster_map_shared(ready, leader));
       }
     }
+  }
   }
 
   if (SPLIT > 1) {
@@ -601,11 +772,9 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
   }
   tc_fence_before();
   __syncwarp();
-  // SPLIT = 1: the peer's last arrivals on the leader's barriers must have landed before the leader leaves, hence the
-  // releasing form.  SPLIT > 1: every remote arrival and copy has been waited for by its receiver, so no CTA's memory is
-  // written or read from outside any more, and the arrival need not wait for the output stores.
-  if (SPLIT == 1) cluster_sync_all();
-  else cluster_sync_relaxed();
+  // Every remote arrival and copy has been waited for by its receiver (the last item's accumulators are not handed back), so no CTA's
+  // memory is written or read from outside any more, and this barrier need not order the output stores.
+  cluster_sync_relaxed();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem, 512);
@@ -672,6 +841,18 @@ int make_map_packed_cols(CUtensorMap* map, const void* base, int64_t n, int64_t 
   return QO_OK;
 }
 
+// outputs [rows, n] of 16 bits (n a multiple of 8); boxes of 32 columns x 32 rows
+int make_map_out(CUtensorMap* map, void* base, int64_t rows, int64_t n) {
+  const cuuint64_t dims[2] = {(cuuint64_t)n, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)(n * 2)};
+  const cuuint32_t box[2] = {32u, 32u};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = unpack_encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                        CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(QO_ERR_CUDA, "int4_matmul: cuTensorMapEncodeTiled failed with code %d", (int)r);
+  return QO_OK;
+}
+
 // clusters of 2 * SPLIT CTAs of this kernel the device runs at once (0 if the query fails); cached per device
 template <typename OutT, bool GATHER, int SPLIT, bool BCOLS>
 int max_clusters(int dev) {
@@ -706,10 +887,15 @@ int launch_typed(const UnpackArgs& p, uint32_t* status, const GatherDsts& dsts, 
   if (clusters <= 0) return QO_ERR_UNSUPPORTED;
   const int64_t ntiles = unpack_tiles(p.t, p.n);
   if (SPLIT > 1 && ntiles > clusters) return QO_ERR_UNSUPPORTED;  // a second wave would cost more than the split saves
-  CUtensorMap a_map, b_map;
+  CUtensorMap a_map, b_map, out_map;
   int rc = make_map_packed(&a_map, p.a, p.t, p.k, p.lda, kBM);
   if (rc) return rc;
   if ((rc = BCOLS ? make_map_packed_cols(&b_map, p.b, p.n, p.k, p.ldb) : make_map_packed(&b_map, p.b, p.n, p.k, p.ldb, kBNh))) return rc;
+  if (SPLIT == 1 && !GATHER) {
+    if ((rc = make_map_out(&out_map, p.out, p.t, p.n))) return rc;
+  } else {
+    out_map = a_map;  // not used
+  }
   const int pairs = (int)(ntiles < clusters ? ntiles : clusters);
   // tiles of a last wave that would occupy at most half of the pairs are cut into halves of 128 columns
   const int64_t whole = (ntiles / pairs) * pairs, rest = ntiles - whole;
@@ -729,7 +915,7 @@ int launch_typed(const UnpackArgs& p, uint32_t* status, const GatherDsts& dsts, 
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  QO_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_s4_unpack_kernel<OutT, GATHER, SPLIT, BCOLS>, a_map, b_map, p.sa, p.sb, reinterpret_cast<OutT*>(p.out),
+  QO_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_s4_unpack_kernel<OutT, GATHER, SPLIT, BCOLS>, a_map, b_map, out_map, p.sa, p.sb, reinterpret_cast<OutT*>(p.out),
                                  p.acc_out, reinterpret_cast<const OutT*>(p.bias), (int)p.t, (int)p.n, (int)p.k, items, cut_from,
                                  p.b_early ? 1 : 0, status, dsts));
   return check_launch("gemm_s4_unpack_kernel");

@@ -1,0 +1,82 @@
+"""Outputs of the GEMM that unpacks inside the kernel where K is not split: the accumulator is handed on before the outputs are
+converted, items of a pair use its tensor memory in turn, and the outputs leave by TMA.  Bits of the kernels that multiply widened
+operands (policy 3), which share none of that, with nothing written past the last row or column."""
+import pytest
+import torch
+
+import quant_ops_b200 as q
+from helpers import N, QD, TD, lib, make_inputs, ptr, stream_ptr
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# one stage per item and many items per pair; two rounds of tiles with a ragged last column tile; halves of tiles in the last round;
+# a single row in the last row block; a single block of eight columns in the last column tile; one tile per pair
+SHAPES = [(2000, 256, 9480), (333, 4096, 14328), (777, 4096, 11008), (4097, 1024, 1032), (1600, 768, 2056), (500, 2048, 9472)]
+
+
+def product(a, b, sa, sb, out, dtype, policy):
+    t, k, n = a.shape[0], a.shape[1] * 8, b.shape[1]
+    ws = torch.empty(lib.qo_int4_matmul_workspace_bytes(t, k, n), dtype=torch.uint8, device=DEV)
+    N.check(lib.qo_set_kernel_policy(policy))
+    try:
+        N.check(lib.qo_int4_matmul(ptr(a), k // 8, ptr(b), b.stride(0), b.stride(1), ptr(sa), ptr(sb), ptr(out), QD[dtype], t, k, n,
+                                   ptr(None), ptr(ws), ws.numel(), stream_ptr()))
+    finally:
+        lib.qo_set_kernel_policy(0)
+    assert lib.qo_device_status(stream_ptr()) == N.QO_OK
+
+
+@pytest.mark.parametrize("t,k,n", SHAPES)
+@pytest.mark.parametrize("layout", ["weights_t_view", "reference_contiguous"])
+def test_outputs_and_nothing_else(t, k, n, layout):
+    g = torch.Generator(device=DEV).manual_seed(t + k + n)
+    words = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, dtype=torch.int64, device=DEV, generator=g).to(torch.int32)
+    a, w = words(t, k // 8), words(n, k // 8)
+    sa, sb = torch.rand(t, device=DEV, generator=g) + 0.01, torch.rand(n, device=DEV, generator=g) * 1e-4
+    b = w.t() if layout == "weights_t_view" else w.t().contiguous()
+    for dtype in ("fp16", "bf16"):
+        ref = torch.empty(t, n, dtype=TD[dtype], device=DEV)
+        product(a, b, sa, sb, ref, dtype, 3)
+        # outputs on a 16-byte boundary that is no 32-byte boundary, fenced on both sides
+        room = torch.full((t * n + 2 * n + 8,), 777.0, dtype=TD[dtype], device=DEV)
+        out = room[8 + n:8 + n + t * n].view(t, n)
+        for _ in range(3):
+            out.fill_(777.0)
+            before = lib.qo_kernel_launch_count()
+            product(a, b, sa, sb, out, dtype, 2)
+            assert lib.qo_kernel_launch_count() - before == 1  # one launch: no widening pass
+            assert torch.equal(out.view(torch.int16), ref.view(torch.int16))
+            assert bool((room[:8 + n] == 777.0).all()) and bool((room[8 + n + t * n:] == 777.0).all())
+
+
+@pytest.mark.parametrize("k", [65536, 65792])
+def test_longest_short_sums_and_shortest_long_ones(k):
+    """Up to K = 65536 a sum is made a float by adding its bits to 1.5 * 2^23's, which holds 22 bits and a sign: codes of -8 on both
+    sides reach 2^22 exactly, and pass it at the next K."""
+    t, n = 256, 38 * 256
+    g = torch.Generator(device=DEV).manual_seed(k)
+    a, w = torch.zeros(t, k // 8, dtype=torch.int32, device=DEV), torch.zeros(n, k // 8, dtype=torch.int32, device=DEV)
+    a[1::2] = -1  # odd rows: codes of 7 on one side, the most negative sums
+    a[2] = torch.randint(-2 ** 31, 2 ** 31, (k // 8,), dtype=torch.int64, device=DEV, generator=g).to(torch.int32)
+    sa, sb = torch.rand(t, device=DEV, generator=g) * 2.0 ** -10, torch.ones(n, device=DEV)
+    ref, out = torch.empty(t, n, dtype=torch.float16, device=DEV), torch.empty(t, n, dtype=torch.float16, device=DEV)
+    product(a, w.t(), sa, sb, ref, "fp16", 3)
+    before = lib.qo_kernel_launch_count()
+    product(a, w.t(), sa, sb, out, "fp16", 2)
+    assert lib.qo_kernel_launch_count() - before == 1
+    assert torch.equal(out.view(torch.int16), ref.view(torch.int16))
+    assert bool((out[0] == (64.0 * k * sa[0]).half()).all())
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("t,k,n", [(400, 4096, 9480), (777, 4096, 11008)])
+def test_bias_is_added_to_the_rounded_output(t, k, n, dtype):
+    x, left, right = (v.to(DEV) for v in make_inputs(t, k, dtype, seed=t + n))
+    g = torch.Generator(device=DEV).manual_seed(n)
+    w = torch.randint(-2 ** 31, 2 ** 31, (n, k // 8), dtype=torch.int64, device=DEV, generator=g).to(torch.int32)
+    sw = torch.rand(n, device=DEV, generator=g) * 1e-3
+    bias = torch.randn(n, device=DEV, generator=g).to(TD[dtype])
+    plain = q.w4a4_linear(x, left, right, w, sw, None, 0.9, TD[dtype])
+    got = q.w4a4_linear(x, left, right, w, sw, bias, 0.9, TD[dtype])
+    assert torch.equal(got, (plain.float() + bias.float()).to(TD[dtype]))
