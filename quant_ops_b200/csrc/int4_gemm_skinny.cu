@@ -91,7 +91,10 @@ int4_gemm_skinny_kernel(const uint32_t* a, int64_t lda, const uint32_t* b, int64
   // Launched with programmatic stream serialization, the kernel may start while its predecessor in the stream (the
   // activation quantizer) still runs.  weights_first: the weights are known not to come from that predecessor, so the
   // first batch of weight loads is issued before the wait and overlaps it; everything else comes after the wait.
-  if (!weights_first) ptx::grid_dependency_wait();
+  if (!weights_first) {
+    ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
+  }
   auto stage_activations = [&]() {
     if (STAGED) {
       const int per_row = nchunks * 4, total = tokens * per_row;
@@ -161,6 +164,7 @@ int4_gemm_skinny_kernel(const uint32_t* a, int64_t lda, const uint32_t* b, int64
   load(0, cb);
   if (weights_first) {
     ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
     stage_activations();
   }
   if (STAGED) {
@@ -242,6 +246,7 @@ int4_gemm_resident_kernel(const uint32_t* a, int64_t lda, const uint32_t* b, int
     for (int r = 0; r < nch; ++r) bulk_copy_g2s(base + (uint32_t)(r * stride4) * 16u, b + (c0 + r) * ldb, row_bytes, bar_a);
   }
   ptx::grid_dependency_wait();  // the codes and their scales are complete now
+  ptx::grid_launch_dependents();
 
   const uint4 zero4 = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);  // eight zeros per word
   const int per = (nchunks + kResWarps - 1) / kResWarps;
@@ -432,6 +437,7 @@ int4_gemm_even_kernel(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t
   const int cb = slice * per, ce = min(nchunks, cb + per);
   const uint4 zero4 = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);  // eight zeros per word
   ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   for (int64_t c0 = (int64_t)blockIdx.x * cpc; c0 < n; c0 += (int64_t)gridDim.x * cpc) {
     const int nch = (int)min((int64_t)cpc, n - c0);
     const int first = grp * cpg, mine = max(0, min(cpg, nch - first));  // this warp's channels of the CTA

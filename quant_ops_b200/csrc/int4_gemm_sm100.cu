@@ -199,6 +199,7 @@ gemm_s8_sm100_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_con
     }
   }
   grid_dependency_wait();
+  grid_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0) {

@@ -96,6 +96,7 @@ gemm_s8_pair_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_cons
   const uint32_t tmem = bars->tmem_base;
   // Launched with programmatic stream serialization: everything above may overlap the tail of the preceding kernel.
   grid_dependency_wait();
+  grid_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0) {

@@ -518,6 +518,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
   if (warp == 0) {
     // ---- TMA producer -------------------------------------------------------------------------------------------
     grid_dependency_wait();
+    grid_launch_dependents();  // the next kernel's launch and set-up overlap this one; it waits before it touches memory
     if (lane == 0) {
       int step = 0;
       bool ok = true;
