@@ -24,6 +24,7 @@
 // Every sum is one chain of fused multiply-adds in ascending k, as in flatquant_generic.cu: the results are the same
 // bits (reference: src/quant_ops/ops/quantization/flatquant/ops.py:99-117).
 #include "qo_internal.cuh"
+#include "sm100_ptx.cuh"
 
 namespace qo {
 namespace {
@@ -142,9 +143,11 @@ __device__ __forceinline__ void product_left(Block& acc, const float* l, int m8,
 // the CTA's teams of `team` threads work on their own groups of tokens; otherwise the CTA is one team.
 template <int MODE, int THREADS, bool RESIDENT>
 __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
-flatquant_f32_kernel(const float* __restrict__ x, int64_t ldx, const float* __restrict__ left, const float* __restrict__ right,
-                     void* __restrict__ codes, void* __restrict__ scales, int64_t tokens, int m, int n, int group, int team, int chunk_rows,
+flatquant_f32_kernel(const float* x, int64_t ldx, const float* left, const float* right, void* __restrict__ codes, void* __restrict__ scales, int64_t tokens, int m, int n, int group, int team, int chunk_rows,
                      float clip, int scale_dtype) {
+  // (launched beside the end of the kernel ahead: 2048 x 4096 55.3 -> 53.4 us, 16 x 4096 13.5 -> 11.5, call behind call)
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
   __shared__ uint32_t ext_all[kMaxTeams][2][kMaxGroup];  // extremes of the teams' tokens
@@ -381,7 +384,7 @@ Shape shape_of(bool resident, int m, int n, int64_t tokens, int sms, int most_th
 }
 
 template <int MODE, int THREADS, bool RESIDENT>
-int launch_sized(const Shape& c, const float* x, int64_t ldx, const float* left, const float* right, void* codes, void* scales, int64_t tokens,
+int launch_sized(const Shape& c, const float* x, int64_t ldx, const float* left, const float* right, void* __restrict__ codes, void* __restrict__ scales, int64_t tokens,
                  int m, int n, float clip, int scale_dtype, int dev, cudaStream_t stream) {
   auto kern = flatquant_f32_kernel<MODE, THREADS, RESIDENT>;
   static bool configured[64] = {};
@@ -391,13 +394,13 @@ int launch_sized(const Shape& c, const float* x, int64_t ldx, const float* left,
   }
   // (resident: a CTA for every group as long as there are SMs, its other teams idle, then a second group for every CTA, ...)
   const int64_t groups = (tokens + c.group - 1) / c.group, room = (int64_t)sm_count(dev) * c.per_sm;
-  kern<<<(unsigned)(groups < room ? groups : room), c.team * c.teams, c.smem, stream>>>(x, ldx, left, right, codes, scales, tokens, m, n, c.group, c.team,
-                                                                                       c.chunk_rows, clip, scale_dtype);
+  QO_CUDA_TRY(launch_beside_tail(kern, (unsigned)(groups < room ? groups : room), (unsigned)(c.team * c.teams), c.smem, stream, x, ldx, left, right,
+                                 codes, scales, tokens, m, n, c.group, c.team, c.chunk_rows, clip, scale_dtype));
   return check_launch("flatquant_f32_kernel");
 }
 
 template <int MODE>
-int launch_mode(const float* x, int64_t ldx, const float* left, const float* right, void* codes, void* scales, int64_t tokens, int m, int n,
+int launch_mode(const float* x, int64_t ldx, const float* left, const float* right, void* __restrict__ codes, void* __restrict__ scales, int64_t tokens, int m, int n,
                 float clip, int scale_dtype, cudaStream_t stream) {
   int dev = 0;
   QO_CUDA_TRY(cudaGetDevice(&dev));

@@ -213,6 +213,23 @@ struct GatherDsts {
   int n_dst;
   long long row_offset;
 };
+// Launch with programmatic stream serialization of a kernel whose first instruction is grid_dependency_wait: its launch overlaps the
+// end of the kernel ahead in the stream.
+template <typename... P, typename... A>
+cudaError_t launch_beside_tail(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // b_early: B was not written by the kernel that precedes the GEMM in the stream
 int launch_gemm_unpack(const int32_t* a, int64_t lda, const int32_t* b, int64_t bsk, int64_t bsn, const float* sa, const float* sb, void* out,
                        int out_dtype, int64_t t, int64_t k, int64_t n, int32_t* acc_out, const void* bias, uint32_t* status,
