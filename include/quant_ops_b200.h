@@ -177,8 +177,14 @@ QO_API int qo_int4_matmul_static(const int32_t* a, int64_t lda, const int32_t* b
  *
  *   out        [tokens, n_out] in out_dtype (QO_F16 / QO_BF16); bias (same dtype, [n_out]) may be NULL
  *   workspace  at least qo_w4a4_linear_workspace_bytes(); NULL = library-owned buffer
+ *
+ * qo_w4a4_linear_in_one_kernel: 1 if a call with these arguments quantizes and multiplies in one kernel (one to four tokens).  It uses no
+ * workspace: NULL then makes the library allocate none either, on any number of streams.
  */
 QO_API size_t qo_w4a4_linear_workspace_bytes(int64_t tokens, int64_t k, int64_t n_out);
+QO_API int qo_w4a4_linear_in_one_kernel(const void* x, int64_t ldx, const void* left, const void* right,
+                                        const int32_t* w_packed, const void* out, int64_t tokens, int m, int n,
+                                        int64_t n_out, float clip_ratio, int in_dtype);
 QO_API int qo_w4a4_linear(const void* x, int64_t ldx, const void* left, const void* right,
                           const int32_t* w_packed, const float* w_scale, const void* bias, void* out,
                           int64_t tokens, int m, int n, int64_t n_out, float clip_ratio, int in_dtype,

@@ -289,6 +289,18 @@ bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
 }
 }  // namespace
 
+// One to four tokens of 64-wide right transforms: every CTA quantizes them itself and multiplies its share of the channels.  (Outputs
+// over the quantizer's inputs stay with two kernels: here one CTA may still read what another has written over.)
+int qo_w4a4_linear_in_one_kernel(const void* x, int64_t ldx, const void* left, const void* right, const int32_t* w_packed, const void* out,
+                                 int64_t tokens, int m, int n, int64_t n_out, float clip_ratio, int in_dtype) {
+  if (t_policy != 0 || !x || !left || !right || !w_packed || !out || m <= 0 || n <= 0 || n_out <= 0 ||
+      !decode_layer_supported(x, ldx, left, right, w_packed, tokens, m, n, n_out, clip_ratio, in_dtype))
+    return 0;
+  const size_t out_bytes = (size_t)tokens * (size_t)n_out * 2;
+  return !overlap(out, out_bytes, x, (size_t)((tokens - 1) * ldx + (int64_t)m * n) * 2) && !overlap(out, out_bytes, left, (size_t)m * m * 2) &&
+         !overlap(out, out_bytes, right, (size_t)n * n * 2);
+}
+
 int qo_w4a4_linear(const void* x, int64_t ldx, const void* left, const void* right, const int32_t* w_packed,
                    const float* w_scale, const void* bias, void* out, int64_t tokens, int m, int n, int64_t n_out,
                    float clip_ratio, int in_dtype, int out_dtype, void* workspace, size_t workspace_bytes,
@@ -304,18 +316,14 @@ int qo_w4a4_linear(const void* x, int64_t ldx, const void* left, const void* rig
   int dev = 0, rc = require_device(&dev);
   if (rc) return rc;
   const size_t need = qo_w4a4_linear_workspace_bytes(tokens, k, n_out);
-  if (workspace == nullptr) {
+  const bool one_kernel = qo_w4a4_linear_in_one_kernel(x, ldx, left, right, w_packed, out, tokens, m, n, n_out, clip_ratio, in_dtype) != 0;
+  if (workspace == nullptr && !one_kernel) {
     if ((rc = scratch_get(g_scratch, dev, need, &workspace))) return rc;
     workspace_bytes = need;
   }
-  if (workspace_bytes < need) return fail(QO_ERR_WORKSPACE, "w4a4_linear: workspace of %zu bytes, need %zu", workspace_bytes, need);
+  if (workspace != nullptr && workspace_bytes < need) return fail(QO_ERR_WORKSPACE, "w4a4_linear: workspace of %zu bytes, need %zu", workspace_bytes, need);
   char* ws = reinterpret_cast<char*>(workspace);
-  // One to four tokens of 64-wide right transforms: every CTA quantizes them itself and multiplies its share of the channels.  (Outputs
-  // over the quantizer's inputs stay with two kernels: here one CTA may still read what another has written over.)
-  const size_t out_bytes = (size_t)tokens * (size_t)n_out * 2;
-  if (t_policy == 0 && decode_layer_supported(x, ldx, left, right, w_packed, tokens, m, n, n_out, clip_ratio, in_dtype) &&
-      !overlap(out, out_bytes, x, (size_t)((tokens - 1) * ldx + k) * 2) && !overlap(out, out_bytes, left, (size_t)m * m * 2) &&
-      !overlap(out, out_bytes, right, (size_t)n * n * 2)) {
+  if (one_kernel) {
     t_quant_path = 2;
     t_gemm_path = 3;
     return launch_decode_layer(x, ldx, left, right, w_packed, w_scale, bias, out, tokens, m, n_out, clip_ratio, in_dtype, out_dtype,

@@ -175,9 +175,13 @@ at::Tensor w4a4_linear(const at::Tensor& x, const at::Tensor& left_trans, const 
   }
   const int64_t tokens = x2.size(0), n_out = w.size(0);
   at::Tensor out = empty_like_device({tokens, n_out}, out_dtype, x);
-  const size_t ws_bytes = qo_w4a4_linear_workspace_bytes(tokens, k, n_out);
+  const int64_t ldx = tokens > 1 ? x2.stride(0) : k;
+  // a decode step in one kernel takes no workspace (an allocation is a tenth of such a call's host time)
+  const bool one_kernel = tokens <= 4 && qo_w4a4_linear_in_one_kernel(x2.data_ptr(), ldx, left.data_ptr(), right.data_ptr(), w.data_ptr<int32_t>(),
+                                                                      out.data_ptr(), tokens, (int)m, (int)n, n_out, (float)clip_ratio, dt);
+  const size_t ws_bytes = one_kernel ? 0 : qo_w4a4_linear_workspace_bytes(tokens, k, n_out);
   at::Tensor ws = ws_bytes ? empty_like_device({(int64_t)ws_bytes}, at::kByte, x) : at::Tensor();
-  check_status(qo_w4a4_linear(x2.data_ptr(), tokens > 1 ? x2.stride(0) : k, left.data_ptr(), right.data_ptr(),
+  check_status(qo_w4a4_linear(x2.data_ptr(), ldx, left.data_ptr(), right.data_ptr(),
                               w.data_ptr<int32_t>(), ws_.data_ptr<float>(), b.defined() ? b.data_ptr() : nullptr,
                               out.data_ptr(), tokens, (int)m, (int)n, n_out, (float)clip_ratio, dt,
                               out_dtype == at::kHalf ? QO_F16 : QO_BF16, ws_bytes ? ws.data_ptr() : nullptr, ws_bytes,
@@ -228,9 +232,18 @@ at::Tensor w4a4_linear_prepared(const at::Tensor& x, const at::Tensor& left_tran
   }
   const int64_t tokens = x2.size(0), n_out = w.size(0);
   at::Tensor out = empty_like_device({tokens, n_out}, out_dtype, x);
+  const int64_t ldx = tokens > 1 ? x2.stride(0) : k;
+  if (tokens <= 4 && qo_w4a4_linear_in_one_kernel(x2.data_ptr(), ldx, left.data_ptr(), right.data_ptr(), w.data_ptr<int32_t>(), out.data_ptr(),
+                                                  tokens, (int)m, (int)n, n_out, (float)clip_ratio, dt)) {
+    check_status(qo_w4a4_linear(x2.data_ptr(), ldx, left.data_ptr(), right.data_ptr(), w.data_ptr<int32_t>(), ws_.data_ptr<float>(),
+                                b.defined() ? b.data_ptr() : nullptr, out.data_ptr(), tokens, (int)m, (int)n, n_out, (float)clip_ratio, dt,
+                                out_dtype == at::kHalf ? QO_F16 : QO_BF16, nullptr, 0, current_stream()),
+                 "w4a4_linear_prepared");
+    return out;
+  }
   const size_t ws_bytes = qo_w4a4_linear_prepared_workspace_bytes(tokens, k, n_out);
   at::Tensor ws = ws_bytes ? empty_like_device({(int64_t)ws_bytes}, at::kByte, x) : at::Tensor();
-  check_status(qo_w4a4_linear_prepared(x2.data_ptr(), tokens > 1 ? x2.stride(0) : k, left.data_ptr(), right.data_ptr(),
+  check_status(qo_w4a4_linear_prepared(x2.data_ptr(), ldx, left.data_ptr(), right.data_ptr(),
                                        w.data_ptr<int32_t>(), w_prepared.data_ptr(), ws_.data_ptr<float>(),
                                        b.defined() ? b.data_ptr() : nullptr, out.data_ptr(), tokens, (int)m, (int)n, n_out,
                                        (float)clip_ratio, dt, out_dtype == at::kHalf ? QO_F16 : QO_BF16,
