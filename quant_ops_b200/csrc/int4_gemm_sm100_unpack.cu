@@ -64,7 +64,8 @@ namespace {
 using namespace ptx;
 
 constexpr int kBM = 128;        // rows per CTA
-constexpr int kBN = 256;        // columns of the pair's tile
+constexpr int kBN = 256;        // columns of the pair's widest tile; a launch chooses a multiple of 32 from kBNLeast on
+constexpr int kBNLeast = 128;
 constexpr int kBNh = kBN / 2;   // B rows staged per CTA
 constexpr int kKStage = 256;    // int4 values per stage = 128 packed bytes = 256 int8 bytes per row
 constexpr int kKWords = kKStage / 8;
@@ -90,8 +91,8 @@ struct Smem {
   static constexpr int kBytes = kOffBar + 128 + 896;  // barriers; room to start on a 1024-byte boundary (the window itself starts on 128)
   static_assert(kBytes <= 227 * 1024, "shared memory of one CTA");
 };
-constexpr int kAccShift = 64;   // the accumulators of successive items start at tensor-memory columns 0 and 64 in turn
-constexpr int kColA = kBN + kAccShift;  // first tensor-memory column of the A operand stages (64 columns each)
+constexpr int kAccCols = 320;   // tensor-memory columns of the accumulators: those of successive items lie at either end in turn
+constexpr int kColA = kAccCols; // first column of the A operand stages (64 columns each)
 constexpr int kShortSums = 65536;  // up to this K a sum fits 22 bits and a sign
 constexpr int kBPiecesA = 3;
 constexpr int kEpiWarp0 = 4, kAWarp0 = 12, kBWarp0 = 24;
@@ -102,7 +103,7 @@ struct Bars {
   uint64_t p_full[kPStages], p_empty[kPStages];
   uint64_t op_ready[kOStages], op_empty[kOStages];
   uint64_t acc_full, acc_empty;
-  uint64_t exchange;  // bytes of the other pairs' partial sums (SPLIT > 1)
+  uint64_t exchange;  // SPLIT > 1: bytes of the other pairs' partial sums; SPLIT = 1: acc_empty of the odd items
   uint32_t tmem_base;
 };
 static_assert(sizeof(Bars) <= 128, "barriers");
@@ -274,6 +275,8 @@ __device__ __forceinline__ bool issue_stage(uint32_t d_tmem, uint32_t a_tmem, ui
   return ok != 0;
 }
 
+// WIDE: tiles of 256 columns as a compile-time fact, which is worth a percent; without it the launch says how many (a multiple of 32).
+//
 // GATHER: the outputs are not stored to `out` but, at row `row_offset + row`, into every buffer of `dsts` -- this GPU's
 // own copy of the gathered output and the peers' copies, mapped into this process (plain stores over NVLink; the
 // all-gather of a row-sharded layer's outputs costs no kernel of its own and no SMs).
@@ -291,13 +294,13 @@ __device__ __forceinline__ bool issue_stage(uint32_t d_tmem, uint32_t a_tmem, ui
 // BCOLS: B is the reference layout [K/8, N] of packed words with N contiguous.  Its box is 32 words of K by 128
 // channels (333 x 4096 x 14336 50.0 -> 27.7 us), a channel's words lie 512 bytes apart in the stage, and a converter thread, which owns a channel, reads
 // them one by one without bank conflicts: no transposing pass over the weights.
-template <typename OutT, bool GATHER, int SPLIT, bool BCOLS>
+template <typename OutT, bool GATHER, int SPLIT, bool BCOLS, bool WIDE>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap b_map,
                       const __grid_constant__ CUtensorMap out_map,
                       const float* sa, const float* sb, OutT* __restrict__ out,
-                      int32_t* __restrict__ acc_out, const OutT* bias, int t, int n, int k, int items, int cut_from,
-                      int b_early, uint32_t* __restrict__ status, const __grid_constant__ GatherDsts dsts) {
+                      int32_t* __restrict__ acc_out, const OutT* bias, int t, int n, int k, int bn_arg, int tiles_arg, int items,
+                      int cut_from, int b_early, uint32_t* __restrict__ status, const __grid_constant__ GatherDsts dsts) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   using S = Smem<SPLIT>;
@@ -309,7 +312,9 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
   const uint32_t leader = SPLIT == 1 ? 0u : (crank & ~1u), other = leader + 1;  // cluster ranks of the pair's CTAs
   // (SPLIT > 1: `pair` counts clusters, each with one tile; kz is the pair's slice of K)
   const int pair = SPLIT == 1 ? blockIdx.x >> 1 : blockIdx.x / (2 * SPLIT), npairs = SPLIT == 1 ? gridDim.x >> 1 : items;
-  const int tiles_n = (n + kBN - 1) / kBN;
+  const int bn = WIDE ? kBN : bn_arg;         // columns of a tile
+  const int tiles_n = WIDE ? (n + kBN - 1) / kBN : tiles_arg;  // tiles side by side
+  const int acc_shift = kAccCols - bn;        // first column of every second item's accumulator
   const int kstages = k / kKStage;  // k is a multiple of 256 (checked by the host)
   const int kz = SPLIT == 1 ? 0 : (int)(crank >> 1);
   const int ks_first = SPLIT == 1 ? 0 : kz * kstages / SPLIT;
@@ -321,9 +326,12 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
   int mine = 0;                              // items of this pair
   if (pair < items) mine = (items - pair + npairs - 1) / npairs;
   const int total_steps = mine * ksteps;
-  // item -> tile index, first column of the item inside the tile (0 or 128), columns of the item (256 or 128)
+  // item -> tile index, first column of the item inside the tile (0 or 128), columns of the item (bn, or 128 of 256)
+  // bytes of a stage: a box of B rows has half a tile's, one of columns always 128 (narrower ones start off the 128-byte lines: 333 x 4096 x
+  // 14336 in tiles of 224 28.6 us, 28.2 with boxes of 128, 27.7 in tiles of 256)
+  const uint32_t stage_bytes = kPABytes + (BCOLS ? kPBBytes : (uint32_t)bn * 64u);
   auto item_of = [&](int item, int& tile, int& col_in_tile, int& width) {
-    if (item < cut_from) { tile = item; col_in_tile = 0; width = kBN; }
+    if (item < cut_from) { tile = item; col_in_tile = 0; width = bn; }
     else { tile = cut_from + ((item - cut_from) >> 1); col_in_tile = ((item - cut_from) & 1) * (kBN / 2); width = kBN / 2; }
   };
 
@@ -332,7 +340,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
     for (int i = 0; i < kOStages; ++i) { mbar_init(smem_u32(&bars->op_ready[i]), 12); mbar_init(smem_u32(&bars->op_empty[i]), 1); }
     mbar_init(smem_u32(&bars->acc_full), 1);
     mbar_init(smem_u32(&bars->acc_empty), 16);
-    mbar_init(smem_u32(&bars->exchange), 1);
+    mbar_init(smem_u32(&bars->exchange), SPLIT == 1 ? 16 : 1);
     fence_barrier_init();
     prefetch_tensormap(&a_map);
     prefetch_tensormap(&b_map);
@@ -350,10 +358,10 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
   int early = 0;  // stages whose B half is already on its way
   if (SPLIT > 1 && b_early && tid == 0) {
     early = min(kPStages, ksteps);
-    const int row_b = (pair % tiles_n) * kBN + (int)rank * kBNh;
+    const int row_b = (pair % tiles_n) * bn + (int)rank * (bn >> 1);
     for (int s = 0; s < early; ++s) {
       const uint32_t bar = smem_u32(&bars->p_full[s]);
-      mbar_arrive_expect_tx(bar, kPStageBytes);
+      mbar_arrive_expect_tx(bar, stage_bytes);
       const uint32_t dst = smem_base + kOffP + s * kPStageBytes + kPABytes;
       if (BCOLS) tma_load_2d(dst, &b_map, bar, row_b, (ks_first + s) * kKWords);
       else tma_load_2d(dst, &b_map, bar, (ks_first + s) * 128, row_b);
@@ -406,16 +414,22 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       item_of(pair + lt * npairs, tile, col_in_tile, width);
       const int mb = tile / tiles_n, nb = tile - mb * tiles_n;
       const int row0 = mb * 2 * kBM + (int)rank * kBM + q * 32;  // first row of this warp
-      const int colt = nb * kBN + col_in_tile;                   // first column of the item
+      const int colt = nb * bn + col_in_tile;                    // first column of the item
       const float s_row = row0 + lane < t ? (SPLIT == 1 ? sa[row0 + lane] : sa[row0 + lane] * 0.00390625f) : 0.f;
-      // blocks of 32 columns in the order in which this warp takes them (a half item has two for each warp)
+      // Blocks of 32 columns in the order in which this warp takes them: its half of those that the next accumulator overlaps (6, 4, 2,
+      // or none of a tile of 256, 224, 192, or up to 160), then every second of the others.  (A half item is a pair's last.)
       const bool last = lt == mine - 1;
-      const bool whole = width == kBN;
-      const int shared_from = (lt & 1) ? 0 : kAccShift / 32;  // first block of those that the next accumulator overlaps
-      auto block = [&](int i) {
-        if (!whole) return 2 * half + i;
-        return i < 2 ? shared_from + 4 * half + i : i == 2 ? shared_from + 2 + half : ((lt & 1) ? 6 : 0) + half;
-      };
+      // (Kept as one register of four-bit numbers.)
+      uint32_t order = 0;
+      int blocks;
+      {
+        const int overlap = width == bn ? max(0, (bn - acc_shift) >> 5) : 0, own = overlap >> 1;
+        blocks = own + (((width >> 5) - overlap + 1 - half) >> 1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          order |= (uint32_t)(i >= blocks ? 0 : i < own ? ((lt & 1) ? 0 : acc_shift >> 5) + half * own + i : ((lt & 1) ? overlap : 0) + 2 * (i - own) + half) << (4 * i);
+      }
+      auto block = [&](int i) { return (int)((order >> (4 * i)) & 15u); };
       // scales and biases of blocks i and i + 1: a lane has one column of each, and a pair of columns of one of them (lanes 0 .. 15 of
       // block i)
       float sb_r[2];
@@ -448,12 +462,12 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_full), lt & 1))) { atomicCAS(status, 0u, 0xA30u); break; }
       if (SPLIT > 1) break;  // every MMA of this pair is done; the partial sums are exchanged below
       tc_fence_after();
-      const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (lt & 1) * kAccShift;
+      const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (lt & 1) * acc_shift;
       auto release = [&] {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          const uint32_t e = smem_u32(&bars->acc_empty);
+          const uint32_t e = smem_u32(lt & 1 ? &bars->exchange : &bars->acc_empty);
           if (rank == 0) mbar_arrive(e); else mbar_arrive_cluster(cluster_map_shared(e, leader));
         }
       };
@@ -479,30 +493,30 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
         uint32_t v[3][32];
         tmem_ld_32x32b_x32(acc + 32 * block(0), v[0]);
         tmem_ld_32x32b_x32(acc + 32 * block(1), v[1]);
-        if (whole) tmem_ld_32x32b_x32(acc + 32 * block(2), v[2]);
+        if (blocks > 2) tmem_ld_32x32b_x32(acc + 32 * block(2), v[2]);
         tmem_ld_wait_for(v[0]);
         tmem_ld_wait_for(v[1]);
         tmem_ld_wait_for(v[2]);
         if (!last) release();
         emit(0, v[0], true);
-        const uint32_t bias_late = whole ? load_columns(2) : 0u;
+        const uint32_t bias_late = blocks > 2 ? load_columns(2) : 0u;
         emit(1, v[1], true);
-        if (whole) {
-          tmem_ld_32x32b_x32(acc + 32 * block(3), v[0]);
+        if (blocks > 2) {
+          tmem_ld_32x32b_x32(acc + 32 * block(3), v[0]);  // (of three blocks: the first again, not used)
           share_columns();
           bias_w = bias_late;
           emit(2, v[2], true);
           tmem_ld_wait_for(v[0]);
-          emit(3, v[0], true);
+          if (blocks > 3) emit(3, v[0], true);
         }
       } else {
         // with the accumulators themselves as a second output, or sums of more bits: block by block
 #pragma unroll 1
-        for (int i = 0; i < (whole ? 4 : 2); ++i) {
+        for (int i = 0; i < blocks; ++i) {
           uint32_t v[32];
           tmem_ld_32x32b_x32(acc + 32 * block(i), v);
           tmem_ld_wait_for(v);
-          if (!last && i == 3) release();  // (a half item is always a pair's last)
+          if (!last && i == blocks - 1) release();
           if (i == 2) {
             bias_w = load_columns(2);
             share_columns();
@@ -527,8 +541,8 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
         int tile, col_in_tile, width;
         item_of(item, tile, col_in_tile, width);
         const int mb = tile / tiles_n, nb = tile - mb * tiles_n;
-        // a CTA stages its half of the item's B rows; the box always has 128 rows, of which a half item uses the first 64
-        const int row_a = mb * 2 * kBM + (int)rank * kBM, row_b = nb * kBN + col_in_tile + (int)rank * (width >> 1);
+        // a CTA stages its half of the item's B rows; the box has half a tile's rows, of which a half item uses the first 64
+        const int row_a = mb * 2 * kBM + (int)rank * kBM, row_b = nb * bn + col_in_tile + (int)rank * (width >> 1);
 #pragma unroll 1
         for (int ks = 0; ks < ksteps; ++ks, ++step) {
           const int ps = step % kPStages, pph = (step / kPStages) & 1;
@@ -539,7 +553,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
             continue;
           }
           if (!mbar_wait(smem_u32(&bars->p_empty[ps]), pph ^ 1)) { atomicCAS(status, 0u, 0xA00u + ps); ok = false; break; }
-          mbar_arrive_expect_tx(bar, kPStageBytes);
+          mbar_arrive_expect_tx(bar, stage_bytes);
           tma_load_2d(dst, &a_map, bar, (ks_first + ks) * 128, row_a);
           if (BCOLS) tma_load_2d(dst + kPABytes, &b_map, bar, row_b, (ks_first + ks) * kKWords);
           else tma_load_2d(dst + kPABytes, &b_map, bar, (ks_first + ks) * 128, row_b);
@@ -549,7 +563,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
   } else if (warp == 1) {
     // ---- MMA issuer (leader CTA only) ----------------------------------------------------------------------------
     if (lane == 0 && rank == 0) {
-      const uint32_t idesc_whole = umma_idesc(2, 1, 1, 0, 0, 2 * kBM, kBN);  // s32 accumulators, s8 x s8, K-major, M = 256 over the pair
+      const uint32_t idesc_whole = umma_idesc(2, 1, 1, 0, 0, 2 * kBM, bn);  // s32 accumulators, s8 x s8, K-major, M = 256 over the pair
       const uint32_t idesc_half = umma_idesc(2, 1, 1, 0, 0, 2 * kBM, kBN / 2);
       // one thread feeds the tensor cores of both SMs, so its instruction count per MMA matters: the B descriptor is
       // built once and advanced by adding to its address field (units of 16 bytes)
@@ -564,8 +578,10 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
         // the item's first operands are looked for before the accumulator, so that the answer comes while that is being drained
         if (!ready && !mbar_wait(smem_u32(&bars->op_ready[step % kOStages]), (step / kOStages) & 1)) { atomicCAS(status, 0u, 0xA20u); break; }
         ready = true;
-        if (lt > 0 && !mbar_wait(smem_u32(&bars->acc_empty), (lt & 1) ^ 1)) { atomicCAS(status, 0u, 0xA10u); break; }
-        const uint32_t d_tmem = tmem + (lt & 1) * kAccShift;
+        // the accumulator this item overlaps: that of the item before, or, where both fit beside one another, of the one before that
+        const int owner = lt - (acc_shift < bn ? 1 : 2);
+        if (owner >= 0 && !mbar_wait(smem_u32(owner & 1 ? &bars->exchange : &bars->acc_empty), (owner >> 1) & 1)) { atomicCAS(status, 0u, 0xA10u); break; }
+        const uint32_t d_tmem = tmem + (lt & 1) * acc_shift;
         const uint32_t idesc = pair + lt * npairs >= cut_from ? idesc_half : idesc_whole;
 #pragma unroll 1
         for (int ks = 0; ks < ksteps; ++ks, ++step) {
@@ -590,6 +606,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
     // the same row of B, so that a stage's converters take about the same time -----------------------------------------------
     const int e = (warp - kAWarp0) >> 2, q = warp & 3, r = q * 32 + lane;  // set 0 .. 2
     const uint32_t sw = (uint32_t)((r & 7) << 4);
+    const bool b_rows = q * 32 < bn >> 1;  // this warp's rows of B are part of the tile
 #pragma unroll 1
     for (int step = e, ph = 0; step < total_steps; step += kSets, ph ^= 1) {
       int s = e;  // the slot of both rings; not known to the compiler, which would keep all of the stage's addresses in registers
@@ -616,12 +633,13 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
           split16(p[o].z, v[8 * c + 4], v[8 * c + 5]);
           split16(p[o].w, v[8 * c + 6], v[8 * c + 7]);
           if (h < 2) p[o] = ld_shared_v4(src ^ (uint32_t)((2 * h + c + 4) << 4));
-          else if (2 * h + c - 4 < kBPiecesA) p[o] = load_b_piece<BCOLS>(stage + kPABytes, r, 8 - kBPiecesA + 2 * h + c - 4);
+          else if (2 * h + c - 4 < kBPiecesA && b_rows) p[o] = load_b_piece<BCOLS>(stage + kPABytes, r, 8 - kBPiecesA + 2 * h + c - 4);
         }
         tmem_st_32x32b_x16(tmem + ((uint32_t)(q * 32) << 16) + kColA + s * 64 + h * 16, v);
       }
+      if (b_rows)
 #pragma unroll
-      for (int i = 0; i < kBPiecesA; ++i) store_b_piece(smem_base + kOffO + s * kOBBytes, r, 8 - kBPiecesA + i, p[i]);
+        for (int i = 0; i < kBPiecesA; ++i) store_b_piece(smem_base + kOffO + s * kOBBytes, r, 8 - kBPiecesA + i, p[i]);
       // The packed stage is released only here, after instructions that consume every loaded value: an arrival placed
       // right behind the ld.shared instructions was measured to let the next TMA overwrite rows that some lanes had
       // not read yet (nothing orders another lane's outstanding loads before lane 0's arrival).
@@ -640,6 +658,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
     // ---- B converters: the first pieces of B's 128 rows, two rows per thread of the set on duty; eight consecutive lanes take
     // eight consecutive rows of one piece, which is conflict-free for the 128-byte-swizzled reads and writes ---------------
     const int f = warp < kBWarp0 ? 0 : 1 + ((warp - kBWarp0) >> 1), bt = (warp & 1) * 32 + lane;  // set 0 .. 2, thread within the set (0 .. 63)
+    const bool second = 64 + (warp & 1) * 32 < bn >> 1;  // the tile has this warp's second rows
 #pragma unroll 1
     for (int step = f, ph = 0; step < total_steps; step += kSets, ph ^= 1) {
       int s = f;  // (as above)
@@ -654,12 +673,14 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       constexpr int kTasks = 2 * (8 - kBPiecesA);
       uint4 p[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) p[i] = load_b_piece<BCOLS>(src, bt + 64 * (i & 1), i >> 1);
+      for (int i = 0; i < 4; ++i)
+        if (!(i & 1) || second) p[i] = load_b_piece<BCOLS>(src, bt + 64 * (i & 1), i >> 1);
 #pragma unroll
-      for (int i = 0; i < kTasks; ++i) {
-        store_b_piece(dst, bt + 64 * (i & 1), i >> 1, p[i & 3]);
-        if (i + 4 < kTasks) p[i & 3] = load_b_piece<BCOLS>(src, bt + 64 * (i & 1), (i + 4) >> 1);
-      }
+      for (int i = 0; i < kTasks; ++i)
+        if (!(i & 1) || second) {
+          store_b_piece(dst, bt + 64 * (i & 1), i >> 1, p[i & 3]);
+          if (i + 4 < kTasks) p[i & 3] = load_b_piece<BCOLS>(src, bt + 64 * (i & 1), (i + 4) >> 1);
+        }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bars->p_empty[s]));  // every loaded value has been consumed by the stores above
       fence_proxy_async_smem();
@@ -673,7 +694,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
   }
 
   if (SPLIT > 1) {
-    // Exchange of the partial sums.  The tile's eight blocks of 32 columns belong to the pairs in turn (block c to pair
+    // Exchange of the partial sums.  The tile's (at most eight) blocks of 32 columns belong to the pairs in turn (block c to pair
     // c % SPLIT); the owner adds the pairs' sums of its blocks and writes the outputs.  A warp takes one block of 32
     // rows x 32 columns out of tensor memory, lays it down as 4 KB (rows of 128 bytes, 16-byte pieces XOR-swizzled by the
     // row) and sends it as ONE bulk copy into the owner's shared memory, which counts the bytes on a barrier: stores of
@@ -681,7 +702,8 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
     const int mb = pair / tiles_n, nb = pair - mb * tiles_n;
     const int row0 = mb * 2 * kBM + (int)rank * kBM;
     const int quads = max(0, min(4, (t - row0 + 31) >> 5));  // lane quadrants with real rows
-    auto owned = [](int z) { return (8 - z + SPLIT - 1) / SPLIT; };
+    const int nblocks = bn >> 5;
+    auto owned = [&](int z) { return (nblocks - z + SPLIT - 1) / SPLIT; };
     const int own = owned(kz);
     const uint32_t staging = smem_base + (uint32_t)(SPLIT * 4 * own) * 4096u;  // behind the slots the other pairs fill
     static_assert((SPLIT * 4 * ((8 + SPLIT - 1) / SPLIT) + 4 * (8 - (8 + SPLIT - 1) / SPLIT)) * 4096 <= S::kOffSb, "slots and staging");
@@ -697,14 +719,14 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       const int q = warp & 3;
       tc_fence_after();
 #pragma unroll 1
-      for (int c = (warp - 2) >> 2; c < 8; c += 4) {
+      for (int c = (warp - 2) >> 2; c < nblocks; c += 4) {
         uint32_t v[32];
         tmem_ld_32x32b_x32(tmem + ((uint32_t)(q * 32) << 16) + c * 32, v);
         tmem_ld_wait();
         const int owner = c % SPLIT, j = c / SPLIT;
         const int before = j + (c % SPLIT > kz ? 1 : 0);  // this pair's own blocks among the first c
         const uint32_t slot = (uint32_t)((kz * 4 + q) * owned(owner) + j) * 4096u;  // in the owner's shared memory
-        const uint32_t dst = owner == kz ? smem_base + slot : staging + (uint32_t)(q * (8 - own) + c - before) * 4096u;
+        const uint32_t dst = owner == kz ? smem_base + slot : staging + (uint32_t)(q * (nblocks - own) + c - before) * 4096u;
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)(lane * 128 + ((i ^ (lane & 7)) << 4))), "r"(v[4 * i]),
@@ -729,7 +751,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
       const int p0 = 2 * (lane & 3);
       for (int unit = warp; unit < own * quads * 4; unit += kThreads / 32) {
         const int j = unit / (quads * 4), rest = unit - j * quads * 4, q = rest >> 2, r = (rest & 3) * 8 + (lane >> 2);
-        const int row = row0 + q * 32 + r, cb = (j * SPLIT + kz) * 32 + 4 * p0, col = nb * kBN + cb;
+        const int row = row0 + q * 32 + r, cb = (j * SPLIT + kz) * 32 + 4 * p0, col = nb * bn + cb;
         if (row >= t || col >= n) continue;
         int v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
@@ -814,7 +836,7 @@ struct UnpackArgs {
   bool b_early;
 };
 
-int64_t unpack_tiles(int64_t t, int64_t n) { return ((t + 2 * kBM - 1) / (2 * kBM)) * ((n + kBN - 1) / kBN); }
+int64_t unpack_tiles(int64_t t, int64_t n, int64_t bn = kBN) { return ((t + 2 * kBM - 1) / (2 * kBM)) * ((n + bn - 1) / bn); }
 
 // packed operand [rows, k / 2 bytes] with a row stride of ld_words 32-bit words; boxes of 128 bytes x box_rows rows
 int make_map_packed(CUtensorMap* map, const void* base, int64_t rows, int64_t k, int64_t ld_words, int box_rows) {
@@ -855,12 +877,12 @@ int make_map_out(CUtensorMap* map, void* base, int64_t rows, int64_t n) {
 }
 
 // clusters of 2 * SPLIT CTAs of this kernel the device runs at once (0 if the query fails); cached per device
-template <typename OutT, bool GATHER, int SPLIT, bool BCOLS>
+template <typename OutT, bool GATHER, int SPLIT, bool BCOLS, bool WIDE>
 int max_clusters(int dev) {
   static int cached[64] = {};
   int& c = cached[dev & 63];
   if (c == 0) {
-    auto kern = gemm_s4_unpack_kernel<OutT, GATHER, SPLIT, BCOLS>;
+    auto kern = gemm_s4_unpack_kernel<OutT, GATHER, SPLIT, BCOLS, WIDE>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<SPLIT>::kBytes) != cudaSuccess) { (void)cudaGetLastError(); c = -1; return 0; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * SPLIT * 74);
@@ -880,18 +902,18 @@ int max_clusters(int dev) {
   return c > 0 ? c : 0;
 }
 
-template <typename OutT, bool GATHER, int SPLIT, bool BCOLS>
-int launch_typed(const UnpackArgs& p, uint32_t* status, const GatherDsts& dsts, cudaStream_t stream) {
+template <typename OutT, bool GATHER, int SPLIT, bool BCOLS, bool WIDE>
+int launch_typed(const UnpackArgs& p, int bn, uint32_t* status, const GatherDsts& dsts, cudaStream_t stream) {
   int dev = 0;
   QO_CUDA_TRY(cudaGetDevice(&dev));
-  const int clusters = max_clusters<OutT, GATHER, SPLIT, BCOLS>(dev);
+  const int clusters = max_clusters<OutT, GATHER, SPLIT, BCOLS, WIDE>(dev);
   if (clusters <= 0) return QO_ERR_UNSUPPORTED;
-  const int64_t ntiles = unpack_tiles(p.t, p.n);
+  const int64_t ntiles = unpack_tiles(p.t, p.n, bn);
   if (SPLIT > 1 && ntiles > clusters) return QO_ERR_UNSUPPORTED;  // a second wave would cost more than the split saves
   CUtensorMap a_map, b_map, out_map;
   int rc = make_map_packed(&a_map, p.a, p.t, p.k, p.lda, kBM);
   if (rc) return rc;
-  if ((rc = BCOLS ? make_map_packed_cols(&b_map, p.b, p.n, p.k, p.ldb) : make_map_packed(&b_map, p.b, p.n, p.k, p.ldb, kBNh))) return rc;
+  if ((rc = BCOLS ? make_map_packed_cols(&b_map, p.b, p.n, p.k, p.ldb) : make_map_packed(&b_map, p.b, p.n, p.k, p.ldb, bn / 2))) return rc;
   if (SPLIT == 1 && !GATHER) {
     if ((rc = make_map_out(&out_map, p.out, p.t, p.n))) return rc;
   } else {
@@ -900,7 +922,7 @@ int launch_typed(const UnpackArgs& p, uint32_t* status, const GatherDsts& dsts, 
   const int pairs = (int)(ntiles < clusters ? ntiles : clusters);
   // tiles of a last wave that would occupy at most half of the pairs are cut into halves of 128 columns
   const int64_t whole = (ntiles / pairs) * pairs, rest = ntiles - whole;
-  const bool cut = SPLIT == 1 && rest > 0 && 2 * rest <= pairs;
+  const bool cut = SPLIT == 1 && bn == kBN && rest > 0 && 2 * rest <= pairs;
   const int items = (int)(cut ? whole + 2 * rest : ntiles), cut_from = cut ? (int)whole : 0x7fffffff;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * SPLIT * pairs));
@@ -916,25 +938,72 @@ int launch_typed(const UnpackArgs& p, uint32_t* status, const GatherDsts& dsts, 
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  QO_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_s4_unpack_kernel<OutT, GATHER, SPLIT, BCOLS>, a_map, b_map, out_map, p.sa, p.sb, reinterpret_cast<OutT*>(p.out),
-                                 p.acc_out, reinterpret_cast<const OutT*>(p.bias), (int)p.t, (int)p.n, (int)p.k, items, cut_from,
+  QO_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_s4_unpack_kernel<OutT, GATHER, SPLIT, BCOLS, WIDE>, a_map, b_map, out_map, p.sa, p.sb, reinterpret_cast<OutT*>(p.out),
+                                 p.acc_out, reinterpret_cast<const OutT*>(p.bias), (int)p.t, (int)p.n, (int)p.k, bn, (int)((p.n + bn - 1) / bn), items, cut_from,
                                  p.b_early ? 1 : 0, status, dsts));
   return check_launch("gemm_s4_unpack_kernel");
 }
 
-// K slices per tile: as many as there are pairs for, while every pair keeps at least two stages of K and all clusters run at
-// once.  256 x 14336 x 4096 (16 tiles): 21.7 us with three slices, the most that run at once;
-// clusters of four pairs do not fit sixteen times on the device.
+// What a call takes with tiles of bn columns and K in `split` slices, in ns (graph replay; `pairs` CTA pairs at a time): rounds of tiles at
+// 408 + 229 bn / 256 per stage of K, the hand-over between rounds, and after the last MMA the outputs of a tile or the
+// exchange of the partial sums, which grows with what a CTA sends and with how many send at once.  Fitted to 710 measurements: 90
+// products of 40 to 1800 rows (K 4096 to 14336, 1024 to 14336 columns) in tiles of 128 to 256 and one to four slices.  What the
+// formula picks is within 1 % of the fastest form in 86 of them, 5 % behind it in the worst.
+double launch_ns(int64_t t, int64_t k, int64_t n, int bn, int split, int pairs) {
+  const int64_t row_blocks = (t + 2 * kBM - 1) / (2 * kBM), tiles = unpack_tiles(t, n, bn), stages = k / kKStage;
+  const double w = bn / 256.0, stage = 408 + 229 * w;
+  if (split > 1) {
+    const int64_t quads = (t + 31) / 32;  // blocks of 32 rows that are exchanged: of a CTA's four, of all
+    const double own = (double)(quads < 4 ? quads : 4) / 4, all = (double)(quads < 8 * row_blocks ? quads : 8 * row_blocks) / (8 * row_blocks);
+    return 2750 + (stages + split - 1) / split * stage + 2240 + w * (split - 1) / split * (3770 * own + 5490 * all * tiles * split / 74);
+  }
+  const int64_t whole = tiles <= pairs ? 1 : tiles / pairs, rest = tiles <= pairs ? 0 : tiles % pairs;
+  if (rest > 0 && bn == kBN && 2 * rest <= pairs) return 2750 + whole * stages * stage + stages * (408 + 229 * 0.5) + whole * 1300 + 4080 * 0.5;
+  const int64_t rounds = whole + (rest > 0);
+  return 2750 + rounds * stages * stage + (rounds - 1) * 1300 * w + 4080 * w;
+}
+
+// Columns of a tile and slices of K.  Tiles of 256 columns and as many slices as run at once, unless the formula promises 3 % (7 % with columns of
+// weights, of which a stage fetches 128 whatever the tile): narrower tiles
+// put more pairs to work and leave each less to exchange or to store, but a stage costs nearly the same for fewer columns.
+// Measured, 256 columns / chosen (graph replay, us): 256 x 14336 x 4096 22.2 / 20.0 (192, three slices), 256 x 4096 x 4096 13.7 / 11.4 (128, two),
+// 128 x 4096 x 1024 11.0 / 8.8 (128, four), 256 x 4096 x 11008 17.1 / 15.5 (160), 600 x 14336 x 4096 41.7 / 37.6 (192).
+// (Clusters of eight CTAs do not fit sixteen times, those of six fit 22 times, of four 33 times: what the device says is asked.)
 template <typename OutT, bool BCOLS>
 int launch_split(const UnpackArgs& p, uint32_t* status, cudaStream_t stream) {
   const GatherDsts none = {};
-  const int64_t tiles = unpack_tiles(p.t, p.n), kstages = p.k / kKStage;
-  int rc = QO_ERR_UNSUPPORTED;
-  if (4 * tiles <= 74 && kstages >= 8) rc = launch_typed<OutT, false, 4, BCOLS>(p, status, none, stream);
-  if (rc == QO_ERR_UNSUPPORTED && 3 * tiles <= 74 && kstages >= 6) rc = launch_typed<OutT, false, 3, BCOLS>(p, status, none, stream);
-  if (rc == QO_ERR_UNSUPPORTED && 2 * tiles <= 74 && kstages >= 4) rc = launch_typed<OutT, false, 2, BCOLS>(p, status, none, stream);
-  if (rc == QO_ERR_UNSUPPORTED) rc = launch_typed<OutT, false, 1, BCOLS>(p, status, none, stream);
-  return rc;
+  int dev = 0;
+  QO_CUDA_TRY(cudaGetDevice(&dev));
+  const int64_t stages = p.k / kKStage;
+  const int pairs = max_clusters<OutT, false, 1, BCOLS, true>(dev);
+  if (pairs <= 0) return QO_ERR_UNSUPPORTED;
+  int bn = kBN, split = 1;
+  double least = 0;
+  for (int c = kBN; c >= kBNLeast; c -= 32) {
+    const int64_t tiles = unpack_tiles(p.t, p.n, c);
+    for (int z = 4; z >= 1; --z) {
+      if (z > 1) {
+        if (z * tiles > pairs || stages < 2 * z) continue;
+        const int fit = z == 4 ? max_clusters<OutT, false, 4, BCOLS, false>(dev)
+                               : (z == 3 ? max_clusters<OutT, false, 3, BCOLS, false>(dev) : max_clusters<OutT, false, 2, BCOLS, false>(dev));
+        if (tiles > fit) continue;
+      }
+      const double ns = launch_ns(p.t, p.k, p.n, c, z, pairs);
+      if (least == 0 || ns < least) {
+        bn = c;
+        split = z;
+        least = c == kBN ? ns * (BCOLS ? 0.93 : 0.97) : ns;
+      }
+      if (c == kBN) break;  // (as many slices as run at once)
+    }
+  }
+  if (split == 4) return launch_typed<OutT, false, 4, BCOLS, false>(p, bn, status, none, stream);
+  if (split == 3 && bn == kBN) return launch_typed<OutT, false, 3, BCOLS, true>(p, bn, status, none, stream);
+  if (split == 3) return launch_typed<OutT, false, 3, BCOLS, false>(p, bn, status, none, stream);
+  if (split == 2 && bn == kBN) return launch_typed<OutT, false, 2, BCOLS, true>(p, bn, status, none, stream);
+  if (split == 2) return launch_typed<OutT, false, 2, BCOLS, false>(p, bn, status, none, stream);
+  if (bn == kBN) return launch_typed<OutT, false, 1, BCOLS, true>(p, bn, status, none, stream);
+  return launch_typed<OutT, false, 1, BCOLS, false>(p, bn, status, none, stream);
 }
 
 }  // namespace
@@ -1016,8 +1085,8 @@ int launch_gemm_unpack(const int32_t* a, int64_t lda, const int32_t* b, int64_t 
     for (int d = 0; d < gather->n_dst; ++d)
       if (!gather->ptr[d] || reinterpret_cast<uintptr_t>(gather->ptr[d]) % 32)
         return fail(QO_ERR_INVALID_ARGUMENT, "w4a4_linear_gather: destination %d is null or not 32-byte aligned", d);
-    if (out_dtype == QO_F16) return launch_typed<__half, true, 1, false>(p, status, *gather, stream);
-    return launch_typed<__nv_bfloat16, true, 1, false>(p, status, *gather, stream);
+    if (out_dtype == QO_F16) return launch_typed<__half, true, 1, false, true>(p, kBN, status, *gather, stream);
+    return launch_typed<__nv_bfloat16, true, 1, false, true>(p, kBN, status, *gather, stream);
   }
   if (reinterpret_cast<uintptr_t>(out) % 16 || (acc_out && reinterpret_cast<uintptr_t>(acc_out) % 16))
     return fail(QO_ERR_INVALID_ARGUMENT, "int4_matmul: outputs of the tcgen05 kernel must be 16-byte aligned");

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import quant_ops_b200 as q
-from helpers import N, QD, TD, lib, make_inputs, ptr, stream_ptr
+from helpers import N, QD, TD, abi_int4_matmul, launched_blocks, lib, make_inputs, ptr, stream_ptr
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -13,6 +13,9 @@ DEV = "cuda:0"
 # one stage per item and many items per pair; two rounds of tiles with a ragged last column tile; halves of tiles in the last round;
 # a single row in the last row block; a single block of eight columns in the last column tile; one tile per pair
 SHAPES = [(2000, 256, 9480), (333, 4096, 14328), (777, 4096, 11008), (4097, 1024, 1032), (1600, 768, 2056), (500, 2048, 9472)]
+# columns of a tile and slices of K that the rule takes, with ragged rows and columns: two rounds and one of narrow tiles, K in slices
+FORMS = [(1100, 4096, 4104, 160, 1), (700, 11008, 4088, 192, 1), (200, 4096, 14328, 224, 1), (256, 4096, 11000, 160, 1), (300, 2816, 4096, 128, 1),
+         (100, 4096, 1032, 128, 4), (256, 14336, 4088, 192, 3), (200, 4096, 4104, 128, 2), (40, 8192, 2048, 160, 4), (130, 2304, 1000, 128, 3)]
 
 
 def product(a, b, sa, sb, out, dtype, policy):
@@ -48,6 +51,26 @@ def test_outputs_and_nothing_else(t, k, n, layout):
             assert lib.qo_kernel_launch_count() - before == 1  # one launch: no widening pass
             assert torch.equal(out.view(torch.int16), ref.view(torch.int16))
             assert bool((room[:8 + n] == 777.0).all()) and bool((room[8 + n + t * n:] == 777.0).all())
+
+
+@pytest.mark.parametrize("layout", ["weights_t_view", "reference_contiguous"])
+@pytest.mark.parametrize("t,k,n,columns,slices", FORMS)
+def test_narrow_tiles(t, k, n, columns, slices, layout):
+    g = torch.Generator(device=DEV).manual_seed(t + k + n)
+    words = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, dtype=torch.int64, device=DEV, generator=g).to(torch.int32)
+    a, w = words(t, k // 8), words(n, k // 8)
+    sa, sb = torch.rand(t, device=DEV, generator=g) + 0.01, torch.rand(n, device=DEV, generator=g) * 1e-4
+    b = w.t() if layout == "weights_t_view" else w.t().contiguous()
+    if layout == "reference_contiguous" and columns == 224:
+        columns = 256  # in this layout a stage fetches as much for the narrower tile
+    tiles = -(-t // 256) * -(-n // columns)
+    assert launched_blocks(lambda: q.int4_matmul(a, b, sa, sb)) == [2 * slices * tiles if slices > 1 else 2 * min(tiles, 74)]
+    ref, ref_acc = abi_int4_matmul(a, b, sa, sb, "bf16", True, policy=3)
+    for _ in range(3):
+        got, acc = abi_int4_matmul(a, b, sa, sb, "bf16", True)
+        assert torch.equal(acc, ref_acc) and torch.equal(got.view(torch.int16), ref.view(torch.int16))
+        assert torch.equal(abi_int4_matmul(a, b, sa, sb, "bf16").view(torch.int16), ref.view(torch.int16))
+    assert lib.qo_device_status(stream_ptr()) == N.QO_OK
 
 
 @pytest.mark.parametrize("k", [65536, 65792])
