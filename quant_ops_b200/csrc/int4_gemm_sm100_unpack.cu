@@ -1031,8 +1031,10 @@ bool gemm_unpack_prefill(int64_t t, int64_t n) {
 
 // Shapes for which the kernel is the better choice: prefill sizes, and everything else with K of 2048 or more.  Measured against
 // widening both operands and multiplying int8 (graph replay): 256 x 14336 x 4096 21.7 against 35.6 us, 600 x 2048 x 1024 11.1
-// against 16.0, 100 x 2048 x 256 10.0 against 11.7, but 100 x 1024 x 1024 9.4 against 7.2 and 300 x 1024 x 2048 9.6 against 7.7:
-// with four stages of K the fill and the exchange outweigh a widening pass that is as short as the product.
+// against 16.0, 100 x 2048 x 256 10.0 against 11.7.  K of 1024 to 2047 since tiles of 128 columns: 40 to 1000 rows by 256 to 11008 columns
+// 0.52 to 0.97 of the time with rows of weights, 0.46 to 0.82 with columns; beside the quantizer of a layer the widening pass is
+// nearly free, and the sides are level up to 4096 columns (0.87 to 1.18), 0.64 to 0.97 from 6144 on.  (Kernel policy 2 keeps
+// these sizes on the int8 kernels.)
 //
 // Few column tiles and a long K are the exception.  K is split four ways at most here, so 1 to 4 tiles occupy 8 to 32 of the
 // 148 SMs; the int8 kernels split it up to eight ways, half as wide tiles for one block of 128 rows, and there is little to
@@ -1044,7 +1046,8 @@ bool gemm_unpack_prefill(int64_t t, int64_t n) {
 // 8192 x 512 0.99.
 bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n, Widening instead) {
   if (gemm_unpack_prefill(t, n)) return true;
-  if (current_kernel_policy() == 3 || n < kBN || k < 2048) return false;
+  if (current_kernel_policy() == 3 || n < kBN || k < 1024) return false;
+  if (k < 2048) return current_kernel_policy() == 0 && (instead != Widening::kWeightsBeside || n >= 6144);
   const int64_t tiles = unpack_tiles(t, n);
   const bool upper_half = t > 96 && t <= 128;
   if (instead == Widening::kColumns) return !(k >= 8192 && tiles <= 2 && upper_half) && !(k >= 14336 && tiles == 1);
@@ -1063,11 +1066,15 @@ bool gemm_unpack_preferred(int64_t t, int64_t k, int64_t n, Widening instead) {
 //     74 of 128 x 256, up to which it is there: 300 x 8192 -> 4352 1.08, 600 x 14336 -> 3072 1.16; on either side 600 x 14336 -> 2816
 //     0.84, 450 x 14336 -> 5120 0.63;
 //   * for K of 4096 with 16 tiles and up to 32 of 128 x 256, 1.02 to 1.05 (1024 x 4096 -> 1024 20.2 / 19.3 us).
-// A second round of tiles: 300 x 4096 -> 11008 30.2 / 22.5.  Up to 128 rows the sides change from shape to shape, 0.80 to 1.31.
+// A second round of tiles: 300 x 4096 -> 11008 30.2 / 22.5.
+// Up to 128 rows, packed / copy over 40, 96, 112 and 128 rows: K of 2048 and 3072 0.72 to 0.97 everywhere, 6144 columns and more 0.82 to 1.01
+// (128 x 4096 -> 11008 19.4 / 22.5 us), up to 1024 columns with K below 8192 0.85 to 0.97 (96 x 4096 -> 1024 11.5 / 13.1); the copy
+// stays for 1025 to 6143 columns with K of 4096 and more, 0.95 to 1.10, and for long K with few columns, 0.99 to 1.15.
 bool gemm_unpack_beats_copy(int64_t t, int64_t k, int64_t n) {
   if (gemm_unpack_prefill(t, n)) return true;
   const int64_t tiles = unpack_tiles(t, n), tiles8 = ((t + 127) / 128) * ((n + 255) / 256);
-  if (t <= 128 || tiles > 74 || !gemm_unpack_preferred(t, k, n, Widening::kWeightsBeside)) return false;
+  if (tiles > 74 || !gemm_unpack_preferred(t, k, n, Widening::kWeightsBeside)) return false;
+  if (t <= 128) return k < 2048 ? n > 8192 : (k < 4096 || n >= 6144 || (n <= 1024 && k < 8192));
   if (k >= 8192) return tiles8 > 14 && (tiles < 34 || tiles8 > 74);
   return !(k >= 4096 && k < 5120 && tiles >= 16 && tiles8 <= 32);
 }

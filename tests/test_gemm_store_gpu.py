@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import quant_ops_b200 as q
-from helpers import N, QD, TD, abi_int4_matmul, launched_blocks, lib, make_inputs, ptr, stream_ptr
+from helpers import N, QD, TD, abi_int4_matmul, launched_blocks, launched_kernels, lib, make_inputs, ptr, stream_ptr
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -103,3 +103,30 @@ def test_bias_is_added_to_the_rounded_output(t, k, n, dtype):
     plain = q.w4a4_linear(x, left, right, w, sw, None, 0.9, TD[dtype])
     got = q.w4a4_linear(x, left, right, w, sw, bias, 0.9, TD[dtype])
     assert torch.equal(got, (plain.float() + bias.float()).to(TD[dtype]))
+
+
+@pytest.mark.parametrize("t,k,n,packed", [(128, 4096, 6144, True), (128, 4096, 6136, False), (96, 4096, 1024, True), (96, 4096, 1032, False), (33, 8192, 1024, False),
+                                          (128, 3072, 2048, True), (64, 14336, 8192, True), (40, 1024, 8200, True), (40, 1024, 8192, False)])
+def test_few_rows_with_kept_weights(t, k, n, packed):
+    x, left, right = (v.to(DEV) for v in make_inputs(t, k, "bf16", seed=t + n))
+    g = torch.Generator(device=DEV).manual_seed(n)
+    w = torch.randint(-2 ** 31, 2 ** 31, (n, k // 8), dtype=torch.int64, device=DEV, generator=g).to(torch.int32)
+    sw, kept = torch.rand(n, device=DEV, generator=g) * 1e-3, q.prepare_weights(w)
+    codes, scales = q.flatquant_dynamic_quantize(x, left, right, 0.9, True)
+    call = lambda: q.w4a4_linear_prepared(x, left, right, w, kept, sw, None, 0.9)
+    assert torch.equal(call(), abi_int4_matmul(codes, w.t(), scales, sw, "bf16", policy=3))
+    assert any("gemm_s4_unpack_kernel" in name for name in launched_kernels(call)) == packed
+
+
+@pytest.mark.parametrize("t,k,n", [(33, 1024, 256), (100, 1280, 1000), (300, 1792, 520), (1000, 1024, 2056)])
+@pytest.mark.parametrize("layout", ["weights_t_view", "reference_contiguous"])
+def test_short_k_without_a_widening_pass(t, k, n, layout):
+    g = torch.Generator(device=DEV).manual_seed(t + k + n)
+    words = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, dtype=torch.int64, device=DEV, generator=g).to(torch.int32)
+    a, w = words(t, k // 8), words(n, k // 8)
+    sa, sb = torch.rand(t, device=DEV, generator=g) + 0.01, torch.rand(n, device=DEV, generator=g) * 1e-4
+    b = w.t() if layout == "weights_t_view" else w.t().contiguous()
+    ref, ref_acc = abi_int4_matmul(a, b, sa, sb, "fp16", True, policy=3)
+    got, acc = abi_int4_matmul(a, b, sa, sb, "fp16", True)
+    assert torch.equal(acc, ref_acc) and torch.equal(got.view(torch.int16), ref.view(torch.int16))
+    assert len(launched_kernels(lambda: q.int4_matmul(a, b, sa, sb))) == 1
