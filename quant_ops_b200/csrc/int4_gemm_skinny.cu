@@ -212,7 +212,16 @@ int4_gemm_skinny_kernel(const uint32_t* a, int64_t lda, const uint32_t* b, int64
 // per token, from L2) are fetched and multiplied.  The weight bytes, the bound of a decode step, move entirely under
 // the quantizer.  Rows are padded by 64 bytes so that the fragment reads are conflict-free; the partial sums of the 16
 // warps (each takes a sixteenth of K) are added through the same shared memory once the weights are no longer needed.
+//
+// ALONE: the stand-alone product.  The weights, too, may come from the kernel ahead, so nothing hides their fetch; a row is therefore
+// fetched in up to four slices of K, a barrier each, and every warp takes a sixteenth of each slice, so that only the last
+// slice's products come after the last weights.  What it gains over the streaming kernel is that all of an SM's weights are in flight at
+// once.  Graph replay, weights from HBM, streaming / this kernel: 8 x 14336 x 4096 11.3 / 10.2 us, 16 x 14336 x 4096 14.5 / 11.4,
+// 24 x 14336 x 4096 22.5 / 14.2, 16 x 11008 x 4096 12.5 / 9.4, 32 x 4096 x 4096 8.3 / 6.9, 16 x 4096 x 1024 4.0 / 3.4; with one slice 12.1 at
+// 16 x 14336 x 4096.  (Inside the layer, where the weights are there first, slices lose: 1 x 14336 -> 4096 10.8 / 11.2, 1 x 4096 -> 14336
+// 11.7 / 13.6.)
 constexpr int kResWarps = 16;
+constexpr int kResSlices = 4;
 
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -220,37 +229,45 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
 }
 
 // NT = 8-token column tiles, TILES = 16-channel row tiles per CTA (TILES * NT <= 8 keeps the accumulators in registers)
-template <int NT, int TILES, typename OutT>
+template <int NT, int TILES, bool ALONE, typename OutT>
 __global__ void __launch_bounds__(kResWarps * 32, 1)
 int4_gemm_resident_kernel(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t ldb,
                           const float* sa, const float* sb, OutT* __restrict__ out,
                           int32_t* __restrict__ acc_out, const OutT* bias, int tokens, int nchunks, int64_t n,
                           int cpc, uint32_t* __restrict__ status) {
   extern __shared__ uint4 wsm[];  // weight rows, row stride nchunks * 4 + 4 uint4; later the partial sums
-  __shared__ uint64_t bar;
+  __shared__ uint64_t bars[ALONE ? kResSlices : 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int64_t c0 = (int64_t)blockIdx.x * cpc;
   const int nch = (int)min((int64_t)cpc, n - c0);  // the grid is sized so that every CTA has at least one channel
   const int stride4 = nchunks * 4 + 4;
-  const uint32_t bar_a = ptx::smem_u32(&bar);
+  const uint32_t bar_a = ptx::smem_u32(bars);
+  // chunks of a slice: whole turns of the warps
+  const int per_slice = ALONE ? (nchunks + kResSlices * kResWarps - 1) / (kResSlices * kResWarps) * kResWarps : nchunks;
   if (threadIdx.x == 0) {
-    ptx::mbar_init(bar_a, 1);
+    for (int i = 0; i < (ALONE ? kResSlices : 1); ++i) ptx::mbar_init(bar_a + 8u * i, 1);
     ptx::fence_barrier_init();
   }
   __syncthreads();
-  // the weights are not written by the kernel before this one (the caller says so): fetch them before the wait
-  if (threadIdx.x == 0) {
-    const uint32_t row_bytes = (uint32_t)nchunks * 64u;
-    ptx::mbar_arrive_expect_tx(bar_a, (uint32_t)nch * row_bytes);
+  if (ALONE) ptx::grid_dependency_wait();
+  // (inside the layer the weights are not written by the kernel before this one, the caller says so: they are fetched before the wait)
+  if (threadIdx.x < (ALONE ? 32 : 1)) {
     const uint32_t base = ptx::smem_u32(wsm);
-    for (int r = 0; r < nch; ++r) bulk_copy_g2s(base + (uint32_t)(r * stride4) * 16u, b + (c0 + r) * ldb, row_bytes, bar_a);
+    for (int i = 0, k0 = 0; k0 < nchunks; ++i, k0 += per_slice) {
+      const uint32_t bytes = (uint32_t)min(per_slice, nchunks - k0) * 64u, bar = bar_a + 8u * i;
+      if (threadIdx.x == 0) ptx::mbar_arrive_expect_tx(bar, (uint32_t)nch * bytes);
+      if (ALONE) __syncwarp();
+      for (int r = threadIdx.x; r < nch; r += ALONE ? 32 : 1)
+        bulk_copy_g2s(base + (uint32_t)(r * stride4) * 16u + (uint32_t)k0 * 64u, b + (c0 + r) * ldb + (int64_t)k0 * kChunkWords, bytes, bar);
+    }
   }
   ptx::grid_dependency_wait();  // the codes and their scales are complete now
   ptx::grid_launch_dependents();
 
   const uint4 zero4 = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);  // eight zeros per word
-  const int per = (nchunks + kResWarps - 1) / kResWarps;
-  const int cb = warp * per, ce = min(nchunks, cb + per);
+  // a warp's chunks: cb, cb + turn, ... below ce
+  const int per = (nchunks + kResWarps - 1) / kResWarps, turn = ALONE ? kResWarps : 1;
+  const int cb = ALONE ? warp : warp * per, ce = ALONE ? nchunks : min(nchunks, cb + per);
   bool tok_ok[NT];
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) tok_ok[nt] = nt * 8 + g < tokens;
@@ -262,10 +279,16 @@ int4_gemm_resident_kernel(const uint32_t* a, int64_t lda, const uint32_t* b, int
   uint4 xa[NT], xb[NT];
   load_x(xa, cb);  // the first codes are requested while the last weight rows may still be arriving
 
-  const bool landed = ptx::mbar_wait(bar_a, 0);
-  if (!__syncthreads_and(landed)) {  // one decision for the whole CTA
+  bool landed = true;
+  int have = 0, limit = 0;  // ALONE: slices seen complete, chunks in them
+  auto give_up = [&] {      // one decision for the whole CTA
+    if (__syncthreads_and(landed)) return false;
     if (threadIdx.x == 0) atomicCAS(status, 0u, 0xB00u);
-    return;  // the outputs stay unwritten; qo_device_status reports the timeout
+    return true;  // the outputs stay unwritten; qo_device_status reports the timeout
+  };
+  if (!ALONE) {
+    landed = ptx::mbar_wait(bar_a, 0);
+    if (give_up()) return;
   }
 
   int acc[TILES][NT][4];
@@ -278,6 +301,8 @@ int4_gemm_resident_kernel(const uint32_t* a, int64_t lda, const uint32_t* b, int
 
   auto compute = [&](const uint4 (&x)[NT], int c) {
     if (c >= ce) return;
+    if (ALONE)
+      for (; c >= limit; ++have, limit += per_slice) landed = ptx::mbar_wait(bar_a + 8u * have, 0) && landed;
 #pragma unroll
     for (int tl = 0; tl < TILES; ++tl) {
       const int r0 = tl * 16 + g, r1 = r0 + 8;
@@ -300,15 +325,19 @@ int4_gemm_resident_kernel(const uint32_t* a, int64_t lda, const uint32_t* b, int
       }
     }
   };
-  for (int c = cb; c < ce; c += 2) {
-    load_x(xb, c + 1);
+  for (int c = cb; c < ce; c += 2 * turn) {
+    load_x(xb, c + turn);
     compute(xa, c);
-    load_x(xa, c + 2);
-    compute(xb, c + 1);
+    load_x(xa, c + 2 * turn);
+    compute(xb, c + turn);
   }
 
   // partial sums of the 16 warps through the shared memory that held the weights
-  __syncthreads();
+  if (ALONE) {
+    if (give_up()) return;  // (every slice has landed: each has a chunk, whose warp has waited for it)
+  } else {
+    __syncthreads();
+  }
   int* red = reinterpret_cast<int*>(wsm);  // [warp][tile][nt][16][9]
 #pragma unroll
   for (int tl = 0; tl < TILES; ++tl)
@@ -338,11 +367,11 @@ int4_gemm_resident_kernel(const uint32_t* a, int64_t lda, const uint32_t* b, int
 }
 
 // the resident-weights kernel for this problem, or QO_ERR_UNSUPPORTED (no message) when its limits do not hold
-template <int NT, int TILES, typename OutT>
+template <int NT, int TILES, bool ALONE, typename OutT>
 int launch_resident_cfg(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t ldb, const float* sa, const float* sb, void* out,
                         int32_t* acc_out, const void* bias, int tokens, int nchunks, int64_t n, int cpc, int grid, size_t smem,
                         uint32_t* status, cudaStream_t stream) {
-  auto kern = int4_gemm_resident_kernel<NT, TILES, OutT>;
+  auto kern = int4_gemm_resident_kernel<NT, TILES, ALONE, OutT>;
   int dev = 0;
   QO_CUDA_TRY(cudaGetDevice(&dev));
   static bool configured[64] = {};
@@ -365,7 +394,7 @@ int launch_resident_cfg(const uint32_t* a, int64_t lda, const uint32_t* b, int64
   return check_launch("int4_gemm_resident_kernel");
 }
 
-template <typename OutT>
+template <bool ALONE, typename OutT>
 int launch_resident(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t ldb, const float* sa, const float* sb, void* out,
                     int32_t* acc_out, const void* bias, int tokens, int nchunks, int64_t n, int taken_sms, cudaStream_t stream) {
   int dev = 0;
@@ -391,9 +420,17 @@ int launch_resident(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t l
   const size_t red = (size_t)kResWarps * tiles * nt * 16 * 9 * sizeof(int);  // the reduction reuses the weight area
   if (red > smem) smem = red;
   if (smem > kSmemOptIn - 64 || tiles * nt > 8 || n < sms) return QO_ERR_UNSUPPORTED;
-  uint32_t* status = device_status_word(dev);
+  // (the first stand-alone product of a process may be under capture, where the status word cannot be allocated: the streaming
+  // kernels need none)
+  uint32_t* status = device_status_word_if_any(dev);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (ALONE && !status && (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)) {
+    (void)cudaGetLastError();
+    return QO_ERR_UNSUPPORTED;
+  }
+  if (!status) status = device_status_word(dev);
   if (!status) return QO_ERR_UNSUPPORTED;
-#define QO_RES(NTV, TLV) return launch_resident_cfg<NTV, TLV, OutT>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, cpc, grid, smem, status, stream)
+#define QO_RES(NTV, TLV) return launch_resident_cfg<NTV, TLV, ALONE, OutT>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, cpc, grid, smem, status, stream)
   if (nt == 1) {
     if (tiles == 1) QO_RES(1, 1);
     if (tiles == 2) QO_RES(1, 2);
@@ -682,6 +719,25 @@ bool gemm_skinny_supported(int64_t t, int64_t k, int64_t n, const void* a, int64
          (reinterpret_cast<uintptr_t>(a) % 16) == 0 && (reinterpret_cast<uintptr_t>(b) % 16) == 0 && n <= (int64_t)16 * 0x7fffffff;
 }
 
+// the kernels that stream the weights
+static int launch_streaming(const uint32_t* a, int64_t lda, const uint32_t* b, int64_t ldb, const float* sa, const float* sb, void* out, int out_dtype, int tokens,
+                     int nchunks, int64_t n, int32_t* acc_out, const void* bias, int weights_first, cudaStream_t stream) {
+  if (out_dtype == QO_F16) return launch_t<__half>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, stream);
+  if (out_dtype == QO_BF16) return launch_t<__nv_bfloat16>(a, lda, b, ldb, sa, sb, out, acc_out, bias, tokens, nchunks, n, weights_first, stream);
+  return fail(QO_ERR_INVALID_ARGUMENT, "int4_matmul: out_dtype must be QO_F16 or QO_BF16");
+}
+
+// The stand-alone product on resident weights: up to 32 channels per SM (above, the even shares hold them in registers), from nine rows and
+// K of 4096 on (2048 with up to 16 channels per SM), and from four rows with K of 11008 and more.  Resident / streaming, graph
+// replay, weights from HBM, 160 to 4736 channels: 9, 16, 17 and 32 rows at K of 4096 0.77 to 0.98, 6144 0.60 to 0.95, 8192 0.57 to 0.98,
+// 11008 0.43 to 0.87, 14336 0.50 to 0.91; K of 2048 up to 2048 channels 0.81 to 1.00, above 0.94 to 1.03; four to eight rows at 11008
+// and 14336 0.71 to 1.03, at 8192 0.85 to 1.13, at 4096 0.92 to 1.03; one row 0.81 to 1.15; K of 1024 0.85 to 1.21, below 0.90 to 1.43.
+static bool resident_alone(int64_t t, int64_t k, int64_t n, int sms) {
+  if (n > 32 * sms) return false;
+  if (k >= 11008) return t >= 4;
+  return t >= 9 && (k >= 4096 || (k >= 2048 && n <= 16 * sms));
+}
+
 int launch_gemm_skinny(const int32_t* a, int64_t lda, const int32_t* b, int64_t bsn, const float* sa, const float* sb, void* out,
                        int out_dtype, int64_t t, int64_t k, int64_t n, int32_t* acc_out, const void* bias, cudaStream_t stream,
                        int taken_sms) {
@@ -692,13 +748,19 @@ int launch_gemm_skinny(const int32_t* a, int64_t lda, const int32_t* b, int64_t 
   if (weights_first) {
     // inside the fused layer: the weights can be fetched in full beside the quantizer that precedes this kernel
     int rc = QO_ERR_UNSUPPORTED;
-    if (out_dtype == QO_F16) rc = launch_resident<__half>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, taken_sms, stream);
-    else if (out_dtype == QO_BF16) rc = launch_resident<__nv_bfloat16>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, taken_sms, stream);
+    if (out_dtype == QO_F16) rc = launch_resident<false, __half>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, taken_sms, stream);
+    else if (out_dtype == QO_BF16) rc = launch_resident<false, __nv_bfloat16>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, taken_sms, stream);
+    if (rc != QO_ERR_UNSUPPORTED) return rc;
+  } else {
+    int dev = 0;
+    QO_CUDA_TRY(cudaGetDevice(&dev));
+    if (!resident_alone(t, k, n, sm_count(dev))) return launch_streaming(ua, lda, ub, bsn, sa, sb, out, out_dtype, (int)t, nchunks, n, acc_out, bias, 0, stream);
+    int rc = QO_ERR_UNSUPPORTED;
+    if (out_dtype == QO_F16) rc = launch_resident<true, __half>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, 0, stream);
+    else if (out_dtype == QO_BF16) rc = launch_resident<true, __nv_bfloat16>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, 0, stream);
     if (rc != QO_ERR_UNSUPPORTED) return rc;
   }
-  if (out_dtype == QO_F16) return launch_t<__half>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, weights_first ? 1 : 0, stream);
-  if (out_dtype == QO_BF16) return launch_t<__nv_bfloat16>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, weights_first ? 1 : 0, stream);
-  return fail(QO_ERR_INVALID_ARGUMENT, "int4_matmul: out_dtype must be QO_F16 or QO_BF16");
+  return launch_streaming(ua, lda, ub, bsn, sa, sb, out, out_dtype, (int)t, nchunks, n, acc_out, bias, weights_first ? 1 : 0, stream);
 }
 
 }  // namespace qo
