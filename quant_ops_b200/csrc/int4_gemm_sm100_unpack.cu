@@ -103,7 +103,7 @@ struct Bars {
   uint64_t p_full[kPStages], p_empty[kPStages];
   uint64_t op_ready[kOStages], op_empty[kOStages];
   uint64_t acc_full, acc_empty;
-  uint64_t exchange;  // SPLIT > 1: bytes of the other pairs' partial sums; SPLIT = 1: acc_empty of the odd items
+  uint64_t exchange;  // bytes of the other pairs' partial sums (SPLIT > 1)
   uint32_t tmem_base;
 };
 static_assert(sizeof(Bars) <= 128, "barriers");
@@ -283,8 +283,8 @@ __device__ __forceinline__ bool issue_stage(uint32_t d_tmem, uint32_t a_tmem, ui
 //
 // SPLIT > 1 (few output tiles: a short activation matrix or a narrow layer): K is split over SPLIT CTA pairs which form
 // one cluster and work on one tile, one work item per pair.  Measured (graph replay, before: widening pass + int8 kernels):
-// 256 x 14336 x 4096 35.6 -> 21.7 us, 64 x 4096 x 4096 15.6 -> 11.2, 512 x 4096 x 4096 22.3 -> 13.9.  What is left behind the
-// last MMA is the exchange, about 5 us of which 2.5 are the copies (18 bytes per cycle and SM), and the first fill, 2 us.
+// 256 x 14336 x 4096 35.6 -> 19.7 us, 64 x 4096 x 4096 15.6 -> 10.1, 512 x 4096 x 4096 22.3 -> 13.5 (there without slices).  What is left
+// behind the last MMA is the exchange, about 4 us of which 2 are the copies (18 bytes per cycle and SM), and the first fill, 2 us.
 // At the end the pairs share out the tile's columns and send
 // each other their int32 partial sums through distributed shared memory (into the rings, which are idle by then).
 // Whole-number sums: exact in any order.
@@ -340,7 +340,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
     for (int i = 0; i < kOStages; ++i) { mbar_init(smem_u32(&bars->op_ready[i]), 12); mbar_init(smem_u32(&bars->op_empty[i]), 1); }
     mbar_init(smem_u32(&bars->acc_full), 1);
     mbar_init(smem_u32(&bars->acc_empty), 16);
-    mbar_init(smem_u32(&bars->exchange), SPLIT == 1 ? 16 : 1);
+    mbar_init(smem_u32(&bars->exchange), 1);
     fence_barrier_init();
     prefetch_tensormap(&a_map);
     prefetch_tensormap(&b_map);
@@ -467,7 +467,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          const uint32_t e = smem_u32(lt & 1 ? &bars->exchange : &bars->acc_empty);
+          const uint32_t e = smem_u32(&bars->acc_empty);
           if (rank == 0) mbar_arrive(e); else mbar_arrive_cluster(cluster_map_shared(e, leader));
         }
       };
@@ -578,9 +578,12 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
         // the item's first operands are looked for before the accumulator, so that the answer comes while that is being drained
         if (!ready && !mbar_wait(smem_u32(&bars->op_ready[step % kOStages]), (step / kOStages) & 1)) { atomicCAS(status, 0u, 0xA20u); break; }
         ready = true;
-        // the accumulator this item overlaps: that of the item before, or, where both fit beside one another, of the one before that
-        const int owner = lt - (acc_shift < bn ? 1 : 2);
-        if (owner >= 0 && !mbar_wait(smem_u32(owner & 1 ? &bars->exchange : &bars->acc_empty), (owner >> 1) & 1)) { atomicCAS(status, 0u, 0xA10u); break; }
+        // The item before has handed over its accumulator.  Where two of them fit beside one another only the one before that is
+        // overwritten, and the wait comes before the commit at the end instead: the epilogue must have seen the item before complete
+        // by then, because a parity wait cannot tell one completion of acc_full from the next but one.
+        const bool beside = acc_shift >= bn;
+        auto handed_over = [&] { return lt == 0 || mbar_wait(smem_u32(&bars->acc_empty), (lt & 1) ^ 1); };
+        if (!beside && !handed_over()) { atomicCAS(status, 0u, 0xA10u); break; }
         const uint32_t d_tmem = tmem + (lt & 1) * acc_shift;
         const uint32_t idesc = pair + lt * npairs >= cut_from ? idesc_half : idesc_whole;
 #pragma unroll 1
@@ -595,6 +598,7 @@ gemm_s4_unpack_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_co
           ready = issue_stage(d_tmem, tmem + kColA + s * 64, b_desc0 + (uint64_t)(s * (kOBBytes >> 4)), idesc, ks != 0,
                               op_empty0 + s * 8, op_empty0_peer + s * 8, smem_u32(&bars->op_ready[sn]), phn) && !last;
         }
+        if (ok && beside && !handed_over()) { atomicCAS(status, 0u, 0xA10u); ok = false; }
         if (ok) {
           mma_commit_pair(acc_full);
           mma_commit_pair(acc_full_peer);
@@ -1030,13 +1034,14 @@ bool gemm_unpack_prefill(int64_t t, int64_t n) {
 }
 
 // Shapes for which the kernel is the better choice: prefill sizes, and everything else with K of 2048 or more.  Measured against
-// widening both operands and multiplying int8 (graph replay): 256 x 14336 x 4096 21.7 against 35.6 us, 600 x 2048 x 1024 11.1
-// against 16.0, 100 x 2048 x 256 10.0 against 11.7.  K of 1024 to 2047 since tiles of 128 columns: 40 to 1000 rows by 256 to 11008 columns
+// widening both operands and multiplying int8 (graph replay): 256 x 14336 x 4096 19.7 against 35.6 us, 600 x 2048 x 1024 11.1
+// against 16.0 (in tiles of 256), 100 x 2048 x 256 10.0 against 11.7 (same).  K of 1024 to 2047 since tiles of 128 columns: 40 to 1000 rows by 256 to 11008 columns
 // 0.52 to 0.97 of the time with rows of weights, 0.46 to 0.82 with columns; beside the quantizer of a layer the widening pass is
 // nearly free, and the sides are level up to 4096 columns (0.87 to 1.18), 0.64 to 0.97 from 6144 on.  (Kernel policy 2 keeps
 // these sizes on the int8 kernels.)
 //
-// Few column tiles and a long K are the exception.  K is split four ways at most here, so 1 to 4 tiles occupy 8 to 32 of the
+// Few column tiles and a long K are the exception (measured in tiles of 256 columns; in narrower ones the unpacking kernel is ahead there
+// too, 0.75 to 0.92, and the lines stay where the tests hold them).  K is split four ways at most here, so 1 to 4 tiles occupy 8 to 32 of the
 // 148 SMs; the int8 kernels split it up to eight ways, half as wide tiles for one block of 128 rows, and there is little to
 // widen.  How little depends on what runs beside it (`instead`).  Measured, unpacking / int8: layer 128 x 4096 -> 256 15.0 /
 // 13.8 us, 128 x 4096 -> 1024 15.2 / 14.3, 128 x 8192 -> 256 1.21 apart, 96 x 8192 -> 512 1.11, 256 x 14336 -> 256 1.02; rows 128 x

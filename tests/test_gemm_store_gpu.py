@@ -15,6 +15,8 @@ DEV = "cuda:0"
 SHAPES = [(2000, 256, 9480), (333, 4096, 14328), (777, 4096, 11008), (4097, 1024, 1032), (1600, 768, 2056), (500, 2048, 9472)]
 # columns of a tile and slices of K that the rule takes, with ragged rows and columns: two rounds and one of narrow tiles, K in slices
 FORMS = [(1100, 4096, 4104, 160, 1), (700, 11008, 4088, 192, 1), (200, 4096, 14328, 224, 1), (256, 4096, 11000, 160, 1), (300, 2816, 4096, 128, 1),
+         # accumulators beside one another, three to nine items per pair, items shorter than their epilogue
+         (1045, 256, 7184, 128, 1), (4498, 256, 4704, 128, 1), (7142, 256, 1640, 128, 1), (7175, 512, 1568, 160, 1), (7537, 768, 1064, 160, 1), (5430, 2816, 1560, 160, 1),
          (100, 4096, 1032, 128, 4), (256, 14336, 4088, 192, 3), (200, 4096, 4104, 128, 2), (40, 8192, 2048, 160, 4), (130, 2304, 1000, 128, 3)]
 
 
