@@ -732,10 +732,11 @@ static int launch_streaming(const uint32_t* a, int64_t lda, const uint32_t* b, i
 // replay, weights from HBM, 160 to 4736 channels: 9, 16, 17 and 32 rows at K of 4096 0.77 to 0.98, 6144 0.60 to 0.95, 8192 0.57 to 0.98,
 // 11008 0.43 to 0.87, 14336 0.50 to 0.91; K of 2048 up to 2048 channels 0.81 to 1.00, above 0.94 to 1.03; four to eight rows at 11008
 // and 14336 0.71 to 1.03, at 8192 0.85 to 1.13, at 4096 0.92 to 1.03; one row 0.81 to 1.15; K of 1024 0.85 to 1.21, below 0.90 to 1.43.
-static bool resident_alone(int64_t t, int64_t k, int64_t n, int sms) {
-  if (n > 32 * sms) return false;
-  if (k >= 11008) return t >= 4;
-  return t >= 9 && (k >= 4096 || (k >= 2048 && n <= 16 * sms));
+static bool resident_alone(int64_t t, int64_t k, int64_t n) {
+  if (t < (k >= 11008 ? 4 : 9) || k < 2048) return false;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+  return n <= (k >= 4096 ? 32 : 16) * sm_count(dev);
 }
 
 int launch_gemm_skinny(const int32_t* a, int64_t lda, const int32_t* b, int64_t bsn, const float* sa, const float* sb, void* out,
@@ -752,9 +753,7 @@ int launch_gemm_skinny(const int32_t* a, int64_t lda, const int32_t* b, int64_t 
     else if (out_dtype == QO_BF16) rc = launch_resident<false, __nv_bfloat16>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, taken_sms, stream);
     if (rc != QO_ERR_UNSUPPORTED) return rc;
   } else {
-    int dev = 0;
-    QO_CUDA_TRY(cudaGetDevice(&dev));
-    if (!resident_alone(t, k, n, sm_count(dev))) return launch_streaming(ua, lda, ub, bsn, sa, sb, out, out_dtype, (int)t, nchunks, n, acc_out, bias, 0, stream);
+    if (!resident_alone(t, k, n)) return launch_streaming(ua, lda, ub, bsn, sa, sb, out, out_dtype, (int)t, nchunks, n, acc_out, bias, 0, stream);
     int rc = QO_ERR_UNSUPPORTED;
     if (out_dtype == QO_F16) rc = launch_resident<true, __half>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, 0, stream);
     else if (out_dtype == QO_BF16) rc = launch_resident<true, __nv_bfloat16>(ua, lda, ub, bsn, sa, sb, out, acc_out, bias, (int)t, nchunks, n, 0, stream);
